@@ -693,9 +693,22 @@ size_t based_tied_attention_scratch_bytes(int B, int L, int H, int G, int d, int
   return tied_decode_scratch_bytes(B, L * (H / G), G, d, max_len);
 }
 
+size_t based_lightning_scratch_bytes(int B, int L, int H, int d, int dv) {
+  if (B <= 0 || L <= 0 || H <= 0 || d <= 0 || dv <= 0 || !lightning_tc_scratch_bytes) return 0;
+  return lightning_tc_scratch_bytes(B, L, H, d, dv);
+}
+
 int based_lightning(const void* q, const void* k, const void* v, const void* decay, void* state, void* out, int B, int L, int H,
                     int d, int dv, const int64_t q_strides[2], const int64_t k_strides[2], const int64_t v_strides[2],
                     const int64_t out_strides[2], const int32_t* offsets, int offset, int io_dtype, int impl, void* stream) {
+  return based_lightning_split(q, k, v, decay, state, out, B, L, H, d, dv, q_strides, k_strides, v_strides, out_strides, offsets,
+                               offset, io_dtype, impl, nullptr, 0, stream);
+}
+
+int based_lightning_split(const void* q, const void* k, const void* v, const void* decay, void* state, void* out, int B, int L,
+                          int H, int d, int dv, const int64_t q_strides[2], const int64_t k_strides[2], const int64_t v_strides[2],
+                          const int64_t out_strides[2], const int32_t* offsets, int offset, int io_dtype, int impl, void* scratch,
+                          size_t scratch_bytes, void* stream) {
   if (!q || !k || !v || !decay || !state || !out || !q_strides || !k_strides || !v_strides || !out_strides) return BASED_ERR_NULL;
   if (!dtype_ok(io_dtype)) return BASED_ERR_DTYPE;
   if (B < 0 || L < 0 || H <= 0 || d <= 0 || d > 512 || dv <= 0 || offset < 0) return BASED_ERR_SHAPE;
@@ -706,7 +719,7 @@ int based_lightning(const void* q, const void* k, const void* v, const void* dec
     if (io_dtype != BASED_BF16 || !launch_lightning_tc) return BASED_ERR_IMPL;
     const int rc = launch_lightning_tc(q, k, v, static_cast<const float*>(decay), static_cast<float*>(state), out, B, L, H, d, dv,
                                        s2(q_strides), s2(k_strides), s2(v_strides), s2(out_strides), offsets, offset,
-                                       static_cast<cudaStream_t>(stream));
+                                       scratch, scratch_bytes, static_cast<cudaStream_t>(stream));
     if (!(autosel && rc == BASED_ERR_IMPL)) return rc;
   }
   if (!launch_lightning_recurrent) return BASED_ERR_IMPL;

@@ -218,7 +218,8 @@ BASED_WEAK int launch_lightning_recurrent(const void* q, const void* k, const vo
                                           Strides2 so, const int32_t* offsets, int offset, int io_dtype, cudaStream_t stream);
 BASED_WEAK int launch_lightning_tc(const void* q, const void* k, const void* v, const float* decay, float* state, void* out, int B,
                                    int L, int H, int d, int dv, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
-                                   const int32_t* offsets, int offset, cudaStream_t stream);
+                                   const int32_t* offsets, int offset, void* scratch, size_t scratch_bytes, cudaStream_t stream);
+BASED_WEAK size_t lightning_tc_scratch_bytes(int B, int L, int H, int d, int dv);
 BASED_WEAK int read_tc_status_lightning(unsigned int* out, int reset);
 BASED_WEAK int launch_lightning_step(const void* q, const void* k, const void* v, const void* gate, int64_t sx,
                                      const float* decay, const void* norm_w, float* state, float* read, int* count, void* out,

@@ -13,6 +13,14 @@
 // 32-bit in the recurrence: the state is the fp32 accumulator and is scaled in fp32; g^(n-1-j) v_j enters as a bf16 pair
 // hi + lo (16 mantissa bits) against k as the activation stored it.  Scores and decays are fp32 until P, and nothing feeds
 // the read-out back.
+//
+// A chunk depends on the one before through the state, so a CTA's time is its number of chunks times the latency of one
+// (3.8 us), whatever the machine could do beside it.  With few (batch, head) pairs the SEQUENCE is cut as well, into segments
+// of whole chunks, in three launches: what each segment alone adds to the state (lightning_segment_kernel: no chain, the decay
+// to the segment's end is multiplied into v), a running sum over the segments in fp32 (lightning_scan_kernel), and this kernel
+// over all segments at once, each from the state before it.  B = 1, 8 heads of 128, L = 6001: 179 us as 32 chains of 47
+// chunks, 43 us as 16 segments (15 + 4 + 23).
+#include <algorithm>
 #include <initializer_list>
 #include <mutex>
 
@@ -36,6 +44,7 @@ constexpr int kStateRegs = 40, kMmaRegs = 40, kLoadRegs = 88;
 constexpr int kItems = C * 16 / kLoaders;   // 16-byte pieces per thread and tensor at 128 columns
 constexpr uint32_t kAtom = 128 * 128;       // bytes of 128 rows x 64 columns
 constexpr int kTables = 32 + 132 + 32;
+constexpr int kMinSplitChunks = 8;
 
 struct Params {
   CUtensorMap mq, mk, mv, mo;               // [B][H][L][.]; q and k for prefetches into L2
@@ -46,6 +55,8 @@ struct Params {
   const int32_t* offsets;
   int64_t qb, ql, kb, kl, ob, ol;
   int offset, L, H, d, dv, cols, tma_out;   // cols: value columns per CTA
+  int nseg, per;                            // segments of the sequence, chunks per segment
+  float* seg;                               // nseg > 1: [B, H, nseg][d][dv], the state each segment starts from
   unsigned int* status;
 };
 
@@ -82,14 +93,32 @@ __device__ __forceinline__ void silu4(uint32_t& u, uint32_t& w) {
   w = pack2(mul2(y, mul2(pair(rcd, rcd), pair(d, c))));
 }
 
+// eight values of v times f as bf16 pairs hi + lo
+__device__ __forceinline__ void decayed(const uint4& v, float f, uint8_t* hi_at, uint8_t* lo_at) {
+  const uint64_t f2 = pair(f, f);
+  uint32_t hi[4], lo[4];
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    float x, y;
+    split(mul2(pair(seq::bf16_lo(w[m]), seq::bf16_hi(w[m])), f2), x, y);
+    hi[m] = pack_bf16(x, y);
+    lo[m] = pack_bf16(x - seq::bf16_lo(hi[m]), y - seq::bf16_hi(hi[m]));
+  }
+  *reinterpret_cast<uint4*>(hi_at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  *reinterpret_cast<uint4*>(lo_at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+}
+
 __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t sb = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = blockIdx.x, b = blockIdx.y, col0 = blockIdx.z * p.cols;
+  const int h = blockIdx.x, b = blockIdx.y, seg = blockIdx.z % p.nseg, col0 = blockIdx.z / p.nseg * p.cols;
   const int cols = min(p.cols, p.dv - col0);
-  const int nc = (p.L + C - 1) / C;
+  const int t0 = seg * p.per * C;                        // this segment's first token
+  const int L = min(p.L - t0, p.per * C);
+  const int nc = (L + C - 1) / C;
   const int aq = (p.d + 63) / 64, av = (p.cols + 63) / 64;
   // shared memory: Q, K (always two atoms: its transpose is a 128-row operand), two of V, hi and lo of the decayed V, S0
   const uint32_t SM_K = aq * kAtom, SM_V = SM_K + 2 * kAtom, SM_W = SM_V + 2 * av * kAtom, SM_S = SM_W + 2 * av * kAtom,
@@ -132,8 +161,8 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
     const int rowq = t >> wq, rowv = t >> wv, colq = t & ((1 << wq) - 1), colv = t & ((1 << wv) - 1);
     const int stepq = kLoaders >> wq, stepv = kLoaders >> wv;
     const bool onq = colq < cq && rowq < C, onv = colv < cv && rowv < C;
-    const bf16* q = p.q + b * p.qb + (int64_t)h * p.d + rowq * p.ql + colq * 8;
-    const bf16* k = p.k + b * p.kb + (int64_t)h * p.d + rowq * p.kl + colq * 8;
+    const bf16* q = p.q + b * p.qb + (int64_t)h * p.d + (t0 + rowq) * p.ql + colq * 8;
+    const bf16* k = p.k + b * p.kb + (int64_t)h * p.d + (t0 + rowq) * p.kl + colq * 8;
     // steps are multiples of 8 rows (or there is one row only): the swizzle is the same for all of a thread's rows
     const uint32_t atq = (colq >> 3) * kAtom + tma::sw128_offset(rowq & (C - 1), colq & 7), atv = (colv >> 3) * kAtom + tma::sw128_offset(rowv & (C - 1), colv & 7);
     uint4 rq[kItems], rk[kItems];
@@ -147,10 +176,10 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
       for (int i = 0; i < kItems; ++i)
         if (i * step < C) { silu4(r[i].x, r[i].y); silu4(r[i].z, r[i].w); }
     };
-    load(rq, q, p.ql, rowq, stepq, onq, min(C, p.L));
-    load(rk, k, p.kl, rowq, stepq, onq, min(C, p.L));
+    load(rq, q, p.ql, rowq, stepq, onq, min(C, L));
+    load(rk, k, p.kl, rowq, stepq, onq, min(C, L));
     for (int c = 0; c < nc; ++c) {
-      const int n = min(C, p.L - c * C);
+      const int n = min(C, L - c * C);
       uint8_t* vb = smem + SM_V + (c & 1) * av * kAtom + atv;
       act(rq, stepq);
       act(rk, stepq);
@@ -181,18 +210,7 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
             uint8_t* dst = smem + SM_W + atv + i * stepv * 128;
             const uint4 r = *reinterpret_cast<const uint4*>(vb + i * stepv * 128);
             const float f = pw[max(n - 1 - rowv - i * stepv, 0)];      // rows past the end are zero
-            const uint64_t f2 = pair(f, f);
-            uint32_t hi[4], lo[4];
-            const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              float x, y;
-              split(mul2(pair(seq::bf16_lo(w[m]), seq::bf16_hi(w[m])), f2), x, y);
-              hi[m] = pack_bf16(x, y);
-              lo[m] = pack_bf16(x - seq::bf16_lo(hi[m]), y - seq::bf16_hi(hi[m]));
-            }
-            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(dst + av * kAtom) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            decayed(r, f, dst, dst + av * kAtom);
           }
       }
       fence_proxy_async();
@@ -200,8 +218,8 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
       if (c + 1 < nc) {
         q += C * p.ql;
         k += C * p.kl;
-        load(rq, q, p.ql, rowq, stepq, onq, min(C, p.L - (c + 1) * C));
-        load(rk, k, p.kl, rowq, stepq, onq, min(C, p.L - (c + 1) * C));
+        load(rq, q, p.ql, rowq, stepq, onq, min(C, L - (c + 1) * C));
+        load(rk, k, p.kl, rowq, stepq, onq, min(C, L - (c + 1) * C));
       }
     }
   } else if (warp >= 8) {
@@ -254,12 +272,12 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
         if (c >= 2) mbar_wait_bounded<false>(B_VF, c & 1, abort_flag, p.status, 1u << 8);   // chunk c - 2 has given its output away
         const uint32_t full = B_R + 8 * (c & 1);
         tma::mbar_expect_tx(full, av * kAtom);
-        for (int a = 0; a < av; ++a) tma::load_4d(sb + SM_V + ((c & 1) * av + a) * kAtom, &p.mv, full, col0 + 64 * a, c * C, h, b);
+        for (int a = 0; a < av; ++a) tma::load_4d(sb + SM_V + ((c & 1) * av + a) * kAtom, &p.mv, full, col0 + 64 * a, t0 + c * C, h, b);
         if (c + 1 < nc) {
-          for (int a = 0; a < av; ++a) tma::prefetch_4d(&p.mv, col0 + 64 * a, (c + 1) * C, h, b);
+          for (int a = 0; a < av; ++a) tma::prefetch_4d(&p.mv, col0 + 64 * a, t0 + (c + 1) * C, h, b);
           for (int a = 0; a < aq; ++a) {
-            tma::prefetch_4d(&p.mq, 64 * a, (c + 1) * C, h, b);
-            tma::prefetch_4d(&p.mk, 64 * a, (c + 1) * C, h, b);
+            tma::prefetch_4d(&p.mq, 64 * a, t0 + (c + 1) * C, h, b);
+            tma::prefetch_4d(&p.mk, 64 * a, t0 + (c + 1) * C, h, b);
           }
         }
       }
@@ -269,10 +287,12 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
     // ---------------- state: one row (key dimension) per thread
     const int row = tid - 128;
     const uint32_t ts = tmem + ((uint32_t)((warp & 3) * 32) << 16) + TM_S;
-    const bool live = row < p.d, fresh = seq::position0(p.offsets, p.offset, b) == 0;
-    float* st = p.state + (((int64_t)b * p.H + h) * p.d + (live ? row : 0)) * p.dv + col0;
+    const bool live = row < p.d, fresh = !p.seg && seq::position0(p.offsets, p.offset, b) == 0;
+    const int64_t at = (int64_t)(live ? row : 0) * p.dv + col0, head = (int64_t)b * p.H + h;
+    float* st = p.state + head * p.d * p.dv + at;
+    const float* from = p.seg ? p.seg + (head * p.nseg + seg) * p.d * p.dv + at : st;
     for (int c = 0; c <= nc; ++c) {
-      const float g = c < nc ? pw[min(C, p.L - c * C)] : 0.f;
+      const float g = c < nc ? pw[min(C, L - c * C)] : 0.f;
       if (c > 0) {
         mbar_wait_bounded(B_S, (c - 1) & 1, abort_flag, p.status, 1u << 5);
         fence_after_sync();
@@ -286,12 +306,12 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
             float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live && !fresh) f = *reinterpret_cast<const float4*>(st + x + i);
+            if (live && !fresh) f = *reinterpret_cast<const float4*>(from + x + i);
             s[i] = __float_as_uint(f.x); s[i + 1] = __float_as_uint(f.y); s[i + 2] = __float_as_uint(f.z); s[i + 3] = __float_as_uint(f.w);
           }
         }
         if (c == nc) {
-          if (live) {
+          if (live && seg == p.nseg - 1) {
 #pragma unroll
             for (int i = 0; i < 16; i += 4)
               *reinterpret_cast<float4*>(st + x + i) = make_float4(__uint_as_float(s[i]), __uint_as_float(s[i + 1]), __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
@@ -321,7 +341,7 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
     // ---------------- scores and read-out: one token per thread
     const int i = tid;
     const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
-    bf16* out = p.out + b * p.ob + (int64_t)h * p.dv + col0;
+    bf16* out = p.out + b * p.ob + t0 * p.ol + (int64_t)h * p.dv + col0;
     for (int c = 0; c < nc; ++c) {
       mbar_wait_bounded(B_A, c & 1, abort_flag, p.status, 1u << 6);
       fence_after_sync();
@@ -359,7 +379,7 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
       mbar_wait_bounded(B_O, c & 1, abort_flag, p.status, 1u << 7);
       fence_after_sync();
       const float g = pw[i + 1];
-      const bool live = c * C + i < p.L;
+      const bool live = c * C + i < L;
       bf16* o = out + (int64_t)(c * C + i) * p.ol;
       uint8_t* tile = smem + SM_V + (c & 1) * av * kAtom;
       for (int x = 0; x < cols; x += 16) {
@@ -387,7 +407,7 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
       asm volatile("bar.sync 1, 128;" ::: "memory");   // these four warps
       if (tid == 0) {
         if (p.tma_out) {               // rows past the sequence and columns past the head are clipped
-          for (int a = 0; a < av; ++a) tma::store_4d(&p.mo, sb + SM_V + ((c & 1) * av + a) * kAtom, col0 + 64 * a, c * C, h, b);
+          for (int a = 0; a < av; ++a) tma::store_4d(&p.mo, sb + SM_V + ((c & 1) * av + a) * kAtom, col0 + 64 * a, t0 + c * C, h, b);
           bulk_commit();
           bulk_wait_read_all();
         }
@@ -405,6 +425,168 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
   }
 }
 
+// What one segment adds to the state by its end: sum_j k_j (g^(end-1-j) v_j)^T over its tokens, without the state before it.
+// grid (H, B, column slices x (segments - 1)).  All warps load, apply silu and write the operands of a chunk into one of two
+// stages; one elected lane issues.  Bound by the loads' latency: a CTA has 2 to 6 chunks, one of them in registers ahead.
+constexpr int kSegThreads = 512;
+__global__ void __launch_bounds__(kSegThreads, 1) lightning_segment_kernel(const __grid_constant__ Params p, const bf16* v, int64_t vb, int64_t vl) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t sb = smem_u32(smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.x, b = blockIdx.y, seg = blockIdx.z % (p.nseg - 1), col0 = blockIdx.z / (p.nseg - 1) * p.cols;
+  const int cols = min(p.cols, p.dv - col0);
+  const int t0 = seg * p.per * C, nc = p.per;            // the last segment is not among these: all chunks are whole
+  const int av = (p.cols + 63) / 64;
+  // shared memory: two stages of K (two atoms), hi and lo of the decayed V
+  const uint32_t STAGE = (2 + 2 * av) * kAtom, SM_POW = 2 * STAGE, SM_BAR = SM_POW + 132 * 4;
+  float* pw = reinterpret_cast<float*>(smem + SM_POW);
+  const uint32_t B_DONE = sb + SM_BAR;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_BAR + 16);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  if (tid == 0) {
+    mbar_init(B_DONE, 1);
+    mbar_init(B_DONE + 8, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (tid <= C) {   // powers by squaring
+    float r = 1.f, x = p.decay[h];
+    for (int e = tid; e > 0; e >>= 1) { if (e & 1) r *= x; x *= x; }
+    pw[tid] = r;
+  }
+  for (uint32_t s = 0; s < 2; ++s)
+    for (uint32_t i = tid * 16; i < 2 * kAtom; i += kSegThreads * 16) *reinterpret_cast<uint4*>(smem + s * STAGE + i) = make_uint4(0, 0, 0, 0);
+  if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 128);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  const int cq = p.d / 8, cv = cols / 8;
+  const int wq = 32 - __clz(cq - 1), wv = 32 - __clz(cv - 1);             // as in the kernel above
+  const int rowq = tid >> wq, rowv = tid >> wv, colq = tid & ((1 << wq) - 1), colv = tid & ((1 << wv) - 1);
+  const int stepq = kSegThreads >> wq, stepv = kSegThreads >> wv;
+  const bool onq = colq < cq && rowq < C, onv = colv < cv && rowv < C;
+  const bf16* k = p.k + b * p.kb + (int64_t)h * p.d + (t0 + rowq) * p.kl + colq * 8;
+  const bf16* vp = v + b * vb + (int64_t)h * p.dv + col0 + (t0 + rowv) * vl + colv * 8;
+  const uint32_t atq = (colq >> 3) * kAtom + tma::sw128_offset(rowq & (C - 1), colq & 7), atv = (colv >> 3) * kAtom + tma::sw128_offset(rowv & (C - 1), colv & 7);
+  constexpr int kPieces = C * 16 / kSegThreads;
+  uint4 rk[kPieces], rv[kPieces];
+  auto load = [&](uint4 (&r)[kPieces], const bf16* src, int64_t stride, int step, bool on) {
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i)
+      if (i * step < C) r[i] = on ? load16(src + i * step * stride) : make_uint4(0, 0, 0, 0);
+  };
+  load(rk, k, p.kl, stepq, onq);
+  load(rv, vp, vl, stepv, onv);
+  const uint32_t id_s = make_idesc_bf16(128, cols, 1, 1);
+  const bool leader = warp == 0 && elect_one_sync();
+  float rest = 1.f;                                        // g^(tokens between this chunk's end and the segment's)
+  for (int c = 1; c < nc; ++c) rest *= pw[C];
+  const float whole = pw[C];
+  for (int c = 0; c < nc; ++c) {
+    uint8_t* st = smem + (c & 1) * STAGE;
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+      if (i * stepq < C) { silu4(rk[i].x, rk[i].y); silu4(rk[i].z, rk[i].w); }
+      if (i * stepv < C) { silu4(rv[i].x, rv[i].y); silu4(rv[i].z, rv[i].w); }
+    }
+    if (c >= 2) mbar_wait_bounded(B_DONE + 8 * (c & 1), ((c >> 1) - 1) & 1, abort_flag, p.status, 1u << 11);
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+      if (onq && i * stepq < C) *reinterpret_cast<uint4*>(st + atq + i * stepq * 128) = rk[i];
+      if (onv && i * stepv < C) {
+        uint8_t* dst = st + 2 * kAtom + atv + i * stepv * 128;
+        const float f = rest * pw[C - 1 - rowv - i * stepv];
+        decayed(rv[i], f, dst, dst + av * kAtom);
+      }
+    }
+    // g^128 may be zero, and rest with it: it is multiplied up again from the end
+    rest = 1.f;
+    for (int m = c + 2; m < nc; ++m) rest *= whole;
+    fence_proxy_async();
+    if (c + 1 < nc) {
+      k += C * p.kl;
+      vp += C * vl;
+      load(rk, k, p.kl, stepq, onq);
+      load(rv, vp, vl, stepv, onv);
+    }
+    __syncthreads();
+    if (leader) {
+      const uint32_t at = sb + (c & 1) * STAGE;
+      const uint64_t dk = make_smem_desc_sw128(at, kAtom, 1024), d0 = make_smem_desc_sw128(at + 2 * kAtom, kAtom, 1024),
+                     d1 = make_smem_desc_sw128(at + (2 + av) * kAtom, kAtom, 1024);
+#pragma unroll
+      for (int m = 0; m < C / 16; ++m) {
+        mma_ss(tmem, dk + 128 * m, d0 + 128 * m, id_s, (c > 0 || m > 0) ? 1u : 0u);
+        mma_ss(tmem, dk + 128 * m, d1 + 128 * m, id_s, 1u);
+      }
+      mma_commit(B_DONE + 8 * (c & 1));
+    }
+    __syncwarp();
+  }
+  mbar_wait_bounded(B_DONE + 8 * ((nc - 1) & 1), ((nc - 1) >> 1) & 1, abort_flag, p.status, 1u << 12);
+  fence_after_sync();
+  // four warps to a quadrant of 32 rows, 16 columns of every 64 each
+  const int row = (warp & 3) * 32 + lane;
+  float* dst = p.seg + (((int64_t)b * p.H + h) * p.nseg + seg + 1) * p.d * p.dv + (int64_t)row * p.dv + col0;
+  for (int x = (warp >> 2) * 16; x < cols; x += 64) {
+    uint32_t s[16];
+    tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + x, s);
+    tmem_ld_wait();
+    if (row < p.d) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4)
+        *reinterpret_cast<float4*>(dst + x + i) = make_float4(__uint_as_float(s[i]), __uint_as_float(s[i + 1]), __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    fence_after_sync();
+    tmem_dealloc(tmem, 128);
+  }
+}
+
+// seg [B H][nseg][n]: slot s + 1 holds what segment s adds; becomes the state before segment s + 1, slot 0 the state of the call.
+// A thread owns four consecutive entries and has eight segments' loads in flight.
+__global__ void __launch_bounds__(256) lightning_scan_kernel(const __grid_constant__ Params p) {
+  const int n = p.d * p.dv, i = (blockIdx.x * 256 + threadIdx.x) * 4, head = blockIdx.y;
+  if (i >= n) return;
+  float g = 1.f, x = p.decay[head % p.H];
+  for (int e = p.per * C; e > 0; e >>= 1) { if (e & 1) g *= x; x *= x; }
+  float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (seq::position0(p.offsets, p.offset, head / p.H) > 0) S = *reinterpret_cast<const float4*>(p.state + (int64_t)head * n + i);
+  float* at = p.seg + (int64_t)head * p.nseg * n + i;
+  *reinterpret_cast<float4*>(at) = S;
+  constexpr int U = 8;
+  for (int s0 = 1; s0 < p.nseg; s0 += U) {
+    float4 a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s0 + u < p.nseg) a[u] = *reinterpret_cast<const float4*>(at + (int64_t)(s0 + u) * n);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s0 + u < p.nseg) {
+        S = make_float4(fmaf(g, S.x, a[u].x), fmaf(g, S.y, a[u].y), fmaf(g, S.z, a[u].z), fmaf(g, S.w, a[u].w));
+        *reinterpret_cast<float4*>(at + (int64_t)(s0 + u) * n) = S;
+      }
+  }
+}
+
+// Segments and chunks per segment of a call.  Cut when every SM can have a segment of at least two chunks and two segments
+// exist: below that the two extra launches (about 6 us) cost more than the shorter chain saves.
+void segments(int B, int L, int H, int dv, int* nseg, int* per) {
+  const int64_t chains = (int64_t)B * H * ((dv + 127) / 128);
+  const int nc = (L + C - 1) / C;
+  *nseg = 1;
+  *per = nc;
+  if (chains * 2 > 148 || nc < kMinSplitChunks) return;
+  const int most = (int)(148 / chains);
+  *per = std::max(2, (nc + most - 1) / most);
+  *nseg = (nc + *per - 1) / *per;
+}
+
 }  // namespace
 
 int read_tc_status_lightning(unsigned int* out, int reset) {
@@ -419,25 +601,37 @@ int read_tc_status_lightning(unsigned int* out, int reset) {
   return (int)e;
 }
 
-// BASED_ERR_IMPL: sizes or strides this kernel does not take.
+// Bytes of the per-segment states; 0 where a call is not cut.
+size_t lightning_tc_scratch_bytes(int B, int L, int H, int d, int dv) {
+  int nseg, per;
+  segments(B, L, H, dv, &nseg, &per);
+  return nseg > 1 ? sizeof(float) * (size_t)B * H * nseg * d * dv : 0;
+}
+
+// With scratch the sequence is cut where that is faster.  BASED_ERR_IMPL: sizes or strides this kernel does not take.
 int launch_lightning_tc(const void* q, const void* k, const void* v, const float* decay, float* state, void* out, int B, int L,
                         int H, int d, int dv, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so, const int32_t* offsets,
-                        int offset, cudaStream_t stream) {
+                        int offset, void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (d % 16 || d > 128 || dv % 16 || B > 65535) return BASED_ERR_IMPL;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(state)) return BASED_ERR_IMPL;
   for (const Strides2& s : {sq, sk, sv, so})
     if (s.h % 8 || (B > 1 && s.b % 8)) return BASED_ERR_IMPL;
   Params p{{}, {}, {}, {}, static_cast<const bf16*>(q), static_cast<const bf16*>(k), decay, state, static_cast<bf16*>(out), offsets,
-           sq.b, sq.h, sk.b, sk.h, so.b, so.h, offset, L, H, d, dv, 0, 0, nullptr};
+           sq.b, sq.h, sk.b, sk.h, so.b, so.h, offset, L, H, d, dv, 0, 0, 1, (L + C - 1) / C, nullptr, nullptr};
+  if (scratch) segments(B, L, H, dv, &p.nseg, &p.per);
+  if (p.nseg > 1) {
+    if (!aligned16(scratch) || scratch_bytes < lightning_tc_scratch_bytes(B, L, H, d, dv)) return BASED_ERR_SCRATCH;
+    p.seg = static_cast<float*>(scratch);
+  }
   // few (batch, head) pairs: their value columns over several CTAs, at least 32 each
   int slices = (dv + 127) / 128;
-  while ((int64_t)B * H * slices * 2 <= 148 && dv / (slices * 2) >= 32) slices *= 2;
+  while (p.nseg == 1 && (int64_t)B * H * slices * 2 <= 148 && dv / (slices * 2) >= 32) slices *= 2;
   p.cols = ((dv + slices - 1) / slices + 15) / 16 * 16;
   slices = (dv + p.cols - 1) / p.cols;
   const int aq = (d + 63) / 64, av = (p.cols + 63) / 64;
   constexpr int kMaxSmem = 227 * 1024;
   const int smem = (aq + 2 + 5 * av) * (int)kAtom + kTables * 4 + 88 + 1024;
-  if (smem > kMaxSmem || slices > 65535) return BASED_ERR_IMPL;
+  if (smem > kMaxSmem || slices * p.nseg > 65535) return BASED_ERR_IMPL;
   {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
@@ -452,6 +646,8 @@ int launch_lightning_tc(const void* q, const void* k, const void* v, const float
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&addr), g_tc_status_lightning);
       if (e != cudaSuccess) return (int)e;
       e = cudaFuncSetAttribute(lightning_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+      if (e != cudaSuccess) return (int)e;
+      e = cudaFuncSetAttribute(lightning_segment_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
       if (e != cudaSuccess) return (int)e;
       status[dev] = addr;
     }
@@ -470,7 +666,12 @@ int launch_lightning_tc(const void* q, const void* k, const void* v, const float
   };
   if (get_map(&p.mq, q, d, sq) || get_map(&p.mk, k, d, sk) || get_map(&p.mv, v, dv, sv) || get_map(&p.mo, out, dv, so)) return BASED_ERR_IMPL;
   p.tma_out = slices == 1 || p.cols % 64 == 0;   // a slice's tile must not reach into the next one
-  lightning_tc_kernel<<<dim3(H, B, slices), NT, smem, stream>>>(p);
+  if (p.nseg > 1) {
+    const int seg_smem = 2 * (2 + 2 * av) * (int)kAtom + 132 * 4 + 24 + 1024;
+    lightning_segment_kernel<<<dim3(H, B, slices * (p.nseg - 1)), kSegThreads, seg_smem, stream>>>(p, static_cast<const bf16*>(v), sv.b, sv.h);
+    lightning_scan_kernel<<<dim3((d * dv / 4 + 255) / 256, B * H), 256, 0, stream>>>(p);
+  }
+  lightning_tc_kernel<<<dim3(H, B, slices * p.nseg), NT, smem, stream>>>(p);
   return (int)cudaGetLastError();
 }
 

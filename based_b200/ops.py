@@ -1153,10 +1153,13 @@ def lightning(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     off, scalar = _position(pos, q)
     if out.numel() == 0:
         return out
+    lib = _capi.lib()
+    need = lib.based_lightning_scratch_bytes(B, L, H, d, dv) if q.dtype == torch.bfloat16 and impl != "simt" else 0
     with torch.cuda.device(q.device):
-        code = _capi.lib().based_lightning(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), B, L,
-                                           H, d, dv, _strides_bl(q), _strides_bl(k), _strides_bl(v), _strides_bl(out), off, scalar,
-                                           _dt(q.dtype), _IMPLS[impl], _stream())
+        scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
+        code = lib.based_lightning_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), B, L,
+                                         H, d, dv, _strides_bl(q), _strides_bl(k), _strides_bl(v), _strides_bl(out), off, scalar,
+                                         _dt(q.dtype), _IMPLS[impl], _ptr(scratch), need, _stream())
     _capi.check(code, "based_lightning")
     return out
 

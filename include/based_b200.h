@@ -607,6 +607,17 @@ int based_lightning(const void* q, const void* k, const void* v, const void* dec
                     const int64_t out_strides[2], const int32_t* offsets, int offset, int io_dtype, int impl, void* stream);
 
 /*
+ * The same with a workspace of based_lightning_scratch_bytes bytes (16-byte aligned, contents do not matter): the chunked kernel
+ * then cuts the sequence into segments that run side by side when few (batch, head) pairs would leave the machine idle.  0 bytes:
+ * this call is not cut.  scratch NULL: as based_lightning.  BASED_ERR_SCRATCH: too small or misaligned.
+ */
+size_t based_lightning_scratch_bytes(int B, int L, int H, int d, int dv);
+int based_lightning_split(const void* q, const void* k, const void* v, const void* decay, void* state, void* out, int B, int L,
+                          int H, int d, int dv, const int64_t q_strides[2], const int64_t k_strides[2], const int64_t v_strides[2],
+                          const int64_t out_strides[2], const int32_t* offsets, int offset, int io_dtype, int impl, void* scratch,
+                          size_t scratch_bytes, void* stream);
+
+/*
  * One token per row, from slices of the packed projection (q, k, v, gate: rows x_row_stride apart) to the gated output in one
  * launch: out = norm over all heads of the read-out * norm_weight * sigmoid(gate).  read [B, H dv] fp32 is workspace, count
  * [B] int32 is zero before the first call and zero again after every call.  BASED_ERR_IMPL for dv % 4 or d above 1024.

@@ -81,6 +81,19 @@ def test_many_heads_fill_the_machine_without_a_split():
     check(args, product(*args, [140], impl="tcgen05"), torch.bfloat16)
 
 
+@pytest.mark.parametrize("d,dv,T,H", [(64, 48, 896, 4), (64, 48, 897, 4), (128, 128, 2047, 2), (128, 160, 1300, 3), (32, 16, 2500, 1), (16, 64, 1025, 37), (48, 64, 1025, 38)])
+def test_a_cut_sequence(d, dv, T, H):
+    """Sequences that run as segments side by side (from eight chunks on, while two segments of every chain find an SM), as a
+    prompt and after a first portion, against the same call in portions that are not cut."""
+    args = case([DECAYS[i % 4] for i in range(H)], d, dv, T, seed=T)
+    whole = product(*args, [T])
+    check(args, whole, torch.bfloat16)
+    check(args, product(*args, [129, T - 129], device_pos=True), torch.bfloat16)
+    few = product(*args, [513])     # no portion below 16 tokens: those take the kernel that does not round its activations
+    assert float((whole[1] - few[1]).abs().max() / few[1].abs().max()) < 2e-5     # bf16 pairs carry 2^-17; fp32 sums
+    assert float((whole[0] - few[0]).abs().max() / few[0].abs().max()) < 1e-2     # one bf16 rounding
+
+
 def test_portions_and_decoding_agree():
     args = case(DECAYS, 64, 48, 600, B=2)
     for cuts in ([600], [2], [128, 128, 1, 127, 3], [500, 1], [31, 33, 200], [15, 17, 16], [129]):
