@@ -49,6 +49,28 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// How many clusters of K CTAs of a kernel are on the device at once (the SMs of a cluster share a GPC, and GPCs differ in
+// size: 148 SMs hold fewer than 148 / K clusters).  0 when the runtime has no answer.  Launchers ask once per K and keep it.
+template <typename... P>
+inline int max_active_clusters(void (*kernel)(P...), int K, int threads, int smem) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = K;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(K);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Launchers implemented one per .cu file; all return a cudaError_t-compatible int (0 = ok).

@@ -9,6 +9,14 @@
 // last, and only then writes S_t * gelu(y_t): the serial part is one multiply-add per 16 tokens.
 // Warp 16 loads u by TMA (two stages) and issues the MMAs (two accumulator buffers); the weights stay in shared memory.
 // Warp 17 loads the y tiles and stores the output tiles, which replace y's values in place.
+//
+// A CTA's time is its number of tiles times the latency of one (3 us): with few rows and blocks most SMs would idle.  There a
+// CLUSTER of 2 to 8 CTAs shares a sequence, a run of tiles each.  A CTA goes over its tiles twice: first for what they make
+// of a state (their decays' product and the end state from zero; no y, no output), then, with its state at the start folded
+// from the CTAs before it over distributed shared memory, for the output.  The first pass takes about two thirds of the
+// second's time, so a run of n / K tiles costs 1.7 n / K.  B = 2, 8 blocks of 128, L = 4096: 190 us
+// with a CTA per block, 67 us with six (of eight-CTA clusters only 15 fit the device, and a second wave took 97 us).
+#include <algorithm>
 #include <initializer_list>
 #include <mutex>
 
@@ -28,6 +36,8 @@ using bf16 = __nv_bfloat16;
 constexpr int TT = 64, GROUPS = 4, TG = TT / GROUPS;   // tokens per tile, groups, tokens per group
 constexpr int NC = 128 * GROUPS, NT = NC + 64;
 constexpr uint32_t kWAtom = 128 * 128, kUAtom = TT * 128;   // bytes of 64 columns x 128 (64) rows
+constexpr uint32_t kSummary = (GROUPS + 1) * 128 * 4;
+constexpr int kMaxCluster = 8;
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct Params {
@@ -36,13 +46,24 @@ struct Params {
   const float* lam;
   float* state;
   const int32_t* offsets;
-  int offset, L, W, n, slices, atoms;
+  int offset, L, W, n, slices, atoms, K;   // K: CTAs per sequence (cluster size)
   unsigned int* status;
 };
 
 __device__ __forceinline__ float ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float sqrt_approx(float x) { float r; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
+// The cluster barrier's two halves, called by diverged threads too.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+__device__ __forceinline__ float ld_peer(uint32_t saddr, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(saddr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
 
 __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -52,11 +73,15 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
     return;
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int blk = blockIdx.x / p.slices, c0 = (blockIdx.x % p.slices) * 128, b = blockIdx.y;
-  const int nt = (p.L + TT - 1) / TT;
+  const int rank = blockIdx.x % p.K, unit = blockIdx.x / p.K;   // consecutive blocks are a cluster
+  const int blk = unit / p.slices, c0 = (unit % p.slices) * 128, b = blockIdx.y;
+  const int tiles = (p.L + TT - 1) / TT, first = tiles * rank / p.K, n2 = tiles * (rank + 1) / p.K - first;
+  const int n1 = rank < p.K - 1 ? n2 : 0, nt = n1 + n2;         // steps: n1 tiles for the summary, then n2 for the output
+  auto token = [&](int t) { return (first + (t < n1 ? t : t - n1)) * TT; };
   // shared memory: W_r, W_i (atoms each), u stages, y stages (two 64-channel atoms each), carries, barriers
+  // and, with K > 1, the summary for the CTAs after this one (a product per group, the end state)
   const uint32_t SM_U = 2u * p.atoms * kWAtom, SM_Y = SM_U + 2u * p.atoms * kUAtom, SM_C = SM_Y + 4u * kUAtom,
-                 SM_BAR = SM_C + GROUPS * 128 * 4;
+                 SM_SUM = SM_C + GROUPS * 128 * 4, SM_BAR = SM_SUM + (p.K > 1 ? kSummary : 0);
   const uint32_t B_W = sb + SM_BAR, B_FULL = B_W + 8, B_D = B_FULL + 16, B_EMPTY = B_D + 16, B_Y = B_EMPTY + 16,
                  B_OUT = B_Y + 16, B_CARRY = B_OUT + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_BAR + 8 * (11 + GROUPS));
@@ -75,6 +100,13 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;   // buffer x: r gates in columns 128 x .., i gates in columns 128 x + 64 ..
 
+  // Cluster barrier 1: the summaries are written (and the call's state is read); 2: they have been read.  Threads that neither
+  // write nor read arrive here at once and wait at the end.
+  const bool writer = n1 > 0 && warp < NC / 32, reader = rank > 0 && warp < 4;
+  float S0 = 0.f;
+  if (warp < 4 && c0 + tid < p.n && seq::position0(p.offsets, p.offset, b) > 0) S0 = p.state[(int64_t)b * p.W + blk * p.n + c0 + tid];
+  if (p.K > 1 && !writer) cluster_arrive();
+
   if (warp == NC / 32) {
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
     const bool leader = elect_one_sync();
@@ -82,7 +114,7 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
       if (leader) {
         tma::mbar_expect_tx(B_FULL + 8 * (t & 1), (uint32_t)p.atoms * kUAtom);
         for (int a = 0; a < p.atoms; ++a)
-          tma::load_4d(sb + SM_U + ((t & 1) * p.atoms + a) * kUAtom, &p.mu, B_FULL + 8 * (t & 1), blk * p.n + 64 * a, t * TT, 0, b);
+          tma::load_4d(sb + SM_U + ((t & 1) * p.atoms + a) * kUAtom, &p.mu, B_FULL + 8 * (t & 1), blk * p.n + 64 * a, token(t), 0, b);
       }
     };
     if (leader) {
@@ -125,16 +157,16 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
       auto load_y = [&](int t) {
         tma::mbar_expect_tx(B_Y + 8 * (t & 1), (uint32_t)na * kUAtom);
         for (int a = 0; a < na; ++a)
-          tma::load_4d(sb + SM_Y + ((t & 1) * 2 + a) * kUAtom, &p.my, B_Y + 8 * (t & 1), c0 + 64 * a, t * TT, blk, b);
+          tma::load_4d(sb + SM_Y + ((t & 1) * 2 + a) * kUAtom, &p.my, B_Y + 8 * (t & 1), c0 + 64 * a, (first + t) * TT, blk, b);
       };
       load_y(0);
-      if (nt > 1) load_y(1);
-      for (int t = 0; t < nt; ++t) {
+      if (n2 > 1) load_y(1);
+      for (int t = 0; t < n2; ++t) {
         mbar_wait_bounded<false>(B_OUT + 8 * (t & 1), (t >> 1) & 1, abort_flag, p.status, 1u << 23);
-        for (int a = 0; a < na; ++a) tma::store_4d(&p.mo, sb + SM_Y + ((t & 1) * 2 + a) * kUAtom, c0 + 64 * a, t * TT, blk, b);
+        for (int a = 0; a < na; ++a) tma::store_4d(&p.mo, sb + SM_Y + ((t & 1) * 2 + a) * kUAtom, c0 + 64 * a, (first + t) * TT, blk, b);
         bulk_commit();
         bulk_wait_read_all();
-        if (t + 2 < nt) load_y(t + 2);
+        if (t + 2 < n2) load_y(t + 2);
       }
       bulk_wait_all();
     }
@@ -153,10 +185,12 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
     const int ychunk = (ch & 63) >> 3;
     const uint8_t* ucol = smem + SM_U + ((c0 + ch) >> 6) * kUAtom + (ch & 7) * 2;   // this channel's column of a stage
     const int chunk = ((c0 + ch) & 63) >> 3;
-    float S0 = 0.f;
-    if (grp == 0 && live && seq::position0(p.offsets, p.offset, b) > 0) S0 = p.state[(int64_t)b * p.W + chan];
+    float* sum = reinterpret_cast<float*>(smem + SM_SUM) + ch;
+    const float given = S0;          // group 0: the state the call starts from
+    if (n1 > 0) S0 = 0.f;
+    float prod = 1.f;
     for (int t = 0; t < nt; ++t) {
-      const int x = t & 1, tok0 = t * TT + t0g;
+      const int x = t & 1, tok0 = token(t) + t0g;
       mbar_wait_bounded(B_D + 8 * x, (t >> 1) & 1, abort_flag, p.status, 1u << 21);
       fence_after_sync();
       uint32_t gr[TG], gi[TG];
@@ -194,11 +228,34 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
         mbar_wait_bounded(from, (grp > 0 ? t : t - 1) & 1, abort_flag, p.status, 1u << 22);
         S0 = *carry_in;
       }
+      if (grp == 0 && t == n1) {     // the output starts from what the CTAs before make of the call's state
+        S0 = given;
+        if (reader) {
+          cluster_wait();
+          for (int r = 0; r < rank; ++r) {
+            float a = 1.f;
+#pragma unroll
+            for (int i = 0; i < GROUPS; ++i) a *= ld_peer(smem_u32(sum + 128 * i), r);
+            S0 = fmaf(a, S0, ld_peer(smem_u32(sum + 128 * GROUPS), r));
+          }
+          cluster_arrive();
+        }
+      }
       const float end = fmaf(pr, S0, sr);
       carry[grp * 128 + ch] = end;
       mbar_arrive(my_carry);
-      mbar_wait_bounded(B_Y + 8 * x, (t >> 1) & 1, abort_flag, p.status, 1u << 24);
-      uint8_t* ys = ycol + x * 2 * kUAtom;
+      if (t < n1) {
+        prod *= pr;
+        if (t == n1 - 1) {
+          sum[128 * grp] = prod;
+          if (grp == GROUPS - 1) sum[128 * GROUPS] = end;
+          cluster_arrive();
+        }
+        continue;
+      }
+      const int yx = (t - n1) & 1;
+      mbar_wait_bounded(B_Y + 8 * yx, ((t - n1) >> 1) & 1, abort_flag, p.status, 1u << 24);
+      uint8_t* ys = ycol + yx * 2 * kUAtom;
       auto at = [&](int i) { return reinterpret_cast<bf16*>(ys + (t0g + i) * 128 + ((ychunk ^ (i & 7)) << 4)); };   // t0g is a multiple of 8
       bf16 yv[TG];   // all read before the first is replaced
 #pragma unroll
@@ -207,9 +264,13 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
       for (int i = 0; i < TG; ++i)     // rows past the sequence and channels past the block are clipped by the store
         *at(i) = __float2bfloat16_rn(fmaf(P[i], S0, s[i]) * seq::gelu_tanh_t<bf16>(__bfloat162float(yv[i])));
       fence_proxy_async();
-      mbar_arrive(B_OUT + 8 * x);
-      if (live && grp == GROUPS - 1 && t == nt - 1) p.state[(int64_t)b * p.W + chan] = end;
+      mbar_arrive(B_OUT + 8 * yx);
+      if (live && grp == GROUPS - 1 && t == nt - 1 && rank == p.K - 1) p.state[(int64_t)b * p.W + chan] = end;
     }
+  }
+  if (p.K > 1) {
+    if (!reader) { cluster_wait(); cluster_arrive(); }
+    cluster_wait();
   }
   __syncwarp();
   fence_before_sync();
@@ -266,12 +327,15 @@ int launch_rglru_tc(const void* u, const void* y, const void* w, const void* rb,
   p.ib = static_cast<const bf16*>(ib);
   p.lam = lam; p.state = state;
   p.offsets = offsets; p.offset = offset; p.L = L; p.W = W; p.n = n;
-  const int smem = 2 * p.atoms * (int)(kWAtom + kUAtom) + 4 * (int)kUAtom + GROUPS * 128 * 4 + 8 * (11 + GROUPS) + 16;
+  int smem = 2 * p.atoms * (int)(kWAtom + kUAtom) + 4 * (int)kUAtom + GROUPS * 128 * 4 + 8 * (11 + GROUPS) + 16;
   if (smem > 227 * 1024) return BASED_ERR_IMPL;
+  const int tiles = (L + TT - 1) / TT;
+  p.K = 1;
   {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
     static unsigned int* status[kMaxDevices] = {};
+    static short room[kMaxDevices][kMaxCluster + 1][4] = {};   // clusters of a size on the device at once, + 1
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -286,9 +350,33 @@ int launch_rglru_tc(const void* u, const void* y, const void* w, const void* rb,
       status[dev] = addr;
     }
     p.status = status[dev];
+    // The largest cluster of which all fit the device at once (a second wave costs more than a smaller cluster) and whose CTAs
+    // have two tiles or more (with one tile each the second pass, the exchange and the launch cost what the shorter chain
+    // saves).  Blocks of 256 leave no room for the summary in shared memory.
+    if (smem + (int)kSummary <= 227 * 1024)
+      for (int K = std::min(kMaxCluster, tiles / 2); K > 1; --K) {
+        const int64_t units = (int64_t)blocks * p.slices * B;
+        if (units * K > 148) continue;
+        short& r = room[dev][K][p.atoms - 1];
+        if (r == 0) r = (short)(1 + max_active_clusters(rglru_tc_kernel, K, NT, smem + (int)kSummary));
+        if (r - 1 < units) continue;
+        p.K = K;
+        smem += kSummary;
+        break;
+      }
   }
-  rglru_tc_kernel<<<dim3(blocks * p.slices, B), NT, smem, stream>>>(p);
-  return (int)cudaGetLastError();
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = p.K;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks * p.slices * p.K, B);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p.K > 1 ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, rglru_tc_kernel, p);
 }
 
 }  // namespace based

@@ -192,6 +192,36 @@ def test_rglru(W, blocks, dtype):
         assert rel_err(out.float().cpu(), ref) < (2e-5 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("W,blocks,L,B", [(128, 1, 193, 2), (512, 2, 257, 1), (144, 1, 449, 1), (96, 1, 512, 2), (512, 4, 961, 1), (1024, 8, 1100, 3), (128, 2, 4096, 2), (256, 1, 700, 1)])
+def test_rglru_shared_sequences(W, blocks, L, B):
+    """Lengths at which 2, 4 or 8 CTAs share a sequence (4, 8 and 16 tiles of 64 tokens and one more), from the start and from a state."""
+    from based_b200 import ops
+    g = torch.Generator().manual_seed(L)
+    n = W // blocks
+    u, y = (torch.randn(B, L, W, generator=g).bfloat16() for _ in range(2))
+    ra, ri = ((torch.randn(blocks, n, n, generator=g) / n ** 0.5).bfloat16() for _ in range(2))
+    rb, ib = ((torch.randn(blocks, n, generator=g) - 1).bfloat16() for _ in range(2))
+    lam = 2 * torch.randn(W, generator=g) - 4
+    ref, last = [], []
+    for i in range(B):
+        ud = u[i].double()
+        r, gi = (torch.sigmoid(R.block_linear(ud, m.double(), c.double())) for m, c in ((ra, rb), (ri, ib)))
+        S = R.rglru_scan(ud, r, gi, lam.double())
+        ref.append(S * R.gelu_tanh(y[i].double()))
+        last.append(S[-1])
+    ref, last = torch.stack(ref), torch.stack(last)
+    gw, ud, yd = torch.stack([ra, ri], 1).contiguous().cuda(), u.cuda(), y.cuda()
+    for parts in ([L], [9, L - 9]):
+        state, out, at = torch.full((B, W), 5.0, device="cuda"), torch.empty(B, L, W, dtype=torch.bfloat16, device="cuda"), 0
+        for m in parts:
+            ops.rglru_gated(ud[:, at:at + m], yd[:, at:at + m], gw, rb.reshape(W).cuda(), ib.reshape(W).cuda(), lam.cuda(), state, pos=at,
+                            out=out[:, at:at + m])
+            at += m
+        ops.check_status()
+        assert rel_err(state.cpu(), last) < 2e-5
+        assert rel_err(out.float().cpu(), ref) < 1e-2
+
+
 @pytest.mark.parametrize("D", [64, 96, 50, 2048, 1031, 7168])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_stream_norm(D, dtype):
