@@ -4,226 +4,433 @@
 //
 // Replaces LinearAttention.parallel_forward's "quadratic" branch
 // (based/models/mixers/linear_attention.py:171-182) and the state hand-off (:220-222) in
-// O(L) memory: the sequence is walked in blocks of T tokens; within a block the causal part
-// uses phi(q).phi(k) = 1 + s + s^2/2 (s = q.k/4), across blocks the [273 x dv] state is
-// carried in registers.
+// O(L) memory: the sequence is walked in chunks of 64 tokens; within a chunk the causal part
+// uses phi(q).phi(k) = 1 + s + s^2/2 (s = q.k/4), across chunks the state is carried in registers.
 //
-// One CTA per (batch, head).  Thread (j, g) with j < dv, g < 4 owns state column j for the
-// features [g*69, g*69+69); one extra warp owns k_state.
+// Bound by the fp32 FMA rate.  The 256 products x_i x_j of the feature map are symmetric: the kernel keeps 153 features (1, x/2,
+// products i <= j) with phi(k) scaled as in the 273 and the products i < j of phi(q) doubled, so that its state is the 273-feature
+// state and every step has 56 % of the multiply-adds.  Per chunk and 64 value columns three register-tiled products run
+// (256 threads, operands in shared memory): O = phi(q) S (4 x 4 per thread), O += P V (4 x 4), S += phi(k)^T V (20 x 2, the
+// accumulators ARE the state): 1.6 M multiply-adds, 12 k cycles at the FMA rate; issue
+// slots are 50 % used (two warps per scheduler, products in registers at 207 of them), so a chunk takes about 25 k.
+//
+// One CTA walks one (batch, head) and up to 64 value columns; with few of those a CLUSTER of 2 to 8 CTAs shares the sequence,
+// a run of chunks each: first what the run adds to the state (the state product alone, 45 % of the work), then, from the sum
+// of the runs before it, read over distributed shared memory in order, the output.  K CTAs take 1.45 / K of the time.
+// B = 2, H = 16, L = 1024, dv = 64: 925 us with a CTA per head and 16-token blocks over 273 features, 98 us like this.
+#include <mutex>
+#include <utility>
+
 #include "common.cuh"
 
 namespace based {
 namespace {
 
-constexpr int G = 4;         // feature groups
-constexpr int FPG = 69;      // features per group (4 * 69 = 276 >= 273)
-constexpr int DP = G * FPG;  // padded feature count, 276
+constexpr int T = 64;          // tokens per chunk
+constexpr int CW = 64;         // value columns per CTA
+constexpr int FP = 160;        // packed features: 153, padded
+constexpr int kPacked = 153;
+constexpr int SP = 68;         // row pitch of the state in shared memory
+constexpr int KP = FP + 4;     // row pitch of phi(k): eight tokens' 16-byte pieces are in different banks
+constexpr int NT = 256;
+constexpr int kMaxCluster = 8;
 
-template <int T>
-struct SmemLayout {
-  // all offsets in floats
-  int q, k, v, phiq, phik, p, part, den, total;
-  __host__ __device__ explicit SmemLayout(int dv) {
-    int o = 0;
-    q = o; o += T * kFeatureDim;
-    k = o; o += T * kFeatureDim;
-    v = o; o += T * dv;
-    phiq = o; o += DP * T;   // [f][t]
-    phik = o; o += DP * T;   // [f][t]
-    p = o; o += T * T;       // [t][s]
-    part = o; o += G * T * dv;  // [g][t][j]
-    den = o; o += T;
-    total = o;
-  }
+struct Smem {
+  float phi[KP * T];           // phi(q) as [feature][token], then phi(k) as [token][feature]
+  float S[FP * SP];            // [feature][column]
+  float v[T * CW];             // [token][column]
+  float p[T * T];              // [key][query]
+  float qt[kFeatureDim * T];   // [dim][token]
+  float k[T * kFeatureDim];    // [token][dim]
+  float den[4 * T];
+  float z[FP];                 // normaliser's state
+  unsigned char at[kExpandedDim + 3];   // packed place of each of the 273
 };
 
-// T = tokens per block step; MAXT = thread-count bound (sets the register budget).
-template <typename IO, typename ST, int T, int MAXT>
-__global__ void __launch_bounds__(MAXT)
-linattn_prefill_simt_kernel(const IO* __restrict__ q, const IO* __restrict__ k, const IO* __restrict__ v,
-                            IO* __restrict__ y, ST* __restrict__ kv_state, ST* __restrict__ k_state, int H, int L,
-                            int dv, Strides3 sq, Strides3 sk, Strides3 sv, Strides3 sy, float eps) {
-  extern __shared__ __align__(16) float smem[];
-  const SmemLayout<T> lay(dv);
-  float* s_q = smem + lay.q;
-  float* s_k = smem + lay.k;
-  float* s_v = smem + lay.v;
-  float* s_phiq = smem + lay.phiq;
-  float* s_phik = smem + lay.phik;
-  float* s_p = smem + lay.p;
-  float* s_part = smem + lay.part;
-  float* s_den = smem + lay.den;
+// Dims of packed feature f >= 17, the products i <= j in rows of i.
+__host__ __device__ constexpr int pair_i(int f) {
+  int i = 0, left = f - 1 - kFeatureDim;
+  while (left >= kFeatureDim - i) left -= kFeatureDim - i++;
+  return i;
+}
+__host__ __device__ constexpr int pair_j(int f) {
+  int i = 0, left = f - 1 - kFeatureDim;
+  while (left >= kFeatureDim - i) left -= kFeatureDim - i++;
+  return i + left;
+}
+// Packed feature F of the 16 values in x (registers: every index is known here); QUERY: products i < j twice, for (j, i) too.
+template <int F, bool QUERY>
+__device__ __forceinline__ float feature(const float (&x)[kFeatureDim]) {
+  if constexpr (F == 0) return 1.f;
+  else if constexpr (F <= kFeatureDim) return x[F - 1] * kC1;
+  else if constexpr (F >= kPacked) return 0.f;
+  else {
+    constexpr int i = pair_i(F), j = pair_j(F);
+    return x[i] * x[j] * (QUERY && i != j ? 2.f * kC2 : kC2);
+  }
+}
+// Features [F0, F0 + 40) of one token: of phi(q) at dst[f * T], of phi(k) at dst[f].
+template <int F0, int... I>
+__device__ __forceinline__ void put_query(float* dst, const float (&x)[kFeatureDim], std::integer_sequence<int, I...>) {
+  ((dst[(F0 + I) * T] = feature<F0 + I, true>(x)), ...);
+}
+template <int F0, int... I>
+__device__ __forceinline__ void put_key(float* dst, const float (&x)[kFeatureDim], bool live, std::integer_sequence<int, I...>) {
+  ((*reinterpret_cast<float4*>(dst + F0 + 4 * I) =
+        live ? make_float4(feature<F0 + 4 * I, false>(x), feature<F0 + 4 * I + 1, false>(x), feature<F0 + 4 * I + 2, false>(x), feature<F0 + 4 * I + 3, false>(x))
+             : make_float4(0.f, 0.f, 0.f, 0.f)), ...);
+}
 
-  const int tid = threadIdx.x, nthreads = blockDim.x;
-  const int bh = blockIdx.x, b = bh / H, h = bh - b * H;
-  const int nkv = G * dv;                 // threads that own kv_state columns
-  const bool is_kv = tid < nkv;
-  const bool is_ks = tid >= nkv;          // the trailing warp
-  const int j = is_kv ? tid % dv : 0;
-  const int g = is_kv ? tid / dv : 0;
-  const int lane = tid & 31;
+template <typename IO>
+struct Args {
+  const IO *q, *k, *v;
+  IO* y;
+  void *kv_state, *k_state;
+  int H, L, dv, K, vec_out, state_bf16;   // K: CTAs per sequence
+  Strides3 sq, sk, sv, sy;
+  float eps;
+};
 
-  const IO* qb = q + b * sq.b + h * sq.h;
-  const IO* kb = k + b * sk.b + h * sk.h;
-  const IO* vb = v + b * sv.b + h * sv.h;
-  IO* yb = y + b * sy.b + h * sy.h;
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* own, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(own)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float ld_peer(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_peer2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
 
-  float S[FPG];
+// acc[a][b] += x[a] * y[b]
+__device__ __forceinline__ void outer4(float (&acc)[4][4], const float4& x, const float4& y) {
+  const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-  for (int i = 0; i < FPG; ++i) S[i] = 0.f;
-  float ks[9];
+  for (int a = 0; a < 4; ++a)
 #pragma unroll
-  for (int i = 0; i < 9; ++i) ks[i] = 0.f;
+    for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(xs[a], ys[b], acc[a][b]);
+}
 
-  for (int t0 = 0; t0 < L; t0 += T) {
-    const int nt = min(T, L - t0);
-    // ---- load the block (zero-filled past the end) ----
-    for (int i = tid; i < T * kFeatureDim; i += nthreads) {
-      const int t = i >> 4, c = i & 15;
-      const bool ok = t < nt;
-      s_q[i] = ok ? to_float(qb[(int64_t)(t0 + t) * sq.l + c]) : 0.f;
-      s_k[i] = ok ? to_float(kb[(int64_t)(t0 + t) * sk.l + c]) : 0.f;
+template <typename IO>
+__global__ void __launch_bounds__(NT, 1) linattn_prefill_simt_kernel(const Args<IO> p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem& s = *reinterpret_cast<Smem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = blockIdx.x % p.K, bh = blockIdx.x / p.K, b = bh / p.H, h = bh - b * p.H;
+  const int c0 = blockIdx.y * CW, cols = min(CW, p.dv - c0);
+  const int chunks = (p.L + T - 1) / T, first = (int)((int64_t)chunks * rank / p.K), n = (int)((int64_t)chunks * (rank + 1) / p.K) - first;
+  const IO* qb = p.q + b * p.sq.b + h * p.sq.h;
+  const IO* kb = p.k + b * p.sk.b + h * p.sk.h;
+  const IO* vb = p.v + b * p.sv.b + h * p.sv.h + c0;
+  for (int f = tid; f < kExpandedDim; f += NT) {
+    if (f <= kFeatureDim) { s.at[f] = (unsigned char)f; continue; }
+    const int i = (f - 1 - kFeatureDim) >> 4, j = (f - 1 - kFeatureDim) & 15, lo = min(i, j), hi = max(i, j);
+    const int at = 1 + kFeatureDim + lo * kFeatureDim - lo * (lo - 1) / 2 + (hi - lo);
+    s.at[f] = (unsigned char)at;
+  }
+  if (tid < FP) s.z[tid] = 0.f;
+
+  // a chunk's inputs wait in registers while the one before is worked on; tokens and columns outside are zero
+  float rq[4], rk[4], rv[16];
+  auto load = [&](int chunk, bool with_q) {
+    const int t0 = chunk * T;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = (tid >> 4) + 16 * i, c = tid & 15;
+      const bool ok = t0 + t < p.L;
+      rk[i] = ok ? to_float(kb[(int64_t)(t0 + t) * p.sk.l + c]) : 0.f;
+      if (with_q) rq[i] = ok ? to_float(qb[(int64_t)(t0 + t) * p.sq.l + c]) : 0.f;
     }
-    for (int i = tid; i < T * dv; i += nthreads) {
-      const int t = i / dv, c = i - t * dv;
-      s_v[i] = (t < nt) ? to_float(vb[(int64_t)(t0 + t) * sv.l + c]) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int t = (tid >> 6) + 4 * i, c = tid & 63;
+      rv[i] = t0 + t < p.L && c < cols ? to_float(vb[(int64_t)(t0 + t) * p.sv.l + c]) : 0.f;
     }
-    __syncthreads();
-    // ---- feature maps (tokens past the end get phi(k) = 0 so they never reach the state) ----
-    for (int i = tid; i < DP * T; i += nthreads) {
-      const int f = i / T, t = i - f * T;
-      float pq = 0.f, pk = 0.f;
-      if (f < kExpandedDim && t < nt) {
-        pq = taylor_feature(s_q + t * kFeatureDim, f);
-        pk = taylor_feature(s_k + t * kFeatureDim, f);
+  };
+  auto put = [&](bool with_q) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = (tid >> 4) + 16 * i, c = tid & 15;
+      s.k[t * kFeatureDim + c] = rk[i];
+      if (with_q) s.qt[c * T + t] = rq[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s.v[((tid >> 6) + 4 * i) * CW + (tid & 63)] = rv[i];
+  };
+  // phi(k) of `nt` tokens as [token][feature]; tokens past the end must not reach the state
+  auto build_k = [&](int nt) {
+    const int t = tid & 63, part = tid >> 6;
+    float x[kFeatureDim];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const float4 y = *reinterpret_cast<const float4*>(s.k + t * kFeatureDim + 4 * m);
+      x[4 * m] = y.x; x[4 * m + 1] = y.y; x[4 * m + 2] = y.z; x[4 * m + 3] = y.w;
+    }
+    float* dst = s.phi + t * KP;
+    constexpr std::make_integer_sequence<int, 10> ten;
+    if (part == 0) put_key<0>(dst, x, t < nt, ten);
+    else if (part == 1) put_key<40>(dst, x, t < nt, ten);
+    else if (part == 2) put_key<80>(dst, x, t < nt, ten);
+    else put_key<120>(dst, x, t < nt, ten);
+  };
+  // the state of this thread: features 20 warp .., columns 2 lane ..
+  float S[20][2];
+#pragma unroll
+  for (int i = 0; i < 20; ++i) S[i][0] = S[i][1] = 0.f;
+  auto update = [&]() {
+    const float* a = s.phi + 20 * warp;
+    const float* v = s.v + 2 * lane;
+    float U[20][2];   // a chunk's sum on its own: fewer roundings at the size of the whole sum
+#pragma unroll
+    for (int i = 0; i < 20; ++i) U[i][0] = U[i][1] = 0.f;
+#pragma unroll 4
+    for (int t = 0; t < T; ++t) {
+      const float2 y = *reinterpret_cast<const float2*>(v + t * CW);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(a + t * KP + 4 * i);
+        U[4 * i][0] = fmaf(x.x, y.x, U[4 * i][0]); U[4 * i][1] = fmaf(x.x, y.y, U[4 * i][1]);
+        U[4 * i + 1][0] = fmaf(x.y, y.x, U[4 * i + 1][0]); U[4 * i + 1][1] = fmaf(x.y, y.y, U[4 * i + 1][1]);
+        U[4 * i + 2][0] = fmaf(x.z, y.x, U[4 * i + 2][0]); U[4 * i + 2][1] = fmaf(x.z, y.y, U[4 * i + 2][1]);
+        U[4 * i + 3][0] = fmaf(x.w, y.x, U[4 * i + 3][0]); U[4 * i + 3][1] = fmaf(x.w, y.y, U[4 * i + 3][1]);
       }
-      s_phiq[i] = pq;
-      s_phik[i] = pk;
     }
-    for (int i = tid; i < T * T; i += nthreads) {
-      const int t = i / T, s = i - t * T;
-      float p = 0.f;
-      if (s <= t && t < nt) {
-        float dot = 0.f;
 #pragma unroll
-        for (int c = 0; c < kFeatureDim; ++c) dot = fmaf(s_q[t * kFeatureDim + c], s_k[s * kFeatureDim + c], dot);
-        const float x = dot * 0.25f;
-        p = 1.f + x + 0.5f * x * x;
+    for (int i = 0; i < 20; ++i) { S[i][0] += U[i][0]; S[i][1] += U[i][1]; }
+    if (tid < FP) {
+      float z[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int t = 0; t < T; t += 4)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) z[i] += s.phi[(t + i) * KP + tid];
+      s.z[tid] += (z[0] + z[1]) + (z[2] + z[3]);
+    }
+  };
+  auto put_state = [&]() {
+#pragma unroll
+    for (int i = 0; i < 20; ++i) *reinterpret_cast<float2*>(s.S + (20 * warp + i) * SP + 2 * lane) = make_float2(S[i][0], S[i][1]);
+  };
+
+  if (p.K > 1) {
+    // ---- what this run of chunks adds to the state (nobody asks the last one)
+    if (rank < p.K - 1) {
+      load(first, false);
+      for (int c = 0; c < n; ++c) {
+        put(false);
+        if (c + 1 < n) load(first + c + 1, false);
+        __syncthreads();
+        build_k(T);            // only the last CTA has a chunk that is not whole
+        __syncthreads();
+        update();
+        __syncthreads();
       }
-      s_p[i] = p;
+      put_state();
     }
+    cluster_sync();
+    // ---- the state before this run: the sum of the runs before it, in order
+#pragma unroll
+    for (int i = 0; i < 20; ++i) S[i][0] = S[i][1] = 0.f;
+    float z = 0.f;
+    for (int r = 0; r < rank; ++r) {
+      const uint32_t at = peer_addr(s.S + 20 * warp * SP + 2 * lane, r);
+#pragma unroll
+      for (int i = 0; i < 20; ++i) {
+        const float2 x = ld_peer2(at + i * SP * 4);
+        S[i][0] += x.x;
+        S[i][1] += x.y;
+      }
+      if (tid < FP) z += ld_peer(peer_addr(s.z + tid, r));
+    }
+    cluster_sync();
+    if (tid < FP) s.z[tid] = z;
+  }
+
+  // ---- the output
+  // this thread's tile of a chunk: tokens ta .., columns ca ..
+  const int ta = (warp & 1) * 32 + (lane >> 2) * 4, ca = (warp >> 1) * 16 + (lane & 3) * 4;
+  load(first, true);
+  for (int c = 0; c < n; ++c) {
+    const int t0 = (first + c) * T, nt = min(T, p.L - t0);
+    const bool some = first + c > 0;   // there is a state
+    put(true);
+    if (c + 1 < n) load(first + c + 1, true);
+    if (some) put_state();
     __syncthreads();
-    // ---- inter-block readout against the carried state, then state update ----
-    if (is_kv) {
-      float acc[T];
+    {  // phi(q), scores: a thread has one token, and a quarter of the features and of the keys
+      const int t = tid & 63, part = tid >> 6;
+      float x[kFeatureDim];
 #pragma unroll
-      for (int t = 0; t < T; ++t) acc[t] = 0.f;
-      float vr[T];
+      for (int i = 0; i < kFeatureDim; ++i) x[i] = s.qt[i * T + t];
+      if (some) {
+        float* dst = s.phi + t;
+        constexpr std::make_integer_sequence<int, 40> forty;
+        if (part == 0) put_query<0>(dst, x, forty);
+        else if (part == 1) put_query<40>(dst, x, forty);
+        else if (part == 2) put_query<80>(dst, x, forty);
+        else put_query<120>(dst, x, forty);
+      }
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int key = part * 16 + i;
+        const float4* kk = reinterpret_cast<const float4*>(s.k + key * kFeatureDim);
+        float d = 0.f;
 #pragma unroll
-      for (int t = 0; t < T; ++t) vr[t] = s_v[t * dv + j];
-      const float4* pq4 = reinterpret_cast<const float4*>(s_phiq + (size_t)g * FPG * T);
-      const float4* pk4 = reinterpret_cast<const float4*>(s_phik + (size_t)g * FPG * T);
-#pragma unroll
-      for (int fi = 0; fi < FPG; ++fi) {
-        float s = S[fi];
-        float upd = 0.f;
-#pragma unroll
-        for (int t4 = 0; t4 < T / 4; ++t4) {
-          const float4 a = pq4[fi * (T / 4) + t4];
-          acc[4 * t4 + 0] = fmaf(a.x, s, acc[4 * t4 + 0]);
-          acc[4 * t4 + 1] = fmaf(a.y, s, acc[4 * t4 + 1]);
-          acc[4 * t4 + 2] = fmaf(a.z, s, acc[4 * t4 + 2]);
-          acc[4 * t4 + 3] = fmaf(a.w, s, acc[4 * t4 + 3]);
-          const float4 c = pk4[fi * (T / 4) + t4];
-          upd = fmaf(c.x, vr[4 * t4 + 0], upd);
-          upd = fmaf(c.y, vr[4 * t4 + 1], upd);
-          upd = fmaf(c.z, vr[4 * t4 + 2], upd);
-          upd = fmaf(c.w, vr[4 * t4 + 3], upd);
+        for (int m = 0; m < 4; ++m) {
+          const float4 y = kk[m];
+          d = fmaf(x[4 * m], y.x, d); d = fmaf(x[4 * m + 1], y.y, d); d = fmaf(x[4 * m + 2], y.z, d); d = fmaf(x[4 * m + 3], y.w, d);
         }
-        S[fi] = s + upd;
+        d *= 0.25f;
+        s.p[key * T + t] = key <= t ? 1.f + d + 0.5f * d * d : 0.f;
+      }
+    }
+    __syncthreads();
+    float o[4][4], o1[4][4];   // two sums: half the roundings at full size
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[i][j] = o1[i][j] = 0.f;
+    if (some) {
+#pragma unroll 4
+      for (int f = 0; f < FP / 2; ++f) {
+        outer4(o, *reinterpret_cast<const float4*>(s.phi + f * T + ta), *reinterpret_cast<const float4*>(s.S + f * SP + ca));
+        outer4(o1, *reinterpret_cast<const float4*>(s.phi + (f + FP / 2) * T + ta), *reinterpret_cast<const float4*>(s.S + (f + FP / 2) * SP + ca));
       }
 #pragma unroll
-      for (int t = 0; t < T; ++t) s_part[(g * T + t) * dv + j] = acc[t];
-    } else if (is_ks) {
-      float acc[T];
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int t = 0; t < T; ++t) acc[t] = 0.f;
+        for (int j = 0; j < 4; ++j) { o[i][j] += o1[i][j]; o1[i][j] = 0.f; }
+    }
+    // a later value must not reach an earlier token, not even times zero: it may be infinite
+#pragma unroll 4
+    for (int t = 0; t < ta; ++t)
+      outer4(o1, *reinterpret_cast<const float4*>(s.p + t * T + ta), *reinterpret_cast<const float4*>(s.v + t * CW + ca));
 #pragma unroll
-      for (int n = 0; n < 9; ++n) {
-        const int f = lane + 32 * n;  // < 288; rows >= 276 are outside the tables
-        if (f < DP) {
-          float upd = 0.f;
+    for (int j = 0; j < 4; ++j) {
+      const float4 y = *reinterpret_cast<const float4*>(s.v + (ta + j) * CW + ca);
 #pragma unroll
-          for (int t = 0; t < T; ++t) {
-            acc[t] = fmaf(s_phiq[f * T + t], ks[n], acc[t]);
-            upd += s_phik[f * T + t];
+      for (int i = j; i < 4; ++i) {
+        const float x = s.p[(ta + j) * T + ta + i];
+        o1[i][0] = fmaf(x, y.x, o1[i][0]); o1[i][1] = fmaf(x, y.y, o1[i][1]); o1[i][2] = fmaf(x, y.z, o1[i][2]); o1[i][3] = fmaf(x, y.w, o1[i][3]);
+      }
+    }
+    {
+      const int t = tid & 63, part = tid >> 6;
+      float d0 = 0.f, d1 = 0.f;
+      if (some)
+#pragma unroll 10
+        for (int f = part * 40; f < part * 40 + 40; f += 2) {
+          d0 = fmaf(s.phi[f * T + t], s.z[f], d0);
+          d1 = fmaf(s.phi[(f + 1) * T + t], s.z[f + 1], d1);
+        }
+#pragma unroll
+      for (int i = 0; i < 16; i += 2) {
+        d0 += s.p[(part * 16 + i) * T + t];
+        d1 += s.p[(part * 16 + i + 1) * T + t];
+      }
+      s.den[part * T + t] = d0 + d1;
+    }
+    __syncthreads();
+    build_k(nt);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = ta + i;
+      if (t < nt) {
+        const float den = (s.den[t] + s.den[T + t]) + (s.den[2 * T + t] + s.den[3 * T + t]) + p.eps;
+        IO* y = p.y + b * p.sy.b + h * p.sy.h + (int64_t)(t0 + t) * p.sy.l + c0 + ca;
+        IO r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = from_float<IO>((o[i][j] + o1[i][j]) / den);
+        if (p.vec_out) {
+          if (ca < cols) {
+            if (sizeof(IO) == 4) *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(r);
+            else *reinterpret_cast<uint2*>(y) = *reinterpret_cast<const uint2*>(r);
           }
-          ks[n] += upd;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (ca + j < cols) y[j] = r[j];
         }
       }
-#pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const float r = warp_sum(acc[t]);
-        if (lane == 0) s_den[t] = r;
-      }
     }
     __syncthreads();
-    // ---- combine: inter-block partials + causal intra-block part, normalise, store ----
-    for (int i = tid; i < nt * dv; i += nthreads) {
-      const int t = i / dv, c = i - t * dv;
-      float num = 0.f;
-#pragma unroll
-      for (int gg = 0; gg < G; ++gg) num += s_part[(gg * T + t) * dv + c];
-      float den = s_den[t];
-      for (int s = 0; s <= t; ++s) {
-        const float p = s_p[t * T + s];
-        num = fmaf(p, s_v[s * dv + c], num);
-        den += p;
-      }
-      yb[(int64_t)(t0 + t) * sy.l + c] = from_float<IO>(num / (den + eps));
-    }
+    update();
     __syncthreads();
   }
-
-  if (kv_state != nullptr && is_kv) {
-    ST* dst = kv_state + ((size_t)bh * dv + j) * kExpandedDim;
-#pragma unroll
-    for (int fi = 0; fi < FPG; ++fi) {
-      const int f = g * FPG + fi;
-      if (f < kExpandedDim) dst[f] = from_float<ST>(S[fi]);
+  if (rank != p.K - 1) return;   // peers read this CTA's memory before the second cluster_sync only
+  // ---- the state after the last token, all 273 features
+  put_state();
+  __syncthreads();
+  if (p.kv_state != nullptr)
+    for (int i = tid; i < cols * kExpandedDim; i += NT) {
+      const int c = i / kExpandedDim, f = i - c * kExpandedDim;
+      const float x = s.S[s.at[f] * SP + c];
+      const int64_t to = ((int64_t)bh * p.dv + c0) * kExpandedDim + i;
+      if (p.state_bf16) static_cast<__nv_bfloat16*>(p.kv_state)[to] = __float2bfloat16_rn(x);
+      else static_cast<float*>(p.kv_state)[to] = x;
     }
-  }
-  if (k_state != nullptr && is_ks) {
-    ST* dst = k_state + (size_t)bh * kExpandedDim;
-#pragma unroll
-    for (int n = 0; n < 9; ++n) {
-      const int f = lane + 32 * n;
-      if (f < kExpandedDim) dst[f] = from_float<ST>(ks[n]);
+  if (p.k_state != nullptr && blockIdx.y == 0)
+    for (int f = tid; f < kExpandedDim; f += NT) {
+      const float x = s.z[s.at[f]];
+      const int64_t to = (int64_t)bh * kExpandedDim + f;
+      if (p.state_bf16) static_cast<__nv_bfloat16*>(p.k_state)[to] = __float2bfloat16_rn(x);
+      else static_cast<float*>(p.k_state)[to] = x;
     }
-  }
 }
 
-template <typename IO, typename ST, int T, int MAXT>
-int launch_cfg(const void* q, const void* k, const void* v, void* y, void* kv_state, void* k_state, int B, int H,
-               int L, int dv, Strides3 sq, Strides3 sk, Strides3 sv, Strides3 sy, float eps, cudaStream_t stream) {
-  const SmemLayout<T> lay(dv);
-  const size_t smem = (size_t)lay.total * sizeof(float);
-  auto kern = linattn_prefill_simt_kernel<IO, ST, T, MAXT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  kern<<<B * H, G * dv + 32, smem, stream>>>(static_cast<const IO*>(q), static_cast<const IO*>(k),
-                                            static_cast<const IO*>(v), static_cast<IO*>(y),
-                                            static_cast<ST*>(kv_state), static_cast<ST*>(k_state), H, L, dv, sq, sk,
-                                            sv, sy, eps);
-  return (int)cudaGetLastError();
-}
-
-template <typename IO, typename ST>
+template <typename IO>
 int launch_typed(const void* q, const void* k, const void* v, void* y, void* kv_state, void* k_state, int B, int H,
-                 int L, int dv, Strides3 sq, Strides3 sk, Strides3 sv, Strides3 sy, float eps,
+                 int L, int dv, Strides3 sq, Strides3 sk, Strides3 sv, Strides3 sy, int state_bf16, float eps,
                  cudaStream_t stream) {
-  if (dv <= 64) return launch_cfg<IO, ST, 16, 288>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
-  return launch_cfg<IO, ST, 8, 544>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
+  auto kern = linattn_prefill_simt_kernel<IO>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+  if (e != cudaSuccess) return (int)e;
+  const bool vec = reinterpret_cast<uintptr_t>(y) % (4 * sizeof(IO)) == 0 && dv % 4 == 0 && sy.b % 4 == 0 && sy.h % 4 == 0 && sy.l % 4 == 0;
+  const int slices = (dv + CW - 1) / CW, chunks = (L + T - 1) / T;
+  if (slices > 65535 || (int64_t)B * H > 0x7fffffff / kMaxCluster) return BASED_ERR_TOO_LARGE;
+  // The largest cluster of which all fit the device at once and whose CTAs have a chunk each: two CTAs with a chunk each take
+  // 1.45 of a chunk's time instead of 2.
+  int K = 1;
+  {
+    constexpr int kMaxDevices = 64;
+    static std::mutex mu;
+    static short room[kMaxDevices][kMaxCluster + 1] = {};   // clusters of a size on the device at once, + 1
+    int dev = 0;
+    e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= kMaxDevices) return BASED_ERR_TOO_LARGE;
+    std::lock_guard<std::mutex> lock(mu);
+    const int64_t units = (int64_t)B * H * slices;
+    for (int k = chunks < kMaxCluster ? chunks : kMaxCluster; k > 1; --k) {
+      if (units * k > 148) continue;
+      short& r = room[dev][k];
+      if (r == 0) r = (short)(1 + max_active_clusters(kern, k, NT, (int)sizeof(Smem)));
+      if (r - 1 < units) continue;
+      K = k;
+      break;
+    }
+  }
+  const Args<IO> args{static_cast<const IO*>(q), static_cast<const IO*>(k), static_cast<const IO*>(v), static_cast<IO*>(y), kv_state, k_state,
+                      H, L, dv, K, vec, state_bf16, sq, sk, sv, sy, eps};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = K;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(B * H * K, slices);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = sizeof(Smem);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = K > 1 ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, kern, args);
 }
 
 }  // namespace
@@ -231,15 +438,10 @@ int launch_typed(const void* q, const void* k, const void* v, void* y, void* kv_
 int launch_linattn_prefill_simt(const void* q, const void* k, const void* v, void* y, void* kv_state, void* k_state,
                                 int B, int H, int L, int dv, Strides3 sq, Strides3 sk, Strides3 sv, Strides3 sy,
                                 int io_dtype, int state_dtype, float eps, cudaStream_t stream) {
-  using bf16 = __nv_bfloat16;
-  if (io_dtype == BASED_F32 && state_dtype == BASED_F32)
-    return launch_typed<float, float>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
-  if (io_dtype == BASED_BF16 && state_dtype == BASED_F32)
-    return launch_typed<bf16, float>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
-  if (io_dtype == BASED_BF16 && state_dtype == BASED_BF16)
-    return launch_typed<bf16, bf16>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
-  if (io_dtype == BASED_F32 && state_dtype == BASED_BF16)
-    return launch_typed<float, bf16>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, eps, stream);
+  if (state_dtype != BASED_F32 && state_dtype != BASED_BF16) return BASED_ERR_DTYPE;
+  const int sb = state_dtype == BASED_BF16;
+  if (io_dtype == BASED_F32) return launch_typed<float>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, sb, eps, stream);
+  if (io_dtype == BASED_BF16) return launch_typed<__nv_bfloat16>(q, k, v, y, kv_state, k_state, B, H, L, dv, sq, sk, sv, sy, sb, eps, stream);
   return BASED_ERR_DTYPE;
 }
 

@@ -57,6 +57,25 @@ def test_linattn_prefill_vs_oracle(ops, impl, dtype, L, dv):
         assert e < tol, (name, e)
 
 
+@pytest.mark.parametrize("B,H,L,dv", [(1, 2, 64, 64), (1, 1, 65, 48), (1, 3, 127, 64), (2, 1, 511, 128), (1, 8, 513, 64), (2, 16, 1024, 64),
+                                       (4, 16, 200, 64), (1, 150, 130, 16), (1, 16, 2047, 112)])
+def test_linattn_prefill_fp32_shared_sequences(ops, B, H, L, dv):
+    """fp32 on CUDA cores at chunk borders (64 tokens) and at sizes where 1 to 8 CTAs share a sequence.  An infinite value
+    shows in no earlier token."""
+    q, k, v = _qkv(B, H, L, dv, torch.float32, seed=L + dv)
+    y_ref, kv_ref, ks_ref = O.linattn_chunked(q.double(), k.double(), v.double(), chunk=128)
+    y, kv, ks = ops.linattn_prefill(q.cuda(), k.cuda(), v.cuda())
+    # sums of at most 2047 products of unit size in fp32, against the oracle's 64 bits
+    assert rel_err(y.cpu(), y_ref) < 1e-5 and rel_err(kv.cpu(), kv_ref) < 1e-5 and rel_err(ks.cpu(), ks_ref) < 1e-5
+    for name, e in {**state_block_errs(kv.cpu(), kv_ref), **{"k_" + n: e for n, e in state_block_errs(ks.cpu(), ks_ref).items()}}.items():
+        assert e < 1e-4, (name, e)
+    at = L // 2 + 1
+    if at < L:
+        v[:, :, at, 3] = float("inf")
+        y2, _, _ = ops.linattn_prefill(q.cuda(), k.cuda(), v.cuda())
+        assert torch.equal(y2[:, :, :at], y[:, :, :at])
+
+
 @pytest.mark.parametrize("B,H,L,dv,nseg", [(1, 2, 1024, 64, 2), (1, 2, 1024 + 77, 64, 3), (2, 1, 4096, 64, 8),
                                             (1, 1, 2048, 32, 4), (1, 1, 2048 + 5, 112, 5), (1, 3, 300, 64, 64),
                                             (1, 1, 128, 64, 4)])
