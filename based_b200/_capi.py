@@ -7,7 +7,7 @@ import ctypes
 import os
 from ctypes import c_float, c_int, c_int32, c_int64, c_void_p, POINTER, c_char_p
 
-from .build import library_path
+from .build import library_path, native_path
 
 BASED_F32 = 0
 BASED_BF16 = 1
@@ -110,6 +110,27 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The extension module that calls the launching entry points with tensors (``csrc_host/native.cpp``)."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+        path = native_path()
+        if not os.path.exists(path):
+            raise BasedLibraryError(f"{path} is missing: build it with `python -m based_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_native", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_native", path, loader=loader))
+        loader.exec_module(module)
+        lib()                        # checks that the library is there and complete
+        module.bind(library_path())
+        _native = module
+    return _native
 
 
 def read_status(reset: bool = True) -> int:

@@ -1,8 +1,10 @@
-"""Compile the CUDA sources in ``based_b200/csrc`` into one C-ABI shared library (sm_100a)."""
+"""Compile the CUDA sources in ``based_b200/csrc`` into one C-ABI shared library (sm_100a), and the host path of its calls
+(``based_b200/csrc_host``) into an extension module."""
 import glob
 import os
 import shutil
 import subprocess
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -37,10 +39,38 @@ def _stale(lib: str) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def native_path() -> str:
+    """Path of the extension module; for one Python and one torch."""
+    import torch
+    tag = f"{sysconfig.get_config_var('SOABI')}-torch{torch.__version__.replace('+', '_')}"
+    return os.path.join(LIBDIR, f"_native.{tag}.so")
+
+
+def build_native(force: bool = False) -> str:
+    """Build (if stale) and return the path of the extension module.  Needs a C++ compiler and torch's headers; no GPU."""
+    import torch
+    path, src = native_path(), os.path.join(PKG, "csrc_host", "native.cpp")
+    deps = [src, os.path.join(ROOT, "include", "based_b200.h")]
+    if not force and os.path.exists(path) and all(os.path.getmtime(d) <= os.path.getmtime(path) for d in deps):
+        return path
+    os.makedirs(LIBDIR, exist_ok=True)
+    t = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + os.path.join(ROOT, "include"), f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include",
+           "-I" + sysconfig.get_paths()["include"], src, "-o", path + ".new", f"-L{t}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building the extension module failed:\n{r.stdout}")
+    os.replace(path + ".new", path)
+    return path
+
+
 def build_library(force: bool = False, verbose: bool = False, part: str = None) -> str:
     """Build (if stale) and return the path of the shared library.  Needs ``nvcc`` only; no GPU.  ``part`` names a subset
     of the kernels that is enough for the caller: only those are compiled, unless the whole library is there already."""
     global _chosen
+    build_native(force)
     if os.environ.get("BASED_B200_LIB"):
         return library_path()  # an explicitly chosen library is used as it is
     lib = os.path.join(LIBDIR, LIBNAME)

@@ -1,0 +1,193 @@
+// The host path of a kernel call, in C++: a module with one function per launching entry point of based_b200.h.
+//
+// Through ctypes a call costs about 20 us of host time (stride arrays, one conversion per argument, the current stream and
+// device looked up in Python): as much as 10 kernels of a short prompt take on the device.  Here an entry point is called with its
+// C arguments in order, without the last one, the stream: a tensor or None for a pointer, a tuple of integers or None for a
+// stride array, numbers for the rest.  The module makes the first tensor's device current and passes that device's current stream.
+// It returns the entry point's code.
+//
+// The entry points are looked up in the library the package has chosen (bind), not linked: a library of a part of the kernels
+// serves as well.
+#include <Python.h>
+#include <ATen/core/Tensor.h>
+#include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <dlfcn.h>
+
+#include <tuple>
+#include <type_traits>
+#include <utility>
+
+#include "based_b200.h"
+
+namespace {
+
+constexpr Py_ssize_t kMaxArray = 8;
+
+// One argument in its C type, with the storage a stride array needs.
+template <typename A>
+struct Arg {
+  A value{};
+  int64_t array[std::is_same_v<A, const int64_t*> ? kMaxArray : 1];
+
+  bool take(PyObject* o, int& device) {
+    if constexpr (std::is_floating_point_v<A>) {
+      const double x = PyFloat_AsDouble(o);
+      if (x == -1.0 && PyErr_Occurred()) return false;
+      value = static_cast<A>(x);
+    } else if constexpr (std::is_integral_v<A>) {
+      const long long x = PyLong_AsLongLong(o);
+      if (x == -1 && PyErr_Occurred()) return false;
+      if (static_cast<long long>(static_cast<A>(x)) != x) {
+        PyErr_SetString(PyExc_OverflowError, "an argument does not fit its C type");
+        return false;
+      }
+      value = static_cast<A>(x);
+    } else if constexpr (std::is_same_v<A, const int64_t*>) {
+      if (o == Py_None) return true;
+      if (!PyTuple_Check(o) || PyTuple_GET_SIZE(o) > kMaxArray) {
+        PyErr_SetString(PyExc_TypeError, "strides must be a tuple of integers");
+        return false;
+      }
+      for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(o); ++i) {
+        array[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(o, i));
+        if (array[i] == -1 && PyErr_Occurred()) return false;
+      }
+      value = array;
+    } else {
+      if (o == Py_None) return true;
+      if (THPVariable_Check(o)) {
+        const at::Tensor& t = THPVariable_Unpack(o);
+        if (!t.is_cuda()) {
+          PyErr_SetString(PyExc_RuntimeError, "based_b200 ops run on CUDA tensors only (there is no CPU path)");
+          return false;
+        }
+        if (device < 0) device = t.get_device();
+        value = static_cast<A>(t.data_ptr());
+        return true;
+      }
+      void* x = PyLong_AsVoidPtr(o);   // an address inside a tensor
+      if (x == nullptr && PyErr_Occurred()) return false;
+      value = static_cast<A>(x);
+    }
+    return true;
+  }
+};
+
+template <typename F>
+struct Caller;
+
+template <typename... A>
+struct Caller<int(A...)> {
+  static constexpr Py_ssize_t kGiven = sizeof...(A) - 1;   // all but the stream
+  using Tuple = std::tuple<Arg<A>...>;
+
+  template <size_t... I>
+  static PyObject* run(int (*fn)(A...), PyObject* const* given, std::index_sequence<I...>) {
+    int code;
+    try {   // a tensor without storage of its own (a tracer's, a vmap's) throws here
+      Tuple args;
+      int device = -1;
+      const bool ok = (std::get<I>(args).take(given[I], device) && ...);
+      if (!ok) return nullptr;
+      if (device < 0) {
+        PyErr_SetString(PyExc_TypeError, "a call needs at least one CUDA tensor");
+        return nullptr;
+      }
+      c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+      std::get<kGiven>(args).value = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
+      code = fn(std::get<I>(args).value..., std::get<kGiven>(args).value);
+    } catch (const std::exception& e) {
+      PyErr_SetString(PyExc_RuntimeError, e.what());
+      return nullptr;
+    }
+    return PyLong_FromLong(code);
+  }
+};
+
+template <typename Entry>
+PyObject* call(PyObject*, PyObject* const* given, Py_ssize_t n) {
+  using C = Caller<typename Entry::Type>;
+  if (Entry::fn == nullptr) {
+    PyErr_Format(PyExc_RuntimeError, "%s: no library is bound", Entry::name);
+    return nullptr;
+  }
+  if (n != C::kGiven) {
+    PyErr_Format(PyExc_TypeError, "%s takes %zd arguments (%zd given)", Entry::name, C::kGiven, n);
+    return nullptr;
+  }
+  return C::run(Entry::fn, given, std::make_index_sequence<C::kGiven>{});
+}
+
+#define ENTRIES(X)                                                                                                          \
+  X(linattn_prefill) X(linattn_prefill_split) X(linattn_decode) X(swa_prefill) X(rotary_apply) X(swa_decode)                \
+  X(gated_conv_prefill) X(gated_conv_step) X(add_rmsnorm) X(gated_act) X(decode_linear) X(rotary_qkv_cache) X(stream_norm)  \
+  X(rmsnorm) X(short_conv) X(latent_prepare) X(split_key_attention) X(latent_prefill) X(latent_decode) X(delta_prefill)     \
+  X(delta_step) X(rglru_gated) X(rglru) X(stream_embed) X(stream_post_norm) X(norm_gate) X(token_gate) X(token_side)        \
+  X(tied_prepare) X(tied_attention) X(lightning_split) X(lightning_step)
+
+#define DECLARE(NAME)                                  \
+  struct Entry_##NAME {                                \
+    using Type = std::remove_pointer_t<decltype(&based_##NAME)>; \
+    static inline Type* fn = nullptr;                  \
+    static constexpr const char* name = "based_" #NAME; \
+  };
+ENTRIES(DECLARE)
+
+// bind(path): take the entry points from this library (loaded before, or now).
+PyObject* bind(PyObject*, PyObject* path) {
+  const char* p = PyUnicode_AsUTF8(path);
+  if (p == nullptr) return nullptr;
+  void* lib = dlopen(p, RTLD_NOW | RTLD_LOCAL);
+  if (lib == nullptr) {
+    PyErr_Format(PyExc_OSError, "%s", dlerror());
+    return nullptr;
+  }
+#define LOOK(NAME)                                                                                       \
+  Entry_##NAME::fn = reinterpret_cast<Entry_##NAME::Type*>(dlsym(lib, Entry_##NAME::name));              \
+  if (Entry_##NAME::fn == nullptr) {                                                                     \
+    PyErr_Format(PyExc_AttributeError, "%s: undefined symbol: %s", p, Entry_##NAME::name);               \
+    return nullptr;                                                                                      \
+  }
+  ENTRIES(LOOK)
+  Py_RETURN_NONE;
+}
+
+// need_cuda(*tensors): CUDA tensors (or None) only, and nothing that wants a gradient under grad mode.
+PyObject* need_cuda(PyObject*, PyObject* const* given, Py_ssize_t n) {
+  bool wants = false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    if (given[i] == Py_None) continue;
+    if (!THPVariable_Check(given[i])) {
+      PyErr_SetString(PyExc_AttributeError, "a tensor is needed");
+      return nullptr;
+    }
+    const at::Tensor& t = THPVariable_Unpack(given[i]);
+    if (!t.is_cuda()) {
+      PyErr_SetString(PyExc_RuntimeError, "based_b200 ops run on CUDA tensors only (there is no CPU path)");
+      return nullptr;
+    }
+    wants |= t.requires_grad();
+  }
+  if (wants && c10::GradMode::is_enabled()) {
+    PyErr_SetString(PyExc_RuntimeError,
+                    "based_b200 kernels are inference-only (no backward): call them under torch.no_grad() or "
+                    "torch.inference_mode(), or detach the inputs");
+    return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+
+#define METHOD(NAME) {#NAME, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&call<Entry_##NAME>)), METH_FASTCALL, "based_" #NAME},
+PyMethodDef methods[] = {
+    ENTRIES(METHOD){"bind", bind, METH_O, "take the entry points from a library"},
+    {"need_cuda", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&need_cuda)), METH_FASTCALL, "check tensors"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Entry points of the kernel library for torch tensors.", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }

@@ -27,15 +27,7 @@ def _need_cuda(*ts):
     """Every op starts here: CUDA tensors only, and no autograd.  The kernels write into fresh buffers through
     raw pointers and register no backward, so under grad mode the result would silently be cut off from the
     graph (the projections before a mixer would get no gradient and nothing would say so)."""
-    for t in ts:
-        if t is not None and not t.is_cuda:
-            raise RuntimeError("based_b200 ops run on CUDA tensors only (there is no CPU path)")
-    if torch.is_grad_enabled():
-        for t in ts:
-            if t is not None and t.requires_grad:
-                raise RuntimeError(
-                    "based_b200 kernels are inference-only (no backward): call them under torch.no_grad() or "
-                    "torch.inference_mode(), or detach the inputs")
+    _capi.native().need_cuda(*ts)
 
 
 def check_status(reset: bool = True) -> int:
@@ -63,6 +55,8 @@ def _rows(t, width):
 
 def flat_rows(t):
     """``t [..., W]`` as ``[M, W]`` without a copy; raises when its rows are not one constant stride apart."""
+    if t.is_contiguous() and t.numel():
+        return t if t.dim() == 2 else t.view(-1, t.shape[-1])
     dims = [(n, st) for n, st in zip(t.shape[:-1], t.stride()[:-1]) if n != 1]
     for (_, outer), (n, inner) in zip(dims, dims[1:]):
         if outer != inner * n:
@@ -71,6 +65,17 @@ def flat_rows(t):
     for n, _ in dims:
         m *= n
     return t.as_strided((m, t.shape[-1]), (dims[-1][1] if dims else t.shape[-1], t.stride(-1)))
+
+
+def _flat(t, width):
+    """``t [..., width]`` for a kernel that takes rows: itself where it is contiguous, else as ``[M, width]`` (a copy where the
+    rows are not one stride apart)."""
+    return t if t.is_contiguous() else t.reshape(-1, width)
+
+
+def _row_stride(t, width):
+    """Elements between the rows of :func:`_flat`'s result."""
+    return width if t.is_contiguous() else t.stride(0)
 
 
 def _position(pos, like):
@@ -142,32 +147,30 @@ def linattn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, eps: f
     can_split = q.dtype == torch.bfloat16 and dv <= 112 and impl in ("auto", "tcgen05")
     if nseg is not None and nseg > 1 and not can_split:
         raise ValueError("nseg > 1 needs bf16 inputs, dv <= 112 and the tensor-core kernel")
-    with torch.cuda.device(q.device):
-        if nseg is None:
-            nseg = lib.based_linattn_prefill_segments(B, H, L) if can_split else 1
-        if nseg > 1:
-            need = lib.based_linattn_prefill_scratch_bytes(B, H, L, dv, nseg)
-            if scratch is None:
-                scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
-            elif scratch.device != q.device or not scratch.is_contiguous():
-                raise ValueError("scratch must be a contiguous tensor on the inputs' device")
-            code = lib.based_linattn_prefill_split(
-                q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                kv_state.data_ptr() if return_state else None, k_state.data_ptr() if return_state else None,
-                B, H, L, d, dv,
-                _capi.strides(*q.stride()[:3]), _capi.strides(*k.stride()[:3]),
-                _capi.strides(*v.stride()[:3]), _capi.strides(*out.stride()[:3]),
-                _dt(sdt), float(eps), int(nseg), scratch.data_ptr(), scratch.numel() * scratch.element_size(),
-                _stream())
-            _capi.check(code, "based_linattn_prefill_split")
-            return out, (kv_state if return_state else None), (k_state if return_state else None)
-        code = lib.based_linattn_prefill(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-            kv_state.data_ptr() if return_state else None, k_state.data_ptr() if return_state else None,
+    if nseg is None:
+        nseg = lib.based_linattn_prefill_segments(B, H, L) if can_split else 1
+    if nseg > 1:
+        need = lib.based_linattn_prefill_scratch_bytes(B, H, L, dv, nseg)
+        if scratch is None:
+            scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
+        elif scratch.device != q.device or not scratch.is_contiguous():
+            raise ValueError("scratch must be a contiguous tensor on the inputs' device")
+        code = _capi.native().linattn_prefill_split(
+            q, k, v, out,
+            kv_state if return_state else None, k_state if return_state else None,
             B, H, L, d, dv,
-            _capi.strides(*q.stride()[:3]), _capi.strides(*k.stride()[:3]),
-            _capi.strides(*v.stride()[:3]), _capi.strides(*out.stride()[:3]),
-            _dt(q.dtype), _dt(sdt), float(eps), _IMPLS[impl], _stream())
+            q.stride()[:3], k.stride()[:3],
+            v.stride()[:3], out.stride()[:3],
+            _dt(sdt), float(eps), int(nseg), scratch, scratch.numel() * scratch.element_size())
+        _capi.check(code, "based_linattn_prefill_split")
+        return out, (kv_state if return_state else None), (k_state if return_state else None)
+    code = _capi.native().linattn_prefill(
+        q, k, v, out,
+        kv_state if return_state else None, k_state if return_state else None,
+        B, H, L, d, dv,
+        q.stride()[:3], k.stride()[:3],
+        v.stride()[:3], out.stride()[:3],
+        _dt(q.dtype), _dt(sdt), float(eps), _IMPLS[impl])
     _capi.check(code, "based_linattn_prefill")
     return out, (kv_state if return_state else None), (k_state if return_state else None)
 
@@ -197,12 +200,11 @@ def linattn_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kv_state: 
     if out is None:
         out = torch.empty(B, 1, H * dv, dtype=q.dtype, device=q.device)
     y = out.view(B, H, dv)
-    with torch.cuda.device(q.device):
-        code = _capi.lib().based_linattn_decode(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), y.data_ptr(), kv_state.data_ptr(), k_state.data_ptr(),
-            B, H, d, dv, _capi.strides(*q.stride()[:2]), _capi.strides(*k.stride()[:2]),
-            _capi.strides(*v.stride()[:2]), _capi.strides(*y.stride()[:2]),
-            _dt(q.dtype), _dt(kv_state.dtype), float(eps), _stream())
+    code = _capi.native().linattn_decode(
+        q, k, v, y, kv_state, k_state,
+        B, H, d, dv, q.stride()[:2], k.stride()[:2],
+        v.stride()[:2], y.stride()[:2],
+        _dt(q.dtype), _dt(kv_state.dtype), float(eps))
     _capi.check(code, "based_linattn_decode")
     return out
 
@@ -223,12 +225,11 @@ def swa_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, window_left: 
     scale = hd ** -0.5 if softmax_scale is None else float(softmax_scale)
     if out.numel() == 0:
         return out
-    with torch.cuda.device(q.device):
-        code = _capi.lib().based_swa_prefill(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), B, L, H, hd,
-            _capi.strides(*q.stride()[:3]), _capi.strides(*k.stride()[:3]),
-            _capi.strides(*v.stride()[:3]), _capi.strides(*out.stride()[:3]),
-            int(window_left), scale, _dt(q.dtype), _IMPLS[impl], _stream())
+    code = _capi.native().swa_prefill(
+        q, k, v, out, B, L, H, hd,
+        q.stride()[:3], k.stride()[:3],
+        v.stride()[:3], out.stride()[:3],
+        int(window_left), scale, _dt(q.dtype), _IMPLS[impl])
     _capi.check(code, "based_swa_prefill")
     return out
 
@@ -256,9 +257,7 @@ def swa_decode(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, kv_cac
     if torch.is_tensor(cache_seqlens):
         if cache_seqlens.dtype != torch.int32 or not cache_seqlens.is_cuda or not cache_seqlens.is_contiguous():
             raise TypeError("cache_seqlens must be a contiguous int32 CUDA tensor")
-        import ctypes
-        lens_ptr = ctypes.cast(cache_seqlens.data_ptr(), ctypes.POINTER(ctypes.c_int32))
-        lens_scalar = 0
+        lens_ptr, lens_scalar = cache_seqlens, 0
     else:
         lens_ptr, lens_scalar = None, int(cache_seqlens)
     rdim = 0
@@ -269,14 +268,13 @@ def swa_decode(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, kv_cac
             raise ValueError("rotary tables must be contiguous")
         rdim = 2 * rotary_cos.shape[-1]
     scale = hd ** -0.5 if softmax_scale is None else float(softmax_scale)
-    with torch.cuda.device(q.device):
-        code = _capi.lib().based_swa_decode(
-            q3.data_ptr(), k3.data_ptr(), v3.data_ptr(), o3.data_ptr(), kv_cache.data_ptr(), lens_ptr, lens_scalar,
-            rotary_cos.data_ptr() if rotary_cos is not None else None,
-            rotary_sin.data_ptr() if rotary_sin is not None else None, rdim,
-            B, H, hd, kv_cache.shape[1], _capi.strides(*q3.stride()[:2]), _capi.strides(*k3.stride()[:2]),
-            _capi.strides(*v3.stride()[:2]), _capi.strides(*o3.stride()[:2]),
-            int(window_left), scale, _dt(q.dtype), _stream())
+    code = _capi.native().swa_decode(
+        q3, k3, v3, o3, kv_cache, lens_ptr, lens_scalar,
+        rotary_cos,
+        rotary_sin, rdim,
+        B, H, hd, kv_cache.shape[1], q3.stride()[:2], k3.stride()[:2],
+        v3.stride()[:2], o3.stride()[:2],
+        int(window_left), scale, _dt(q.dtype))
     _capi.check(code, "based_swa_decode")
     return out
 
@@ -294,19 +292,17 @@ def rotary_apply_(x: torch.Tensor, rotary_cos: torch.Tensor, rotary_sin: torch.T
     if x.numel() == 0:
         return x
     if torch.is_tensor(seqlen_offset):
-        import ctypes
         if seqlen_offset.dtype != torch.int32 or not seqlen_offset.is_cuda:
             raise TypeError("seqlen_offset tensor must be int32 on CUDA")
-        off_ptr, off_scalar = ctypes.cast(seqlen_offset.data_ptr(), ctypes.POINTER(ctypes.c_int32)), 0
+        off_ptr, off_scalar = seqlen_offset, 0
         max_pos = None
     else:
         off_ptr, off_scalar = None, int(seqlen_offset)
         if off_scalar + L > rotary_cos.shape[0]:
             raise ValueError("rotary tables are shorter than seqlen_offset + L")
-    with torch.cuda.device(x.device):
-        code = _capi.lib().based_rotary_apply(
-            x.data_ptr(), B, L, H, hd, _capi.strides(*x.stride()[:3]), rotary_cos.data_ptr(), rotary_sin.data_ptr(),
-            2 * rotary_cos.shape[-1], off_ptr, off_scalar, _dt(x.dtype), _stream())
+    code = _capi.native().rotary_apply(
+        x, B, L, H, hd, x.stride()[:3], rotary_cos, rotary_sin,
+        2 * rotary_cos.shape[-1], off_ptr, off_scalar, _dt(x.dtype))
     _capi.check(code, "based_rotary_apply")
     return x
 
@@ -340,13 +336,10 @@ def gated_conv_prefill(u: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
         if state is not None:
             state.zero_()
         return out
-    u1, u2 = u[..., :di], u[..., di:]
-    with torch.cuda.device(u.device):
-        code = _capi.lib().based_gated_conv_prefill(
-            u1.data_ptr(), u2.data_ptr(), out.data_ptr(), state.data_ptr() if state is not None else None,
-            weight.data_ptr(), bias.data_ptr() if bias is not None else None, B, L, di, k,
-            _capi.strides(*u1.stride()[:2]), _capi.strides(*u2.stride()[:2]), _capi.strides(*out.stride()[:2]),
-            _dt(u.dtype), _dt(weight.dtype), _stream())
+    su = u.stride()[:2]
+    code = _capi.native().gated_conv_prefill(
+        u, u.data_ptr() + di * u.element_size(), out, state, weight, bias, B, L, di, k, su, su, out.stride()[:2],
+        _dt(u.dtype), _dt(weight.dtype))
     _capi.check(code, "based_gated_conv_prefill")
     return out
 
@@ -371,12 +364,9 @@ def gated_conv_step(u: torch.Tensor, state: torch.Tensor, weight: torch.Tensor,
         out = torch.empty(B, di, dtype=u.dtype, device=u.device)
     if B == 0:
         return out
-    u1, u2 = u[:, :di], u[:, di:]
-    with torch.cuda.device(u.device):
-        code = _capi.lib().based_gated_conv_step(
-            u1.data_ptr(), u2.data_ptr(), out.data_ptr(), state.data_ptr(), weight.data_ptr(),
-            bias.data_ptr() if bias is not None else None, B, di, k, u1.stride(0), u2.stride(0), out.stride(0),
-            _dt(u.dtype), _dt(weight.dtype), _stream())
+    code = _capi.native().gated_conv_step(
+        u, u.data_ptr() + di * u.element_size(), out, state, weight, bias, B, di, k, u.stride(0), u.stride(0), out.stride(0),
+        _dt(u.dtype), _dt(weight.dtype))
     _capi.check(code, "based_gated_conv_step")
     return out
 
@@ -390,34 +380,31 @@ def add_rmsnorm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     norm (the unfused ``norm(residual.to(weight.dtype))`` of block.py:134-137).  x ``[..., D]``."""
     _need_cuda(x, weight, bias, residual)
     D = x.shape[-1]
-    x2 = x.reshape(-1, D)
+    x2 = _flat(x, D)
     _inner_contig(x2, "x")
-    M = x2.shape[0]
-    res2 = None
+    M = x.numel() // D
+    res2, sr = None, 0
     if residual is not None:
         if residual.shape != x.shape:
             raise ValueError("residual must have x's shape")
-        res2 = residual.reshape(-1, D)
+        res2 = _flat(residual, D)
         _inner_contig(res2, "residual")
     res_dtype = torch.float32 if (residual_in_fp32 or (residual is not None and residual.dtype == torch.float32)) else x.dtype
-    if res2 is not None and res2.dtype != res_dtype:
-        res2 = res2.to(res_dtype)
+    if res2 is not None:
+        if res2.dtype != res_dtype:
+            res2 = res2.to(res_dtype)
+        sr = _row_stride(res2, D)
     weight = weight.contiguous()
     if bias is not None:
         bias = bias.to(weight.dtype).contiguous()
-    out = torch.empty(M, D, dtype=x.dtype, device=x.device)
-    res_out = torch.empty(M, D, dtype=res_dtype, device=x.device) if prenorm else None
+    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    res_out = torch.empty(x.shape, dtype=res_dtype, device=x.device) if prenorm else None
     if M > 0:
-        with torch.cuda.device(x.device):
-            code = _capi.lib().based_add_rmsnorm(
-                x2.data_ptr(), res2.data_ptr() if res2 is not None else None, weight.data_ptr(),
-                bias.data_ptr() if bias is not None else None, out.data_ptr(),
-                res_out.data_ptr() if res_out is not None else None, M, D, x2.stride(0),
-                res2.stride(0) if res2 is not None else 0, out.stride(0), res_out.stride(0) if res_out is not None else 0,
-                float(eps), _dt(x.dtype), _dt(res_dtype), _dt(weight.dtype), int(round_input), _stream())
+        code = _capi.native().add_rmsnorm(
+            x2, res2, weight, bias, out, res_out, M, D, _row_stride(x2, D), sr, D, D if prenorm else 0,
+            eps, _dt(x.dtype), _dt(res_dtype), _dt(weight.dtype), round_input)
         _capi.check(code, "based_add_rmsnorm")
-    out = out.reshape(x.shape)
-    return (out, res_out.reshape(x.shape)) if prenorm else out
+    return (out, res_out) if prenorm else out
 
 
 _ACTS = {"silu": 0, "swiglu": 0, "sigmoid": 1, "glu": 1}
@@ -429,17 +416,20 @@ def gated_act(y: torch.Tensor, activation: str = "silu", out: Optional[torch.Ten
     _need_cuda(y, out)
     F2 = y.shape[-1]
     F = F2 // 2
-    y2 = y.reshape(-1, F2)
+    y2 = _flat(y, F2)
     _inner_contig(y2, "y")
-    M = y2.shape[0]
-    out = torch.empty(M, F, dtype=y.dtype, device=y.device) if out is None else _rows(out, F)
-    if M > 0:
-        a, g = y2[:, :F], y2[:, F:]
-        with torch.cuda.device(y.device):
-            code = _capi.lib().based_gated_act(a.data_ptr(), g.data_ptr(), out.data_ptr(), M, F, a.stride(0),
-                                               g.stride(0), out.stride(0), _ACTS[activation], _dt(y.dtype), _stream())
+    M = y.numel() // F2 if F2 else 0
+    if out is None:
+        out = o2 = torch.empty(*y.shape[:-1], F, dtype=y.dtype, device=y.device)
+    else:
+        o2 = _rows(out, F)
+        out = o2.reshape(*y.shape[:-1], F)
+    if M > 0 and F > 0:
+        sy = _row_stride(y2, F2)
+        code = _capi.native().gated_act(y2, y2.data_ptr() + F * y2.element_size(), o2, M, F, sy, sy, _row_stride(o2, F),
+                                        _ACTS[activation], _dt(y.dtype))
         _capi.check(code, "based_gated_act")
-    return out.reshape(*y.shape[:-1], F)
+    return out
 
 
 DECODE_LINEAR_MAX_ROWS = 64  # beyond this the library GEMM is the better tool
@@ -480,12 +470,11 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
         if conv_state.shape != (M, n_out, ck) or conv_state.dtype != torch.bfloat16 or not conv_state.is_contiguous():
             raise ValueError("conv_state must be a contiguous bfloat16 [M, N/2, k] tensor")
     if M > 0:
-        with torch.cuda.device(x.device):
-            code = _capi.lib().based_decode_linear(
-                x2.data_ptr(), weight.data_ptr(), bias.data_ptr() if bias is not None else None, out.data_ptr(),
-                M, N, K, x2.stride(0), out.stride(0), epi, _ACTS[activation],
-                conv_state.data_ptr() if epi == 2 else None, conv_weight.data_ptr() if epi == 2 else None,
-                conv_bias.data_ptr() if (epi == 2 and conv_bias is not None) else None, ck, cw_dt, _stream())
+        code = _capi.native().decode_linear(
+            x2, weight, bias, out,
+            M, N, K, x2.stride(0), out.stride(0), epi, _ACTS[activation],
+            conv_state if epi == 2 else None, conv_weight if epi == 2 else None,
+            conv_bias if (epi == 2 and conv_bias is not None) else None, ck, cw_dt)
         _capi.check(code, "based_decode_linear")
     return out.reshape(*x.shape[:-1], n_out)
 
@@ -524,10 +513,9 @@ def rotary_qkv_cache_(qkv: torch.Tensor, rotary_cos: torch.Tensor, rotary_sin: t
         raise ValueError("kv_cache must be [>= B, >= L, 2, H, hd] with the last three dims contiguous")
     if qkv.numel() == 0:
         return qkv
-    with torch.cuda.device(qkv.device):
-        code = _capi.lib().based_rotary_qkv_cache(
-            qkv.data_ptr(), B, L, H, hd, _capi.strides(*qkv.stride()[:4]), rotary_cos.data_ptr(), rotary_sin.data_ptr(),
-            kv_cache.data_ptr(), _capi.strides(*kv_cache.stride()[:2]), _stream())
+    code = _capi.native().rotary_qkv_cache(
+        qkv, B, L, H, hd, qkv.stride()[:4], rotary_cos, rotary_sin,
+        kv_cache, kv_cache.stride()[:2])
     _capi.check(code, "based_rotary_qkv_cache")
     return qkv
 
@@ -642,10 +630,9 @@ def stream_norm(residual: torch.Tensor, w1: torch.Tensor, w2: Optional[torch.Ten
         if t is not None and (t.dtype != w1.dtype or (t is not branch and not t.is_contiguous())):
             raise TypeError("weights, table and branch must share a dtype and be contiguous")
     if M > 0:
-        with torch.cuda.device(residual.device):
-            code = _capi.lib().based_stream_norm(
-                _ptr(tokens), _ptr(table), _ptr(table_norm), V, _ptr(branch), sb, float(mult), residual.data_ptr(),
-                w1.data_ptr(), _ptr(w2), out1.data_ptr(), _ptr(out2), M, D, float(eps), _dt(w1.dtype), _stream())
+        code = _capi.native().stream_norm(
+            tokens, table, table_norm, V, branch, sb, float(mult), residual,
+            w1, w2, out1, out2, M, D, float(eps), _dt(w1.dtype))
         _capi.check(code, "based_stream_norm")
     return out1, out2
 
@@ -660,9 +647,8 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     if weight.dtype != x.dtype:
         raise TypeError("weight must be in x's dtype")
     if out.numel() > 0:
-        with torch.cuda.device(x.device):
-            code = _capi.lib().based_rmsnorm(x2.data_ptr(), weight.data_ptr(), out.data_ptr(), x2.shape[0], D, x2.stride(0), D,
-                                             float(eps), _dt(x.dtype), _stream())
+        code = _capi.native().rmsnorm(x2, weight, out, x2.shape[0], D, x2.stride(0), D,
+                                         float(eps), _dt(x.dtype))
         _capi.check(code, "based_rmsnorm")
     return out
 
@@ -683,10 +669,9 @@ def short_conv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     if y.numel() == 0:
         return y
     off, scalar = _position(pos, x)
-    with torch.cuda.device(x.device):
-        code = _capi.lib().based_short_conv(x.data_ptr(), y.data_ptr(), _ptr(ring), weight.data_ptr(), _ptr(bias), B, L, C, taps,
-                                            _capi.strides(*x.stride()[:2]), _capi.strides(*y.stride()[:2]), off, scalar,
-                                            int(silu), _dt(x.dtype), _stream())
+    code = _capi.native().short_conv(x, y, ring, weight, bias, B, L, C, taps,
+                                        x.stride()[:2], y.stride()[:2], off, scalar,
+                                        int(silu), _dt(x.dtype))
     _capi.check(code, "based_short_conv")
     return y
 
@@ -707,14 +692,13 @@ def latent_prepare_(q: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, dim: 
         _inner_contig(z, "z")
         if z.dtype != q.dtype or cache.dtype != q.dtype or cache.shape[0] < B or cache.shape[2] != kv_rank + rd or cache.stride(2) != 1:
             raise ValueError("cache must be [>= B, max_len, kv_rank + rot] in the inputs' dtype")
-        zs, cs, max_len = _capi.strides(*z.stride()[:2]), _capi.strides(*cache.stride()[:2]), cache.shape[1]
+        zs, cs, max_len = z.stride()[:2], cache.stride()[:2], cache.shape[1]
     if q.numel() == 0:
         return q
     off, scalar = _position(pos, q)
-    with torch.cuda.device(q.device):
-        code = _capi.lib().based_latent_prepare(_ptr(z), _ptr(norm_weight), _ptr(cache), q.data_ptr(), cos.data_ptr(), sin.data_ptr(),
-                                                cos.shape[0], B, L, H, int(kv_rank), rd, int(dim), max_len, zs, cs,
-                                                _capi.strides(*q.stride()[:2]), off, scalar, float(eps), _dt(q.dtype), _stream())
+    code = _capi.native().latent_prepare(z, norm_weight, cache, q, cos, sin,
+                                            cos.shape[0], B, L, H, int(kv_rank), rd, int(dim), max_len, zs, cs,
+                                            q.stride()[:2], off, scalar, float(eps), _dt(q.dtype))
     _capi.check(code, "based_latent_prepare")
     return q
 
@@ -732,17 +716,16 @@ def split_key_attention(q1, q2, k1, k2, v, scale: float, *, gate: Optional[torch
     off, scalar = _position(pos, q1)
     if off is None and k1.shape[1] < scalar + L:
         raise ValueError("fewer keys than the last query sees")
-    gs = _capi.strides(*gate.stride()[:2]) if gate is not None else None
+    gs = gate.stride()[:2] if gate is not None else None
     if gate is not None:
         _inner_contig(gate, "gate")
     if out.numel() == 0:
         return out
-    with torch.cuda.device(q1.device):
-        code = _capi.lib().based_split_key_attention(
-            q1.data_ptr(), q2.data_ptr(), k1.data_ptr(), k2.data_ptr(), v.data_ptr(), _ptr(gate), out.data_ptr(), B, L, H, d1,
-            q2.shape[-1], v.shape[-1], _capi.strides(*q1.stride()[:3]), _capi.strides(*q2.stride()[:3]),
-            _capi.strides(*k1.stride()[:3]), _capi.strides(*k2.stride()[:3]), _capi.strides(*v.stride()[:3]),
-            _capi.strides(*out.stride()[:3]), gs, off, scalar, float(scale), _dt(q1.dtype), _stream())
+    code = _capi.native().split_key_attention(
+        q1, q2, k1, k2, v, gate, out, B, L, H, d1,
+        q2.shape[-1], v.shape[-1], q1.stride()[:3], q2.stride()[:3],
+        k1.stride()[:3], k2.stride()[:3], v.stride()[:3],
+        out.stride()[:3], gs, off, scalar, float(scale), _dt(q1.dtype))
     _capi.check(code, "based_split_key_attention")
     return out
 
@@ -761,13 +744,12 @@ def latent_prefill(q1, q2, k1, k2, v, scale: float, *, gate: Optional[torch.Tens
         _inner_contig(gate, "gate")
     if out.numel() == 0:
         return out
-    with torch.cuda.device(q1.device):
-        code = _capi.lib().based_latent_prefill(
-            q1.data_ptr(), q2.data_ptr(), k1.data_ptr(), k2.data_ptr(), v.data_ptr(), _ptr(gate), out.data_ptr(), B, L, k1.shape[1],
-            H, d1, q2.shape[-1], v.shape[-1], _capi.strides(*q1.stride()[:3]), _capi.strides(*q2.stride()[:3]),
-            _capi.strides(*k1.stride()[:3]), _capi.strides(*k2.stride()[:2]), _capi.strides(*v.stride()[:3]),
-            _capi.strides(*out.stride()[:3]), _capi.strides(*gate.stride()[:2]) if gate is not None else None, int(pos),
-            float(scale), _dt(q1.dtype), _IMPLS[impl], _stream())
+    code = _capi.native().latent_prefill(
+        q1, q2, k1, k2, v, gate, out, B, L, k1.shape[1],
+        H, d1, q2.shape[-1], v.shape[-1], q1.stride()[:3], q2.stride()[:3],
+        k1.stride()[:3], k2.stride()[:2], v.stride()[:3],
+        out.stride()[:3], gate.stride()[:2] if gate is not None else None, int(pos),
+        float(scale), _dt(q1.dtype), _IMPLS[impl])
     _capi.check(code, "based_latent_prefill")
     return out
 
@@ -790,15 +772,14 @@ def latent_decode(qa, qr, cache, scale: float, *, gate: Optional[torch.Tensor] =
     if out.numel() == 0:
         return out
     off, scalar = _position(pos, qa)
-    with torch.cuda.device(qa.device):
-        lib = _capi.lib()
-        need = lib.based_latent_decode_scratch_bytes(B, L, H, r, cache.shape[1])
-        scratch = torch.empty(need, dtype=torch.uint8, device=qa.device) if need else None
-        code = lib.based_latent_decode(
-            qa.data_ptr(), qr.data_ptr(), cache.data_ptr(), _ptr(gate), out.data_ptr(), _ptr(scratch), need, B, L, H, r, rd,
-            cache.shape[1], _capi.strides(*qa.stride()[:3]), _capi.strides(*qr.stride()[:3]), _capi.strides(*cache.stride()[:2]),
-            _capi.strides(*out.stride()[:3]), _capi.strides(*gate.stride()[:2]) if gate is not None else None, off, scalar,
-            float(scale), _dt(qa.dtype), _stream())
+    lib = _capi.lib()
+    need = lib.based_latent_decode_scratch_bytes(B, L, H, r, cache.shape[1])
+    scratch = torch.empty(need, dtype=torch.uint8, device=qa.device) if need else None
+    code = _capi.native().latent_decode(
+        qa, qr, cache, gate, out, scratch, need, B, L, H, r, rd,
+        cache.shape[1], qa.stride()[:3], qr.stride()[:3], cache.stride()[:2],
+        out.stride()[:3], gate.stride()[:2] if gate is not None else None, off, scalar,
+        float(scale), _dt(qa.dtype))
     _capi.check(code, "based_latent_decode")
     return out
 
@@ -828,15 +809,14 @@ def delta_prefill(q, k, v, z, a, b, A_log, dt_bias, norm_weight, state, *, pos=0
     off, scalar = _position(pos, q)
     if out.numel() == 0:
         return out
-    with torch.cuda.device(q.device):
-        need = _capi.lib().based_delta_prefill_scratch_bytes(B, L, H, d, dv) if q.dtype == torch.bfloat16 and impl != "simt" else 0
-        scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-        code = _capi.lib().based_delta_prefill(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), z.data_ptr(), a.data_ptr(), b.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
-            norm_weight.data_ptr(), state.data_ptr(), out.data_ptr(), B, L, H, Hk, d, dv, _capi.strides(*q.stride()[:2]),
-            _capi.strides(*k.stride()[:2]), _capi.strides(*v.stride()[:2]), _capi.strides(*z.stride()[:2]),
-            _capi.strides(*a.stride()[:2]), _capi.strides(*out.stride()[:2]), off, scalar, float(eps), _dt(q.dtype), _IMPLS[impl],
-            _ptr(scratch), need, _stream())
+    need = _capi.lib().based_delta_prefill_scratch_bytes(B, L, H, d, dv) if q.dtype == torch.bfloat16 and impl != "simt" else 0
+    scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
+    code = _capi.native().delta_prefill(
+        q, k, v, z, a, b, A_log, dt_bias,
+        norm_weight, state, out, B, L, H, Hk, d, dv, q.stride()[:2],
+        k.stride()[:2], v.stride()[:2], z.stride()[:2],
+        a.stride()[:2], out.stride()[:2], off, scalar, float(eps), _dt(q.dtype), _IMPLS[impl],
+        scratch, need)
     _capi.check(code, "based_delta_prefill")
     return out
 
@@ -856,11 +836,10 @@ def delta_step(x, conv_weight, ring, a, b, A_log, dt_bias, norm_weight, state, k
     off, scalar = _position(pos, x)
     if B == 0:
         return True
-    with torch.cuda.device(x.device):
-        code = _capi.lib().based_delta_step(
-            x.data_ptr(), conv_weight.data_ptr(), ring.data_ptr(), a.data_ptr(), b.data_ptr(), A_log.data_ptr(), dt_bias.data_ptr(),
-            norm_weight.data_ptr(), state.data_ptr(), out.data_ptr(), B, H, int(kv_heads), d, dv, taps, x.stride(0), a.stride(0),
-            out.stride(0), off, scalar, float(eps), _dt(x.dtype), _stream())
+    code = _capi.native().delta_step(
+        x, conv_weight, ring, a, b, A_log, dt_bias,
+        norm_weight, state, out, B, H, int(kv_heads), d, dv, taps, x.stride(0), a.stride(0),
+        out.stride(0), off, scalar, float(eps), _dt(x.dtype))
     if code == _capi.ERR_IMPL:
         return False
     _capi.check(code, "based_delta_step")
@@ -893,11 +872,10 @@ def rglru(u, y, gates, r_bias, i_bias, lam, state, *, pos=0, out: torch.Tensor) 
     off, scalar = _position(pos, u)
     if out.numel() == 0:
         return out
-    with torch.cuda.device(u.device):
-        code = _capi.lib().based_rglru(
-            u.data_ptr(), y.data_ptr(), gates.data_ptr(), r_bias.data_ptr(), i_bias.data_ptr(), lam.data_ptr(), state.data_ptr(),
-            out.data_ptr(), B, L, W, n2 // 2, _capi.strides(*u.stride()[:2]), _capi.strides(*y.stride()[:2]),
-            _capi.strides(*out.stride()[:2]), _capi.strides(gates.stride(0), gates.stride(1)), off, scalar, _dt(u.dtype), _stream())
+    code = _capi.native().rglru(
+        u, y, gates, r_bias, i_bias, lam, state,
+        out, B, L, W, n2 // 2, u.stride()[:2], y.stride()[:2],
+        out.stride()[:2], (gates.stride(0), gates.stride(1)), off, scalar, _dt(u.dtype))
     _capi.check(code, "based_rglru")
     return out
 
@@ -919,11 +897,10 @@ def rglru_gated(u, y, gate_weight, r_bias, i_bias, lam, state, *, pos=0, out: to
         for t, name in ((u, "u"), (y, "y"), (out, "out")):
             _inner_contig(t, name)
         off, scalar = _position(pos, u)
-        with torch.cuda.device(u.device):
-            code = _capi.lib().based_rglru_gated(
-                u.data_ptr(), y.data_ptr(), gate_weight.data_ptr(), r_bias.data_ptr(), i_bias.data_ptr(), lam.data_ptr(),
-                state.data_ptr(), out.data_ptr(), B, L, W, n, _capi.strides(*u.stride()[:2]), _capi.strides(*y.stride()[:2]),
-                _capi.strides(*out.stride()[:2]), off, scalar, _dt(u.dtype), _stream())
+        code = _capi.native().rglru_gated(
+            u, y, gate_weight, r_bias, i_bias, lam,
+            state, out, B, L, W, n, u.stride()[:2], y.stride()[:2],
+            out.stride()[:2], off, scalar, _dt(u.dtype))
         if code != _capi.ERR_IMPL:
             _capi.check(code, "based_rglru_gated")
             return out
@@ -933,7 +910,7 @@ def rglru_gated(u, y, gate_weight, r_bias, i_bias, lam, state, *, pos=0, out: to
 # --------------------------------------------------------------------------- post-norm stacks
 
 def _strides_bl(t):
-    return _capi.strides(*t.stride()[:2])
+    return t.stride()[:2]
 
 
 def _same_dtype(like, **tensors):
@@ -958,10 +935,9 @@ def stream_embed(residual: torch.Tensor, tokens: torch.Tensor, table: torch.Tens
     off, scalar = _position(pos, residual)
     if residual.numel() > 0:
         tokens = tokens.contiguous()
-        with torch.cuda.device(residual.device):
-            code = _capi.lib().based_stream_embed(
-                tokens.data_ptr(), table.data_ptr(), table.shape[0], float(scale), pos_table.data_ptr(), pos_table.shape[0],
-                residual.data_ptr(), None if out is residual else out.data_ptr(), B, L, D, off, scalar, _dt(table.dtype), _stream())
+        code = _capi.native().stream_embed(
+            tokens, table, table.shape[0], float(scale), pos_table, pos_table.shape[0],
+            residual, None if out is residual else out, B, L, D, off, scalar, _dt(table.dtype))
         _capi.check(code, "based_stream_embed")
     return out
 
@@ -982,9 +958,8 @@ def stream_post_norm(residual: torch.Tensor, branch: torch.Tensor, weight: torch
     alias = out_weight is None and branch.dtype == torch.float32
     out = residual if alias else torch.empty(residual.shape, dtype=branch.dtype, device=residual.device)
     if M > 0:
-        with torch.cuda.device(residual.device):
-            code = _capi.lib().based_stream_post_norm(b2.data_ptr(), b2.stride(0), weight.data_ptr(), residual.data_ptr(), _ptr(out_weight),
-                                                      None if alias else out.data_ptr(), M, D, float(eps), _dt(branch.dtype), _stream())
+        code = _capi.native().stream_post_norm(b2, b2.stride(0), weight, residual, out_weight,
+                                                  None if alias else out, M, D, float(eps), _dt(branch.dtype))
         _capi.check(code, "based_stream_post_norm")
     return out
 
@@ -999,9 +974,8 @@ def norm_gate(x: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, eps: fl
     if g2.shape != x2.shape or o2.shape != x2.shape or weight.shape != (D,):
         raise ValueError("gate and out must have x's shape and the weight its width")
     if x2.numel() > 0:
-        with torch.cuda.device(x.device):
-            code = _capi.lib().based_norm_gate(x2.data_ptr(), x2.stride(0), weight.data_ptr(), g2.data_ptr(), g2.stride(0), o2.data_ptr(),
-                                               o2.stride(0), x2.shape[0], D, float(eps), _dt(x.dtype), _stream())
+        code = _capi.native().norm_gate(x2, x2.stride(0), weight, g2, g2.stride(0), o2,
+                                           o2.stride(0), x2.shape[0], D, float(eps), _dt(x.dtype))
         _capi.check(code, "based_norm_gate")
     return out
 
@@ -1017,9 +991,8 @@ def token_gate(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, colum
     out = torch.empty(z.shape, dtype=z.dtype, device=z.device)
     if out.numel() > 0:
         tokens = tokens.contiguous()
-        with torch.cuda.device(z.device):
-            code = _capi.lib().based_token_gate(z2.data_ptr(), z2.stride(0), tokens.data_ptr(), table.data_ptr(), table.shape[0],
-                                                table.stride(0), int(column), out.data_ptr(), z2.shape[0], n, _dt(z.dtype), _stream())
+        code = _capi.native().token_gate(z2, z2.stride(0), tokens, table, table.shape[0],
+                                            table.stride(0), int(column), out, z2.shape[0], n, _dt(z.dtype))
         _capi.check(code, "based_token_gate")
     return out
 
@@ -1049,11 +1022,10 @@ def token_side_step(residual: torch.Tensor, x: torch.Tensor, tokens: torch.Tenso
         raise ValueError("norm weights must have the stream's width")
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
     tokens = tokens.contiguous()
-    with torch.cuda.device(x.device):
-        code = _capi.lib().based_token_side(
-            x2.data_ptr(), x2.stride(0), tokens.data_ptr(), gate_weight.data_ptr(), proj_weight.data_ptr(), table.data_ptr(), table.shape[0],
-            table.stride(0), int(column), norm_weight.data_ptr(), residual.data_ptr(), _ptr(out_weight), out.data_ptr(), M, W, n, float(eps),
-            _dt(x.dtype), _stream())
+    code = _capi.native().token_side(
+        x2, x2.stride(0), tokens, gate_weight, proj_weight, table, table.shape[0],
+        table.stride(0), int(column), norm_weight, residual, out_weight, out, M, W, n, float(eps),
+        _dt(x.dtype))
     if code == _capi.ERR_IMPL:
         return None
     _capi.check(code, "based_token_side")
@@ -1091,11 +1063,10 @@ def tied_prepare_(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_we
         raise ValueError("k must be [B, L, G d]")
     off, scalar = _position(pos, q)
     if q.numel() > 0:
-        with torch.cuda.device(q.device):
-            code = _capi.lib().based_tied_prepare(
-                q.data_ptr(), k.data_ptr(), q_weight.data_ptr(), k_weight.data_ptr(), cache.data_ptr(), factor.data_ptr(), B, L, H, G, d,
-                cache.shape[1], _strides_bl(q), _strides_bl(k), _strides_bl(cache), _strides_bl(factor), off, scalar, float(eps),
-                float(temp_coef), float(temp_every), _dt(q.dtype), _stream())
+        code = _capi.native().tied_prepare(
+            q, k, q_weight, k_weight, cache, factor, B, L, H, G, d,
+            cache.shape[1], _strides_bl(q), _strides_bl(k), _strides_bl(cache), _strides_bl(factor), off, scalar, float(eps),
+            float(temp_coef), float(temp_every), _dt(q.dtype))
         _capi.check(code, "based_tied_prepare")
     return q
 
@@ -1118,15 +1089,14 @@ def tied_attention(q: torch.Tensor, cache: torch.Tensor, factor: torch.Tensor, c
     off, scalar = _position(pos, q)
     if out.numel() == 0:
         return out
-    with torch.cuda.device(q.device):
-        need = 0
-        if q.dtype == torch.bfloat16 and (impl == "decode" or impl == "auto" and (off is not None or L * (heads // G) <= _capi.TIED_DECODE_ROWS)):
-            need = _capi.lib().based_tied_attention_scratch_bytes(B, L, heads, G, d, cache.shape[1])
-        scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-        code = _capi.lib().based_tied_attention(
-            q.data_ptr(), cache.data_ptr(), factor.data_ptr(), _ptr(gate), out.data_ptr(), B, L, heads, G, d, cache.shape[1],
-            _strides_bl(q), _strides_bl(cache), _strides_bl(factor), _strides_bl(gate) if gate is not None else None, _strides_bl(out),
-            off, scalar, float(scale), float(sink), _dt(q.dtype), _IMPLS[impl], _ptr(scratch), need, count.data_ptr(), count.numel(), _stream())
+    need = 0
+    if q.dtype == torch.bfloat16 and (impl == "decode" or impl == "auto" and (off is not None or L * (heads // G) <= _capi.TIED_DECODE_ROWS)):
+        need = _capi.lib().based_tied_attention_scratch_bytes(B, L, heads, G, d, cache.shape[1])
+    scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
+    code = _capi.native().tied_attention(
+        q, cache, factor, gate, out, B, L, heads, G, d, cache.shape[1],
+        _strides_bl(q), _strides_bl(cache), _strides_bl(factor), _strides_bl(gate) if gate is not None else None, _strides_bl(out),
+        off, scalar, float(scale), float(sink), _dt(q.dtype), _IMPLS[impl], scratch, need, count, count.numel())
     _capi.check(code, "based_tied_attention")
     return out
 
@@ -1155,11 +1125,10 @@ def lightning(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         return out
     lib = _capi.lib()
     need = lib.based_lightning_scratch_bytes(B, L, H, d, dv) if q.dtype == torch.bfloat16 and impl != "simt" else 0
-    with torch.cuda.device(q.device):
-        scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-        code = lib.based_lightning_split(q.data_ptr(), k.data_ptr(), v.data_ptr(), decay.data_ptr(), state.data_ptr(), out.data_ptr(), B, L,
-                                         H, d, dv, _strides_bl(q), _strides_bl(k), _strides_bl(v), _strides_bl(out), off, scalar,
-                                         _dt(q.dtype), _IMPLS[impl], _ptr(scratch), need, _stream())
+    scratch = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
+    code = _capi.native().lightning_split(q, k, v, decay, state, out, B, L,
+                                     H, d, dv, _strides_bl(q), _strides_bl(k), _strides_bl(v), _strides_bl(out), off, scalar,
+                                     _dt(q.dtype), _IMPLS[impl], scratch, need)
     _capi.check(code, "based_lightning")
     return out
 
@@ -1182,11 +1151,10 @@ def lightning_step(q, k, v, gate, decay, norm_weight, state, read, count, *, pos
     off, scalar = _position(pos, q)
     if B == 0:
         return True
-    with torch.cuda.device(q.device):
-        code = _capi.lib().based_lightning_step(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), q.stride(0), decay.data_ptr(), norm_weight.data_ptr(),
-            state.data_ptr(), read.data_ptr(), count.data_ptr(), out.data_ptr(), out.stride(0), B, H, d, dv, off, scalar, float(eps),
-            _dt(q.dtype), _stream())
+    code = _capi.native().lightning_step(
+        q, k, v, gate, q.stride(0), decay, norm_weight,
+        state, read, count, out, out.stride(0), B, H, d, dv, off, scalar, float(eps),
+        _dt(q.dtype))
     if code == _capi.ERR_IMPL:
         return False
     _capi.check(code, "based_lightning_step")
