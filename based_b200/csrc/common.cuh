@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "based_b200.h"
 
 namespace based {
@@ -69,6 +71,33 @@ inline int max_active_clusters(void (*kernel)(P...), int K, int threads, int sme
     return 0;
   }
   return n;
+}
+
+// Programmatic launches: a kernel started by launch_pdl may begin while the kernel before it in the stream still runs (once all of
+// that one's blocks have called pdl_trigger or left).  Every such kernel calls pdl_wait, in every block, before it touches memory that
+// another kernel writes or reads: it returns when the kernels before have ended and their writes are visible.  What stands
+// before it (launch latency, set-up, prefetches of weights into L2) overlaps with them.  Without the attribute both do nothing.
+// Data of other kernels is read by coherent loads only: the read-only path is for what no kernel in flight writes.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// 16-byte aligned, a multiple of 16 bytes
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
+}
+
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -7,24 +7,31 @@
 //   CONV    u = x W^T + b, [u1 | u2] = u; the BaseConv decode step on u1 (shift the [B, d, k] state,
 //           append, dot with the taps), silu, gate by u2       in_proj + ShortConvolution.step + gate
 //                                                           (based/models/mixers/convolution.py:88-109, :205-211)
-// With M <= 16 the work is reading W once: HBM-bound (2 bytes per weight, 2 M flops per weight).
-// A warp owns 8 output columns (one n8 tile of mma.sync.m16n8k16; M = 16 is exactly the tile
-// height) and a quarter of K; the four warps of a block reduce through shared memory.  Each lane
-// reads 16 contiguous bytes of one weight row per step -- the K order inside a 32-wide block is
-// permuted identically for x and W, which a dot product does not notice -- so a warp's load
-// covers 8 rows x 64 bytes, and x (a few KB, L1/L2 resident) is read the same way.
+//   F32     PLAIN with an fp32 result
+// The work is reading W once, 2 to 26 MB: 0.3 to 4 us at the HBM rate, so a launch of its own is mostly latency: the launch, the
+// first bytes from HBM, the sum over the split of K.  Two things against that:
+//  * The launch is programmatic: the blocks start while the kernel before still runs, bring their part of W into L2 (a hint;
+//    nothing is read that an earlier kernel may still write), and only then wait for that kernel's end.  The HBM stream of a
+//    chain of such launches does not stop between them.
+//  * All or half of a warp's loads are in flight at once for the usual K: eight or sixteen warps split K, a block owns 8 output
+//    columns (for two halves that an epilogue combines 8 of each; two or four times that where N would need more blocks than
+//    the device holds) and 16 or 32 rows (one or two m16n8k16 tiles, W read once for both).  Each lane reads 16 contiguous
+//    bytes of one weight row per step -- the K order inside a 32-wide block is permuted identically for x and W, which a dot
+//    product does not notice -- so a warp's load covers 8 rows x 64 bytes; x (a few KB, L2 resident) is read the same way.
+// In a chain of such launches, W from HBM, 16 rows (us; cuBLAS's kernel, this one, W at the HBM rate): 1024 x 1024 4.6, 2.9, 0.3;
+// 1024 x 2048 6.6, 2.6, 0.6; 4096 x 1024 4.7, 3.1, 1.3 (with the gated activation 6.8, 3.1); 7168 x 1792 7.4, 6.9, 3.9.
 #include "common.cuh"
 
 namespace based {
 namespace {
 
-constexpr int WARPS = 4;  // split of K inside a block
-enum Epi { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_CONV = 2 };
+constexpr int kSms = 148;
+enum Epi { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_CONV = 2, EPI_F32 = 3 };
 
 struct LinParams {
   const __nv_bfloat16 *x, *w, *bias;
-  __nv_bfloat16* out;
-  int M, N, K;          // N = rows of W (PLAIN: outputs; SWIGLU / CONV: 2 x outputs)
+  void* out;
+  int M, N, K;          // N = rows of W (SWIGLU / CONV: 2 x outputs)
   int64_t sx, so;       // row strides of x and out
   int act;              // SWIGLU: 0 silu, 1 sigmoid
   // CONV
@@ -44,103 +51,170 @@ __device__ __forceinline__ float ld_w(const void* p, int bf16, int i) {
   return bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]) : static_cast<const float*>(p)[i];
 }
 
-// NTILE = 1: one n8 tile per warp; 2: two tiles, columns n0.. and n0 + N/2.. (the two halves an epilogue combines)
-// grid = (outputs / 8, ceil(M / 16)), block = WARPS x 32
-template <int NTILE, int EPI>
-__global__ void __launch_bounds__(WARPS * 32) decode_linear_kernel(const LinParams p) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// CT: 8-column tiles of outputs per block; an epilogue of two halves reads two tiles of W for each, N/2 rows apart.
+// MT: tiles of 16 rows of x.  U: 32-wide blocks of K whose loads are issued together.
+// grid = (ceil(outputs / (8 CT)), ceil(M / (16 MT))), block = WARPS x 32
+template <int CT, int EPI, int MT, int U, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) decode_linear_kernel(const LinParams p) {
+  pdl_trigger();
+  constexpr bool kTwo = EPI == EPI_SWIGLU || EPI == EPI_CONV;
+  constexpr int kCols = 8 * CT, NT8 = kTwo ? 2 * CT : CT;   // output columns of the block, tiles of W: tile i of a second half is CT + i
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 8, m0 = blockIdx.y * 16;
-  const int half = p.N / 2;
+  const int n0 = blockIdx.x * kCols, m0 = blockIdx.y * 16 * MT;
+  const int half = p.N / 2, outputs = kTwo ? half : p.N;
+  // first row of W of a tile; the last block's may not be full
+  auto w_row = [&](int tile) { return min(n0 + (tile % CT) * 8, outputs - 8) + (tile >= CT ? half : 0); };
   // K slice of this warp, in blocks of 32
   const int kblocks = p.K / 32, per = (kblocks + WARPS - 1) / WARPS;
   const int kb0 = warp * per, kb1 = min(kb0 + per, kblocks);
-  const int r0 = m0 + g, r1 = m0 + g + 8;
-  const bool v0 = r0 < p.M, v1 = r1 < p.M;
-  const __nv_bfloat16* xa = p.x + (int64_t)(v0 ? r0 : 0) * p.sx + 8 * t;
-  const __nv_bfloat16* xb = p.x + (int64_t)(v1 ? r1 : 0) * p.sx + 8 * t;
-  const __nv_bfloat16* wr[NTILE];
+  const __nv_bfloat16* wr[NT8];
 #pragma unroll
-  for (int i = 0; i < NTILE; ++i) wr[i] = p.w + (int64_t)(n0 + g + i * half) * p.K + 8 * t;
-  float acc[NTILE][4];
+  for (int i = 0; i < NT8; ++i) wr[i] = p.w + (int64_t)(w_row(i) + g) * p.K + 8 * t;
+  // this warp's part of W into L2, a row segment per lane
+  if (lane < 8 * NT8 && kb0 < kb1) prefetch_l2(p.w + (int64_t)(w_row(lane >> 3) + (lane & 7)) * p.K + kb0 * 32, (kb1 - kb0) * 64);
+  pdl_wait();
+  const __nv_bfloat16* xr[2 * MT];
+  bool live[2 * MT];
 #pragma unroll
-  for (int i = 0; i < NTILE; ++i)
+  for (int m = 0; m < 2 * MT; ++m) {
+    live[m] = m0 + g + 8 * m < p.M;
+    xr[m] = p.x + (int64_t)(live[m] ? m0 + g + 8 * m : 0) * p.sx + 8 * t;
+  }
+  float acc[NT8][MT][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
-  constexpr int U = 4;  // K blocks per round: their loads are issued together
+  for (int i = 0; i < NT8; ++i)
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][m][e] = 0.f;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   for (int kb = kb0; kb < kb1; kb += U) {
-    uint4 wv[U][NTILE], a0[U], a1[U];
+    uint4 wv[U][NT8], xv[U][2 * MT];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool ok = kb + u < kb1;
       const int ko = (kb + u) * 32;
 #pragma unroll
-      for (int i = 0; i < NTILE; ++i) wv[u][i] = ok ? __ldg(reinterpret_cast<const uint4*>(wr[i] + ko)) : zero;
-      a0[u] = (ok && v0) ? __ldg(reinterpret_cast<const uint4*>(xa + ko)) : zero;
-      a1[u] = (ok && v1) ? __ldg(reinterpret_cast<const uint4*>(xb + ko)) : zero;
+      for (int i = 0; i < NT8; ++i) wv[u][i] = ok ? __ldg(reinterpret_cast<const uint4*>(wr[i] + ko)) : zero;
+#pragma unroll
+      for (int m = 0; m < 2 * MT; ++m) xv[u][m] = ok && live[m] ? *reinterpret_cast<const uint4*>(xr[m] + ko) : zero;
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t fa[4] = {a0[u].x, a1[u].x, a0[u].y, a1[u].y};
-      const uint32_t fb[4] = {a0[u].z, a1[u].z, a0[u].w, a1[u].w};
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int i = 0; i < NTILE; ++i) {
-        mma_16816(acc[i], fa, wv[u][i].x, wv[u][i].y);
-        mma_16816(acc[i], fb, wv[u][i].z, wv[u][i].w);
+      for (int m = 0; m < MT; ++m) {
+        const uint4 lo = xv[u][2 * m], hi = xv[u][2 * m + 1];
+        const uint32_t fa[4] = {lo.x, hi.x, lo.y, hi.y}, fb[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int i = 0; i < NT8; ++i) {
+          mma_16816(acc[i][m], fa, wv[u][i].x, wv[u][i].y);
+          mma_16816(acc[i][m], fb, wv[u][i].z, wv[u][i].w);
+        }
       }
+  }
+  // ---- the K slices' sums meet in shared memory, [warp][tile][row][column]; lanes hold rows g, g + 8 and columns 2t, 2t + 1
+  __shared__ float red[WARPS][NT8][16 * MT * 8];
+#pragma unroll
+  for (int i = 0; i < NT8; ++i)
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      *reinterpret_cast<float2*>(&red[warp][i][(16 * m + g) * 8 + 2 * t]) = make_float2(acc[i][m][0], acc[i][m][1]);
+      *reinterpret_cast<float2*>(&red[warp][i][(16 * m + g + 8) * 8 + 2 * t]) = make_float2(acc[i][m][2], acc[i][m][3]);
+    }
+  // outputs (tile, row, column) over the threads
+  constexpr int kIn = 16 * MT * 8, kOut = kIn * CT, kThreads = WARPS * 32, kPer = (kOut + kThreads - 1) / kThreads;
+  float bias[kPer][2], cs[kPer][8], cw[kPer][8], cb[kPer];
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int o = tid + r * kThreads, in = o % kIn, col = n0 + o / kIn * 8 + (in & 7), row = m0 + (in >> 3);
+    bias[r][0] = bias[r][1] = cb[r] = 0.f;
+    if (o < kOut && col < outputs && p.bias) {
+      bias[r][0] = __bfloat162float(p.bias[col]);
+      if (kTwo) bias[r][1] = __bfloat162float(p.bias[col + half]);
+    }
+    if (EPI == EPI_CONV && o < kOut && row < p.M && col < outputs) {   // these loads' latency passes with the barrier
+      const __nv_bfloat16* st = p.state + ((int64_t)row * half + col) * p.ck;
+      if (p.cb) cb[r] = ld_w(p.cb, p.cw_bf16, col);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < p.ck) {
+          cs[r][j] = __bfloat162float(st[j]);
+          cw[r][j] = ld_w(p.cw, p.cw_bf16, col * p.ck + j);
+        }
     }
   }
-  // ---- reduce the K slices
-  __shared__ float red[WARPS][NTILE][4][32];
-#pragma unroll
-  for (int i = 0; i < NTILE; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) red[warp][i][e][lane] = acc[i][e];
   __syncthreads();
-  if (warp != 0) return;
 #pragma unroll
-  for (int i = 0; i < NTILE; ++i)
+  for (int r = 0; r < kPer; ++r) {
+    const int o = tid + r * kThreads, tile = o / kIn, in = o % kIn, col = n0 + tile * 8 + (in & 7), row = m0 + (in >> 3);
+    if (o >= kOut || row >= p.M || col >= outputs) continue;
+    float y = 0.f, y2 = 0.f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) s += red[w][i][e][lane];
-      acc[i][e] = s;
+    for (int w = 0; w < WARPS; ++w) {
+      y += red[w][tile][in];
+      if (kTwo) y2 += red[w][(kTwo ? CT : 0) + tile][in];
     }
-  // this lane holds rows r0 (e = 0, 1) and r1 (e = 2, 3), columns c0 = n0 + 2t and c0 + 1 of each tile
-  const int c0 = n0 + 2 * t;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int row = e < 2 ? r0 : r1, col = c0 + (e & 1);
-    if (row >= p.M) continue;
+    y += bias[r][0];
+    y2 += bias[r][1];
+    const int64_t at = (int64_t)row * p.so + col;
+    if (EPI == EPI_F32) {
+      static_cast<float*>(p.out)[at] = y;
+      continue;
+    }
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + at;
     if (EPI == EPI_PLAIN) {
-      float y = acc[0][e];
-      if (p.bias) y += __bfloat162float(p.bias[col]);
-      p.out[(int64_t)row * p.so + col] = __float2bfloat16_rn(y);
+      *out = __float2bfloat16_rn(y);
     } else if (EPI == EPI_SWIGLU) {
-      float y = acc[0][e], gt = acc[NTILE - 1][e];
-      if (p.bias) { y += __bfloat162float(p.bias[col]); gt += __bfloat162float(p.bias[col + half]); }
-      y = bf16_round(y); gt = bf16_round(gt);  // fc1's output is a bf16 tensor in the unfused sequence
-      const float s = sigmoid_f(gt);
-      p.out[(int64_t)row * p.so + col] = __float2bfloat16_rn(y * (p.act == 0 ? gt * s : s));
+      y = bf16_round(y);                          // fc1's output is a bf16 tensor in the unfused sequence
+      const float gt = bf16_round(y2), s = sigmoid_f(gt);
+      *out = __float2bfloat16_rn(y * (p.act == 0 ? gt * s : s));
     } else {
-      float u1 = acc[0][e], u2 = acc[NTILE - 1][e];
-      if (p.bias) { u1 += __bfloat162float(p.bias[col]); u2 += __bfloat162float(p.bias[col + half]); }
-      const __nv_bfloat16 u1b = __float2bfloat16_rn(u1);
-      u2 = bf16_round(u2);
       __nv_bfloat16* st = p.state + ((int64_t)row * half + col) * p.ck;
-      float c = p.cb ? ld_w(p.cb, p.cw_bf16, col) : 0.f;
-      for (int j = 0; j + 1 < p.ck; ++j) {
-        const __nv_bfloat16 h = st[j + 1];
-        st[j] = h;
-        c = fmaf(ld_w(p.cw, p.cw_bf16, col * p.ck + j), __bfloat162float(h), c);
-      }
-      st[p.ck - 1] = u1b;
-      c = fmaf(ld_w(p.cw, p.cw_bf16, col * p.ck + p.ck - 1), __bfloat162float(u1b), c);
-      p.out[(int64_t)row * p.so + col] = __float2bfloat16_rn(c * sigmoid_f(c) * u2);
+      const __nv_bfloat16 u1 = __float2bfloat16_rn(y);
+      float c = cb[r];
+#pragma unroll
+      for (int j = 0; j < 7; ++j)
+        if (j < p.ck - 1) {
+          st[j] = __float2bfloat16_rn(cs[r][j + 1]);   // exact: it was a bf16 value
+          c = fmaf(cw[r][j], cs[r][j + 1], c);
+        }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j == p.ck - 1) {
+          st[j] = u1;
+          c = fmaf(cw[r][j], __bfloat162float(u1), c);
+        }
+      *out = __float2bfloat16_rn(c * sigmoid_f(c) * bf16_round(y2));
     }
   }
+}
+
+template <int EPI, int CT>
+int launch_tiles(const LinParams& p, int outputs, cudaStream_t stream) {
+  constexpr int NT8 = (EPI == EPI_SWIGLU || EPI == EPI_CONV ? 2 : 1) * CT;
+  constexpr int U1 = NT8 == 1 ? 8 : NT8 == 2 ? 4 : 2, U2 = NT8 == 1 ? 4 : 2;
+  const int gx = (outputs / 8 + CT - 1) / CT;
+  const dim3 g1(gx, 1), g2(gx, (p.M + 31) / 32);
+  // 16 warps to a block where K is long and every block has an SM: a warp's loads are one round again
+  if constexpr (CT == 1) {
+    if (p.K > 1024 && gx <= kSms) {
+      if (p.M <= 16) return launch_pdl(decode_linear_kernel<CT, EPI, 1, 4, 16>, g1, dim3(512), 0, stream, p);
+      return launch_pdl(decode_linear_kernel<CT, EPI, 2, U2, 16>, g2, dim3(512), 0, stream, p);
+    }
+  }
+  if (p.M <= 16) return launch_pdl(decode_linear_kernel<CT, EPI, 1, U1, 8>, g1, dim3(256), 0, stream, p);
+  return launch_pdl(decode_linear_kernel<CT, EPI, 2, U2, 8>, g2, dim3(256), 0, stream, p);
+}
+
+// Column tiles per block: as few as let all blocks be on the device at once, two to an SM; a block that starts later starts
+// its share of W later, and the kernel after this one cannot start its own before it.
+template <int EPI>
+int launch_epi(const LinParams& p, int outputs, cudaStream_t stream) {
+  const int tiles = outputs / 8;
+  if constexpr (EPI == EPI_PLAIN || EPI == EPI_F32)
+    if (tiles > 4 * kSms) return launch_tiles<EPI, 4>(p, outputs, stream);
+  return tiles > 2 * kSms ? launch_tiles<EPI, 2>(p, outputs, stream) : launch_tiles<EPI, 1>(p, outputs, stream);
 }
 
 }  // namespace
@@ -149,17 +223,17 @@ int launch_decode_linear(const void* x, const void* w, const void* bias, void* o
                          int64_t so, int epilogue, int act, void* conv_state, const void* conv_weight,
                          const void* conv_bias, int conv_k, int conv_w_dtype, cudaStream_t stream) {
   if (K % 32 != 0 || sx % 8 != 0 || !aligned16(x) || !aligned16(w)) return BASED_ERR_ALIGN;
-  const int outputs = epilogue == EPI_PLAIN ? N : N / 2;
-  if (outputs % 8 != 0 || (epilogue != EPI_PLAIN && N % 2 != 0)) return BASED_ERR_SHAPE;
+  const bool two = epilogue == EPI_SWIGLU || epilogue == EPI_CONV;
+  const int outputs = two ? N / 2 : N;
+  if (outputs % 8 != 0 || (two && N % 2 != 0)) return BASED_ERR_SHAPE;
   LinParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
-              static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(out), M, N, K, sx, so, act,
+              static_cast<const __nv_bfloat16*>(bias), out, M, N, K, sx, so, act,
               static_cast<__nv_bfloat16*>(conv_state), conv_weight, conv_bias, conv_k, conv_w_dtype == BASED_BF16};
-  const dim3 grid(outputs / 8, (M + 15) / 16);
-  if (epilogue == EPI_PLAIN) decode_linear_kernel<1, EPI_PLAIN><<<grid, WARPS * 32, 0, stream>>>(p);
-  else if (epilogue == EPI_SWIGLU) decode_linear_kernel<2, EPI_SWIGLU><<<grid, WARPS * 32, 0, stream>>>(p);
-  else if (epilogue == EPI_CONV) decode_linear_kernel<2, EPI_CONV><<<grid, WARPS * 32, 0, stream>>>(p);
-  else return BASED_ERR_SHAPE;
-  return (int)cudaGetLastError();
+  if (epilogue == EPI_PLAIN) return launch_epi<EPI_PLAIN>(p, outputs, stream);
+  if (epilogue == EPI_SWIGLU) return launch_epi<EPI_SWIGLU>(p, outputs, stream);
+  if (epilogue == EPI_CONV) return launch_epi<EPI_CONV>(p, outputs, stream);
+  if (epilogue == EPI_F32) return launch_epi<EPI_F32>(p, outputs, stream);
+  return BASED_ERR_SHAPE;
 }
 
 }  // namespace based

@@ -109,6 +109,8 @@ __device__ __forceinline__ void load_taps(const void* weight, int w_bf16, int ch
 // grid = (ceil(di / (N * NTH)), ceil(L / (TT * TY)), B), block = (NTH, TY)
 template <typename T, int K>
 __global__ void __launch_bounds__(NTH * TY, 3) gated_conv_prefill_kernel(const ConvParams p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Vec<T>::N;
   const int ch = (blockIdx.x * NTH + threadIdx.x) * N;
   const int l0 = (blockIdx.y * TY + threadIdx.y) * TT, b = blockIdx.z;
@@ -171,6 +173,8 @@ __global__ void __launch_bounds__(NTH * TY, 3) gated_conv_prefill_kernel(const C
 // One decode step: thread per (batch, channel); the state row of a channel is K contiguous elements.
 template <typename T, int K>
 __global__ void __launch_bounds__(256) gated_conv_step_kernel(const ConvParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int idx = blockIdx.x * 256 + threadIdx.x;
   if (idx >= p.B * p.di) return;
   const int b = idx / p.di, ch = idx - b * p.di;
@@ -195,10 +199,10 @@ int launch_prefill_t(const ConvParams& p, int k, cudaStream_t stream) {
   constexpr int N = Vec<T>::N;
   const dim3 grid((p.di / N + NTH - 1) / NTH, (p.L + TT * TY - 1) / (TT * TY), p.B), block(NTH, TY);
   switch (k) {
-    case 1: gated_conv_prefill_kernel<T, 1><<<grid, block, 0, stream>>>(p); break;
-    case 2: gated_conv_prefill_kernel<T, 2><<<grid, block, 0, stream>>>(p); break;
-    case 3: gated_conv_prefill_kernel<T, 3><<<grid, block, 0, stream>>>(p); break;
-    case 4: gated_conv_prefill_kernel<T, 4><<<grid, block, 0, stream>>>(p); break;
+    case 1: launch_pdl(gated_conv_prefill_kernel<T, 1>, grid, block, 0, stream, p); break;
+    case 2: launch_pdl(gated_conv_prefill_kernel<T, 2>, grid, block, 0, stream, p); break;
+    case 3: launch_pdl(gated_conv_prefill_kernel<T, 3>, grid, block, 0, stream, p); break;
+    case 4: launch_pdl(gated_conv_prefill_kernel<T, 4>, grid, block, 0, stream, p); break;
     default: return BASED_ERR_SHAPE;
   }
   return (int)cudaGetLastError();
@@ -207,10 +211,10 @@ template <typename T>
 int launch_step_t(const ConvParams& p, int k, cudaStream_t stream) {
   const int grid = (int)(((int64_t)p.B * p.di + 255) / 256);
   switch (k) {
-    case 1: gated_conv_step_kernel<T, 1><<<grid, 256, 0, stream>>>(p); break;
-    case 2: gated_conv_step_kernel<T, 2><<<grid, 256, 0, stream>>>(p); break;
-    case 3: gated_conv_step_kernel<T, 3><<<grid, 256, 0, stream>>>(p); break;
-    case 4: gated_conv_step_kernel<T, 4><<<grid, 256, 0, stream>>>(p); break;
+    case 1: launch_pdl(gated_conv_step_kernel<T, 1>, grid, 256, 0, stream, p); break;
+    case 2: launch_pdl(gated_conv_step_kernel<T, 2>, grid, 256, 0, stream, p); break;
+    case 3: launch_pdl(gated_conv_step_kernel<T, 3>, grid, 256, 0, stream, p); break;
+    case 4: launch_pdl(gated_conv_step_kernel<T, 4>, grid, 256, 0, stream, p); break;
     default: return BASED_ERR_SHAPE;
   }
   return (int)cudaGetLastError();

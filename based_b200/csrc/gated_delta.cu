@@ -138,6 +138,8 @@ struct StepP {
 // NR float4 rows of the state per thread; thread t owns columns 4 (t mod dv/4) .. +3 of rows t / (dv/4), + R, ...
 template <typename T, int NR>
 __global__ void __launch_bounds__(kThreads, NR <= 8 ? 3 : NR <= 16 ? 2 : 1) delta_step_kernel(const StepP p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int hk = h / (p.H / p.Hk);
@@ -258,12 +260,12 @@ int launch_step_t(const StepP& p, cudaStream_t st) {
   const int C4 = p.dv / 4, R = kThreads / C4, nr = (p.d + R - 1) / R;
   const size_t smem = sizeof(float) * (2 * p.d + p.dv + 24) + sizeof(float4) * R * C4;
   const dim3 grid(p.H, p.B);
-  if (nr <= 1) delta_step_kernel<T, 1><<<grid, kThreads, smem, st>>>(p);
-  else if (nr <= 2) delta_step_kernel<T, 2><<<grid, kThreads, smem, st>>>(p);
-  else if (nr <= 4) delta_step_kernel<T, 4><<<grid, kThreads, smem, st>>>(p);
-  else if (nr <= 8) delta_step_kernel<T, 8><<<grid, kThreads, smem, st>>>(p);
-  else if (nr <= 16) delta_step_kernel<T, 16><<<grid, kThreads, smem, st>>>(p);
-  else delta_step_kernel<T, 32><<<grid, kThreads, smem, st>>>(p);
+  if (nr <= 1) launch_pdl(delta_step_kernel<T, 1>, grid, kThreads, smem, st, p);
+  else if (nr <= 2) launch_pdl(delta_step_kernel<T, 2>, grid, kThreads, smem, st, p);
+  else if (nr <= 4) launch_pdl(delta_step_kernel<T, 4>, grid, kThreads, smem, st, p);
+  else if (nr <= 8) launch_pdl(delta_step_kernel<T, 8>, grid, kThreads, smem, st, p);
+  else if (nr <= 16) launch_pdl(delta_step_kernel<T, 16>, grid, kThreads, smem, st, p);
+  else launch_pdl(delta_step_kernel<T, 32>, grid, kThreads, smem, st, p);
   return (int)cudaGetLastError();
 }
 

@@ -31,6 +31,8 @@ struct PrepP {
 
 template <typename T>
 __global__ void __launch_bounds__(kPrepThreads) latent_prepare_kernel(const PrepP p) {
+  pdl_trigger();
+  pdl_wait();
   const int l = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int pos = position0(p.offsets, p.offset, b) + l;
   if (pos < 0 || pos >= p.max_len || pos >= p.table_len) return;
@@ -168,8 +170,8 @@ int launch_latent_prepare(const void* z, const void* norm_w, void* cache, void* 
   const PrepP p{z, norm_w, cache, q, cosv, sinv, offsets, offset, B, L, H, r, rd, d, max_len, table_len,
                 zb, zl, cb, cl, qb, ql, eps};
   const dim3 grid(L, B);
-  if (io_dtype == BASED_BF16) latent_prepare_kernel<__nv_bfloat16><<<grid, kPrepThreads, 0, stream>>>(p);
-  else latent_prepare_kernel<float><<<grid, kPrepThreads, 0, stream>>>(p);
+  if (io_dtype == BASED_BF16) launch_pdl(latent_prepare_kernel<__nv_bfloat16>, grid, kPrepThreads, 0, stream, p);
+  else launch_pdl(latent_prepare_kernel<float>, grid, kPrepThreads, 0, stream, p);
   return (int)cudaGetLastError();
 }
 

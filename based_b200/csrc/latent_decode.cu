@@ -41,6 +41,8 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 // NW: 8-column groups of the context per warp
 template <int NW>
 __global__ void __launch_bounds__(kThreads, 2) latent_decode_kernel(const P p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int split = blockIdx.x, row0 = blockIdx.y * 16, b = blockIdx.z;
@@ -194,6 +196,8 @@ __global__ void __launch_bounds__(kThreads, 2) latent_decode_kernel(const P p) {
 // G groups of splits times 128 / G column pairs per block; grid (R, B, ceil(r / (256 / G)))
 template <int G>
 __global__ void __launch_bounds__(128) latent_decode_merge_kernel(const P p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int W = 128 / G;
   const int row = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, grp = tid / W, lane = tid % W;
   const int c = blockIdx.z * 2 * W + 2 * lane;
@@ -249,9 +253,9 @@ template <int NW>
 int launch_nw(const P& p, cudaStream_t st) {
   const cudaError_t e = cudaFuncSetAttribute(latent_decode_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return (int)e;
-  latent_decode_kernel<NW><<<dim3(p.splits, (p.R + 15) / 16, p.B), kThreads, smem_bytes(p.r + p.rd), st>>>(p);
-  if (p.splits > 16) latent_decode_merge_kernel<8><<<dim3(p.R, p.B, (p.r + 31) / 32), 128, 0, st>>>(p);
-  else if (p.splits > 1) latent_decode_merge_kernel<1><<<dim3(p.R, p.B, (p.r + 255) / 256), 128, 0, st>>>(p);
+  launch_pdl(latent_decode_kernel<NW>, dim3(p.splits, (p.R + 15) / 16, p.B), kThreads, smem_bytes(p.r + p.rd), st, p);
+  if (p.splits > 16) launch_pdl(latent_decode_merge_kernel<8>, dim3(p.R, p.B, (p.r + 31) / 32), 128, 0, st, p);
+  else if (p.splits > 1) launch_pdl(latent_decode_merge_kernel<1>, dim3(p.R, p.B, (p.r + 255) / 256), 128, 0, st, p);
   return (int)cudaGetLastError();
 }
 

@@ -106,6 +106,8 @@ struct StepP {
 // are in flight.
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, V <= 8 ? 3 : 2) lightning_step_kernel(const StepP p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, col0 = blockIdx.z * p.cols, tid = threadIdx.x;
   const int quads = p.cols / 4, R = kThreads / quads, row4 = p.dv / 4;
@@ -216,10 +218,10 @@ int launch_step_t(const StepP& p, int B, cudaStream_t st) {
   const int quads = p.cols / 4, R = kThreads / quads, rows = (p.d + R - 1) / R;
   const size_t smem = sizeof(float) * (2 * p.d + p.cols + (size_t)R * p.cols);
   const dim3 grid(p.H, B, p.dv / p.cols);
-  if (rows <= 2) lightning_step_kernel<T, 2><<<grid, kThreads, smem, st>>>(p);
-  else if (rows <= 4) lightning_step_kernel<T, 4><<<grid, kThreads, smem, st>>>(p);
-  else if (rows <= 8) lightning_step_kernel<T, 8><<<grid, kThreads, smem, st>>>(p);
-  else lightning_step_kernel<T, 16><<<grid, kThreads, smem, st>>>(p);
+  if (rows <= 2) launch_pdl(lightning_step_kernel<T, 2>, grid, kThreads, smem, st, p);
+  else if (rows <= 4) launch_pdl(lightning_step_kernel<T, 4>, grid, kThreads, smem, st, p);
+  else if (rows <= 8) launch_pdl(lightning_step_kernel<T, 8>, grid, kThreads, smem, st, p);
+  else launch_pdl(lightning_step_kernel<T, 16>, grid, kThreads, smem, st, p);
   return (int)cudaGetLastError();
 }
 

@@ -58,9 +58,11 @@ template <> struct VecOps<__nv_bfloat16> {
 
 template <typename IO, typename ST, int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads <= 192 ? 3 : 2)
-linattn_decode_kernel(const IO* __restrict__ q, const IO* __restrict__ k, const IO* __restrict__ v,
-                      IO* __restrict__ y, ST* __restrict__ kv_state, ST* __restrict__ k_state,
+linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
+                      IO* y, ST* kv_state, ST* k_state,
                       int H, int dv, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 sy, float eps) {
+  pdl_trigger();
+  pdl_wait();
   using VO = VecOps<ST>;
   constexpr int VEC = VO::kVec;
   constexpr int RPG = VEC;  // rows per 16-byte-aligned group
@@ -184,11 +186,11 @@ int launch_typed(const void* q, const void* k, const void* v, void* y, void* kv_
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if ((long long)B * H >= 6LL * sms) {  // at least two waves of three CTAs per SM
-    linattn_decode_kernel<IO, ST, 192><<<B * H, 192, 0, stream>>>(
+    launch_pdl(linattn_decode_kernel<IO, ST, 192>, B * H, 192, 0, stream, 
         static_cast<const IO*>(q), static_cast<const IO*>(k), static_cast<const IO*>(v), static_cast<IO*>(y),
         static_cast<ST*>(kv_state), static_cast<ST*>(k_state), H, dv, sq, sk, sv, sy, eps);
   } else {
-    linattn_decode_kernel<IO, ST, 256><<<B * H, 256, 0, stream>>>(
+    launch_pdl(linattn_decode_kernel<IO, ST, 256>, B * H, 256, 0, stream, 
         static_cast<const IO*>(q), static_cast<const IO*>(k), static_cast<const IO*>(v), static_cast<IO*>(y),
         static_cast<ST*>(kv_state), static_cast<ST*>(k_state), H, dv, sq, sk, sv, sy, eps);
   }

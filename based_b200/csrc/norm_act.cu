@@ -102,6 +102,8 @@ constexpr int NORM_THREADS = 128;
 // between the reduction and the scaling, so the row is read once).
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(const NormParams p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t row = blockIdx.x;
   const int ngroups = p.D >> 3;
   float z[VPT][8];
@@ -197,6 +199,8 @@ struct StreamParams {
 // One row per block; N values per access (8, or 1 for any D), VPT accesses per thread kept in registers.
 template <typename T, int N, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamParams p) {
+  pdl_trigger();
+  pdl_wait();
   using seq::Pack;
   const int64_t row = blockIdx.x;
   const int groups = p.D / N;
@@ -284,6 +288,8 @@ struct PostNormParams {
 
 template <typename T, int N, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const PostNormParams p) {
+  pdl_trigger();
+  pdl_wait();
   using seq::Pack;
   const int64_t row = blockIdx.x;
   const int groups = p.D / N;
@@ -347,6 +353,8 @@ struct EmbedParams {
 
 template <typename T, int N>
 __global__ void __launch_bounds__(NORM_THREADS) stream_embed_kernel(const EmbedParams p) {
+  pdl_trigger();
+  pdl_wait();
   using seq::Pack;
   const int64_t row = (int64_t)blockIdx.y * p.L + blockIdx.x;
   const int64_t tok = p.tokens[row], at = (int64_t)seq::position0(p.offsets, p.offset, blockIdx.y) + blockIdx.x;
@@ -374,6 +382,8 @@ struct NormGateParams {
 
 template <typename T, int N, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS) norm_gate_kernel(const NormGateParams p) {
+  pdl_trigger();
+  pdl_wait();
   using seq::Pack;
   const int64_t row = blockIdx.x;
   const int groups = p.D / N;
@@ -414,6 +424,8 @@ struct TokenGateParams {
 
 template <typename T, int N>
 __global__ void __launch_bounds__(256) token_gate_kernel(const TokenGateParams p) {
+  pdl_trigger();
+  pdl_wait();
   using seq::Pack;
   const int per = p.n / N;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -446,6 +458,8 @@ __device__ __forceinline__ float act_fn(float g, int act) {
 // warp's accesses are contiguous, all loads of a thread are issued before any arithmetic.
 template <typename T, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS) gated_act_kernel(const ActParams p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = V16<T>::N;
   const int nvec = p.F / N;
   const int64_t row = blockIdx.x;
@@ -493,14 +507,14 @@ int launch_stream_norm_t(const StreamParams& p, cudaStream_t stream) {
                    aligned16(p.out2) && p.sb % 8 == 0;
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   if (vec) {
-    if (vpt <= 1) stream_norm_kernel<T, 8, 1><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 2) stream_norm_kernel<T, 8, 2><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 4) stream_norm_kernel<T, 8, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 8) stream_norm_kernel<T, 8, 8><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 1) launch_pdl(stream_norm_kernel<T, 8, 1>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 2) launch_pdl(stream_norm_kernel<T, 8, 2>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 4) launch_pdl(stream_norm_kernel<T, 8, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 8) launch_pdl(stream_norm_kernel<T, 8, 8>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 8192 wide
   } else {
-    if (vpt <= 4) stream_norm_kernel<T, 1, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 32) stream_norm_kernel<T, 1, 32><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 4) launch_pdl(stream_norm_kernel<T, 1, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 32) launch_pdl(stream_norm_kernel<T, 1, 32>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 4096 wide
   }
   return (int)cudaGetLastError();
@@ -513,14 +527,14 @@ int launch_post_norm_t(const PostNormParams& p, int64_t M, cudaStream_t stream) 
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
   if (vec) {
-    if (vpt <= 1) stream_post_norm_kernel<T, 8, 1><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 2) stream_post_norm_kernel<T, 8, 2><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 4) stream_post_norm_kernel<T, 8, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 8) stream_post_norm_kernel<T, 8, 8><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 1) launch_pdl(stream_post_norm_kernel<T, 8, 1>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 2) launch_pdl(stream_post_norm_kernel<T, 8, 2>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 4) launch_pdl(stream_post_norm_kernel<T, 8, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 8) launch_pdl(stream_post_norm_kernel<T, 8, 8>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 8192 wide
   } else {
-    if (vpt <= 4) stream_post_norm_kernel<T, 1, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 32) stream_post_norm_kernel<T, 1, 32><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 4) launch_pdl(stream_post_norm_kernel<T, 1, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 32) launch_pdl(stream_post_norm_kernel<T, 1, 32>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 4096 wide
   }
   return (int)cudaGetLastError();
@@ -530,9 +544,9 @@ template <typename T>
 int launch_embed_t(const EmbedParams& p, int B, cudaStream_t stream) {
   const dim3 grid((unsigned)p.L, (unsigned)B);
   if (p.D % 8 == 0 && aligned16(p.table) && aligned16(p.pos) && aligned16(p.residual) && aligned16(p.out))
-    stream_embed_kernel<T, 8><<<grid, NORM_THREADS, 0, stream>>>(p);
+    launch_pdl(stream_embed_kernel<T, 8>, grid, NORM_THREADS, 0, stream, p);
   else
-    stream_embed_kernel<T, 1><<<grid, NORM_THREADS, 0, stream>>>(p);
+    launch_pdl(stream_embed_kernel<T, 1>, grid, NORM_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -543,14 +557,14 @@ int launch_norm_gate_t(const NormGateParams& p, int64_t M, cudaStream_t stream) 
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
   if (vec) {
-    if (vpt <= 1) norm_gate_kernel<T, 8, 1><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 2) norm_gate_kernel<T, 8, 2><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 4) norm_gate_kernel<T, 8, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 8) norm_gate_kernel<T, 8, 8><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 1) launch_pdl(norm_gate_kernel<T, 8, 1>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 2) launch_pdl(norm_gate_kernel<T, 8, 2>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 4) launch_pdl(norm_gate_kernel<T, 8, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 8) launch_pdl(norm_gate_kernel<T, 8, 8>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;
   } else {
-    if (vpt <= 4) norm_gate_kernel<T, 1, 4><<<grid, NORM_THREADS, 0, stream>>>(p);
-    else if (vpt <= 32) norm_gate_kernel<T, 1, 32><<<grid, NORM_THREADS, 0, stream>>>(p);
+    if (vpt <= 4) launch_pdl(norm_gate_kernel<T, 1, 4>, grid, NORM_THREADS, 0, stream, p);
+    else if (vpt <= 32) launch_pdl(norm_gate_kernel<T, 1, 32>, grid, NORM_THREADS, 0, stream, p);
     else return BASED_ERR_SHAPE;
   }
   return (int)cudaGetLastError();
@@ -562,8 +576,8 @@ int launch_token_gate_t(const TokenGateParams& p, cudaStream_t stream) {
                    aligned16(p.out);
   const int64_t work = p.M * (p.n / (vec ? 8 : 1)), blocks = (work + 255) / 256;
   if (blocks > 2147483647LL) return BASED_ERR_TOO_LARGE;
-  if (vec) token_gate_kernel<T, 8><<<(unsigned)blocks, 256, 0, stream>>>(p);
-  else token_gate_kernel<T, 1><<<(unsigned)blocks, 256, 0, stream>>>(p);
+  if (vec) launch_pdl(token_gate_kernel<T, 8>, (unsigned)blocks, 256, 0, stream, p);
+  else launch_pdl(token_gate_kernel<T, 1>, (unsigned)blocks, 256, 0, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -618,10 +632,10 @@ int launch_add_rmsnorm(const void* x, const void* residual, const void* weight, 
                io_dtype == BASED_BF16, res_dtype == BASED_BF16, w_dtype == BASED_BF16, round_input != 0, eps};
   const int groups = D / 8, vpt = (groups + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
-  if (vpt <= 1) add_rmsnorm_kernel<1><<<grid, NORM_THREADS, 0, stream>>>(p);
-  else if (vpt <= 2) add_rmsnorm_kernel<2><<<grid, NORM_THREADS, 0, stream>>>(p);
-  else if (vpt <= 4) add_rmsnorm_kernel<4><<<grid, NORM_THREADS, 0, stream>>>(p);
-  else add_rmsnorm_kernel<8><<<grid, NORM_THREADS, 0, stream>>>(p);
+  if (vpt <= 1) launch_pdl(add_rmsnorm_kernel<1>, grid, NORM_THREADS, 0, stream, p);
+  else if (vpt <= 2) launch_pdl(add_rmsnorm_kernel<2>, grid, NORM_THREADS, 0, stream, p);
+  else if (vpt <= 4) launch_pdl(add_rmsnorm_kernel<4>, grid, NORM_THREADS, 0, stream, p);
+  else launch_pdl(add_rmsnorm_kernel<8>, grid, NORM_THREADS, 0, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -654,11 +668,11 @@ int launch_gated_act(const void* y, const void* gate, void* out, int64_t M, int 
   }
 #define BASED_LAUNCH_ACT(T)                                                                      \
   do {                                                                                           \
-    if (vpt <= 1) gated_act_kernel<T, 1><<<grid, NORM_THREADS, 0, stream>>>(p);                  \
-    else if (vpt <= 2) gated_act_kernel<T, 2><<<grid, NORM_THREADS, 0, stream>>>(p);             \
-    else if (vpt <= 4) gated_act_kernel<T, 4><<<grid, NORM_THREADS, 0, stream>>>(p);             \
-    else if (vpt <= 8) gated_act_kernel<T, 8><<<grid, NORM_THREADS, 0, stream>>>(p);             \
-    else gated_act_kernel<T, 16><<<grid, NORM_THREADS, 0, stream>>>(p);                          \
+    if (vpt <= 1) launch_pdl(gated_act_kernel<T, 1>, grid, NORM_THREADS, 0, stream, p);                  \
+    else if (vpt <= 2) launch_pdl(gated_act_kernel<T, 2>, grid, NORM_THREADS, 0, stream, p);             \
+    else if (vpt <= 4) launch_pdl(gated_act_kernel<T, 4>, grid, NORM_THREADS, 0, stream, p);             \
+    else if (vpt <= 8) launch_pdl(gated_act_kernel<T, 8>, grid, NORM_THREADS, 0, stream, p);             \
+    else launch_pdl(gated_act_kernel<T, 16>, grid, NORM_THREADS, 0, stream, p);                          \
   } while (0)
   if (io_dtype == BASED_BF16) BASED_LAUNCH_ACT(__nv_bfloat16);
   else BASED_LAUNCH_ACT(float);

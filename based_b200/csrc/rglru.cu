@@ -27,6 +27,8 @@ constexpr int kThreads = 64;
 
 template <typename T, int U>
 __global__ void __launch_bounds__(kThreads) rglru_kernel(const RgP p) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * kThreads + threadIdx.x, b = blockIdx.y;
   if (c >= p.W) return;
   const int blk = c / p.bw, j = c - blk * p.bw;
@@ -68,11 +70,11 @@ int launch_rglru(const void* u, const void* y, const float* gates, const void* r
   const RgP p{u, y, rb, ib, gates, lam, state, out, offsets, offset, B, L, W, bw, su, sy, so, g_block, g_row};
   const dim3 grid((W + kThreads - 1) / kThreads, B);
   if (io_dtype == BASED_BF16) {
-    if (L == 1) rglru_kernel<__nv_bfloat16, 1><<<grid, kThreads, 0, stream>>>(p);
-    else rglru_kernel<__nv_bfloat16, 8><<<grid, kThreads, 0, stream>>>(p);
+    if (L == 1) launch_pdl(rglru_kernel<__nv_bfloat16, 1>, grid, kThreads, 0, stream, p);
+    else launch_pdl(rglru_kernel<__nv_bfloat16, 8>, grid, kThreads, 0, stream, p);
   } else {
-    if (L == 1) rglru_kernel<float, 1><<<grid, kThreads, 0, stream>>>(p);
-    else rglru_kernel<float, 8><<<grid, kThreads, 0, stream>>>(p);
+    if (L == 1) launch_pdl(rglru_kernel<float, 1>, grid, kThreads, 0, stream, p);
+    else launch_pdl(rglru_kernel<float, 8>, grid, kThreads, 0, stream, p);
   }
   return (int)cudaGetLastError();
 }

@@ -91,6 +91,8 @@ __global__ void __launch_bounds__(kThreads) short_conv_kernel(const ConvP p) {
 // are used, so that a thread's loads are all in flight together, and the taps of its channels are TAPS 16-byte loads.
 template <typename T, int TT, int TAPS>
 __global__ void __launch_bounds__(kThreads, 5) short_conv_vec_kernel(const ConvP p) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Wide<T>::N;
   const int c = (blockIdx.x * kThreads + threadIdx.x) * N;
   const int l0 = blockIdx.y * TT, b = blockIdx.z;
@@ -152,6 +154,8 @@ __global__ void __launch_bounds__(kThreads, 5) short_conv_vec_kernel(const ConvP
 // the last min(L, taps) inputs of the call into their slots
 template <typename T>
 __global__ void __launch_bounds__(kThreads) ring_update_kernel(const ConvP p) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * kThreads + threadIdx.x, b = blockIdx.z;
   if (c >= p.C) return;
   const int pos0 = position0(p.offsets, p.offset, b);
@@ -166,9 +170,9 @@ bool launch_vec(const ConvP& p, cudaStream_t st) {
   constexpr int N = Wide<T>::N;
   const dim3 grid((p.C / N + kThreads - 1) / kThreads, (p.L + TT - 1) / TT, p.B);
   switch (p.taps) {
-    case 2: short_conv_vec_kernel<T, TT, 2><<<grid, kThreads, 0, st>>>(p); return true;
-    case 3: short_conv_vec_kernel<T, TT, 3><<<grid, kThreads, 0, st>>>(p); return true;
-    case 4: short_conv_vec_kernel<T, TT, 4><<<grid, kThreads, 0, st>>>(p); return true;
+    case 2: launch_pdl(short_conv_vec_kernel<T, TT, 2>, grid, kThreads, 0, st, p); return true;
+    case 3: launch_pdl(short_conv_vec_kernel<T, TT, 3>, grid, kThreads, 0, st, p); return true;
+    case 4: launch_pdl(short_conv_vec_kernel<T, TT, 4>, grid, kThreads, 0, st, p); return true;
     default: return false;
   }
 }
@@ -195,7 +199,7 @@ int launch_t(const ConvP& p, cudaStream_t st) {
     else launch_taps<T, 1, 4>(p, st);
   }
   if (p.ring && p.L > 1)
-    ring_update_kernel<T><<<dim3((p.C + kThreads - 1) / kThreads, p.L < p.taps ? p.L : p.taps, p.B), kThreads, 0, st>>>(p);
+    launch_pdl(ring_update_kernel<T>, dim3((p.C + kThreads - 1) / kThreads, p.L < p.taps ? p.L : p.taps, p.B), kThreads, 0, st, p);
   return (int)cudaGetLastError();
 }
 

@@ -107,11 +107,13 @@ __device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_ca
 // One warp per (batch, head).  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
 template <typename IO>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-swa_decode_kernel(const IO* __restrict__ q, const IO* __restrict__ k_new, const IO* __restrict__ v_new,
-                  IO* __restrict__ o, IO* __restrict__ kv_cache, const int32_t* __restrict__ cache_seqlens,
-                  int cache_seqlen_scalar, const IO* __restrict__ rcos, const IO* __restrict__ rsin, int rotary_dim,
+swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
+                  IO* o, IO* kv_cache, const int32_t* cache_seqlens,
+                  int cache_seqlen_scalar, const IO* rcos, const IO* rsin, int rotary_dim,
                   int BH, int H, int hd, int max_seqlen, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
                   int window_left, float scale) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float s_q[kWarpsPerBlock][kMaxHd];
   __shared__ float s_k[kWarpsPerBlock][kMaxHd];
   __shared__ float s_p[kWarpsPerBlock][kMaxKeysPerLane * 32];
@@ -291,6 +293,8 @@ __global__ void __launch_bounds__(256)
 rotary_qkv_cache_kernel(__nv_bfloat16* __restrict__ qkv, int L, int H, int hd, int64_t sb, int64_t sl, int64_t s3,
                         int64_t sh, const __nv_bfloat16* __restrict__ rcos, const __nv_bfloat16* __restrict__ rsin,
                         __nv_bfloat16* __restrict__ cache, int64_t cb, int64_t cl, long long total) {
+  pdl_trigger();
+  pdl_wait();
   using IO = __nv_bfloat16;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
@@ -342,7 +346,7 @@ int launch_rotary_qkv_cache(void* qkv, int B, int L, int H, int hd, int64_t sb, 
   if (total == 0) return 0;
   const long long blocks = (total + 255) / 256;
   if (blocks > 2147483647LL) return BASED_ERR_TOO_LARGE;
-  rotary_qkv_cache_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
+  launch_pdl(rotary_qkv_cache_kernel, (unsigned)blocks, 256, 0, stream, 
       static_cast<__nv_bfloat16*>(qkv), L, H, hd, sb, sl, s3, sh, static_cast<const __nv_bfloat16*>(rcos),
       static_cast<const __nv_bfloat16*>(rsin), static_cast<__nv_bfloat16*>(cache), cb, cl, total);
   return (int)cudaGetLastError();
@@ -425,12 +429,12 @@ int launch_swa_decode(const void* q, const void* k_new, const void* v_new, void*
   const int grid = (BH + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (io_dtype == BASED_BF16) {
     using T = __nv_bfloat16;
-    swa_decode_kernel<T><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
+    launch_pdl(swa_decode_kernel<T>, grid, kWarpsPerBlock * 32, 0, stream, 
         static_cast<const T*>(q), static_cast<const T*>(k_new), static_cast<const T*>(v_new), static_cast<T*>(o),
         static_cast<T*>(kv_cache), cache_seqlens, cache_seqlen_scalar, static_cast<const T*>(rotary_cos),
         static_cast<const T*>(rotary_sin), rotary_dim, BH, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
   } else if (io_dtype == BASED_F32) {
-    swa_decode_kernel<float><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
+    launch_pdl(swa_decode_kernel<float>, grid, kWarpsPerBlock * 32, 0, stream, 
         static_cast<const float*>(q), static_cast<const float*>(k_new), static_cast<const float*>(v_new),
         static_cast<float*>(o), static_cast<float*>(kv_cache), cache_seqlens, cache_seqlen_scalar,
         static_cast<const float*>(rotary_cos), static_cast<const float*>(rotary_sin), rotary_dim, BH, H, hd,

@@ -28,6 +28,8 @@ struct PrepP {
 
 template <typename T, int N, int VPT>
 __global__ void __launch_bounds__(kThreads) tied_prepare_kernel(const PrepP p) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t task = (int64_t)blockIdx.x * (kThreads / kLanes) + threadIdx.x / kLanes;
   const int lane = threadIdx.x % kLanes, heads = p.H + p.G;
   const bool live = task < p.tasks;     // every lane stays for the reductions
@@ -86,11 +88,11 @@ int launch_t(const PrepP& p, cudaStream_t st) {
   const unsigned grid = (unsigned)blocks;
   const bool vec = p.d % 8 == 0 && aligned16(p.q) && aligned16(p.k) && aligned16(p.wq) && aligned16(p.wk) && aligned16(p.cache) &&
                    p.qb % 8 == 0 && p.ql % 8 == 0 && p.kb % 8 == 0 && p.kl % 8 == 0 && p.cb % 8 == 0 && p.cl % 8 == 0;
-  if (vec && p.d <= 128) tied_prepare_kernel<T, 8, 1><<<grid, kThreads, 0, st>>>(p);
-  else if (vec && p.d <= 256) tied_prepare_kernel<T, 8, 2><<<grid, kThreads, 0, st>>>(p);
-  else if (vec && p.d <= 512) tied_prepare_kernel<T, 8, 4><<<grid, kThreads, 0, st>>>(p);
-  else if (p.d <= 128) tied_prepare_kernel<T, 1, 8><<<grid, kThreads, 0, st>>>(p);
-  else if (p.d <= 512) tied_prepare_kernel<T, 1, 32><<<grid, kThreads, 0, st>>>(p);
+  if (vec && p.d <= 128) launch_pdl(tied_prepare_kernel<T, 8, 1>, grid, kThreads, 0, st, p);
+  else if (vec && p.d <= 256) launch_pdl(tied_prepare_kernel<T, 8, 2>, grid, kThreads, 0, st, p);
+  else if (vec && p.d <= 512) launch_pdl(tied_prepare_kernel<T, 8, 4>, grid, kThreads, 0, st, p);
+  else if (p.d <= 128) launch_pdl(tied_prepare_kernel<T, 1, 8>, grid, kThreads, 0, st, p);
+  else if (p.d <= 512) launch_pdl(tied_prepare_kernel<T, 1, 32>, grid, kThreads, 0, st, p);
   else return BASED_ERR_SHAPE;
   return (int)cudaGetLastError();
 }

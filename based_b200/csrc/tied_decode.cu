@@ -64,6 +64,8 @@ __device__ __forceinline__ float weight(float m, float base) { return m == -INFI
 // d <= 16 * NK, a multiple of 16; 8 * NR rows per CTA
 template <int NK, int NR>
 __global__ void __launch_bounds__(kThreads, NK <= 4 ? 4 : (NK <= 8 ? 2 : 1)) tied_decode_kernel(const __grid_constant__ P p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   constexpr int kRows = 8 * NR;
@@ -345,7 +347,7 @@ int launch_k(const P& p, cudaStream_t st) {
   const cudaError_t e = cudaFuncSetAttribute(tied_decode_kernel<NK, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(16 * NK));
   if (e != cudaSuccess) return (int)e;
   const int rows = 8 * NR;
-  tied_decode_kernel<NK, NR><<<dim3(p.splits, (p.L * p.group + rows - 1) / rows, p.B * p.G), kThreads, smem_bytes(p.d), st>>>(p);
+  launch_pdl(tied_decode_kernel<NK, NR>, dim3(p.splits, (p.L * p.group + rows - 1) / rows, p.B * p.G), kThreads, smem_bytes(p.d), st, p);
   return (int)cudaGetLastError();
 }
 

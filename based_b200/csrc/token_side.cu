@@ -40,11 +40,14 @@ __device__ __forceinline__ void mma32(float (&c)[4], const uint4& lo, const uint
   mma16816(c, lo.x, hi.x, lo.y, hi.y, b.x, b.y);
   mma16816(c, lo.z, hi.z, lo.w, hi.w, b.z, b.w);
 }
+// weights only
 __device__ __forceinline__ uint4 load16(const bf16* p, bool ok) { return ok ? __ldg(reinterpret_cast<const uint4*>(p)) : make_uint4(0, 0, 0, 0); }
 
 // NT: projection tiles of 8 columns per warp
 template <int NT>
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) token_side_kernel(const P p) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
@@ -101,7 +104,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) tok
   for (int k0 = warp * 32; k0 < p.W; k0 += kWarps * 32) {
     const int k = k0 + t4 * 8;
     const bool ok = k < p.W;
-    const uint4 lo = load16(xa + k, ok), hi = load16(xb + k, ok);
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const uint4 lo = ok ? *reinterpret_cast<const uint4*>(xa + k) : zero, hi = ok ? *reinterpret_cast<const uint4*>(xb + k) : zero;
     uint4 w[kMaxGateTiles];
 #pragma unroll
     for (int i = 0; i < kMaxGateTiles; ++i) {
@@ -226,7 +230,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) tok
 template <int NT>
 int launch_nt(const P& p, cudaStream_t st) {
   const size_t smem = (size_t)kRows * (p.n + 8) * 2 + sizeof(float) * (kWarps * kRows * kMaxGateTiles * 8 + 2 * kCluster * kRows + kWarps * kRows);
-  token_side_kernel<NT><<<(p.M + kRows - 1) / kRows * kCluster, kThreads, smem, st>>>(p);
+  launch_pdl(token_side_kernel<NT>, (p.M + kRows - 1) / kRows * kCluster, kThreads, smem, st, p);
   return (int)cudaGetLastError();
 }
 

@@ -122,7 +122,7 @@ class BaseConv(nn.Module):
         fills the convolution state and later single-token calls step it."""
         if inference_params is not None and inference_params.seqlen_offset > 0:
             state = self.conv._get_state(inference_params)
-            if (ops.DECODE_LINEAR_USE["conv"] and ops._decode_rows(u, self.in_proj.weight)
+            if (ops._decode_rows(u, self.in_proj.weight, fused=True)
                     and state.dtype == torch.bfloat16 and state.is_contiguous()
                     and state.shape[0] == u.shape[0] and u.shape[1] == 1 and self.d_inner % 8 == 0):
                 # decode step: in_proj, the convolution step on the state, silu and the gate in one launch

@@ -8,6 +8,9 @@ from typing import Optional, Tuple
 
 import torch
 
+from torch._C._functorch import is_functorch_wrapped_tensor as _wrapped
+from torch.autograd import forward_ad as _forward_ad
+
 from . import _capi
 from ._capi import BASED_BF16, BASED_F32, IMPL_AUTO, IMPL_DECODE, IMPL_SIMT, IMPL_TCGEN05  # noqa: F401
 
@@ -432,11 +435,12 @@ def gated_act(y: torch.Tensor, activation: str = "silu", out: Optional[torch.Ten
     return out
 
 
-DECODE_LINEAR_MAX_ROWS = 64  # beyond this the library GEMM is the better tool
-# Which decode-step products the mixers and the MLP hand to decode_linear instead of cuBLAS (+ a separate
-# elementwise launch).  Measured on the 360M model at batch 16 with the weights streaming from HBM
-# (ms per decode step): none 1.146, gated 1.089, gated + conv 1.145, all three 1.329 -- only fc1 + SwiGLU pays.
-DECODE_LINEAR_USE = {"plain": False, "gated": True, "conv": False}
+# Where a product goes to decode_linear; beyond, the library GEMM is the better tool.  us a launch in a chain of such launches with
+# the weights from HBM, cuBLAS / ours (N x K, rows): 1024 x 1024 4.6 / 2.9 (16), 4.2 / 3.6 (32); 4096 x 1024 4.7 / 3.1, 4.8 / 4.3,
+# 4.8 / 8.3 (64); 1024 x 3072 8.6 / 3.5, 7.2 / 5.3; 1792 x 1792 5.2 / 3.6, 5.2 / 5.8; 7168 x 1792 7.4 / 6.9, 7.5 / 8.0, with the gated
+# activation 9.9 / 7.0, 9.9 / 8.5; 50280 x 1024 21 / 30.  So: up to 16 rows whatever K; up to 32 for a short K, for few enough
+# outputs that every block of the kernel has an SM, and where the epilogue saves a launch.
+DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_OUTPUTS = 32, 8192
 
 
 def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, *,
@@ -444,7 +448,7 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
                   conv_weight: Optional[torch.Tensor] = None, conv_bias: Optional[torch.Tensor] = None,
                   out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x W^T (+ bias)`` for the few rows of a decode step (bf16), with a fused epilogue:
-    ``"plain"``; ``"gated"`` -> ``first_half * act(second_half)`` (mlp.py:146-154); ``"conv"`` -> the BaseConv
+    ``"plain"``; ``"f32"``: plain with an fp32 result; ``"gated"`` -> ``first_half * act(second_half)`` (mlp.py:146-154); ``"conv"`` -> the BaseConv
     decode step on the first half (``conv_state [M, N/2, k]`` updated in place), silu, gate by the second half
     (convolution.py:88-109, :205-211).  x ``[..., K]``; returns ``[..., N]`` or ``[..., N/2]``."""
     _need_cuda(x, weight, bias, conv_state, conv_weight, conv_bias)
@@ -456,9 +460,12 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
     M, N = x2.shape[0], weight.shape[0]
     if weight.shape[1] != K or not weight.is_contiguous():
         raise ValueError("weight must be a contiguous [N, K] tensor")
-    epi = {"plain": 0, "gated": 1, "conv": 2}[epilogue]
-    n_out = N if epi == 0 else N // 2
-    out = torch.empty(M, n_out, dtype=torch.bfloat16, device=x.device) if out is None else _rows(out, n_out)
+    epi = {"plain": 0, "gated": 1, "conv": 2, "f32": 3}[epilogue]
+    n_out = N // 2 if epi in (1, 2) else N
+    dtype = torch.float32 if epi == 3 else torch.bfloat16
+    out = torch.empty(M, n_out, dtype=dtype, device=x.device) if out is None else _rows(out, n_out)
+    if out.dtype != dtype:
+        raise TypeError(f"out must be {dtype}")
     if bias is not None:
         bias = bias.to(torch.bfloat16).contiguous()
     ck, cw_dt = 0, BASED_BF16
@@ -479,17 +486,31 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
     return out.reshape(*x.shape[:-1], n_out)
 
 
-def _decode_rows(x: torch.Tensor, weight: torch.Tensor) -> bool:
-    """True when ``x W^T`` is a decode-step product the library's own kernel should run."""
-    rows = x.numel() // x.shape[-1] if x.numel() else 0
-    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and 0 < rows <= DECODE_LINEAR_MAX_ROWS
-            and x.shape[-1] % 32 == 0 and weight.shape[0] % 8 == 0 and weight.is_contiguous() and x.stride(-1) == 1
-            and not torch.is_grad_enabled())
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> bool:
+    """True when ``x W^T`` is a decode-step product the library's own kernel should run: a few bf16 rows in a layout it takes, and
+    nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing).
+    ``fused``: its epilogue takes the place of another launch."""
+    K = x.shape[-1] if x.dim() else 0
+    if not (0 < x.numel() <= K * DECODE_LINEAR_MAX_ROWS and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16):
+        return False
+    if type(x) is not torch.Tensor or type(weight) not in _PLAIN_TYPES or weight.dim() != 2 or weight.shape[0] > DECODE_LINEAR_MAX_OUTPUTS:
+        return False
+    if x.numel() > 16 * K and not (K <= 1024 or (weight.shape[0] <= 8 * 148 and K <= 3072) or (fused and K <= 2048)):
+        return False
+    return (K % 32 == 0 and weight.shape[1] == K and weight.shape[0] % 8 == 0 and weight.is_contiguous()
+            and (x.is_contiguous() or (x.stride(-1) == 1 and all(st % 8 == 0 for st in x.stride()[:-1])))
+            and x.device == weight.device and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+            and _forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
+            and not _wrapped(x) and not _wrapped(weight) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``nn.functional.linear`` for the mixers: the decode-step kernel for a few bf16 rows, cuBLAS otherwise."""
-    if DECODE_LINEAR_USE["plain"] and _decode_rows(x, weight):
+    if _decode_rows(x, weight) and (bias is None or (type(bias) in _PLAIN_TYPES and bias.dtype == torch.bfloat16
+                                                     and bias.shape == weight.shape[:1] and bias.device == x.device)):
         return decode_linear(x, weight, bias)
     return torch.nn.functional.linear(x, weight, bias)
 
@@ -599,6 +620,8 @@ def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     _need_cuda(x, weight)
     if x.dtype == torch.float32:
         return torch.nn.functional.linear(x, weight)
+    if _decode_rows(x, weight):
+        return decode_linear(x, weight, epilogue="f32")
     y = torch.mm(x.reshape(-1, x.shape[-1]), weight.t(), out_dtype=torch.float32)
     return y.view(*x.shape[:-1], weight.shape[0])
 
@@ -997,6 +1020,7 @@ def token_gate(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, colum
     return out
 
 
+TOKEN_SIDE_MAX_ROWS = 64
 TOKEN_SIDE_MAX_WEIGHT = 200_000   # elements of one matrix up to which one cluster per 16 rows beats the separate launches
 
 
@@ -1008,7 +1032,7 @@ def token_side_step(residual: torch.Tensor, x: torch.Tensor, tokens: torch.Tenso
     _need_cuda(residual, x, tokens, gate_weight, proj_weight, table, norm_weight, out_weight)
     n, W = gate_weight.shape
     M = x.numel() // W if W else 0
-    if x.dtype != torch.bfloat16 or not 0 < M <= DECODE_LINEAR_MAX_ROWS or n * W > TOKEN_SIDE_MAX_WEIGHT:
+    if x.dtype != torch.bfloat16 or not 0 < M <= TOKEN_SIDE_MAX_ROWS or n * W > TOKEN_SIDE_MAX_WEIGHT:
         return None
     _same_dtype(x, x=x, gate_weight=gate_weight, proj_weight=proj_weight, table=table, norm_weight=norm_weight, out_weight=out_weight)
     x2 = flat_rows(x)

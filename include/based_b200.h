@@ -333,6 +333,7 @@ int based_rotary_qkv_cache(void* qkv, int B, int L, int H, int hd, const int64_t
 #define BASED_EPI_PLAIN 0  /* out[M, N]   = x W^T + bias */
 #define BASED_EPI_GATED 1  /* out[M, N/2] = (x W1^T + b1) * act(x W2^T + b2), W = [W1; W2], act as in based_gated_act */
 #define BASED_EPI_CONV 2   /* out[M, N/2] = silu(conv_step(u1)) * u2 with [u1 | u2] = x W^T + bias */
+#define BASED_EPI_F32 3    /* as PLAIN, out in fp32 */
 
 /*
  * A linear layer on the few rows of a decode step (one token per sequence), bf16, with the
@@ -347,10 +348,10 @@ int based_rotary_qkv_cache(void* qkv, int B, int L, int H, int hd, const int64_t
  *          conv_bias [N/2] (or NULL) are in conv_w_dtype
  * which the reference runs as separate cuBLAS and elementwise launches.
  *
- *   x [M, K], W [N, K] (nn.Linear layout, contiguous), bias [N] or NULL, out as above; all bf16;
+ *   x [M, K], W [N, K] (nn.Linear layout, contiguous), bias [N] or NULL, out as above; all bf16 (but F32's out);
  *   row strides in elements.  K a multiple of 32; the number of outputs a multiple of 8;
- *   x and W 16-byte aligned, x_row_stride a multiple of 8.  Built for M <= 16 (weights are read
- *   once per 16 rows); larger M works and re-reads W from L2 per 16 rows.
+ *   x and W 16-byte aligned, x_row_stride a multiple of 8.  Built for M <= 32 (weights are read
+ *   once per 32 rows); larger M works and re-reads W from L2 per 32 rows.
  */
 int based_decode_linear(const void* x, const void* w, const void* bias, void* out,
                         int M, int N, int K, int64_t x_row_stride, int64_t out_row_stride,

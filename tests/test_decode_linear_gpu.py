@@ -82,3 +82,51 @@ def test_decode_linear_rejects_what_it_cannot_run(ops):
         ops.decode_linear(torch.randn(4, 64, device="cuda").bfloat16(), torch.randn(12, 64, device="cuda").bfloat16())
     with pytest.raises(TypeError):
         ops.decode_linear(torch.randn(4, 64, device="cuda"), torch.randn(16, 64, device="cuda"))
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33])
+@pytest.mark.parametrize("N,K", [(8 * 148, 1056), (8 * 149, 2048), (8 * 297, 64), (8 * 593, 96), (8 * 1189, 32)])
+def test_decode_linear_tilings(ops, M, N, K):
+    """Where the number of column tiles per block, of row tiles and of warps changes, with a last block that is not full; every
+    epilogue, outputs against the sum in 64 bits to their last rounding plus the sum's own in fp32."""
+    x, w, b = _mk(M, N, K, M + N + K, True)
+    ref = x.double() @ w.double().T
+    xd, wd, bd = x.cuda(), w.cuda(), b.cuda()
+    f32 = ops.decode_linear(xd, wd, epilogue="f32")
+    assert f32.dtype == torch.float32 and rel_err(f32.cpu(), ref) < 1e-5
+    y = ops.decode_linear(xd, wd, bd)
+    assert rel_err(y.cpu().double(), ref + b.double()) < 2 ** -8
+    w2 = torch.cat([w, w.flip(0)])
+    u = (torch.cat([ref, ref.flip(1)], 1) + torch.cat([b, b]).double()).bfloat16().double()
+    got = ops.decode_linear(xd, w2.cuda(), torch.cat([bd, bd]), epilogue="gated")
+    assert rel_err(got.cpu().double(), O.gated_act(u, "silu")) < 2e-2
+    g = torch.Generator().manual_seed(N)
+    state, cw = torch.randn(M, N, 8, generator=g).bfloat16(), (torch.randn(N, 8, generator=g) * 0.3).bfloat16()
+    st = state.cuda()
+    want_state = state.double()
+    want = O.gated_conv_step(u, want_state, cw.double(), None)
+    got = ops.decode_linear(xd, w2.cuda(), torch.cat([bd, bd]), epilogue="conv", conv_state=st, conv_weight=cw.cuda())
+    assert rel_err(got.cpu().double(), want) < 2e-2 and torch.equal(st[..., :-1].cpu(), state[..., 1:])
+
+
+def test_linear_takes_the_kernel_only_where_it_can(ops):
+    """Layouts, alignments and surroundings that the kernel does not serve give what torch gives."""
+    import torch.nn.functional as F
+    w = (torch.randn(64, 96, device="cuda") / 10).bfloat16()
+    buf = torch.randn(4 * 200 + 8, device="cuda").bfloat16()
+    odd = [buf[1:1 + 4 * 96].view(4, 96), buf[:4 * 100].view(4, 100)[:, :96], buf[:4 * 96].view(96, 4).t(), buf[:96], buf[:96].expand(3, 96),
+           buf[:4 * 192].view(4, 192)[:, ::2]]
+    with torch.no_grad():
+        for x in odd:
+            assert rel_err(ops.linear(x, w).float().cpu(), F.linear(x.float(), w.float()).cpu()) < 2 ** -7
+        assert rel_err(ops.linear(odd[3], w[1:, :].contiguous()).float().cpu(), F.linear(odd[3].float(), w[1:].float()).cpu()) < 2 ** -7
+        x = buf[:4 * 96].view(4, 96)
+        assert torch.equal(torch.func.vmap(lambda r: ops.linear(r, w))(x), torch.func.vmap(lambda r: F.linear(r, w))(x))
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert ops.linear(x, w).dtype == torch.float16
+        with torch.autograd.forward_ad.dual_level():
+            d = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+            assert torch.autograd.forward_ad.unpack_dual(ops.linear(d, w)).tangent is not None
+    xg = x.clone().requires_grad_()
+    ops.linear(xg, w).sum().backward()
+    assert xg.grad is not None
