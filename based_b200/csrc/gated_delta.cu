@@ -139,9 +139,11 @@ struct StepP {
 template <typename T, int NR>
 __global__ void __launch_bounds__(kThreads, NR <= 8 ? 3 : NR <= 16 ? 2 : 1) delta_step_kernel(const StepP p) {
   pdl_trigger();
-  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  // this CTA's state into L2 before the kernel ahead has ended, a row per thread (dv is a multiple of 4, the state aligned)
+  for (int i = tid; i < p.d; i += kThreads) prefetch_l2(p.state + (((int64_t)b * p.H + h) * p.d + i) * p.dv, p.dv * 4);
+  pdl_wait();
   const int hk = h / (p.H / p.Hk);
   const int d = p.d, dv = p.dv, C4 = dv / 4, R = kThreads / C4;
   const int c4 = tid % C4, rg = tid / C4;

@@ -107,9 +107,12 @@ struct StepP {
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, V <= 8 ? 3 : 2) lightning_step_kernel(const StepP p) {
   pdl_trigger();
-  pdl_wait();
   extern __shared__ float sm[];
   const int h = blockIdx.x, b = blockIdx.y, col0 = blockIdx.z * p.cols, tid = threadIdx.x;
+  // this CTA's state into L2 before the kernel ahead has ended
+  if (p.cols % 4 == 0 && p.dv % 4 == 0)
+    for (int i = tid; i < p.d; i += kThreads) prefetch_l2(p.state + (((int64_t)b * p.H + h) * p.d + i) * p.dv + col0, p.cols * 4);
+  pdl_wait();
   const int quads = p.cols / 4, R = kThreads / quads, row4 = p.dv / 4;
   const int c = tid % quads, rg = tid / quads;
   const bool mine = rg < R;

@@ -62,6 +62,10 @@ linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
                       IO* y, ST* kv_state, ST* k_state,
                       int H, int dv, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 sy, float eps) {
   pdl_trigger();
+  if (kThreads > 192) {   // few blocks: their state into L2 before the kernel ahead has ended, a whole number of 16-byte vectors
+    const uint32_t bytes = dv * kExpandedDim * sizeof(ST), piece = ((bytes + kThreads - 1) / kThreads + 15) & ~15u, at = threadIdx.x * piece;
+    if (at < bytes) prefetch_l2(reinterpret_cast<const char*>(kv_state) + (size_t)blockIdx.x * bytes + at, min(piece, bytes - at));
+  }
   pdl_wait();
   using VO = VecOps<ST>;
   constexpr int VEC = VO::kVec;
@@ -81,6 +85,16 @@ linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
   const int bh = blockIdx.x;
   const int b = bh / H, h = bh - b * H;
 
+  // a warp's first rows of the state are in flight while the feature tables are built
+  const int ngroups = dv / RPG;
+  uint4 r[kIters];
+  auto fetch = [&](int g) {
+    const uint4* base = reinterpret_cast<const uint4*>(kv_state + ((size_t)bh * dv + (size_t)g * RPG) * kExpandedDim);
+#pragma unroll
+    for (int n = 0; n < kIters; ++n)
+      if (lane + 32 * n < kVecPerGroup) r[n] = __ldcs(base + lane + 32 * n);
+  };
+  if (kThreads > 192 && warp < ngroups) fetch(warp);
   if (tid < kFeatureDim) {
     s_x[0][tid] = to_float(q[b * sq.b + h * sq.h + tid]);
   } else if (tid < 2 * kFeatureDim) {
@@ -117,15 +131,9 @@ linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
     if (lane == 0) s_den = den;
   }
 
-  const int ngroups = dv / RPG;
   for (int g = warp; g < ngroups; g += kWarps) {
     uint4* base = reinterpret_cast<uint4*>(kv_state + ((size_t)bh * dv + (size_t)g * RPG) * kExpandedDim);
-    uint4 r[kIters];
-#pragma unroll
-    for (int n = 0; n < kIters; ++n) {
-      const int idx = lane + 32 * n;
-      if (idx < kVecPerGroup) r[n] = __ldcs(base + idx);
-    }
+    if (kThreads <= 192 || g != warp) fetch(g);
     float acc[RPG];
 #pragma unroll
     for (int rr = 0; rr < RPG; ++rr) acc[rr] = 0.f;

@@ -72,165 +72,181 @@ swa_prefill_simt_kernel(const IO* __restrict__ q, const IO* __restrict__ k, cons
   }
 }
 
-// dot product of a cached key row with the query held in shared memory (fp32); 16-byte loads
-__device__ __forceinline__ float dot_row(const __nv_bfloat16* kc, const float* sq, int hd) {
-  float dot = 0.f;
-  for (int c = 0; c < hd; c += 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(kc + c);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+// 8 consecutive values of a cached row
+struct Row8 {
+  float x[8];
+};
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, uint4 (&r)[1]) { r[0] = *reinterpret_cast<const uint4*>(p); }
+__device__ __forceinline__ void load8(const float* p, uint4 (&r)[2]) {
+  r[0] = *reinterpret_cast<const uint4*>(p);
+  r[1] = *reinterpret_cast<const uint4*>(p + 4);
+}
+__device__ __forceinline__ Row8 unpack8(const uint4 (&r)[1]) {
+  const uint32_t w[4] = {r[0].x, r[0].y, r[0].z, r[0].w};
+  Row8 y;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      dot = fmaf(sq[c + 2 * i], __uint_as_float(w[i] << 16), dot);
-      dot = fmaf(sq[c + 2 * i + 1], __uint_as_float(w[i] & 0xFFFF0000u), dot);
-    }
+  for (int i = 0; i < 4; ++i) {
+    y.x[2 * i] = __uint_as_float(w[i] << 16);
+    y.x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
   }
-  return dot;
+  return y;
 }
-__device__ __forceinline__ float dot_row(const float* kc, const float* sq, int hd) {
-  float dot = 0.f;
-  for (int c = 0; c < hd; c += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(kc + c);
-    dot = fmaf(sq[c], v.x, dot);
-    dot = fmaf(sq[c + 1], v.y, dot);
-    dot = fmaf(sq[c + 2], v.z, dot);
-    dot = fmaf(sq[c + 3], v.w, dot);
-  }
-  return dot;
+__device__ __forceinline__ Row8 unpack8(const uint4 (&r)[2]) {
+  return Row8{{__uint_as_float(r[0].x), __uint_as_float(r[0].y), __uint_as_float(r[0].z), __uint_as_float(r[0].w),
+               __uint_as_float(r[1].x), __uint_as_float(r[1].y), __uint_as_float(r[1].z), __uint_as_float(r[1].w)}};
 }
-// two adjacent value columns of a cached row
-__device__ __forceinline__ float2 load2(const __nv_bfloat16* p) {
-  const uint32_t w = *reinterpret_cast<const uint32_t*>(p);
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
-}
-__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
-// One warp per (batch, head).  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
-template <typename IO>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+// One block per (batch, head).  A step's bytes (a window of keys and values, 16 KB a head) take less than a microsecond; what
+// it takes is the chain load - scores - softmax - values.  So the window is spread over the block: LPK lanes share a cached
+// row, 8 values (16 or 32 bytes) each, a group of lanes has every (32 / LPK * WARPS)-th key, and its first four keys AND values
+// are in flight before the query is rotated.  Each group keeps a running maximum, sum and weighted row of its own keys; the
+// groups meet once at the end.  16 heads, 16 rows, hd = 64, 64 keys: 10.6 us with one warp per head (keys, softmax, values in
+// turn), @SWA@ us like this.  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
+template <typename IO, int LPK, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
                   IO* o, IO* kv_cache, const int32_t* cache_seqlens,
                   int cache_seqlen_scalar, const IO* rcos, const IO* rsin, int rotary_dim,
-                  int BH, int H, int hd, int max_seqlen, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
+                  int H, int hd, int max_seqlen, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
                   int window_left, float scale) {
   pdl_trigger();
   pdl_wait();
-  __shared__ float s_q[kWarpsPerBlock][kMaxHd];
-  __shared__ float s_k[kWarpsPerBlock][kMaxHd];
-  __shared__ float s_p[kWarpsPerBlock][kMaxKeysPerLane * 32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int bh = blockIdx.x * kWarpsPerBlock + warp;
-  if (bh >= BH) return;
-  const int b = bh / H, h = bh - b * H;
+  constexpr int kGroups = WARPS * 32 / LPK, U = 4, kVec = sizeof(IO) / 2;
+  __shared__ float s_q[kMaxHd], s_k[kMaxHd], s_v[kMaxHd], s_r[2][kMaxHd];
+  __shared__ float s_o[WARPS][kMaxHd], s_m[WARPS], s_l[WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.x / H, h = blockIdx.x - b * H;
   const int pos = cache_seqlens ? cache_seqlens[b] : cache_seqlen_scalar;
   if (pos < 0 || pos >= max_seqlen) return;  // nothing sensible to do; the host validates the scalar case
+  const size_t row = (size_t)2 * H * hd;  // elements per cached position
+  IO* cache_b = kv_cache + (size_t)b * max_seqlen * row;
+  const int lo = max(0, pos - window_left), old = pos - lo;   // cached keys; the new one comes on top
+  const int group = tid / LPK, c = 8 * (tid % LPK);
+  const bool on = c < hd;
+  const IO* kc = cache_b + (size_t)lo * row + (size_t)h * hd + c;
+  uint4 kx[U][kVec], vx[U][kVec];
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = j0 + u * kGroups + group;
+      if (on && j < old) {
+        load8(kc + (size_t)j * row, kx[u]);
+        load8(kc + (size_t)j * row + (size_t)H * hd, vx[u]);
+      }
+    }
+  };
+  fetch(0);
+  // the new token: RoPE in fp32, result rounded to the I/O dtype like the reference kernel's store, and its row of the cache
   const IO* qp = q + b * sq.b + h * sq.h;
   const IO* kp = k_new + b * sk.b + h * sk.h;
   const IO* vp = v_new + b * sv.b + h * sv.h;
-  for (int c = lane; c < hd; c += 32) {
-    s_q[warp][c] = to_float(qp[c]);
-    s_k[warp][c] = to_float(kp[c]);
+  for (int i = tid; i < hd; i += WARPS * 32) {
+    s_r[0][i] = to_float(qp[i]);
+    s_r[1][i] = to_float(kp[i]);
+    s_v[i] = to_float(vp[i]);
   }
-  __syncwarp();
-  const size_t row = (size_t)2 * H * hd;  // elements per cached position
-  IO* cache_b = kv_cache + (size_t)b * max_seqlen * row;
-  IO* knew = cache_b + (size_t)pos * row + (size_t)h * hd;
-  IO* vnew = knew + (size_t)H * hd;
-  // RoPE in fp32, result rounded to the I/O dtype like the reference kernel's store.
+  __syncthreads();
   const int half = rcos ? rotary_dim / 2 : 0;
-  float qr[kMaxHd / 32], kr[kMaxHd / 32];
-#pragma unroll
-  for (int n = 0; n < kMaxHd / 32; ++n) {
-    const int c = lane + 32 * n;
-    if (c < hd) {
-      float qv = s_q[warp][c], kv = s_k[warp][c];
-      if (c < 2 * half) {
-        const int cc = c < half ? c : c - half;
-        const float cs = to_float(rcos[(size_t)pos * half + cc]);
-        const float sn = to_float(rsin[(size_t)pos * half + cc]);
-        if (c < half) {
-          qv = s_q[warp][c] * cs - s_q[warp][c + half] * sn;
-          kv = s_k[warp][c] * cs - s_k[warp][c + half] * sn;
-        } else {
-          qv = s_q[warp][c - half] * sn + s_q[warp][c] * cs;
-          kv = s_k[warp][c - half] * sn + s_k[warp][c] * cs;
-        }
-      }
-      qr[n] = to_float(from_float<IO>(qv));
-      kr[n] = to_float(from_float<IO>(kv));
+  for (int i = tid; i < 2 * hd; i += WARPS * 32) {
+    const int which = i >= hd, cc = which ? i - hd : i;
+    const float* x = s_r[which];
+    float y = x[cc];
+    if (cc < 2 * half) {
+      const int a = cc < half ? cc : cc - half;
+      const float cs = to_float(rcos[(size_t)pos * half + a]), sn = to_float(rsin[(size_t)pos * half + a]);
+      y = cc < half ? x[cc] * cs - x[cc + half] * sn : x[cc - half] * sn + x[cc] * cs;
+    }
+    const IO r = from_float<IO>(y);
+    (which ? s_k : s_q)[cc] = to_float(r);
+    if (which) {
+      IO* knew = cache_b + (size_t)pos * row + (size_t)h * hd;
+      knew[cc] = r;
+      knew[(size_t)H * hd + cc] = vp[cc];
     }
   }
-  __syncwarp();
+  __syncthreads();
+  float qv[8], acc[8], m = -INFINITY, l = 0.f;
 #pragma unroll
-  for (int n = 0; n < kMaxHd / 32; ++n) {
-    const int c = lane + 32 * n;
-    if (c < hd) {
-      s_q[warp][c] = qr[n];
-      knew[c] = from_float<IO>(kr[n]);
-      vnew[c] = vp[c];
+  for (int i = 0; i < 8; ++i) { qv[i] = on ? s_q[c + i] : 0.f; acc[i] = 0.f; }
+  auto score = [&](const Row8& x) {
+    float d = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d = fmaf(qv[i], x.x[i], d);
+#pragma unroll
+    for (int x2 = LPK / 2; x2 > 0; x2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, x2);
+    return d * scale;
+  };
+  auto take = [&](const float (&sc)[U], const Row8 (&x)[U]) {   // scores of -inf stand for no key
+    float top = m;
+#pragma unroll
+    for (int u = 0; u < U; ++u) top = fmaxf(top, sc[u]);
+    const float base = top == -INFINITY ? 0.f : top, f = __expf(m - base);
+    m = top;
+    l *= f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float w = __expf(sc[u] - base);
+      l += w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(w, x[u].x[i], acc[i]);
     }
+  };
+  const Row8 none{};
+  for (int j0 = 0; j0 < old; j0 += U * kGroups) {
+    if (j0 > 0) fetch(j0);
+    float sc[U];
+    Row8 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool live = j0 + u * kGroups + group < old;
+      const float d = score(on && live ? unpack8(kx[u]) : none);
+      sc[u] = live ? d : -INFINITY;
+      x[u] = on && live ? unpack8(vx[u]) : none;
+    }
+    take(sc, x);
   }
-  __syncwarp();  // orders this warp's cache writes before its reads below
-  const int lo = max(0, pos - window_left);
-  const int nk = pos - lo + 1;
-  float sc[kMaxKeysPerLane];
-  float m = -INFINITY;
+  {  // the new key belongs to the first group
+    Row8 x = none, y = none;
+    if (on)
 #pragma unroll
-  for (int n = 0; n < kMaxKeysPerLane; ++n) {
-    const int jj = lane + 32 * n;
-    sc[n] = -INFINITY;
-    if (jj < nk) {
-      const IO* kc = cache_b + (size_t)(lo + jj) * row + (size_t)h * hd;
-      sc[n] = dot_row(kc, s_q[warp], hd) * scale;
-      m = fmaxf(m, sc[n]);
-    }
+      for (int i = 0; i < 8; ++i) { x.x[i] = s_k[c + i]; y.x[i] = s_v[c + i]; }
+    const float d = score(x), ninf = -INFINITY;
+    const float sc[U] = {group == 0 ? d : ninf, ninf, ninf, ninf};
+    const Row8 v[U] = {group == 0 ? y : none, none, none, none};
+    take(sc, v);
   }
-  m = warp_max(m);
-  float sum = 0.f;
+  // groups of a warp, then the warps
+  float top = m;
 #pragma unroll
-  for (int n = 0; n < kMaxKeysPerLane; ++n) {
-    const int jj = lane + 32 * n;
-    if (jj < nk) {
-      const float p = __expf(sc[n] - m);
-      s_p[warp][jj] = p;
-      sum += p;
-    }
+  for (int x = LPK; x < 32; x <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
+  float f = m == -INFINITY ? 0.f : __expf(m - top);
+  l *= f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] *= f;
+#pragma unroll
+  for (int x = LPK; x < 32; x <<= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], x);
   }
-  sum = warp_sum(sum);
-  __syncwarp();
-  const float inv = 1.f / sum;
-  // a lane owns two adjacent value columns; sixteen (then four) rows per round so that their loads overlap
-  for (int c = 2 * lane; c < hd; c += 64) {
-    const IO* vc = cache_b + (size_t)lo * row + (size_t)(H + h) * hd + c;
-    float a0 = 0.f, a1 = 0.f;
-    int jj = 0;
-    for (; jj + 16 <= nk; jj += 16) {  // sixteen rows in flight: the loop is latency-bound
-      float2 x[16];
+  if (lane < LPK && on)
 #pragma unroll
-      for (int u = 0; u < 16; ++u) x[u] = load2(vc + (size_t)(jj + u) * row);
+    for (int i = 0; i < 8; ++i) s_o[warp][c + i] = acc[i];
+  if (lane == 0) { s_m[warp] = top; s_l[warp] = l; }
+  __syncthreads();
+  for (int i = tid; i < hd; i += WARPS * 32) {
+    float mm = s_m[0], sum = 0.f, y = 0.f;
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        a0 = fmaf(s_p[warp][jj + u], x[u].x, a0);
-        a1 = fmaf(s_p[warp][jj + u], x[u].y, a1);
-      }
+    for (int w = 1; w < WARPS; ++w) mm = fmaxf(mm, s_m[w]);
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float g = s_m[w] == -INFINITY ? 0.f : __expf(s_m[w] - mm);
+      sum = fmaf(g, s_l[w], sum);
+      y = fmaf(g, s_o[w][i], y);
     }
-    for (; jj + 4 <= nk; jj += 4) {
-      float2 x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = load2(vc + (size_t)(jj + u) * row);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a0 = fmaf(s_p[warp][jj + u], x[u].x, a0);
-        a1 = fmaf(s_p[warp][jj + u], x[u].y, a1);
-      }
-    }
-    for (; jj < nk; ++jj) {
-      const float2 x = load2(vc + (size_t)jj * row);
-      a0 = fmaf(s_p[warp][jj], x.x, a0);
-      a1 = fmaf(s_p[warp][jj], x.y, a1);
-    }
-    IO* op = o + b * so.b + h * so.h + c;
-    op[0] = from_float<IO>(a0 * inv);
-    op[1] = from_float<IO>(a1 * inv);
+    o[b * so.b + h * so.h + i] = from_float<IO>(y * (1.f / sum));
   }
 }
 
@@ -425,24 +441,18 @@ int launch_swa_decode(const void* q, const void* k_new, const void* v_new, void*
                       cudaStream_t stream) {
   if (window_left + 1 > kMaxKeysPerLane * 32) return BASED_ERR_TOO_LARGE;
   if (!aligned16(kv_cache) || hd % 8 != 0) return BASED_ERR_ALIGN;  // 16-byte reads of cached rows
-  const int BH = B * H;
-  const int grid = (BH + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  if (io_dtype == BASED_BF16) {
-    using T = __nv_bfloat16;
-    launch_pdl(swa_decode_kernel<T>, grid, kWarpsPerBlock * 32, 0, stream, 
+  if ((int64_t)B * H > 0x7fffffff) return BASED_ERR_TOO_LARGE;
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    auto kern = hd <= 64 ? swa_decode_kernel<T, 8, 4> : swa_decode_kernel<T, 16, 8>;   // 64 keys in the first round either way
+    return launch_pdl(kern, dim3(B * H), dim3(hd <= 64 ? 128 : 256), 0, stream,
         static_cast<const T*>(q), static_cast<const T*>(k_new), static_cast<const T*>(v_new), static_cast<T*>(o),
         static_cast<T*>(kv_cache), cache_seqlens, cache_seqlen_scalar, static_cast<const T*>(rotary_cos),
-        static_cast<const T*>(rotary_sin), rotary_dim, BH, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
-  } else if (io_dtype == BASED_F32) {
-    launch_pdl(swa_decode_kernel<float>, grid, kWarpsPerBlock * 32, 0, stream, 
-        static_cast<const float*>(q), static_cast<const float*>(k_new), static_cast<const float*>(v_new),
-        static_cast<float*>(o), static_cast<float*>(kv_cache), cache_seqlens, cache_seqlen_scalar,
-        static_cast<const float*>(rotary_cos), static_cast<const float*>(rotary_sin), rotary_dim, BH, H, hd,
-        max_seqlen, sq, sk, sv, so, window_left, scale);
-  } else {
-    return BASED_ERR_DTYPE;
-  }
-  return (int)cudaGetLastError();
+        static_cast<const T*>(rotary_sin), rotary_dim, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
+  };
+  if (io_dtype == BASED_BF16) return run(__nv_bfloat16{});
+  if (io_dtype == BASED_F32) return run(float{});
+  return BASED_ERR_DTYPE;
 }
 
 }  // namespace based

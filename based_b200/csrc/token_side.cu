@@ -47,11 +47,20 @@ __device__ __forceinline__ uint4 load16(const bf16* p, bool ok) { return ok ? __
 template <int NT>
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) token_side_kernel(const P p) {
   pdl_trigger();
-  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
   const int rank = (int)cluster.block_rank(), row0 = (blockIdx.x / kCluster) * kRows;
+  // this CTA's weights into L2 before the kernel ahead has ended: a row of the gate or of the projection per thread
+  for (int i = tid; i < kMaxGateTiles * 8; i += kThreads) {
+    const int t = rank + (i >> 3) * kCluster;
+    if (t < p.n / 8) prefetch_l2(p.wg + (int64_t)(t * 8 + (i & 7)) * p.W, p.W * 2);
+  }
+  for (int i = tid; i < kWarps * NT * 8; i += kThreads) {
+    const int r = rank * kWarps * NT * 8 + i;
+    if (r < p.W) prefetch_l2(p.wp + (int64_t)r * p.n, p.n * 2);
+  }
+  pdl_wait();
   const int ldg = p.n + 8;                                                    // rows of G: an odd number of 16-byte units
   bf16* G = reinterpret_cast<bf16*>(smem);                                    // [16][ldg]
   float* part = reinterpret_cast<float*>(smem + kRows * ldg * 2);             // [warps][16][kMaxGateTiles * 8]
@@ -61,11 +70,6 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads) tok
   const int tile0 = (rank * kWarps + warp) * NT;                              // this warp's projection tiles
 
   auto started = cluster.barrier_arrive();   // the others' shared memory is written below
-  // weights of the projection into L2
-  for (int i = lane; i < NT * 8 * ((p.n + 63) / 64); i += 32) {
-    const int r = i % (NT * 8), c = i / (NT * 8), row = tile0 * 8 + r;
-    if (row < p.W) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.wp + (int64_t)row * p.n + c * 64));
-  }
   // the token vectors' values this thread will multiply by
   constexpr int ldp = kMaxGateTiles * 8, kMine = kRows * ldp / kThreads;
   float ev[kMine];
