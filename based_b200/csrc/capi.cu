@@ -555,6 +555,19 @@ int based_rglru(const void* u, const void* y, const void* gates, const void* r_b
                       static_cast<cudaStream_t>(stream));
 }
 
+int based_rglru_step(const void* x, const void* y, const void* conv_weight, const void* conv_bias, void* ring,
+                     const void* gate_weight, const void* r_bias, const void* i_bias, const void* lam, void* state, void* out,
+                     int B, int W, int block_width, int taps, int64_t x_row_stride, int64_t y_row_stride, int64_t out_row_stride,
+                     const int32_t* offsets, int offset, void* stream) {
+  if (!x || !y || !conv_weight || !ring || !gate_weight || !r_bias || !i_bias || !lam || !state || !out) return BASED_ERR_NULL;
+  if (B < 0 || W <= 0 || block_width <= 0 || W % block_width || taps < 1 || offset < 0) return BASED_ERR_SHAPE;
+  if (B == 0) return BASED_OK;
+  if (!launch_rglru_step) return BASED_ERR_IMPL;
+  return launch_rglru_step(x, y, conv_weight, conv_bias, ring, gate_weight, r_bias, i_bias, static_cast<const float*>(lam),
+                           static_cast<float*>(state), out, B, W, block_width, taps, x_row_stride, y_row_stride, out_row_stride,
+                           offsets, offset, static_cast<cudaStream_t>(stream));
+}
+
 int based_rglru_gated(const void* u, const void* y, const void* gate_weight, const void* r_bias, const void* i_bias,
                       const void* lam, void* state, void* out, int B, int L, int W, int block_width,
                       const int64_t u_strides[2], const int64_t y_strides[2], const int64_t out_strides[2],

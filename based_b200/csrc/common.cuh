@@ -206,6 +206,10 @@ BASED_WEAK int launch_delta_step(const void* x, const void* conv_w, void* ring, 
                       const float* dt_bias, const void* norm_w, float* state, void* out, int B, int H, int Hk, int d,
                       int dv, int taps, int64_t sx, int64_t sg, int64_t so, const int32_t* offsets, int offset, float eps,
                       int io_dtype, cudaStream_t stream);
+BASED_WEAK int launch_rglru_step(const void* x, const void* y, const void* cw, const void* cb, void* ring, const void* gw,
+                                 const void* rb, const void* ib, const float* lam, float* state, void* out, int B, int W, int n,
+                                 int taps, int64_t sx, int64_t sy, int64_t so, const int32_t* offsets, int offset,
+                                 cudaStream_t stream);
 BASED_WEAK int launch_rglru(const void* u, const void* y, const float* gates, const void* rb, const void* ib, const float* lam,
                  float* state, void* out, int B, int L, int W, int bw, Strides2 su, Strides2 sy, Strides2 so,
                  int64_t g_block, int64_t g_row, const int32_t* offsets, int offset, int io_dtype, cudaStream_t stream);

@@ -54,6 +54,9 @@ class RGLRU(StatefulMixer):
         st = self.state(inference_params, h.dtype)
         pos = self.position(inference_params, L)
         x = self.in_proj(h)
+        if L == 1 and ops.rglru_step(self.in_proj.slice(x, "x")[:, 0], self.in_proj.slice(x, "y")[:, 0], self.conv_weight, self.conv_bias,
+                                     st["ring"], self.gate_weight, self.r_bias, self.i_bias, self.lam, st["state"], pos=pos, out=out[:, 0]):
+            return
         u = ops.short_conv(self.in_proj.slice(x, "x"), self.conv_weight, self.conv_bias, ring=st["ring"], pos=pos)
         ops.rglru_gated(u, self.in_proj.slice(x, "y"), self.gate_weight, self.r_bias, self.i_bias, self.lam, st["state"], pos=pos,
                         out=out)

@@ -930,6 +930,37 @@ def rglru_gated(u, y, gate_weight, r_bias, i_bias, lam, state, *, pos=0, out: to
     return rglru(u, y, block_gates(u, gate_weight), r_bias, i_bias, lam, state, pos=pos, out=out)
 
 
+def rglru_step(x, y, conv_weight, conv_bias, ring, gate_weight, r_bias, i_bias, lam, state, *, pos, out: torch.Tensor) -> bool:
+    """One token per row in one launch: ``x, y [B, W]`` column slices of the packed projection through :func:`short_conv`,
+    :func:`block_gates` and :func:`rglru`; ``ring [B, taps, W]`` and ``state [B, W]`` are updated IN PLACE, ``out [B, W]``.  Returns
+    False, nothing launched, for dtypes, sizes or layouts it does not take."""
+    _need_cuda(x, y, conv_weight, conv_bias, ring, gate_weight, r_bias, i_bias, lam, state, out)
+    B, W = x.shape
+    nb, two, n, n2 = gate_weight.shape
+    taps = conv_weight.shape[1]
+    if any(t.dtype != torch.bfloat16 for t in (x, y, conv_weight, ring, gate_weight, r_bias, i_bias, out)) or (
+            conv_bias is not None and conv_bias.dtype != torch.bfloat16):
+        return False
+    if (two != 2 or n2 != n or nb * n != W or y.shape != (B, W) or out.shape != (B, W) or conv_weight.shape[0] != W
+            or ring.shape[0] < B or ring.shape[1:] != (taps, W) or state.shape[0] < B or state.shape[1] != W
+            or state.dtype != torch.float32 or lam.dtype != torch.float32):
+        raise ValueError("x, y, out must be [B, W], ring [>= B, taps, W], gate_weight [blocks, 2, n, n], state [>= B, W] and lam float32")
+    if not all(t.is_contiguous() for t in (conv_weight, ring, gate_weight, state, r_bias, i_bias, lam)) or (
+            conv_bias is not None and not conv_bias.is_contiguous()):
+        return False
+    for t, name in ((x, "x"), (y, "y"), (out, "out")):
+        _inner_contig(t, name)
+    off, scalar = _position(pos, x)
+    if B == 0:
+        return True
+    code = _capi.native().rglru_step(x, y, conv_weight, conv_bias, ring, gate_weight, r_bias, i_bias, lam, state, out, B, W, n, taps,
+                                     x.stride(0), y.stride(0), out.stride(0), off, scalar)
+    if code == _capi.ERR_IMPL:
+        return False
+    _capi.check(code, "based_rglru_step")
+    return True
+
+
 # --------------------------------------------------------------------------- post-norm stacks
 
 def _strides_bl(t):

@@ -518,6 +518,17 @@ int based_rglru(const void* u, const void* y, const void* gates, const void* r_b
                 const int32_t* offsets, int offset, int io_dtype, void* stream);
 
 /*
+ * One token per row from the packed projection to the gated output in one launch, bf16: u = conv(x) over the ring (as
+ * based_short_conv, conv_bias [W] or NULL), gates gate_weight [blocks, 2, n, n] u (as based_rglru_gated), recurrence and gate by
+ * gelu(y).  ring [B, taps, W] and state [B, W] fp32 are updated.  BASED_ERR_IMPL for block widths that are not multiples of 32 or
+ * above 256, taps outside 2..4, an x row stride that is no multiple of 8, and x, weights or ring that are not 16-byte aligned.
+ */
+int based_rglru_step(const void* x, const void* y, const void* conv_weight, const void* conv_bias, void* ring,
+                     const void* gate_weight, const void* r_bias, const void* i_bias, const void* lam, void* state, void* out,
+                     int B, int W, int block_width, int taps, int64_t x_row_stride, int64_t y_row_stride, int64_t out_row_stride,
+                     const int32_t* offsets, int offset, void* stream);
+
+/*
  * The same with the gate products inside (tensor cores, bf16): gate_weight [blocks, 2, n, n], r and i matrices stored
  * [out, in], n = block_width.  BASED_ERR_IMPL for fp32, n not a multiple of 16 or above 256, or unaligned u.
  */

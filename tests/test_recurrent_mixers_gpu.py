@@ -222,6 +222,32 @@ def test_rglru_shared_sequences(W, blocks, L, B):
         assert rel_err(out.float().cpu(), ref) < 1e-2
 
 
+@pytest.mark.parametrize("W,blocks,taps,B", [(1024, 8, 4, 16), (64, 2, 4, 1), (256, 1, 2, 17), (96, 1, 3, 5), (480, 3, 4, 33)])
+def test_rglru_step(W, blocks, taps, B):
+    """The fused step against the three launches it stands for, rows at positions of their own (two of them fresh, one within the
+    convolution's reach of the start): the same values in all but the order of the gates' sums."""
+    from based_b200 import ops
+    g = torch.Generator().manual_seed(W)
+    n = W // blocks
+    packed = torch.randn(B, 2 * W + 8, generator=g).bfloat16().cuda()
+    x, y = packed[:, :W], packed[:, W + 8:]
+    cw, cb = (torch.randn(W, taps, generator=g) / 2).bfloat16().cuda(), (torch.randn(W, generator=g) / 4).bfloat16().cuda()
+    gw = (torch.randn(blocks, 2, n, n, generator=g) / n ** 0.5).bfloat16().cuda()
+    rb, ib = ((torch.randn(W, generator=g) - 1).bfloat16().cuda() for _ in range(2))
+    lam = (2 * torch.randn(W, generator=g) - 4).cuda()
+    ring, state = torch.randn(B + 1, taps, W, generator=g).bfloat16().cuda(), torch.randn(B + 1, W, generator=g).cuda()
+    for pos in (torch.tensor([(0, 1, 7, 0, 2, 900, 3)[i % 7] for i in range(B)], dtype=torch.int32, device="cuda"), 0, 5):
+        r1, s1, r2, s2 = ring.clone(), state.clone(), ring.clone(), state.clone()
+        got, want = torch.empty(B, W, dtype=torch.bfloat16, device="cuda"), torch.empty(B, 1, W, dtype=torch.bfloat16, device="cuda")
+        assert ops.rglru_step(x, y, cw, cb, r1, gw, rb, ib, lam, s1, pos=pos, out=got)
+        u = ops.short_conv(x[:, None], cw, cb, ring=r2, pos=pos)
+        ops.rglru(u, y[:, None], ops.block_gates(u, gw), rb, ib, lam, s2, pos=pos, out=want)
+        assert torch.equal(r1, r2) and torch.equal(s1[B], state[B])
+        assert rel_err(s1.cpu(), s2.cpu()) < 1e-5 and rel_err(got.float().cpu(), want[:, 0].float().cpu()) < 1e-2
+    for bad in (dict(x=x.float()), dict(gw=gw.float()), dict(x=packed[:, 1:W + 1])):   # another dtype; not 16-byte aligned
+        assert not ops.rglru_step(bad.get("x", x), y, cw, cb, ring, bad.get("gw", gw), rb, ib, lam, state, pos=0, out=got)
+
+
 @pytest.mark.parametrize("D", [64, 96, 50, 2048, 1031, 7168])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_stream_norm(D, dtype):
