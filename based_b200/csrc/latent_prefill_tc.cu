@@ -63,8 +63,9 @@ __global__ void __launch_bounds__(NT, 1) latent_prefill_tc_kernel(const __grid_c
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t sb = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * (2 * TQ);   // longest rows first
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * (2 * TQ);   // longest rows first, of all heads: a head that starts late ends late.
+                                                                      // B = 2, 8 heads, L = 4096: 184 us with a head's tiles in a row, 122 like this
   const int off = seq::position0(p.offsets, p.offset, b);
   const int na = p.a1 + p.a2;
   const uint32_t SM_RING = 2u * na * kAtom, SM_BAR = SM_RING + (uint32_t)p.ring * kAtom;
@@ -328,7 +329,7 @@ int launch_latent_prefill_tc(const void* q1, const void* q2, const void* k1, con
                          fix(sv.h, H), fix(sv.l, T), fix(so.b, B), fix(so.h, H), fix(so.l, L)};
   for (int64_t s : all)
     if (s % 8 != 0 || s <= 0) return BASED_ERR_IMPL;
-  if (B > 65535 || H > 65535) return BASED_ERR_IMPL;
+  if (B > 65535 || H > 65535 || (L - 1) / (2 * TQ) >= 65535) return BASED_ERR_IMPL;
   Params p;
   p.a1 = (d1 + 63) / 64; p.a2 = (d2 + 63) / 64; p.av = (dv + 63) / 64;
   const int na = p.a1 + p.a2;
@@ -376,7 +377,7 @@ int launch_latent_prefill_tc(const void* q1, const void* q2, const void* k1, con
     p.status = status[dev];
   }
   const int smem = 2 * na * (int)kAtom + p.ring * (int)kAtom + kFixed;
-  latent_prefill_tc_kernel<<<dim3((L + 2 * TQ - 1) / (2 * TQ), H, B), NT, smem, stream>>>(p);
+  latent_prefill_tc_kernel<<<dim3(H, B, (L + 2 * TQ - 1) / (2 * TQ)), NT, smem, stream>>>(p);
   return (int)cudaGetLastError();
 }
 

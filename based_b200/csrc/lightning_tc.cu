@@ -110,6 +110,7 @@ __device__ __forceinline__ void decayed(const uint4& v, float f, uint8_t* hi_at,
 }
 
 __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_constant__ Params p) {
+  pdl_wait();   // before the TMEM allocation: what is waited for may hold all of it
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t sb = smem_u32(smem);
@@ -430,6 +431,8 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
 // stages; one elected lane issues.  Bound by the loads' latency: a CTA has 2 to 6 chunks, one of them in registers ahead.
 constexpr int kSegThreads = 512;
 __global__ void __launch_bounds__(kSegThreads, 1) lightning_segment_kernel(const __grid_constant__ Params p, const bf16* v, int64_t vb, int64_t vl) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t sb = smem_u32(smem);
@@ -551,6 +554,8 @@ __global__ void __launch_bounds__(kSegThreads, 1) lightning_segment_kernel(const
 // seg [B H][nseg][n]: slot s + 1 holds what segment s adds; becomes the state before segment s + 1, slot 0 the state of the call.
 // A thread owns four consecutive entries and has eight segments' loads in flight.
 __global__ void __launch_bounds__(256) lightning_scan_kernel(const __grid_constant__ Params p) {
+  pdl_trigger();
+  pdl_wait();
   const int n = p.d * p.dv, i = (blockIdx.x * 256 + threadIdx.x) * 4, head = blockIdx.y;
   if (i >= n) return;
   float g = 1.f, x = p.decay[head % p.H];
@@ -668,10 +673,10 @@ int launch_lightning_tc(const void* q, const void* k, const void* v, const float
   p.tma_out = slices == 1 || p.cols % 64 == 0;   // a slice's tile must not reach into the next one
   if (p.nseg > 1) {
     const int seg_smem = 2 * (2 + 2 * av) * (int)kAtom + 132 * 4 + 24 + 1024;
-    lightning_segment_kernel<<<dim3(H, B, slices * (p.nseg - 1)), kSegThreads, seg_smem, stream>>>(p, static_cast<const bf16*>(v), sv.b, sv.h);
-    lightning_scan_kernel<<<dim3((d * dv / 4 + 255) / 256, B * H), 256, 0, stream>>>(p);
+    launch_pdl(lightning_segment_kernel, dim3(H, B, slices * (p.nseg - 1)), kSegThreads, seg_smem, stream, p, static_cast<const bf16*>(v), sv.b, sv.h);
+    launch_pdl(lightning_scan_kernel, dim3((d * dv / 4 + 255) / 256, B * H), 256, 0, stream, p);
   }
-  lightning_tc_kernel<<<dim3(H, B, slices * p.nseg), NT, smem, stream>>>(p);
+  launch_pdl(lightning_tc_kernel, dim3(H, B, slices * p.nseg), NT, smem, stream, p);
   return (int)cudaGetLastError();
 }
 

@@ -17,7 +17,8 @@ namespace {
 
 // CTA size: 192 threads (three CTAs per SM, 96 registers) when there are many (batch, head) blocks -- measured
 // 0.1052 ms against 0.1091 ms at B=256, H=16, fp32 state -- and 256 threads (two per SM) when there are few, where
-// one block's latency is what counts (B=16, H=16, bf16 state: 10.6 us against 17.3 us).
+// one block's latency is what counts (B=16, H=16, bf16 state: 10.6 us against 17.3 us); 512 where every block has an SM of its
+// own and more than eight row groups (B=8, H=16, dv=112, bf16 state, in a chain of launches: 10.5 us with 256, 6.6 with 512).
 constexpr int kTab = 288;     // table length: 273 + wrap-around + padding, multiple of 4
 constexpr int kVecPerGroup = kExpandedDim;  // 273 vectors of 16 B per row group
 constexpr int kIters = (kVecPerGroup + 31) / 32;  // 9
@@ -57,13 +58,13 @@ template <> struct VecOps<__nv_bfloat16> {
 };
 
 template <typename IO, typename ST, int kThreads>
-__global__ void __launch_bounds__(kThreads, kThreads <= 192 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, kThreads <= 192 ? 3 : kThreads <= 256 ? 2 : 1)
 linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
                       IO* y, ST* kv_state, ST* k_state,
                       int H, int dv, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 sy, float eps) {
   pdl_trigger();
-  if (kThreads > 192) {   // few blocks: their state into L2 before the kernel ahead has ended, a whole number of 16-byte vectors
-    const uint32_t bytes = dv * kExpandedDim * sizeof(ST), piece = ((bytes + kThreads - 1) / kThreads + 15) & ~15u, at = threadIdx.x * piece;
+  if (kThreads > 192 && threadIdx.x < 32) {   // few blocks: their state into L2 before the kernel ahead has ended; whole 16-byte vectors
+    const uint32_t bytes = dv * kExpandedDim * sizeof(ST), piece = (bytes / 32 + 15) & ~15u, at = threadIdx.x * piece;
     if (at < bytes) prefetch_l2(reinterpret_cast<const char*>(kv_state) + (size_t)blockIdx.x * bytes + at, min(piece, bytes - at));
   }
   pdl_wait();
@@ -195,6 +196,10 @@ int launch_typed(const void* q, const void* k, const void* v, void* y, void* kv_
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if ((long long)B * H >= 6LL * sms) {  // at least two waves of three CTAs per SM
     launch_pdl(linattn_decode_kernel<IO, ST, 192>, B * H, 192, 0, stream, 
+        static_cast<const IO*>(q), static_cast<const IO*>(k), static_cast<const IO*>(v), static_cast<IO*>(y),
+        static_cast<ST*>(kv_state), static_cast<ST*>(k_state), H, dv, sq, sk, sv, sy, eps);
+  } else if ((long long)B * H <= sms && dv / VecOps<ST>::kVec > 8) {   // a block per SM: all its row groups at once
+    launch_pdl(linattn_decode_kernel<IO, ST, 512>, B * H, 512, 0, stream,
         static_cast<const IO*>(q), static_cast<const IO*>(k), static_cast<const IO*>(v), static_cast<IO*>(y),
         static_cast<ST*>(kv_state), static_cast<ST*>(k_state), H, dv, sq, sk, sv, sy, eps);
   } else {

@@ -106,13 +106,15 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(const NormPar
   pdl_wait();
   const int64_t row = blockIdx.x;
   const int ngroups = p.D >> 3;
-  float z[VPT][8];
+  constexpr bool kEarly = VPT <= 2;   // the weights' latency passes with the row's
+  float z[VPT][8], wv[kEarly ? VPT : 1][8];
   float ss = 0.f;
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int g = threadIdx.x + v * NORM_THREADS;
     if (g < ngroups) {
       load8(p.x, p.io_bf16, row * p.sx + 8 * g, z[v]);
+      if (kEarly) load8(p.weight, p.w_bf16, 8 * g, wv[kEarly ? v : 0]);
       if (p.residual) {
         float r[8];
         load8(p.residual, p.res_bf16, row * p.sr + 8 * g, r);
@@ -148,9 +150,9 @@ __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(const NormPar
     const int g = threadIdx.x + v * NORM_THREADS;
     if (g < ngroups) {
       float w[8], o[8];
-      load8(p.weight, p.w_bf16, 8 * g, w);
+      if (!kEarly) load8(p.weight, p.w_bf16, 8 * g, w);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = z[v][i] * rstd * w[i];
+      for (int i = 0; i < 8; ++i) o[i] = z[v][i] * rstd * (kEarly ? wv[kEarly ? v : 0][i] : w[i]);
       if (p.bias) {
         load8(p.bias, p.w_bf16, 8 * g, w);
 #pragma unroll
@@ -205,7 +207,8 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamP
   const int64_t row = blockIdx.x;
   const int groups = p.D / N;
   float* res = p.residual + row * p.D;
-  float z[VPT][N];
+  constexpr bool kEarly = VPT <= 2;   // the weights' latency passes with the row's
+  float z[VPT][N], w1[kEarly ? VPT : 1][N], w2[kEarly ? VPT : 1][N];
   auto load_res = [&](int g, float (&v)[N]) {
     if constexpr (N == 8) load8(res, 0, 8 * g, v);
     else v[0] = res[g];
@@ -226,6 +229,10 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamP
       float b[N];
       if (p.tokens || p.branch) Pack<T, N>::load(src + (int64_t)g * N, b);
       if (!p.tokens) load_res(g, z[v]);
+      if (kEarly) {
+        Pack<T, N>::load(static_cast<const T*>(p.w1) + (int64_t)g * N, w1[kEarly ? v : 0]);
+        if (p.out2) Pack<T, N>::load(static_cast<const T*>(p.w2) + (int64_t)g * N, w2[kEarly ? v : 0]);
+      }
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         if (p.tokens) z[v][i] = known ? b[i] : 0.f;
@@ -260,15 +267,16 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamP
   for (int v = 0; v < VPT; ++v) {
     const int g = threadIdx.x + v * NORM_THREADS;
     if (g < groups) {
-      float w[N], o[N];
-      Pack<T, N>::load(static_cast<const T*>(p.w1) + (int64_t)g * N, w);
+      float o[N];
+      float (&u1)[N] = w1[kEarly ? v : 0], (&u2)[N] = w2[kEarly ? v : 0];
+      if (!kEarly) Pack<T, N>::load(static_cast<const T*>(p.w1) + (int64_t)g * N, u1);
 #pragma unroll
-      for (int i = 0; i < N; ++i) o[i] = z[v][i] * rstd * w[i];
+      for (int i = 0; i < N; ++i) o[i] = z[v][i] * rstd * u1[i];
       Pack<T, N>::store(static_cast<T*>(p.out1) + row * p.D + (int64_t)g * N, o);
       if (p.out2) {
-        Pack<T, N>::load(static_cast<const T*>(p.w2) + (int64_t)g * N, w);
+        if (!kEarly) Pack<T, N>::load(static_cast<const T*>(p.w2) + (int64_t)g * N, u2);
 #pragma unroll
-        for (int i = 0; i < N; ++i) o[i] = z[v][i] * rstd * w[i];
+        for (int i = 0; i < N; ++i) o[i] = z[v][i] * rstd * u2[i];
         Pack<T, N>::store(static_cast<T*>(p.out2) + row * p.D + (int64_t)g * N, o);
       }
     }
@@ -295,7 +303,8 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const Po
   const int groups = p.D / N;
   float* res = p.residual + row * p.D;
   const T* br = static_cast<const T*>(p.branch) + row * p.sb;
-  float z[VPT][N], r[VPT][N];
+  constexpr bool kEarly = VPT <= 2;   // the weight's latency passes with the row's
+  float z[VPT][N], r[VPT][N], w0[kEarly ? VPT : 1][N];
   float ss = 0.f;
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
@@ -303,6 +312,7 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const Po
     if (g < groups) {
       Pack<T, N>::load(br + (int64_t)g * N, z[v]);
       Pack<float, N>::load(res + (int64_t)g * N, r[v]);
+      if (kEarly) Pack<T, N>::load(static_cast<const T*>(p.w) + (int64_t)g * N, w0[kEarly ? v : 0]);
 #pragma unroll
       for (int i = 0; i < N; ++i) ss = fmaf(z[v][i], z[v][i], ss);
     }
@@ -313,8 +323,8 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const Po
   for (int v = 0; v < VPT; ++v) {
     const int g = threadIdx.x + v * NORM_THREADS;
     if (g < groups) {
-      float w[N];
-      Pack<T, N>::load(static_cast<const T*>(p.w) + (int64_t)g * N, w);
+      float (&w)[N] = w0[kEarly ? v : 0];
+      if (!kEarly) Pack<T, N>::load(static_cast<const T*>(p.w) + (int64_t)g * N, w);
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         r[v][i] = fmaf(z[v][i] * rstd, w[i], r[v][i]);

@@ -10,7 +10,8 @@
 //    block has 32 channels of one gate block and 16 rows, takes the convolution of the whole gate block for itself (a few KB,
 //    cheaper than a second launch that shares it) and multiplies it by its 64 rows of the gate matrices, one 8-row tile per
 //    warp, whose loads are in flight before the convolution.  Three launches, the middle one a library product that ends a
-//    chain of programmatic launches, took @OLD@ us a layer in a step of 16 rows, this one @NEW@.
+//    chain of programmatic launches, took 6.5 us in a chain of their own at 16 rows of 1024 (7.2 without programmatic launches),
+//    this one 4.2; a step of 17 such layers 731 -> 662 us.
 #include <initializer_list>
 
 #include "seq_common.cuh"

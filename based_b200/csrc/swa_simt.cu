@@ -101,7 +101,7 @@ __device__ __forceinline__ Row8 unpack8(const uint4 (&r)[2]) {
 // row, 8 values (16 or 32 bytes) each, a group of lanes has every (32 / LPK * WARPS)-th key, and its first four keys AND values
 // are in flight before the query is rotated.  Each group keeps a running maximum, sum and weighted row of its own keys; the
 // groups meet once at the end.  16 heads, 16 rows, hd = 64, 64 keys: 10.6 us with one warp per head (keys, softmax, values in
-// turn), about 4 us like this.  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
+// turn), 4.4 us like this.  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
 template <typename IO, int LPK, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
