@@ -142,7 +142,10 @@ BASED_WEAK int launch_rotary_qkv_cache(void* qkv, int B, int L, int H, int hd, i
                             cudaStream_t stream);
 int launch_decode_linear(const void* x, const void* w, const void* bias, void* out, int M, int N, int K, int64_t sx,
                          int64_t so, int epilogue, int act, void* conv_state, const void* conv_weight,
-                         const void* conv_bias, int conv_k, int conv_w_dtype, cudaStream_t stream);
+                         const void* conv_bias, int conv_k, int conv_w_dtype, const float* row_ss, int n_ss, float eps,
+                         cudaStream_t stream);
+int launch_decode_linear_add(const void* x, const void* w, const void* bias, int M, int N, int K, int64_t sx, float* residual,
+                             const void* norm, void* out, float* ss, cudaStream_t stream);
 
 BASED_WEAK int launch_tp_outproj_allreduce(const void* const* x, const void* const* w, const void* bias, void* const* out,
                                 void* const* workspaces, int M, int N, int K, int64_t sx, int64_t so, int Mmax,

@@ -8,6 +8,10 @@
 //           append, dot with the taps), silu, gate by u2       in_proj + ShortConvolution.step + gate
 //                                                           (based/models/mixers/convolution.py:88-109, :205-211)
 //   F32     PLAIN with an fp32 result
+//   ADD     y = x W^T + b joins the fp32 residual stream in place (z = residual + y), and z times the weights of the
+//           norm that comes next goes out in bf16, with the sums of z^2 over 8 columns beside it
+// A product of up to 16 rows may take ADD's outputs for x: the norm's 1 / rms is one factor per row, so it is applied to the
+// sums (row_ss), and no launch stands between the product before a norm and the one after it.
 // The work is reading W once, 2 to 26 MB: 0.3 to 4 us at the HBM rate, so a launch of its own is mostly latency: the launch, the
 // first bytes from HBM, the sum over the split of K.  Two things against that:
 //  * The launch is programmatic: the blocks start while the kernel before still runs, bring their part of W into L2 (a hint;
@@ -26,7 +30,7 @@ namespace based {
 namespace {
 
 constexpr int kSms = 148;
-enum Epi { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_CONV = 2, EPI_F32 = 3 };
+enum Epi { EPI_PLAIN = 0, EPI_SWIGLU = 1, EPI_CONV = 2, EPI_F32 = 3, EPI_ADD = 4 };
 
 struct LinParams {
   const __nv_bfloat16 *x, *w, *bias;
@@ -38,6 +42,13 @@ struct LinParams {
   __nv_bfloat16* state;            // [M, N/2, ck]
   const void *cw, *cb;             // taps [N/2, ck], bias [N/2] or null
   int ck, cw_bf16;
+  // x is scaled per row by 1 / sqrt(sum of the row's n_ss entries / K + eps); null: it is not
+  const float* row_ss;             // [M, n_ss]
+  int n_ss;
+  float eps;
+  // ADD
+  float *residual, *ss;            // [M, N] fp32; [M, N / 8]
+  const __nv_bfloat16* norm;       // [N]
 };
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -113,6 +124,18 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) decode_linear_k
         }
       }
   }
+  // ---- the rows' factors, a few threads to a row
+  __shared__ float factor[16 * MT];
+  if (MT == 1 && p.row_ss) {
+    constexpr int kTo = WARPS * 2;   // threads per row
+    const int row = tid / kTo, j0 = tid % kTo;
+    float sum = 0.f;
+    if (m0 + row < p.M)
+      for (int j = j0; j < p.n_ss; j += kTo) sum += p.row_ss[(int64_t)(m0 + row) * p.n_ss + j];
+#pragma unroll
+    for (int o = kTo / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (j0 == 0) factor[row] = rsqrtf(sum / (float)p.K + p.eps);
+  }
   // ---- the K slices' sums meet in shared memory, [warp][tile][row][column]; lanes hold rows g, g + 8 and columns 2t, 2t + 1
   __shared__ float red[WARPS][NT8][16 * MT * 8];
 #pragma unroll
@@ -143,6 +166,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) decode_linear_k
           cw[r][j] = ld_w(p.cw, p.cw_bf16, col * p.ck + j);
         }
     }
+    if (EPI == EPI_ADD && o < kOut && row < p.M && col < outputs) {
+      cs[r][0] = p.residual[(int64_t)row * p.N + col];
+      cw[r][0] = __bfloat162float(p.norm[col]);
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -155,6 +182,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) decode_linear_k
       y += red[w][tile][in];
       if (kTwo) y2 += red[w][(kTwo ? CT : 0) + tile][in];
     }
+    if (MT == 1 && p.row_ss) {
+      y *= factor[in >> 3];
+      y2 *= factor[in >> 3];
+    }
     y += bias[r][0];
     y2 += bias[r][1];
     const int64_t at = (int64_t)row * p.so + col;
@@ -163,7 +194,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) decode_linear_k
       continue;
     }
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + at;
-    if (EPI == EPI_PLAIN) {
+    if (EPI == EPI_ADD) {
+      const float z = cs[r][0] + y;     // fp32: the branch is not rounded on its way
+      p.residual[(int64_t)row * p.N + col] = z;
+      *out = __float2bfloat16_rn(z * cw[r][0]);
+      float ss = z * z;            // eight neighbouring threads have a row's eight columns, and take this way together
+#pragma unroll
+      for (int d = 1; d < 8; d <<= 1) ss += __shfl_xor_sync(0xffu << (lane & 24), ss, d);
+      if ((in & 7) == 0) p.ss[(int64_t)row * (p.N / 8) + col / 8] = ss;
+    } else if (EPI == EPI_PLAIN) {
       *out = __float2bfloat16_rn(y);
     } else if (EPI == EPI_SWIGLU) {
       y = bf16_round(y);                          // fc1's output is a bf16 tensor in the unfused sequence
@@ -212,7 +251,7 @@ int launch_tiles(const LinParams& p, int outputs, cudaStream_t stream) {
 template <int EPI>
 int launch_epi(const LinParams& p, int outputs, cudaStream_t stream) {
   const int tiles = outputs / 8;
-  if constexpr (EPI == EPI_PLAIN || EPI == EPI_F32)
+  if constexpr (EPI == EPI_PLAIN || EPI == EPI_F32 || EPI == EPI_ADD)
     if (tiles > 4 * kSms) return launch_tiles<EPI, 4>(p, outputs, stream);
   return tiles > 2 * kSms ? launch_tiles<EPI, 2>(p, outputs, stream) : launch_tiles<EPI, 1>(p, outputs, stream);
 }
@@ -221,19 +260,32 @@ int launch_epi(const LinParams& p, int outputs, cudaStream_t stream) {
 
 int launch_decode_linear(const void* x, const void* w, const void* bias, void* out, int M, int N, int K, int64_t sx,
                          int64_t so, int epilogue, int act, void* conv_state, const void* conv_weight,
-                         const void* conv_bias, int conv_k, int conv_w_dtype, cudaStream_t stream) {
+                         const void* conv_bias, int conv_k, int conv_w_dtype, const float* row_ss, int n_ss, float eps,
+                         cudaStream_t stream) {
   if (K % 32 != 0 || sx % 8 != 0 || !aligned16(x) || !aligned16(w)) return BASED_ERR_ALIGN;
   const bool two = epilogue == EPI_SWIGLU || epilogue == EPI_CONV;
   const int outputs = two ? N / 2 : N;
-  if (outputs % 8 != 0 || (two && N % 2 != 0)) return BASED_ERR_SHAPE;
+  if (outputs % 8 != 0 || (two && N % 2 != 0) || (row_ss && M > 16)) return BASED_ERR_SHAPE;
   LinParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
               static_cast<const __nv_bfloat16*>(bias), out, M, N, K, sx, so, act,
-              static_cast<__nv_bfloat16*>(conv_state), conv_weight, conv_bias, conv_k, conv_w_dtype == BASED_BF16};
+              static_cast<__nv_bfloat16*>(conv_state), conv_weight, conv_bias, conv_k, conv_w_dtype == BASED_BF16,
+              row_ss, n_ss, eps, nullptr, nullptr, nullptr};
   if (epilogue == EPI_PLAIN) return launch_epi<EPI_PLAIN>(p, outputs, stream);
   if (epilogue == EPI_SWIGLU) return launch_epi<EPI_SWIGLU>(p, outputs, stream);
   if (epilogue == EPI_CONV) return launch_epi<EPI_CONV>(p, outputs, stream);
   if (epilogue == EPI_F32) return launch_epi<EPI_F32>(p, outputs, stream);
   return BASED_ERR_SHAPE;
+}
+
+int launch_decode_linear_add(const void* x, const void* w, const void* bias, int M, int N, int K, int64_t sx, float* residual,
+                             const void* norm, void* out, float* ss,
+                             cudaStream_t stream) {
+  if (K % 32 != 0 || sx % 8 != 0 || !aligned16(x) || !aligned16(w)) return BASED_ERR_ALIGN;
+  if (N % 8 != 0 || M > 16) return BASED_ERR_SHAPE;
+  LinParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
+              static_cast<const __nv_bfloat16*>(bias), out, M, N, K, sx, N, 0, nullptr, nullptr, nullptr, 0, 0,
+              nullptr, 0, 0.f, residual, ss, static_cast<const __nv_bfloat16*>(norm)};
+  return launch_epi<EPI_ADD>(p, N, stream);
 }
 
 }  // namespace based

@@ -117,9 +117,15 @@ class BaseConv(nn.Module):
         if device is not None or dtype is not None:
             self.conv.to(device=device, dtype=dtype)
 
-    def forward(self, u, position_ids=None, inference_params=None, *args, **kwargs):
+    def step_weights(self):
+        """(weight, bias) of the products of a decode step, the output projection last; None where a step has another form."""
+        return [(m.weight, m.bias) for m in (self.in_proj, self.out_proj)]
+
+    def forward(self, u, position_ids=None, inference_params=None, *args, finish=None, **kwargs):
         """u ``[B, L, d_model]`` -> ``[B, L, d_model]``; with ``inference_params`` the prompt pass
-        fills the convolution state and later single-token calls step it."""
+        fills the convolution state and later single-token calls step it.  ``finish(v, weight, bias)``, when
+        given, stands for the product with out_proj and what comes behind it."""
+        finish = finish or ops.linear
         if inference_params is not None and inference_params.seqlen_offset > 0:
             state = self.conv._get_state(inference_params)
             if (ops._decode_rows(u, self.in_proj.weight, fused=True)
@@ -128,10 +134,10 @@ class BaseConv(nn.Module):
                 # decode step: in_proj, the convolution step on the state, silu and the gate in one launch
                 v = ops.decode_linear(u, self.in_proj.weight, self.in_proj.bias, epilogue="conv", conv_state=state,
                                       conv_weight=self.conv.conv.weight, conv_bias=self.conv.conv.bias)
-                return ops.linear(v, self.out_proj.weight, self.out_proj.bias)
+                return finish(v, self.out_proj.weight, self.out_proj.bias)
         u = ops.linear(u, self.in_proj.weight, self.in_proj.bias)
         v = self.conv.gated(u, inference_params=inference_params)
-        return ops.linear(v, self.out_proj.weight, self.out_proj.bias)
+        return finish(v, self.out_proj.weight, self.out_proj.bias)
 
     def allocate_inference_cache(self, batch_size: int, max_seqlen: int, dtype=None, **kwargs):
         return {"conv": self.conv.allocate_inference_cache(batch_size, max_seqlen, dtype=dtype, **kwargs)}

@@ -112,7 +112,13 @@ class LinearAttention(nn.Module):
         self.proj_v = nn.Linear(self.d_model, self.num_heads * self.head_dim, bias=False, **fk)
         self.out_proj = nn.Linear(self.num_heads * self.head_dim, self.d_model, bias=False, **fk)
 
-    def forward(self, hidden_states: torch.Tensor, inference_params=None, *args, **kwargs):
+    def step_weights(self):
+        """(weight, bias) of the products of a decode step, the output projection last; None where a step has another form."""
+        if not self.fuse_qkv or self.training or self.process_group is not None:
+            return None
+        return [(self.proj_q.weight, None), (self.proj_k.weight, None), (self.proj_v.weight, None), (self.out_proj.weight, self.out_proj.bias)]
+
+    def forward(self, hidden_states: torch.Tensor, inference_params=None, *args, finish=None, **kwargs):
         """hidden_states ``[B, L, d_model]`` -> ``[B, L, d_model]`` (linear_attention.py:115-150).
         Extra keyword arguments the model passes to every mixer (``position_ids``, ``decay``,
         ``stream``, ``seqlen``) are accepted and ignored, as in the reference."""
@@ -134,7 +140,7 @@ class LinearAttention(nn.Module):
             return self.parallel_forward(hidden_states, q, k, v)
         if inference_params.seqlen_offset > 0:
             kv_state, k_state = self._get_inference_cache(inference_params)
-            return self.recurrent_forward(hidden_states, kv_state, k_state, q, k, v)
+            return self.recurrent_forward(hidden_states, kv_state, k_state, q, k, v, finish=finish)
         cached = inference_params.key_value_memory_dict.get(self.layer_idx)
         if cached is not None and cached[0].shape[0] == b:
             # pre-allocated (CUDA-graph) cache: the kernel writes the states in place
@@ -173,7 +179,7 @@ class LinearAttention(nn.Module):
             return out, kv_state, k_state
         return out
 
-    def recurrent_forward(self, hidden_states, kv_state, k_state, q, k, v, decay=None):
+    def recurrent_forward(self, hidden_states, kv_state, k_state, q, k, v, decay=None, finish=None):
         """One token (linear_attention.py:230-252).  ``q``/``k`` are the RAW ``[B, H, 1, 16]``
         projections: the kernel applies the feature map itself (the reference maps them
         first, :139).  ``kv_state``/``k_state`` are updated in place."""
@@ -181,6 +187,8 @@ class LinearAttention(nn.Module):
         assert l == 1, f"q.shape is {q.shape} but should be ({b}, {h}, 1, {d})"
         eps = 1e-6 if "fla" in self.parallel_implementation else 1e-12
         y = ops.linattn_decode(q, k, v, kv_state, k_state, eps=eps)
+        if finish is not None:   # stands for the product with out_proj and what comes behind it
+            return finish(y, self.out_proj.weight, self.out_proj.bias)
         return row_parallel_decode_linear(self, y, self.out_proj.weight, self.out_proj.bias, self.process_group)
 
     def expanded_size(self):

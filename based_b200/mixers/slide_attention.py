@@ -147,8 +147,14 @@ class SlidingAttention(nn.Module):
                                             self.num_heads_kv, self.head_dim, dtype=like.dtype, device=like.device)
         return d[self.layer_idx]
 
+    def step_weights(self):
+        """(weight, bias) of the products of a decode step, the output projection last; None where a step has another form."""
+        if self.process_group is not None or self.return_residual:
+            return None
+        return [(m.weight, m.bias) for m in (self.Wqkv, self.out_proj)]
+
     def forward(self, x, x_kv=None, key_padding_mask=None, cu_seqlens=None, max_seqlen=None, mixer_subset=None,
-                inference_params=None, **kwargs):
+                inference_params=None, finish=None, **kwargs):
         """x ``[B, L, embed_dim]`` -> ``[B, L, embed_dim]`` (slide_attention.py:483-600)."""
         if x_kv is not None or key_padding_mask is not None or cu_seqlens is not None or mixer_subset is not None:
             raise NotImplementedError("only the dense self-attention path of the Based model is implemented")
@@ -197,6 +203,8 @@ class SlidingAttention(nn.Module):
             context = ops.swa_decode(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], cache, lens, w, self.softmax_scale,
                                      rotary_cos=cos, rotary_sin=sin)
         context = context.to(in_dtype).reshape(batch, seqlen, self.num_heads * self.head_dim)
+        if finish is not None:   # stands for the product with out_proj and what comes behind it
+            return finish(context, self.out_proj.weight, self.out_proj.bias)
         if seqlen == 1 and inference_params is not None and inference_params.seqlen_offset > 0:
             out = row_parallel_decode_linear(self, context, self.out_proj.weight, self.out_proj.bias, self.process_group)
         else:

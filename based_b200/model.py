@@ -93,6 +93,34 @@ class Block(nn.Module):
     def allocate_inference_cache(self, batch_size, max_seqlen, dtype=None, **kwargs):
         return self.mixer.allocate_inference_cache(batch_size, max_seqlen, dtype=dtype, **kwargs)
 
+    def step_ok(self, width):
+        """True when a decode step may run without launches of their own for the norms: the stream is fp32, nobody watches the
+        modules, and the products around them are ones :func:`ops.linear_add_norm` and :func:`ops.decode_linear` take."""
+        norms = (self.norm1, self.norm2)
+        weights = self.mixer.step_weights() if type(self.mixer) in (BaseConv, LinearAttention, SlidingAttention) else None
+        if weights is None or not self.residual_in_fp32 or type(self.mlp) is not GatedMlp or self.mlp.return_residual:
+            return False
+        if any(m._forward_hooks or m._forward_pre_hooks for m in (self, self.mixer, self.mlp, *norms)):
+            return False
+        if any(type(n) is not RMSNorm or n.bias is not None or n.weight.dtype != torch.bfloat16 for n in norms):
+            return False
+        weights = weights + [(self.mlp.fc1.weight, self.mlp.fc1.bias), (self.mlp.fc2.weight, self.mlp.fc2.bias)]
+        return (all(ops.step_weight(*w) for w in weights) and self.mlp.fc1.weight.shape[0] % 16 == 0
+                and weights[-3][0].shape[0] == weights[-1][0].shape[0] == width)
+
+    def step(self, hidden_states, residual, inference_params, next_norm):
+        """:meth:`forward` for a decode step where :meth:`step_ok`: ``residual`` is updated in place, ``hidden_states`` may be what
+        the block before returned, and with ``next_norm`` this one returns what the next block's norm gives.  The norms see the fp32
+        stream: the rounding to the activations' dtype comes once, behind the norm's weight."""
+        if type(hidden_states) is not ops.NormRows:
+            hidden_states, residual = self.norm1(hidden_states, residual=residual, prenorm=True, residual_in_fp32=True, round_input=True)
+
+        def into(norm):
+            return lambda x, weight, bias: ops.linear_add_norm(x, weight, bias, residual, norm.weight, eps=norm.eps)
+
+        hidden_states = self.mixer(hidden_states, inference_params=inference_params, finish=into(self.norm2))
+        return self.mlp(hidden_states, finish=None if next_norm is None else into(next_norm)), residual
+
     def forward(self, hidden_states, residual=None, inference_params=None):
         # block.py:134-137: residual = hidden + residual; hidden = norm(residual.to(weight dtype)); residual kept in fp32
         hidden_states, residual = self.norm1(hidden_states, residual=residual, prenorm=True,
@@ -124,10 +152,20 @@ class BasedModel(nn.Module):
         return {i: layer.allocate_inference_cache(batch_size, max_seqlen, dtype=dtype, **kwargs)
                 for i, layer in enumerate(self.layers)}
 
+    def _step_ok(self, h):
+        return (h.dim() == 3 and h.shape[1] == 1 and h.shape[0] <= ops.STEP_MAX_ROWS and len(self.layers) > 0
+                and ops._decode_rows(h, self.layers[0].mlp.fc1.weight) and not torch.nn.modules.module._has_any_global_hook()
+                and all(type(layer) is Block and layer.step_ok(h.shape[-1]) for layer in self.layers))
+
     def forward(self, input_ids, inference_params=None):
         hidden_states, residual = self.embeddings(input_ids), None
-        for layer in self.layers:
-            hidden_states, residual = layer(hidden_states, residual, inference_params=inference_params)
+        if inference_params is not None and inference_params.seqlen_offset > 0 and self._step_ok(hidden_states):
+            following = [layer.norm1 for layer in self.layers[1:]] + [None]
+            for layer, norm in zip(self.layers, following):
+                hidden_states, residual = layer.step(hidden_states, residual, inference_params, norm)
+        else:
+            for layer in self.layers:
+                hidden_states, residual = layer(hidden_states, residual, inference_params=inference_params)
         # gpt.py:676-690: last add, then the final norm on the sum cast to the weights' dtype
         return self.ln_f(hidden_states, residual=residual, residual_in_fp32=self.config.residual_in_fp32,
                          round_input=True)

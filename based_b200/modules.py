@@ -60,8 +60,9 @@ class GatedMlp(nn.Module):
         if ops._decode_rows(x, self.fc1.weight, fused=True) and self.fc1.weight.shape[0] % 16 == 0:
             # decode step: fc1 and the gated activation in one launch
             return ops.decode_linear(x, self.fc1.weight, self.fc1.bias, epilogue="gated", activation=act, out=out)
-        return ops.gated_act(self.fc1(x), act, out=out)
+        return ops.gated_act(self.fc1(ops.dense(x)), act, out=out)
 
-    def forward(self, x):
-        y = ops.linear(self.hidden(x), self.fc2.weight, self.fc2.bias)
+    def forward(self, x, finish=None):
+        """``finish(hidden, weight, bias)``, when given, stands for the product with fc2 and what comes behind it."""
+        y = (finish or ops.linear)(self.hidden(x), self.fc2.weight, self.fc2.bias)
         return y if not self.return_residual else (y, x)

@@ -451,6 +451,9 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
     ``"plain"``; ``"f32"``: plain with an fp32 result; ``"gated"`` -> ``first_half * act(second_half)`` (mlp.py:146-154); ``"conv"`` -> the BaseConv
     decode step on the first half (``conv_state [M, N/2, k]`` updated in place), silu, gate by the second half
     (convolution.py:88-109, :205-211).  x ``[..., K]``; returns ``[..., N]`` or ``[..., N/2]``."""
+    rows = None
+    if type(x) is NormRows:
+        rows, x = x, x.x
     _need_cuda(x, weight, bias, conv_state, conv_weight, conv_bias)
     if x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
         raise TypeError("decode_linear takes bfloat16 activations and weights")
@@ -477,13 +480,72 @@ def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
         if conv_state.shape != (M, n_out, ck) or conv_state.dtype != torch.bfloat16 or not conv_state.is_contiguous():
             raise ValueError("conv_state must be a contiguous bfloat16 [M, N/2, k] tensor")
     if M > 0:
-        code = _capi.native().decode_linear(
+        code = _capi.native().decode_linear_scaled(
             x2, weight, bias, out,
             M, N, K, x2.stride(0), out.stride(0), epi, _ACTS[activation],
             conv_state if epi == 2 else None, conv_weight if epi == 2 else None,
-            conv_bias if (epi == 2 and conv_bias is not None) else None, ck, cw_dt)
+            conv_bias if (epi == 2 and conv_bias is not None) else None, ck, cw_dt,
+            rows.ss if rows is not None else None, rows.ss.shape[1] if rows is not None else 0, rows.eps if rows is not None else 0.0)
         _capi.check(code, "based_decode_linear")
     return out.reshape(*x.shape[:-1], n_out)
+
+
+class NormRows:
+    """The normed rows of a decode step before their norm's last factor: ``x [..., D]`` bf16 is the stream times the norm's weight,
+    ``ss [rows, D / 8]`` the sums of the stream's squares.  The products of this module take it for a tensor (they apply the
+    factor to their sums); nothing else does.  :func:`dense` gives the tensor it stands for."""
+    __slots__ = ("x", "ss", "eps")
+
+    def __init__(self, x, ss, eps):
+        self.x, self.ss, self.eps = x, ss, eps
+
+    shape = property(lambda self: self.x.shape)
+    dtype = property(lambda self: self.x.dtype)
+    device = property(lambda self: self.x.device)
+
+    def size(self, *dim):
+        return self.x.size(*dim)
+
+
+def dense(x):
+    """``x``, or the normed tensor a :class:`NormRows` stands for."""
+    if type(x) is not NormRows:
+        return x
+    rstd = torch.rsqrt(x.ss.sum(1) / x.x.shape[-1] + x.eps)
+    return (x.x.float() * rstd.view(*x.x.shape[:-1], 1)).to(x.x.dtype)
+
+
+STEP_MAX_ROWS = 16
+
+
+def step_weight(weight, bias=None) -> bool:
+    """True for a weight (and bias) that :func:`decode_linear` and :func:`linear_add_norm` take for a few rows."""
+    return (type(weight) in _PLAIN_TYPES and weight.dtype == torch.bfloat16 and weight.dim() == 2 and weight.is_contiguous()
+            and weight.shape[1] % 32 == 0 and weight.shape[0] % 8 == 0 and weight.shape[0] <= DECODE_LINEAR_MAX_OUTPUTS
+            and weight.data_ptr() % 16 == 0
+            and (bias is None or (type(bias) in _PLAIN_TYPES and bias.dtype == torch.bfloat16 and bias.is_contiguous())))
+
+
+def linear_add_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], residual: torch.Tensor, norm_weight: torch.Tensor,
+                    *, eps: float) -> NormRows:
+    """``x W^T (+ bias)`` of at most 16 bf16 rows joins the fp32 stream ``residual [..., N]`` IN PLACE, unrounded; returns the
+    stream's norm with the weights ``norm_weight``."""
+    _need_cuda(x, weight, bias, residual, norm_weight)
+    N, K = weight.shape
+    M = x.numel() // K
+    if x.dtype != torch.bfloat16 or not step_weight(weight, bias) or x.shape[-1] != K or not 0 < M <= STEP_MAX_ROWS:
+        raise ValueError("linear_add_norm takes at most 16 bfloat16 rows and a contiguous bfloat16 [N, K] weight")
+    if residual.dtype != torch.float32 or not residual.is_contiguous() or residual.shape != (*x.shape[:-1], N):
+        raise TypeError("residual must be a contiguous float32 tensor with the product's shape")
+    if norm_weight.dtype != torch.bfloat16 or norm_weight.shape != (N,) or not norm_weight.is_contiguous():
+        raise TypeError("norm weights must be contiguous bfloat16 [N]")
+    x2 = _flat(x, K)
+    _inner_contig(x2, "x")
+    out = torch.empty(residual.shape, dtype=torch.bfloat16, device=x.device)
+    ss = torch.empty(M, N // 8, dtype=torch.float32, device=x.device)
+    code = _capi.native().decode_linear_add(x2, weight, bias, M, N, K, _row_stride(x2, K), residual, norm_weight, out, ss)
+    _capi.check(code, "based_decode_linear_add")
+    return NormRows(out, ss, eps)
 
 
 _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
@@ -493,6 +555,8 @@ def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> 
     """True when ``x W^T`` is a decode-step product the library's own kernel should run: a few bf16 rows in a layout it takes, and
     nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing).
     ``fused``: its epilogue takes the place of another launch."""
+    if type(x) is NormRows:
+        x = x.x
     K = x.shape[-1] if x.dim() else 0
     if not (0 < x.numel() <= K * DECODE_LINEAR_MAX_ROWS and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16):
         return False
@@ -512,7 +576,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if _decode_rows(x, weight) and (bias is None or (type(bias) in _PLAIN_TYPES and bias.dtype == torch.bfloat16
                                                      and bias.shape == weight.shape[:1] and bias.device == x.device)):
         return decode_linear(x, weight, bias)
-    return torch.nn.functional.linear(x, weight, bias)
+    return torch.nn.functional.linear(dense(x), weight, bias)
 
 
 def rotary_qkv_cache_(qkv: torch.Tensor, rotary_cos: torch.Tensor, rotary_sin: torch.Tensor,
@@ -617,11 +681,12 @@ def tp_outproj_allreduce_emulated(xs, weights, bias, workspaces, max_rows: int):
 
 def linear_f32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x W^T`` with an fp32 result (fp32 accumulation of the operands' products, not rounded to their dtype)."""
+    if _decode_rows(x, weight):
+        return decode_linear(x, weight, epilogue="f32")
+    x = dense(x)
     _need_cuda(x, weight)
     if x.dtype == torch.float32:
         return torch.nn.functional.linear(x, weight)
-    if _decode_rows(x, weight):
-        return decode_linear(x, weight, epilogue="f32")
     y = torch.mm(x.reshape(-1, x.shape[-1]), weight.t(), out_dtype=torch.float32)
     return y.view(*x.shape[:-1], weight.shape[0])
 

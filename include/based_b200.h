@@ -360,6 +360,19 @@ int based_decode_linear(const void* x, const void* w, const void* bias, void* ou
                         int conv_k, int conv_w_dtype, void* stream);
 
 /*
+ * The product before a norm and the one after it, for up to 16 rows, without a launch between them.
+ * _add: y = x W^T + bias is added to the fp32 stream residual [M, N] in place; out = bf16(stream * norm_weight[N]), contiguous
+ * [M, N]; ss [M, N / 8] fp32 = sums of the stream's squares over 8 columns.  _scaled: based_decode_linear with row i of x scaled by
+ * 1 / sqrt(sum of row_ss[i, 0 .. n_ss) / K + eps) (row_ss NULL: not scaled, any M).
+ */
+int based_decode_linear_add(const void* x, const void* w, const void* bias, int M, int N, int K, int64_t x_row_stride,
+                            void* residual, const void* norm_weight, void* out, void* ss, void* stream);
+int based_decode_linear_scaled(const void* x, const void* w, const void* bias, void* out, int M, int N, int K,
+                               int64_t x_row_stride, int64_t out_row_stride, int epilogue, int act, void* conv_state,
+                               const void* conv_weight, const void* conv_bias, int conv_k, int conv_w_dtype,
+                               const void* row_ss, int n_ss, float eps, void* stream);
+
+/*
  * Tensor-parallel decode step: row-parallel output projection fused with the all-reduce that follows it.
  *
  *   out[M, N] = sum over ranks r of x_r[M, K] W_r[N, K]^T (+ bias)        bf16 in / out, fp32 partials and sum

@@ -130,3 +130,27 @@ def test_linear_takes_the_kernel_only_where_it_can(ops):
     xg = x.clone().requires_grad_()
     ops.linear(xg, w).sum().backward()
     assert xg.grad is not None
+
+
+@pytest.mark.parametrize("M,D,K,F", [(16, 1024, 2048, 256), (1, 8, 32, 16), (5, 1792, 96, 64), (16, 2400, 64, 8)])
+def test_products_around_a_norm(ops, M, D, K, F):
+    """The product that adds to the stream and the products of its norm, against 64 bits: the stream to fp32, the normed rows and
+    their products to bf16's rounding of the rows (2^-9 each, averaged in the sums)."""
+    g = torch.Generator().manual_seed(D)
+    x, w, b = _mk(M, D, K, D + K, True)
+    res, n = torch.randn(M, D, generator=g) * 3, (1 + 0.1 * torch.randn(D, generator=g)).bfloat16()
+    z = res.double() + x.double() @ w.double().T + b.double()
+    want = z / torch.sqrt(z.square().mean(-1, keepdim=True) + 1e-5) * n.double()
+    stream = res.cuda()
+    rows = ops.linear_add_norm(x.cuda(), w.cuda(), b.cuda(), stream, n.cuda(), eps=1e-5)
+    assert type(rows) is ops.NormRows and rows.shape == (M, D) and rel_err(stream.cpu(), z) < 1e-5
+    assert rel_err(ops.dense(rows).double().cpu(), want) < 1e-2
+    if D % 32 == 0:
+        _, w3, b3 = _mk(1, 2 * F, D, F, True)
+        ref = want @ w3.double().T
+        assert rel_err(ops.decode_linear(rows, w3.cuda(), epilogue="f32").cpu(), ref) < 5e-3
+        assert rel_err(ops.linear(rows, w3.cuda(), b3.cuda()).double().cpu(), ref + b3.double()) < 1e-2
+        gated = ops.decode_linear(rows, w3.cuda(), b3.cuda(), epilogue="gated")
+        assert rel_err(gated.double().cpu(), O.gated_act(ref + b3.double(), "silu")) < 2e-2
+    odd = torch.randn(5, D, generator=g).bfloat16()      # not a weight of the kernel's: the rows are normed for torch
+    assert rel_err(ops.linear(rows, odd.cuda()).double().cpu(), want @ odd.double().T) < 2e-2

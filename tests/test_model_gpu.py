@@ -102,3 +102,22 @@ def test_generate_with_sampling():
     assert torch.equal(m.generate(ids, max_new_tokens=8, top_k=20, temperature=1e-4), greedy)
     g = m.generate(ids, max_new_tokens=8, cg=True, top_k=20, top_p=0.9, temperature=0.8)
     assert g.shape == (3, 28) and int(g.max()) < 211 and torch.equal(g[:, :20], ids)
+
+
+def test_steps_without_norm_launches_equal_watched_ones():
+    """A hook on a norm makes the step launch its norms; the logits and states agree to bf16 rounding either way."""
+    from based_b200 import ops
+    m = _small_model(seed=3)
+    ids = torch.randint(0, 211, (2, 9), device="cuda")
+    logits, seen = [], []
+    for watched in (False, True):
+        handle = m.transformer.layers[2].norm2.register_forward_hook(lambda *a: seen.append(1)) if watched else None
+        with torch.inference_mode():
+            ip = m.new_inference_params(2, 16)
+            m.advance(ids[:, :6], ip)
+            before = len(seen)
+            logits.append(torch.cat([m.advance(ids[:, i:i + 1], ip) for i in range(6, 9)], 1))
+        if watched:
+            assert len(seen) == before + 3
+            handle.remove()
+    assert rel_err(logits[0].float().cpu(), logits[1].float().cpu()) < 3e-2
