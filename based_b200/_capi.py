@@ -88,6 +88,9 @@ SIGNATURES = {
     "based_lightning": (c_int, [c_void_p] * 6 + [c_int] * 5 + [_I64P] * 4 + _POS + [c_int, c_int, c_void_p]),
     "based_lightning_scratch_bytes": (ctypes.c_size_t, [c_int] * 5),
     "based_lightning_split": (c_int, [c_void_p] * 6 + [c_int] * 5 + [_I64P] * 4 + _POS + [c_int, c_int, c_void_p, ctypes.c_size_t, c_void_p]),
+    "based_lightning_step_pieces": (c_int, [c_int] * 3),
+    "based_lightning_step_rows": (c_int, [c_void_p] * 4 + [c_int64] + [c_void_p] * 4 + [c_int64, c_void_p] + [c_int] * 5 + _POS
+                                  + [c_int, c_void_p]),
     "based_lightning_step": (c_int, [c_void_p] * 4 + [c_int64] + [c_void_p] * 6 + [c_int64] + [c_int] * 4 + _POS
                              + [c_float, c_int, c_void_p]),
 }

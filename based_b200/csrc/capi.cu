@@ -770,7 +770,26 @@ int based_lightning_step(const void* q, const void* k, const void* v, const void
   if (!launch_lightning_step) return BASED_ERR_IMPL;
   return launch_lightning_step(q, k, v, gate, x_row_stride, static_cast<const float*>(decay), norm_weight,
                                static_cast<float*>(state), static_cast<float*>(read), static_cast<int*>(count), out,
-                               out_row_stride, B, H, d, dv, offsets, offset, eps, io_dtype, static_cast<cudaStream_t>(stream));
+                               out_row_stride, nullptr, B, H, d, dv, offsets, offset, eps, io_dtype, static_cast<cudaStream_t>(stream));
+}
+
+int based_lightning_step_pieces(int B, int H, int dv) {
+  if (B <= 0 || H <= 0 || dv <= 0 || !lightning_step_pieces) return 0;
+  return lightning_step_pieces(B, H, dv);
+}
+
+int based_lightning_step_rows(const void* q, const void* k, const void* v, const void* gate, int64_t x_row_stride, const void* decay,
+                              const void* norm_weight, void* state, void* out, int64_t out_row_stride, void* ss, int n_ss, int B,
+                              int H, int d, int dv, const int32_t* offsets, int offset, int io_dtype, void* stream) {
+  if (!q || !k || !v || !gate || !decay || !norm_weight || !state || !out || !ss) return BASED_ERR_NULL;
+  if (!dtype_ok(io_dtype)) return BASED_ERR_DTYPE;
+  if (B < 0 || H <= 0 || d <= 0 || dv <= 0 || offset < 0) return BASED_ERR_SHAPE;
+  if (B == 0) return BASED_OK;
+  if (!launch_lightning_step) return BASED_ERR_IMPL;
+  if (n_ss != based_lightning_step_pieces(B, H, dv)) return BASED_ERR_SHAPE;
+  return launch_lightning_step(q, k, v, gate, x_row_stride, static_cast<const float*>(decay), norm_weight, static_cast<float*>(state),
+                               nullptr, nullptr, out, out_row_stride, static_cast<float*>(ss), B, H, d, dv, offsets, offset, 0.f,
+                               io_dtype, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

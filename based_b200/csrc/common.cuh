@@ -279,9 +279,10 @@ BASED_WEAK int launch_lightning_tc(const void* q, const void* k, const void* v, 
                                    const int32_t* offsets, int offset, void* scratch, size_t scratch_bytes, cudaStream_t stream);
 BASED_WEAK size_t lightning_tc_scratch_bytes(int B, int L, int H, int d, int dv);
 BASED_WEAK int read_tc_status_lightning(unsigned int* out, int reset);
+BASED_WEAK int lightning_step_pieces(int B, int H, int dv);
 BASED_WEAK int launch_lightning_step(const void* q, const void* k, const void* v, const void* gate, int64_t sx,
                                      const float* decay, const void* norm_w, float* state, float* read, int* count, void* out,
-                                     int64_t so, int B, int H, int d, int dv, const int32_t* offsets, int offset, float eps,
+                                     int64_t so, float* ss, int B, int H, int d, int dv, const int32_t* offsets, int offset, float eps,
                                      int io_dtype, cudaStream_t stream);
 
 }  // namespace based

@@ -46,11 +46,27 @@ class LightningAttention(StatefulMixer):
                 "read": torch.zeros(batch_size, H * dv, dtype=torch.float32, device=dev),     # workspace of a decode step
                 "count": torch.zeros(batch_size, dtype=torch.int32, device=dev)}
 
+    def forward(self, h, inference_params=None):
+        if (inference_params is not None and h.shape[1] == 1 and h.shape[0] <= ops.STEP_MAX_ROWS and ops.step_weight(self.out_proj.weight)
+                and ops._decode_rows(h, self.in_proj.weight)):
+            st = self.state(inference_params, h.dtype)
+            x = self.in_proj(h)
+            q, k, v, g = (self.in_proj.slice(x[:, 0], n) for n in "qkvg")
+            # the output projection takes the norm's factor per row: no block waits for all heads
+            rows = ops.lightning_step_rows(q, k, v, g, self.decay, self.norm_weight, st["state"], pos=self.position(inference_params, 1), eps=self.eps)
+            if rows is None:
+                rows = torch.empty(h.shape[0], 1, self.inner, dtype=h.dtype, device=h.device)
+                self._read_out(x, inference_params, rows)
+            return ops.linear(rows, self.out_proj.weight)
+        return super().forward(h, inference_params)
+
     def heads(self, h, inference_params, out):
-        L = h.shape[1]
-        st = self.state(inference_params, h.dtype)
+        self._read_out(self.in_proj(h), inference_params, out)
+
+    def _read_out(self, x, inference_params, out):
+        L = x.shape[1]
+        st = self.state(inference_params, x.dtype)
         pos = self.position(inference_params, L)
-        x = self.in_proj(h)
         q, k, v, g = (self.in_proj.slice(x, n) for n in "qkvg")
         if L == 1 and ops.lightning_step(q[:, 0], k[:, 0], v[:, 0], g[:, 0], self.decay, self.norm_weight, st["state"], st["read"],
                                          st["count"], pos=pos, eps=self.eps, out=out[:, 0]):

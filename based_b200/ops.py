@@ -1279,3 +1279,29 @@ def lightning_step(q, k, v, gate, decay, norm_weight, state, read, count, *, pos
         return False
     _capi.check(code, "based_lightning_step")
     return True
+
+
+def lightning_step_rows(q, k, v, gate, decay, norm_weight, state, *, pos, eps: float) -> Optional[NormRows]:
+    """:func:`lightning_step` with the norm's factor left to the product behind it: :class:`NormRows` ``[B, 1, H dv]`` for
+    :func:`decode_linear`.  None, nothing launched, for dtypes and sizes it does not take."""
+    _need_cuda(q, k, v, gate, decay, norm_weight, state)
+    B = q.shape[0]
+    _, H, d, dv = state.shape
+    if q.dtype != torch.bfloat16 or not 0 < B <= STEP_MAX_ROWS:
+        return None
+    _check_lightning(state, decay, B, H, d, dv)
+    _same_dtype(q, q=q, k=k, v=v, gate=gate, norm_weight=norm_weight)
+    if q.shape[1] != H * d or k.shape != q.shape or v.shape != (B, H * dv) or gate.shape != v.shape or norm_weight.shape != (H * dv,):
+        raise ValueError("q, k must be [B, H d] and v, gate [B, H dv]")
+    if len({t.stride(0) for t in (q, k, v, gate)}) > 1 and B > 1:
+        raise ValueError("q, k, v and gate must be slices of one tensor")
+    off, scalar = _position(pos, q)
+    pieces = _capi.lib().based_lightning_step_pieces(B, H, dv)
+    out = torch.empty(B, 1, H * dv, dtype=q.dtype, device=q.device)
+    ss = torch.empty(B, pieces, dtype=torch.float32, device=q.device)
+    code = _capi.native().lightning_step_rows(q, k, v, gate, q.stride(0), decay, norm_weight, state, out, H * dv, ss, pieces, B, H, d, dv,
+                                              off, scalar, _dt(q.dtype))
+    if code == _capi.ERR_IMPL:
+        return None
+    _capi.check(code, "based_lightning_step_rows")
+    return NormRows(out, ss, eps)

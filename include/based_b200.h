@@ -650,6 +650,14 @@ int based_lightning_split(const void* q, const void* k, const void* v, const voi
 int based_lightning_step(const void* q, const void* k, const void* v, const void* gate, int64_t x_row_stride, const void* decay,
                          const void* norm_weight, void* state, void* read, void* count, void* out, int64_t out_row_stride, int B,
                          int H, int d, int dv, const int32_t* offsets, int offset, float eps, int io_dtype, void* stream);
+/*
+ * The same with the norm's factor left to the product behind it (based_decode_linear_scaled): out = read-out * norm_weight *
+ * sigmoid(gate), ss [B, n_ss] the sums of the read-out's squares, n_ss = based_lightning_step_pieces.
+ */
+int based_lightning_step_pieces(int B, int H, int dv);
+int based_lightning_step_rows(const void* q, const void* k, const void* v, const void* gate, int64_t x_row_stride, const void* decay,
+                              const void* norm_weight, void* state, void* out, int64_t out_row_stride, void* ss, int n_ss, int B,
+                              int H, int d, int dv, const int32_t* offsets, int offset, int io_dtype, void* stream);
 
 #ifdef __cplusplus
 }

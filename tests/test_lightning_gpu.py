@@ -254,3 +254,26 @@ def test_token_input_in_one_launch(M, W, n):
     assert ops.token_side_step(stream.cuda(), x.float().cuda(), ids.cuda(), wg.float().cuda(), wp.float().cuda(), table.float().cuda(), n, norm.float().cuda()) is None
     big = torch.zeros(128, 2048).bfloat16().cuda()     # too much weight for one cluster
     assert ops.token_side_step(torch.zeros(1, 2048, device="cuda"), big[:1], ids[:1].cuda(), big, big.view(2048, 128), table.cuda().repeat(1, 128), 0, big[0]) is None
+
+
+@pytest.mark.parametrize("B,H,d,dv", [(1, 8, 128, 128), (16, 3, 64, 48), (5, 2, 16, 64), (2, 1, 256, 640)])
+def test_step_with_the_norm_left_to_the_product(B, H, d, dv):
+    """Read-out times weight and gate, and the sums of squares, against the step that norms: the rows they stand for to two
+    roundings to bf16, the states to the bit; and what it does not take."""
+    from based_b200 import ops
+    g = torch.Generator().manual_seed(d + dv)
+    packed = torch.randn(B, 2 * H * (d + dv), generator=g).bfloat16().cuda()
+    q, k, v, gate = packed.split([H * d, H * d, H * dv, H * dv], -1)
+    w = (1 + 0.2 * torch.randn(H * dv, generator=g)).bfloat16().cuda()
+    dec = torch.tensor([0.5 + 0.4 * i / H for i in range(H)], dtype=torch.float32, device="cuda")
+    S = torch.randn(B, H, d, dv, generator=g).cuda()
+    S1, S2, out = S.clone(), S.clone(), torch.empty(B, H * dv, dtype=torch.bfloat16, device="cuda")
+    read, count = torch.empty(B, H * dv, device="cuda"), torch.zeros(B, dtype=torch.int32, device="cuda")
+    pos = torch.tensor([i % 3 for i in range(B)], dtype=torch.int32, device="cuda")
+    assert ops.lightning_step(q, k, v, gate, dec, w, S1, read, count, pos=pos, eps=EPS, out=out)
+    rows = ops.lightning_step_rows(q, k, v, gate, dec, w, S2, pos=pos, eps=EPS)
+    assert torch.equal(S1, S2) and rows.shape == (B, 1, H * dv)
+    got = ops.dense(rows)[:, 0].double()
+    assert float((got - out.double()).abs().max() / out.double().abs().max()) < 2 ** -7
+    z = lambda *s: torch.zeros(*s, device="cuda")
+    assert ops.lightning_step_rows(z(1, 16), z(1, 16), z(1, 8), z(1, 8), z(2), z(8), z(1, 2, 8, 4), pos=0, eps=EPS) is None   # fp32
