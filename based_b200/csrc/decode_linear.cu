@@ -19,7 +19,7 @@
 //    chain of such launches does not stop between them.
 //  * All or half of a warp's loads are in flight at once for the usual K: eight or sixteen warps split K, a block owns 8 output
 //    columns (for two halves that an epilogue combines 8 of each; two or four times that where N would need more blocks than
-//    the device holds) and 16 or 32 rows (one or two m16n8k16 tiles, W read once for both).  Each lane reads 16 contiguous
+//    the device holds) and 16, 32 or 64 rows (m16n8k16 tiles, W read once for all).  Each lane reads 16 contiguous
 //    bytes of one weight row per step -- the K order inside a 32-wide block is permuted identically for x and W, which a dot
 //    product does not notice -- so a warp's load covers 8 rows x 64 bytes; x (a few KB, L2 resident) is read the same way.
 // In a chain of such launches, W from HBM, 16 rows (us; cuBLAS's kernel, this one, W at the HBM rate): 1024 x 1024 4.6, 2.9, 0.3;
@@ -235,6 +235,11 @@ int launch_tiles(const LinParams& p, int outputs, cudaStream_t stream) {
   constexpr int U1 = NT8 == 1 ? 8 : NT8 == 2 ? 4 : 2, U2 = NT8 == 1 ? 4 : 2;
   const int gx = (outputs / 8 + CT - 1) / CT;
   const dim3 g1(gx, 1), g2(gx, (p.M + 31) / 32);
+  // more rows: four tiles of 16, W read once for all of them, where registers and shared memory allow it (4096 x 1024 gated, 64
+  // rows: 8.3 us with two tiles and W read twice, 6.4 like this)
+  if constexpr (NT8 <= 2 && EPI != EPI_CONV && EPI != EPI_ADD) {
+    if (p.M > 32) return launch_pdl(decode_linear_kernel<CT, EPI, 4, 1, 8>, dim3(gx, (p.M + 63) / 64), dim3(256), 0, stream, p);
+  }
   // 16 warps to a block where K is long and every block has an SM: a warp's loads are one round again
   if constexpr (CT == 1) {
     if (p.K > 1024 && gx <= kSms) {

@@ -440,7 +440,9 @@ def gated_act(y: torch.Tensor, activation: str = "silu", out: Optional[torch.Ten
 # 4.8 / 8.3 (64); 1024 x 3072 8.6 / 3.5, 7.2 / 5.3; 1792 x 1792 5.2 / 3.6, 5.2 / 5.8; 7168 x 1792 7.4 / 6.9, 7.5 / 8.0, with the gated
 # activation 9.9 / 7.0, 9.9 / 8.5; 50280 x 1024 21 / 30.  So: up to 16 rows whatever K; up to 32 for a short K, for few enough
 # outputs that every block of the kernel has an SM, and where the epilogue saves a launch.
-DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_OUTPUTS = 32, 8192
+# With the gated activation and one round of blocks, some more: 4096 x 1024 and the library's 1024 x 2048 behind it 13.1 / 12.3 (33 rows),
+# 12.4 / 12.6 (48), 12.4 / 13.0 (64).
+DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_ROWS_GATED, DECODE_LINEAR_MAX_OUTPUTS = 32, 40, 8192
 
 
 def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, *,
@@ -551,14 +553,15 @@ def linear_add_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
 _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 
 
-def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False) -> bool:
+def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False, gated: bool = False) -> bool:
     """True when ``x W^T`` is a decode-step product the library's own kernel should run: a few bf16 rows in a layout it takes, and
     nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing).
-    ``fused``: its epilogue takes the place of another launch."""
+    ``fused``: its epilogue takes the place of another launch; ``gated``: that launch is the gated activation."""
     if type(x) is NormRows:
         x = x.x
     K = x.shape[-1] if x.dim() else 0
-    if not (0 < x.numel() <= K * DECODE_LINEAR_MAX_ROWS and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16):
+    most = DECODE_LINEAR_MAX_ROWS_GATED if gated and K <= 1024 and weight.shape[0] <= 2 * 8 * 296 else DECODE_LINEAR_MAX_ROWS
+    if not (0 < x.numel() <= K * most and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16):
         return False
     if type(x) is not torch.Tensor or type(weight) not in _PLAIN_TYPES or weight.dim() != 2 or weight.shape[0] > DECODE_LINEAR_MAX_OUTPUTS:
         return False

@@ -350,8 +350,8 @@ int based_rotary_qkv_cache(void* qkv, int B, int L, int H, int hd, const int64_t
  *
  *   x [M, K], W [N, K] (nn.Linear layout, contiguous), bias [N] or NULL, out as above; all bf16 (but F32's out);
  *   row strides in elements.  K a multiple of 32; the number of outputs a multiple of 8;
- *   x and W 16-byte aligned, x_row_stride a multiple of 8.  Built for M <= 32 (weights are read
- *   once per 32 rows); larger M works and re-reads W from L2 per 32 rows.
+ *   x and W 16-byte aligned, x_row_stride a multiple of 8.  Built for M <= 64 (weights are read
+ *   once per 32 or 64 rows); larger M works and re-reads W from L2.
  */
 int based_decode_linear(const void* x, const void* w, const void* bias, void* out,
                         int M, int N, int K, int64_t x_row_stride, int64_t out_row_stride,

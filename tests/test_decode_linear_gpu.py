@@ -84,7 +84,7 @@ def test_decode_linear_rejects_what_it_cannot_run(ops):
         ops.decode_linear(torch.randn(4, 64, device="cuda"), torch.randn(16, 64, device="cuda"))
 
 
-@pytest.mark.parametrize("M", [1, 16, 17, 32, 33])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65])
 @pytest.mark.parametrize("N,K", [(8 * 148, 1056), (8 * 149, 2048), (8 * 297, 64), (8 * 593, 96), (8 * 1189, 32)])
 def test_decode_linear_tilings(ops, M, N, K):
     """Where the number of column tiles per block, of row tiles and of warps changes, with a last block that is not full; every
