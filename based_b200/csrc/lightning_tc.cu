@@ -70,10 +70,11 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; a
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ uint32_t pack2(uint64_t v) { float lo, hi; split(v, lo, hi); return pack_bf16(lo, hi); }
 
-// volatile: stays where it is written, a chunk ahead of its use
+// volatile: stays where it is written, a chunk ahead of its use.  Not .nc: these kernels are programmatic launches, and a kernel that
+// triggers early may still be writing the activations when their blocks arrive.
 __device__ __forceinline__ uint4 load16(const bf16* src) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src));
+  asm volatile("ld.global.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src));
   return v;
 }
 

@@ -277,3 +277,35 @@ def test_step_with_the_norm_left_to_the_product(B, H, d, dv):
     assert float((got - out.double()).abs().max() / out.double().abs().max()) < 2 ** -7
     z = lambda *s: torch.zeros(*s, device="cuda")
     assert ops.lightning_step_rows(z(1, 16), z(1, 16), z(1, 8), z(1, 8), z(2), z(8), z(1, 2, 8, 4), pos=0, eps=EPS) is None   # fp32
+
+
+@pytest.mark.parametrize("L", [16, 24, 32, 1100])
+def test_inputs_written_by_the_launch_before(L):
+    """Chains in which the kernel before, which lets its successor start early, writes q, k and v into buffers that the call
+    before read: equal to the bit to the same chain with the device drained between the launches.  16 to 32 tokens: the
+    projection is a decode product; 1100: eight chunks and more, cut into segments."""
+    from based_b200 import ops
+    g = torch.Generator().manual_seed(L)
+    H, d, dv, n = 4, 64, 64, 12
+    width = H * (2 * d + dv)
+    w = (torch.randn(width, 512, generator=g) / 512 ** 0.5).bfloat16().cuda()
+    xs = [torch.randn(1, L, 512 if L <= 32 else 2 * width, generator=g).bfloat16().cuda() for _ in range(n)]
+    dec = torch.tensor([0.9, 0.5, 0.999, 1.0], dtype=torch.float32, device="cuda")
+
+    def chain(after):
+        packed, S, outs = torch.zeros(1, L, width, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, H, d, dv, device="cuda"), []
+        for i, x in enumerate(xs):
+            if L <= 32:
+                ops.decode_linear(x, w, out=packed)
+            else:
+                ops.gated_act(x, out=packed)
+            after()
+            outs.append(ops.lightning(*packed.split([H * d, H * d, H * dv], -1), dec, S, pos=i * L, impl="tcgen05"))
+            after()
+        return torch.stack(outs), S
+
+    want = chain(torch.cuda.synchronize)
+    for _ in range(8):
+        got = chain(lambda: None)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    ops.check_status()
