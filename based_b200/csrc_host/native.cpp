@@ -4,7 +4,8 @@
 // device looked up in Python): as much as 10 kernels of a short prompt take on the device.  Here an entry point is called with its
 // C arguments in order, without the last one, the stream: a tensor or None for a pointer, a tuple of integers or None for a
 // stride array, numbers for the rest.  The module makes the first tensor's device current and passes that device's current stream.
-// It returns the entry point's code.
+// It returns the entry point's code.  The interpreter lock is released around it, as by ctypes: a launch waits while the stream's
+// queue is full, and what empties the queue may need another Python thread.
 //
 // The entry points are looked up in the library the package has chosen (bind), not linked: a library of a part of the kernels
 // serves as well.
@@ -76,6 +77,11 @@ struct Arg {
   }
 };
 
+struct Unlocked {   // the interpreter lock comes back before an exception is caught
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 template <typename F>
 struct Caller;
 
@@ -96,6 +102,7 @@ struct Caller<int(A...)> {
         PyErr_SetString(PyExc_TypeError, "a call needs at least one CUDA tensor");
         return nullptr;
       }
+      Unlocked unlocked;   // the caller's references keep the tensors
       c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
       std::get<kGiven>(args).value = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream();
       code = fn(std::get<I>(args).value..., std::get<kGiven>(args).value);
