@@ -76,6 +76,20 @@ def test_linattn_prefill_fp32_shared_sequences(ops, B, H, L, dv):
         assert torch.equal(y2[:, :, :at], y[:, :, :at])
 
 
+@pytest.mark.parametrize("L", [60, 128, 129, 300, 512, 513, 1024, 2048])
+@pytest.mark.parametrize("dv", [64, 112])
+def test_linattn_prefill_fp32_state_roundings(ops, L, dv):
+    """The fp32 state sums L products in runs, whose length keeps the number of roundings near its least: run / 2 and L / run / 2
+    of them at full size in the sense of squares, sqrt(L) together at run = sqrt(L), and one for the products, each 2^-25 in
+    the mean.  64 CTAs of one sequence each: no cluster shortens the sums."""
+    q, k, v = (x.cuda() for x in _qkv(4, 16, L, dv, torch.float32, seed=L, qscale=1.0))
+    _, kv, _ = ops.linattn_prefill(q, k, v)
+    K = k.double()
+    phi = torch.cat([torch.ones_like(K[..., :1]), K / 2, (K.unsqueeze(-1) * K.unsqueeze(-2)).flatten(-2) / 2 ** 0.5 / 4], -1)
+    ref = v.double().transpose(-1, -2) @ phi
+    assert ((kv[:, :, 0].double() - ref).norm() / ref.norm()).item() < 2 ** -25 * (L ** 0.5 + 1) ** 0.5
+
+
 @pytest.mark.parametrize("B,H,L,dv,nseg", [(1, 2, 1024, 64, 2), (1, 2, 1024 + 77, 64, 3), (2, 1, 4096, 64, 8),
                                             (1, 1, 2048, 32, 4), (1, 1, 2048 + 5, 112, 5), (1, 3, 300, 64, 64),
                                             (1, 1, 128, 64, 4)])
