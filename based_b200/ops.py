@@ -10,6 +10,7 @@ import torch
 
 from torch._C._functorch import is_functorch_wrapped_tensor as _wrapped
 from torch.autograd import forward_ad as _forward_ad
+from torch.utils._device import DeviceContext as _DeviceContext
 
 from . import _capi
 from ._capi import BASED_BF16, BASED_F32, IMPL_AUTO, IMPL_DECODE, IMPL_SIMT, IMPL_TCGEN05  # noqa: F401
@@ -553,9 +554,17 @@ def linear_add_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
 _PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
 
 
+def _observed() -> bool:
+    """True while a dispatch or function mode (a FLOP counter, ``make_fx``, a logger) watches torch's operators: a product must then be
+    one of them.  ``torch.device`` as a context is a function mode too, but only sets the device of new tensors."""
+    n = torch._C._len_torch_function_stack()
+    return torch._C._len_torch_dispatch_stack() > 0 or (
+        n > 0 and any(type(torch._C._get_function_stack_at(i)) is not _DeviceContext for i in range(n)))
+
+
 def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False, gated: bool = False) -> bool:
     """True when ``x W^T`` is a decode-step product the library's own kernel should run: a few bf16 rows in a layout it takes, and
-    nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing).
+    nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing, modes).
     ``fused``: its epilogue takes the place of another launch; ``gated``: that launch is the gated activation."""
     if type(x) is NormRows:
         x = x.x
@@ -571,7 +580,7 @@ def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False, gat
             and (x.is_contiguous() or (x.stride(-1) == 1 and all(st % 8 == 0 for st in x.stride()[:-1])))
             and x.device == weight.device and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
             and _forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
-            and not _wrapped(x) and not _wrapped(weight) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+            and not _observed() and not _wrapped(x) and not _wrapped(weight) and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -132,6 +132,35 @@ def test_linear_takes_the_kernel_only_where_it_can(ops):
     assert xg.grad is not None
 
 
+def test_modes_see_the_products(ops, monkeypatch):
+    """A FLOP counter and a function mode find every product of a few rows, as they do for many; a device context is no
+    reason to leave the kernel."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils.flop_counter import FlopCounterMode
+    w = (torch.randn(64, 96, device="cuda") / 10).bfloat16()
+    x = torch.randn(4, 96, device="cuda").bfloat16()
+
+    class Names(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            names.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+
+    names, ran = [], []
+    kernel = ops.decode_linear
+    monkeypatch.setattr(ops, "decode_linear", lambda *a, **k: ran.append(1) or kernel(*a, **k))
+    with torch.no_grad():
+        for product in (ops.linear, ops.linear_f32):
+            with FlopCounterMode(display=False) as flops:
+                product(x, w)
+            assert flops.get_total_flops() == 2 * 4 * 96 * 64
+        with Names():
+            ops.linear(x, w)
+        assert "linear" in names and not ran
+        with torch.device("cuda"):
+            ops.linear(x, w)
+        assert len(ran) == 1
+
+
 @pytest.mark.parametrize("M,D,K,F", [(16, 1024, 2048, 256), (1, 8, 32, 16), (5, 1792, 96, 64), (16, 2400, 64, 8)])
 def test_products_around_a_norm(ops, M, D, K, F):
     """The product that adds to the stream and the products of its norm, against 64 bits: the stream to fp32, the normed rows and

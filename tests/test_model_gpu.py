@@ -121,3 +121,17 @@ def test_steps_without_norm_launches_equal_watched_ones():
             assert len(seen) == before + 3
             handle.remove()
     assert rel_err(logits[0].float().cpu(), logits[1].float().cpu()) < 3e-2
+
+
+def test_flop_counter_sees_a_decode_step():
+    """Every product of a step is one of torch's operators while a mode watches: two operations per weight and row."""
+    from torch.utils.flop_counter import FlopCounterMode
+    m = _small_model(seed=5)
+    weights = sum(mod.weight.numel() for mod in m.modules() if type(mod) is torch.nn.Linear)
+    ids = torch.randint(0, 211, (2, 7), device="cuda")
+    with torch.inference_mode():
+        ip = m.new_inference_params(2, 16)
+        m.advance(ids[:, :6], ip)
+        with FlopCounterMode(display=False) as flops:
+            m.advance(ids[:, 6:], ip)
+    assert flops.get_total_flops() == 2 * 2 * weights
