@@ -235,10 +235,13 @@ int launch_tiles(const LinParams& p, int outputs, cudaStream_t stream) {
   constexpr int U1 = NT8 == 1 ? 8 : NT8 == 2 ? 4 : 2, U2 = NT8 == 1 ? 4 : 2;
   const int gx = (outputs / 8 + CT - 1) / CT;
   const dim3 g1(gx, 1), g2(gx, (p.M + 31) / 32);
-  // more rows: four tiles of 16, W read once for all of them, where registers and shared memory allow it (4096 x 1024 gated, 64
-  // rows: 8.3 us with two tiles and W read twice, 6.4 like this)
+  // More rows: four tiles of 16, W read once for all of them, where registers and shared memory allow it (64 rows, us with two tiles
+  // and W read twice / like this: 4096 x 1024 8.2 / 6.3, with the gated activation the same; 1792 x 1792 10.8 / 7.1).  Not with the
+  // gated activation while two tiles need no second round of blocks: 2048 x 1024 4.2 / 5.2 (33 rows), 4.2 / 6.0 (64).
   if constexpr (NT8 <= 2 && EPI != EPI_CONV && EPI != EPI_ADD) {
-    if (p.M > 32) return launch_pdl(decode_linear_kernel<CT, EPI, 4, 1, 8>, dim3(gx, (p.M + 63) / 64), dim3(256), 0, stream, p);
+    const int resident = CT == 1 && p.K > 1024 && gx <= kSms ? kSms : 2 * kSms;
+    const bool once = EPI == EPI_SWIGLU && (int64_t)gx * g2.y <= resident;
+    if (p.M > 32 && !once) return launch_pdl(decode_linear_kernel<CT, EPI, 4, 1, 8>, dim3(gx, (p.M + 63) / 64), dim3(256), 0, stream, p);
   }
   // 16 warps to a block where K is long and every block has an SM: a warp's loads are one round again
   if constexpr (CT == 1) {

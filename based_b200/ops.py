@@ -438,11 +438,12 @@ def gated_act(y: torch.Tensor, activation: str = "silu", out: Optional[torch.Ten
 
 # Where a product goes to decode_linear; beyond, the library GEMM is the better tool.  us a launch in a chain of such launches with
 # the weights from HBM, cuBLAS / ours (N x K, rows): 1024 x 1024 4.6 / 2.9 (16), 4.2 / 3.6 (32); 4096 x 1024 4.7 / 3.1, 4.8 / 4.3,
-# 4.8 / 8.3 (64); 1024 x 3072 8.6 / 3.5, 7.2 / 5.3; 1792 x 1792 5.2 / 3.6, 5.2 / 5.8; 7168 x 1792 7.4 / 6.9, 7.5 / 8.0, with the gated
+# 4.9 / 6.3 (64); 1024 x 3072 8.6 / 3.5, 7.2 / 5.3; 1792 x 1792 5.2 / 3.6, 5.2 / 5.8; 7168 x 1792 7.4 / 6.9, 7.5 / 8.0, with the gated
 # activation 9.9 / 7.0, 9.9 / 8.5; 50280 x 1024 21 / 30.  So: up to 16 rows whatever K; up to 32 for a short K, for few enough
 # outputs that every block of the kernel has an SM, and where the epilogue saves a launch.
-# With the gated activation and one round of blocks, some more: 4096 x 1024 and the library's 1024 x 2048 behind it 13.1 / 12.3 (33 rows),
-# 12.4 / 12.6 (48), 12.4 / 13.0 (64).
+# With the gated activation and one round of blocks, some more.  An MLP whose second product is the library's, library / ours (width x
+# hidden, 33 and 40 rows): 512 x 1024 9.5 / 8.1, 9.5 / 8.2; 768 x 1536 10.9 / 10.5, 10.9 / 10.6; 1024 x 1024 10.3 / 9.2, 10.3 / 9.4;
+# 1024 x 2048 12.3 / 12.2, 12.3 / 12.3, behind a norm 14.4 / 12.9, 14.4 / 13.1.  At 48 rows 1024 x 2048 is 12.4 / 12.6.
 DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_ROWS_GATED, DECODE_LINEAR_MAX_OUTPUTS = 32, 40, 8192
 
 

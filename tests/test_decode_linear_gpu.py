@@ -85,7 +85,7 @@ def test_decode_linear_rejects_what_it_cannot_run(ops):
 
 
 @pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65])
-@pytest.mark.parametrize("N,K", [(8 * 148, 1056), (8 * 149, 2048), (8 * 297, 64), (8 * 593, 96), (8 * 1189, 32)])
+@pytest.mark.parametrize("N,K", [(8 * 148, 1056), (8 * 148, 96), (8 * 149, 2048), (8 * 297, 64), (8 * 593, 96), (8 * 1189, 32)])
 def test_decode_linear_tilings(ops, M, N, K):
     """Where the number of column tiles per block, of row tiles and of warps changes, with a last block that is not full; every
     epilogue, outputs against the sum in 64 bits to their last rounding plus the sum's own in fp32."""
