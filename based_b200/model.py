@@ -95,12 +95,13 @@ class Block(nn.Module):
 
     def step_ok(self, width):
         """True when a decode step may run without launches of their own for the norms: the stream is fp32, nobody watches the
-        modules, and the products around them are ones :func:`ops.linear_add_norm` and :func:`ops.decode_linear` take."""
+        modules or has put another forward on them, and the products around them are ones :func:`ops.linear_add_norm` and
+        :func:`ops.decode_linear` take."""
         norms = (self.norm1, self.norm2)
         weights = self.mixer.step_weights() if type(self.mixer) in (BaseConv, LinearAttention, SlidingAttention) else None
         if weights is None or not self.residual_in_fp32 or type(self.mlp) is not GatedMlp or self.mlp.return_residual:
             return False
-        if any(m._forward_hooks or m._forward_pre_hooks for m in (self, self.mixer, self.mlp, *norms)):
+        if any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in (self, self.mixer, self.mlp, *norms)):
             return False
         if any(type(n) is not RMSNorm or n.bias is not None or n.weight.dtype != torch.bfloat16 for n in norms):
             return False

@@ -135,3 +135,21 @@ def test_flop_counter_sees_a_decode_step():
         with FlopCounterMode(display=False) as flops:
             m.advance(ids[:, 6:], ip)
     assert flops.get_total_flops() == 2 * 2 * weights
+
+
+@pytest.mark.parametrize("where", ["layer", "mixer", "mlp", "norm1", "norm2"])
+def test_a_forward_put_on_a_module_runs_in_steps(where):
+    """A module whose ``forward`` was replaced on the instance (as libraries do that move weights around a call) is called through
+    it, in prompts and in steps."""
+    m = _small_model(seed=6)
+    layer = m.transformer.layers[2]
+    module = layer if where == "layer" else getattr(layer, where)
+    calls, own = [], module.forward
+    module.forward = lambda *a, **k: calls.append(1) or own(*a, **k)
+    ids = torch.randint(0, 211, (2, 8), device="cuda")
+    with torch.inference_mode():
+        ip = m.new_inference_params(2, 16)
+        m.advance(ids[:, :6], ip)
+        for i in (6, 7):
+            m.advance(ids[:, i:i + 1], ip)
+    assert len(calls) == 3
