@@ -100,6 +100,13 @@ inline int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, 
   return (int)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// A launcher's answer where it has the launch's own code: the runtime keeps a copy of an error for the next cudaGetLastError, which
+// would report it for a launch that went well.
+inline int launched(int code) {
+  if (code != 0) cudaGetLastError();
+  return code;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Launchers implemented one per .cu file; all return a cudaError_t-compatible int (0 = ok).

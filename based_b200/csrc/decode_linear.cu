@@ -278,10 +278,10 @@ int launch_decode_linear(const void* x, const void* w, const void* bias, void* o
               static_cast<const __nv_bfloat16*>(bias), out, M, N, K, sx, so, act,
               static_cast<__nv_bfloat16*>(conv_state), conv_weight, conv_bias, conv_k, conv_w_dtype == BASED_BF16,
               row_ss, n_ss, eps, nullptr, nullptr, nullptr};
-  if (epilogue == EPI_PLAIN) return launch_epi<EPI_PLAIN>(p, outputs, stream);
-  if (epilogue == EPI_SWIGLU) return launch_epi<EPI_SWIGLU>(p, outputs, stream);
-  if (epilogue == EPI_CONV) return launch_epi<EPI_CONV>(p, outputs, stream);
-  if (epilogue == EPI_F32) return launch_epi<EPI_F32>(p, outputs, stream);
+  if (epilogue == EPI_PLAIN) return launched(launch_epi<EPI_PLAIN>(p, outputs, stream));
+  if (epilogue == EPI_SWIGLU) return launched(launch_epi<EPI_SWIGLU>(p, outputs, stream));
+  if (epilogue == EPI_CONV) return launched(launch_epi<EPI_CONV>(p, outputs, stream));
+  if (epilogue == EPI_F32) return launched(launch_epi<EPI_F32>(p, outputs, stream));
   return BASED_ERR_SHAPE;
 }
 
@@ -293,7 +293,7 @@ int launch_decode_linear_add(const void* x, const void* w, const void* bias, int
   LinParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w),
               static_cast<const __nv_bfloat16*>(bias), out, M, N, K, sx, N, 0, nullptr, nullptr, nullptr, 0, 0,
               nullptr, 0, 0.f, residual, ss, static_cast<const __nv_bfloat16*>(norm)};
-  return launch_epi<EPI_ADD>(p, N, stream);
+  return launched(launch_epi<EPI_ADD>(p, N, stream));
 }
 
 }  // namespace based

@@ -443,7 +443,7 @@ int launch_typed(const void* q, const void* k, const void* v, void* y, void* kv_
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = K > 1 ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, kern, args);
+  return launched((int)cudaLaunchKernelEx(&cfg, kern, args));
 }
 
 }  // namespace

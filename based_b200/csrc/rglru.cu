@@ -195,7 +195,7 @@ int launch_rglru_step(const void* x, const void* y, const void* cw, const void* 
                   static_cast<const T*>(gw), static_cast<const T*>(rb), static_cast<const T*>(ib), lam, static_cast<T*>(ring),
                   static_cast<T*>(out), state, offsets, sx, sy, so, offset, B, W, n, taps};
   auto kern = taps == 2 ? rglru_step_kernel<2> : taps == 3 ? rglru_step_kernel<3> : rglru_step_kernel<4>;
-  return launch_pdl(kern, dim3(W / kStepCh, (B + 15) / 16), dim3(kStepThreads), 0, stream, p);
+  return launched(launch_pdl(kern, dim3(W / kStepCh, (B + 15) / 16), dim3(kStepThreads), 0, stream, p));
 }
 
 int launch_rglru(const void* u, const void* y, const float* gates, const void* rb, const void* ib, const float* lam,

@@ -376,7 +376,7 @@ int launch_rglru_tc(const void* u, const void* y, const void* w, const void* rb,
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = p.K > 1 ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, rglru_tc_kernel, p);
+  return launched((int)cudaLaunchKernelEx(&cfg, rglru_tc_kernel, p));
 }
 
 }  // namespace based

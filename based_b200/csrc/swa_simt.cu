@@ -450,8 +450,8 @@ int launch_swa_decode(const void* q, const void* k_new, const void* v_new, void*
         static_cast<T*>(kv_cache), cache_seqlens, cache_seqlen_scalar, static_cast<const T*>(rotary_cos),
         static_cast<const T*>(rotary_sin), rotary_dim, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
   };
-  if (io_dtype == BASED_BF16) return run(__nv_bfloat16{});
-  if (io_dtype == BASED_F32) return run(float{});
+  if (io_dtype == BASED_BF16) return launched(run(__nv_bfloat16{}));
+  if (io_dtype == BASED_F32) return launched(run(float{}));
   return BASED_ERR_DTYPE;
 }
 

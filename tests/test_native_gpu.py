@@ -63,3 +63,47 @@ def test_errors_after_a_call_and_before_one(stub):
         module.gated_act(x.cpu(), x, x, 1, 8, 16, 16, 16, 0, 0)
     lib.release()
     assert module.gated_act(x, x, x, 1, 8, 16, 16, 16, 0, 0) == 0
+
+
+def _launchers():
+    from based_b200 import ops
+    g = torch.Generator("cuda").manual_seed(0)
+    r = lambda *s, dtype=torch.bfloat16: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    W, n, B = 64, 32, 2
+    rg = [r(W // n, 2, n, n), r(W), r(W), r(W, dtype=torch.float32)]
+    x, w, o = r(2, 64), r(16, 64), r(2, 16)
+    q, k, v, y = r(1, 2, 70, 16, dtype=torch.float32), r(1, 2, 70, 16, dtype=torch.float32), r(1, 2, 70, 16, dtype=torch.float32), r(1, 2, 70, 16, dtype=torch.float32)
+    cache, h, ctx = r(B, 8, 2, 2, 16), r(B, 1, 2, 16), r(B, 1, 2, 16)
+    u, out, S, ring, taps = r(B, 16, W), r(B, 16, W), r(B, W, dtype=torch.float32), r(B, 4, W), r(W, 4)
+    return {
+        "decode_linear": lambda: ops.decode_linear(x, w, out=o),
+        "linattn_prefill": lambda: ops.linattn_prefill(q, k, v, out=y, return_state=False),
+        "swa_decode": lambda: ops.swa_decode(h, h, h, cache, 3, 4, out=ctx),
+        "rglru_gated": lambda: ops.rglru_gated(u, u, *rg, S, pos=0, out=out),
+        "rglru_step": lambda: ops.rglru_step(u[:, 0], u[:, 1], taps, None, ring, *rg, S, pos=1, out=out[:, 0]),
+    }
+
+
+@pytest.mark.parametrize("name", ["decode_linear", "linattn_prefill", "swa_decode", "rglru_gated", "rglru_step"])
+def test_a_refused_launch_leaves_no_error_behind(name):
+    """A launch into a capture that has been invalidated (by waiting for its stream) is refused by the runtime; the calls after it
+    answer for themselves."""
+    from based_b200 import ops
+    launch = _launchers()[name]
+    launch()                                    # first uses load modules and set attributes
+    other, gate = torch.randn(2, 32, device="cuda"), torch.empty(2, 16, device="cuda")
+    torch.cuda.synchronize()
+    rt, s = ctypes.CDLL("libcudart.so.12"), torch.cuda.Stream()
+    stream, graph = ctypes.c_void_p(s.cuda_stream), ctypes.c_void_p()
+    with torch.cuda.stream(s):
+        assert rt.cudaStreamBeginCapture(stream, 2) == 0
+        assert rt.cudaStreamSynchronize(stream) != 0
+        try:
+            with pytest.raises(_capi.BasedLibraryError):
+                launch()
+        finally:
+            rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+            rt.cudaGetLastError()
+    got = ops.gated_act(other, out=gate)
+    assert torch.equal(got, gate)
+    torch.cuda.synchronize()
