@@ -1,4 +1,5 @@
-"""The host path of the kernel calls (csrc_host/native.cpp) on a second copy of the module that is bound to a stub library."""
+"""The host path of the kernel calls (csrc_host/native.cpp), in part on a second copy of the module that is bound to a stub
+library, and chains of programmatic launches."""
 import ctypes
 import importlib.machinery
 import importlib.util
@@ -107,3 +108,62 @@ def test_a_refused_launch_leaves_no_error_behind(name):
     got = ops.gated_act(other, out=gate)
     assert torch.equal(got, gate)
     torch.cuda.synchronize()
+
+
+class Drained:
+    """The extension module with the device drained after every call."""
+
+    def __init__(self, module):
+        self.module = module
+
+    def __getattr__(self, name):
+        fn = getattr(self.module, name)
+
+        def call(*args):
+            code = fn(*args)
+            torch.cuda.synchronize()
+            return code
+        return call
+
+
+def _tensors(x):
+    if torch.is_tensor(x):
+        return [x]
+    return [t for y in (x.values() if isinstance(x, dict) else x) for t in _tensors(y)]
+
+
+@pytest.mark.parametrize("stack,B", [("based", 1), ("based", 16), ("based", 20), ("razesun", 3), ("vubenex", 1), ("vubenex", 17)])
+def test_chains_equal_the_same_launches_one_at_a_time(stack, B, monkeypatch):
+    """Prompt, portions and decode steps, whose kernels start under the ones before them, give to the bit the logits and states
+    of the same calls with nothing in flight between them."""
+    if stack == "based":
+        from test_model_gpu import _small_model
+        m = _small_model(seed=11)
+    elif stack == "razesun":
+        from test_razesun_gpu import build
+        m = build("mixed", torch.bfloat16)[2]
+    else:
+        import vubenex_models
+        from test_vubenex_gpu import build
+        m = build(vubenex_models.configs()["wide"], torch.bfloat16)[1]
+    g = torch.Generator().manual_seed(B)
+    pieces = [40] + [1] * 8 if stack == "based" else [40, 24, 1, 1, 16] + [1] * 6
+    ids = torch.randint(0, 90, (B, sum(pieces)), generator=g).cuda()
+
+    @torch.inference_mode()
+    def run():
+        ip = m.new_inference_params(B, sum(pieces))
+        for t in _tensors(ip.key_value_memory_dict):
+            t.zero_()
+        out, at = [], 0
+        for n in pieces:
+            out.append(m.advance(ids[:, at:at + n], ip))
+            at += n
+        return out + _tensors(ip.key_value_memory_dict)
+
+    real = _capi.native()
+    with monkeypatch.context() as patch:
+        patch.setattr(_capi, "native", lambda: Drained(real))
+        want = run()
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(run(), want, strict=True))
