@@ -118,3 +118,23 @@ def test_norm_act_full_size_properties(ops):
     h = ops.gated_act(y, "silu")
     assert torch.equal(ops.gated_act(y[777:900], "silu"), h[777:900])
     assert rel_err(h[:64].cpu().double(), O.gated_act(y[:64].cpu().double(), "silu")) < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("D", [512, 1024, 1792, 4096, 8192])
+def test_many_rows_equal_few(ops, D):
+    """Few rows run as a programmatic launch with the weights loaded early, many without either: the same arithmetic, so rows
+    of a large call equal those of a small one to the bit.  1185 rows is one above the gated activation's border; the norms'
+    lies between the two sizes for every width."""
+    g = torch.Generator("cuda").manual_seed(D)
+    r = lambda *s, dtype=torch.bfloat16: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    M, m = 1185, 5
+    x, res, w, w2, gate = r(M, D), r(M, D, dtype=torch.float32), r(D), r(D), r(M, D)
+
+    def all_ops(n):
+        stream, post = res[:n].clone(), res[:n].clone()
+        return [*ops.add_rmsnorm(x[:n], w, residual=res[:n], prenorm=True, residual_in_fp32=True), ops.rmsnorm(x[:n], w, 1e-6),
+                *ops.stream_norm(stream, w, w2, branch=x[:n]), stream, ops.stream_post_norm(post, x[:n], w, out_weight=w2, eps=1e-5), post,
+                ops.norm_gate(x[:n], w, gate[:n], 1e-5), ops.gated_act(x[:n])]
+
+    for many, few in zip(all_ops(M), all_ops(m), strict=True):
+        assert torch.equal(many[:m], few)
