@@ -96,26 +96,36 @@ __device__ __forceinline__ Row8 unpack8(const uint4 (&r)[2]) {
                __uint_as_float(r[1].x), __uint_as_float(r[1].y), __uint_as_float(r[1].z), __uint_as_float(r[1].w)}};
 }
 
-// One block per (batch, head).  A step's bytes (a window of keys and values, 16 KB a head) take less than a microsecond; what
-// it takes is the chain load - scores - softmax - values.  So the window is spread over the block: LPK lanes share a cached
-// row, 8 values (16 or 32 bytes) each, a group of lanes has every (32 / LPK * WARPS)-th key, and its first four keys AND values
-// are in flight before the query is rotated.  Each group keeps a running maximum, sum and weighted row of its own keys; the
-// groups meet once at the end.  16 heads, 16 rows, hd = 64, 64 keys: 10.6 us with one warp per head (keys, softmax, values in
-// turn), 4.4 us like this.  hd is a multiple of 8 and the cache 16-byte aligned (checked by the launcher).
-template <typename IO, int LPK, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+// A (batch, head) has a block of WARPS warps, or HEADS of them share a block, a warp each.  A step's bytes (a window of keys and
+// values, 16 KB a head) take less than a microsecond; what it takes is the chain load - scores - softmax - values.  So the window
+// is spread over the warps: LPK lanes share a cached row, 8 values (16 or 32 bytes) each, a group of lanes has every
+// (32 / LPK * WARPS)-th key, and its first four keys AND values are in flight before the query is rotated.  Each group keeps a
+// running maximum, sum and weighted row of its own keys; the groups meet once at the end.  16 heads, 16 rows, hd = 64, 64 keys: 6.5 us
+// with one warp per head (keys, softmax, values in turn), 3.6 us like this, in a chain of such launches.  hd is a multiple of 8 and
+// the cache 16-byte aligned (checked by the launcher).
+template <typename IO, int LPK, int WARPS, int HEADS>
+__global__ void __launch_bounds__(WARPS * HEADS * 32)
 swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
                   IO* o, IO* kv_cache, const int32_t* cache_seqlens,
                   int cache_seqlen_scalar, const IO* rcos, const IO* rsin, int rotary_dim,
-                  int H, int hd, int max_seqlen, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
+                  int BH, int H, int hd, int max_seqlen, Strides2 sq, Strides2 sk, Strides2 sv, Strides2 so,
                   int window_left, float scale) {
   pdl_trigger();
   pdl_wait();
   constexpr int kGroups = WARPS * 32 / LPK, U = 4, kVec = sizeof(IO) / 2;
-  __shared__ float s_q[kMaxHd], s_k[kMaxHd], s_v[kMaxHd], s_r[2][kMaxHd];
-  __shared__ float s_o[WARPS][kMaxHd], s_m[WARPS], s_l[WARPS];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int b = blockIdx.x / H, h = blockIdx.x - b * H;
+  static_assert(HEADS == 1 || WARPS == 1, "heads of a block leave it on their own");
+  __shared__ float sq_[HEADS][kMaxHd], sk_[HEADS][kMaxHd], sv_[HEADS][kMaxHd], sr_[HEADS][2][kMaxHd];
+  __shared__ float so_[HEADS][WARPS][kMaxHd], sm_[HEADS][WARPS], sl_[HEADS][WARPS];
+  const int slot = HEADS == 1 ? 0 : threadIdx.x >> 5, tid = HEADS == 1 ? threadIdx.x : threadIdx.x & 31, lane = tid & 31, warp = tid >> 5;
+  float *s_q = sq_[slot], *s_k = sk_[slot], *s_v = sv_[slot], *s_m = sm_[slot], *s_l = sl_[slot];
+  float (*s_r)[kMaxHd] = sr_[slot], (*s_o)[kMaxHd] = so_[slot];
+  auto sync = [] {
+    if constexpr (WARPS == 1) __syncwarp();
+    else __syncthreads();
+  };
+  const int bh = blockIdx.x * HEADS + slot;
+  if (bh >= BH) return;
+  const int b = bh / H, h = bh - b * H;
   const int pos = cache_seqlens ? cache_seqlens[b] : cache_seqlen_scalar;
   if (pos < 0 || pos >= max_seqlen) return;  // nothing sensible to do; the host validates the scalar case
   const size_t row = (size_t)2 * H * hd;  // elements per cached position
@@ -145,7 +155,7 @@ swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
     s_r[1][i] = to_float(kp[i]);
     s_v[i] = to_float(vp[i]);
   }
-  __syncthreads();
+  sync();
   const int half = rcos ? rotary_dim / 2 : 0;
   for (int i = tid; i < 2 * hd; i += WARPS * 32) {
     const int which = i >= hd, cc = which ? i - hd : i;
@@ -164,7 +174,7 @@ swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
       knew[(size_t)H * hd + cc] = vp[cc];
     }
   }
-  __syncthreads();
+  sync();
   float qv[8], acc[8], m = -INFINITY, l = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) { qv[i] = on ? s_q[c + i] : 0.f; acc[i] = 0.f; }
@@ -235,7 +245,7 @@ swa_decode_kernel(const IO* q, const IO* k_new, const IO* v_new,
 #pragma unroll
     for (int i = 0; i < 8; ++i) s_o[warp][c + i] = acc[i];
   if (lane == 0) { s_m[warp] = top; s_l[warp] = l; }
-  __syncthreads();
+  sync();
   for (int i = tid; i < hd; i += WARPS * 32) {
     float mm = s_m[0], sum = 0.f, y = 0.f;
 #pragma unroll
@@ -442,13 +452,33 @@ int launch_swa_decode(const void* q, const void* k_new, const void* v_new, void*
   if (window_left + 1 > kMaxKeysPerLane * 32) return BASED_ERR_TOO_LARGE;
   if (!aligned16(kv_cache) || hd % 8 != 0) return BASED_ERR_ALIGN;  // 16-byte reads of cached rows
   if ((int64_t)B * H > 0x7fffffff) return BASED_ERR_TOO_LARGE;
+  const int BH = B * H;
   auto run = [&](auto zero) {
     using T = decltype(zero);
-    auto kern = hd <= 64 ? swa_decode_kernel<T, 8, 4> : swa_decode_kernel<T, 16, 8>;   // 64 keys in the first round either way
-    return launch_pdl(kern, dim3(B * H), dim3(hd <= 64 ? 128 : 256), 0, stream,
-        static_cast<const T*>(q), static_cast<const T*>(k_new), static_cast<const T*>(v_new), static_cast<T*>(o),
-        static_cast<T*>(kv_cache), cache_seqlens, cache_seqlen_scalar, static_cast<const T*>(rotary_cos),
-        static_cast<const T*>(rotary_sin), rotary_dim, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
+    auto go = [&](auto kern, int warps, int heads) {
+      return launch_pdl(kern, dim3((BH - 1) / heads + 1), dim3(warps * heads * 32), 0, stream,
+          static_cast<const T*>(q), static_cast<const T*>(k_new), static_cast<const T*>(v_new), static_cast<T*>(o),
+          static_cast<T*>(kv_cache), cache_seqlens, cache_seqlen_scalar, static_cast<const T*>(rotary_cos),
+          static_cast<const T*>(rotary_sin), rotary_dim, BH, H, hd, max_seqlen, sq, sk, sv, so, window_left, scale);
+    };
+    // Warps per head: few heads want the window in flight at once, many heads fewer blocks and warps.  us with 1 / 2 / 4 / 8 warps (one
+    // warp: four heads to a block), windows of 16, 32, 64, 128 keys.  hd = 64: 16 heads 3.2 / 2.6 / 2.6, 3.7 / 2.7 / 2.7, 5.0 / 3.2 / 2.7,
+    // 7.5 / 4.2 / 3.2; 512 heads 3.5 / 4.0 / 4.5, 4.2 / 4.0 / 4.6, 5.5 / 4.9 / 4.6, 8.2 / 6.8 / 6.0; 4096 heads 7.6 / 10.6 / 16, 9.5 / 10.8 / 17,
+    // 15.9 / 15.1 / 17.6, 31 / 28 / 28.  hd = 112: 16 heads - / 3.0 / 2.8 / 3.2, - / 3.6 / 2.8 / 3.4, - / 4.8 / 3.4 / 3.4, - / 7.1 / 4.6 / 4.0; 4096 heads
+    // 12.5 / 12.4 / 19 / 36, 18.5 / 16.7 / 20 / 37, 33 / 27 / 29 / 41, 56 / 47 / 46 / 56.
+    const int keys = window_left + 1;
+    const bool many = BH > 5 * 148;
+    if (hd <= 64) {
+      const int warps = many ? (keys <= 40 ? 1 : keys <= 80 ? 2 : 4) : (keys <= 40 ? 2 : 4);
+      if (warps == 1) return go(swa_decode_kernel<T, 8, 1, 4>, 1, 4);
+      if (warps == 2) return go(swa_decode_kernel<T, 8, 2, 1>, 2, 1);
+      return go(swa_decode_kernel<T, 8, 4, 1>, 4, 1);
+    }
+    const int warps = many ? (keys <= 9 ? 1 : keys <= 40 ? 2 : 4) : (keys <= 80 ? 4 : 8);
+    if (warps == 1) return go(swa_decode_kernel<T, 16, 1, 4>, 1, 4);
+    if (warps == 2) return go(swa_decode_kernel<T, 16, 2, 1>, 2, 1);
+    if (warps == 4) return go(swa_decode_kernel<T, 16, 4, 1>, 4, 1);
+    return go(swa_decode_kernel<T, 16, 8, 1>, 8, 1);
   };
   if (io_dtype == BASED_BF16) return launched(run(__nv_bfloat16{}));
   if (io_dtype == BASED_F32) return launched(run(float{}));

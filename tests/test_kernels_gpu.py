@@ -465,3 +465,29 @@ def test_rotary_qkv_cache_equals_rotary_then_copy(ops, B, L, H, hd):
     assert (cache[0] == 7).all() and (cache[1:, L:] == 7).all()          # nothing else is touched
     ref_q = O.apply_rotary(qkv[:, :, 0], cos, sin, 0)
     assert rel_err(a[:, :, 0].cpu().float(), ref_q.float()) < 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hd", [48, 64, 112, 128])
+@pytest.mark.parametrize("B,H", [(5, 3), (247, 3)])
+@pytest.mark.parametrize("w", [8, 9, 39, 40, 79, 80, 255])
+def test_swa_decode_shapes_of_the_work(ops, B, H, hd, w, dtype):
+    """Every split of the window over warps and of heads over blocks (741 heads: one above the border, and a last block that is
+    not full), at the windows on both sides of each border; rows at positions of their own, one of them outside the cache."""
+    g = torch.Generator("cuda").manual_seed(B + hd + w)
+    maxL = 300
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    cache, q, k, v = r(B, maxL, 2, H, hd), r(B, 1, H, hd), r(B, 1, H, hd), r(B, 1, H, hd)
+    lens = torch.randint(0, maxL, (B,), generator=g, device="cuda", dtype=torch.int32)
+    lens[0], lens[1], lens[2], lens[3] = 0, maxL - 1, -1, min(w, maxL - 1)
+    out, before = torch.full((B, 1, H, hd), 7.0, device="cuda").to(dtype), cache.clone()
+    ops.swa_decode(q, k, v, cache, lens, w, out=out)
+    ok = lens >= 0
+    rows, at = torch.arange(B, device="cuda")[ok], lens[ok].long()
+    before[rows, at, 0], before[rows, at, 1] = k[ok, 0], v[ok, 0]
+    assert torch.equal(cache, before) and bool((out[2] == 7).all())
+    j = torch.arange(maxL, device="cuda")
+    s = torch.einsum("bhd,bthd->bht", q[ok, 0].double(), before[rows, :, 0].double()) * hd ** -0.5
+    s = s.masked_fill(((j[None] > at[:, None]) | (j[None] < at[:, None] - w))[:, None], float("-inf"))
+    ref = torch.einsum("bht,bthd->bhd", s.softmax(-1), before[rows, :, 1].double())
+    assert rel_err(out[ok, 0].cpu(), ref.cpu()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
