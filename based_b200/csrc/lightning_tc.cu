@@ -580,15 +580,17 @@ __global__ void __launch_bounds__(256) lightning_scan_kernel(const __grid_consta
   }
 }
 
-// Segments and chunks per segment of a call.  Cut when every SM can have a segment of at least two chunks and two segments
-// exist: below that the two extra launches (about 6 us) cost more than the shorter chain saves.
+// Segments and chunks per segment of a call.  Uncut, a chain of more than 64 value columns spreads them over two CTAs instead, so it is cut
+// from eight chunks on only where four segments of every chain find an SM, from twelve where three do, and not where two do.
+// us uncut / cut, 128 columns: 37 chains 41 / 35 (8 chunks), 289 / 158 (64); 48 chains 40 / 42 (8), 56 / 53 (12), 136 / 115 (32); 64 chains 43 / 53
+// (8), 145 / 158 (32).  64 columns: 48 chains 31 / 28 (8); 64 chains 36 / 35 (8), 51 / 47 (12), 118 / 112 (32).
 void segments(int B, int L, int H, int dv, int* nseg, int* per) {
   const int64_t chains = (int64_t)B * H * ((dv + 127) / 128);
   const int nc = (L + C - 1) / C;
   *nseg = 1;
   *per = nc;
-  if (chains * 2 > 148 || nc < kMinSplitChunks) return;
-  const int most = (int)(148 / chains);
+  const int most = (int)(148 / chains);   // segments of every chain that find an SM
+  if (most < 2 || nc < kMinSplitChunks || (dv > 64 && (most == 2 || (most == 3 && nc < 12)))) return;
   *per = std::max(2, (nc + most - 1) / most);
   *nseg = (nc + *per - 1) / *per;
 }

@@ -81,10 +81,11 @@ def test_many_heads_fill_the_machine_without_a_split():
     check(args, product(*args, [140], impl="tcgen05"), torch.bfloat16)
 
 
-@pytest.mark.parametrize("d,dv,T,H", [(64, 48, 896, 4), (64, 48, 897, 4), (128, 128, 2047, 2), (128, 160, 1300, 3), (32, 16, 2500, 1), (16, 64, 1025, 37), (48, 64, 1025, 38)])
+@pytest.mark.parametrize("d,dv,T,H", [(64, 48, 896, 4), (64, 48, 897, 4), (128, 128, 2047, 2), (128, 160, 1300, 3), (32, 16, 2500, 1), (16, 64, 1025, 37), (48, 64, 1025, 38),
+                                        (32, 64, 1025, 74), (32, 128, 1408, 48), (32, 128, 1409, 48), (32, 112, 1537, 50)])
 def test_a_cut_sequence(d, dv, T, H):
-    """Sequences that run as segments side by side (from eight chunks on, while two segments of every chain find an SM), as a
-    prompt and after a first portion, against the same call in portions that are not cut."""
+    """Sequences that run as segments side by side, and their neighbours that do not (above 64 value columns: eleven chunks of 48
+    chains, any of 50), as a prompt and after a first portion, against the same call in portions that are not cut."""
     args = case([DECAYS[i % 4] for i in range(H)], d, dv, T, seed=T)
     whole = product(*args, [T])
     check(args, whole, torch.bfloat16)
