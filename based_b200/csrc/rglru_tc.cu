@@ -13,8 +13,8 @@
 // A CTA's time is its number of tiles times the latency of one (3 us): with few rows and blocks most SMs would idle.  There a
 // CLUSTER of 2 to 8 CTAs shares a sequence, a run of tiles each.  A CTA goes over its tiles twice: first for what they make
 // of a state (their decays' product and the end state from zero; no y, no output), then, with its state at the start folded
-// from the CTAs before it over distributed shared memory, for the output.  The first pass takes about two thirds of the
-// second's time, so a run of n / K tiles costs 1.7 n / K.  B = 2, 8 blocks of 128, L = 4096: 190 us
+// from the CTAs before it over distributed shared memory, for the output.  A tile takes 2.4 us in the first pass and
+// 3.0 in the second, so a run of n / K tiles costs 1.8 n / K.  B = 2, 8 blocks of 128, L = 4096: 190 us
 // with a CTA per block, 67 us with six (of eight-CTA clusters only 15 fit the device, and a second wave took 97 us).
 #include <algorithm>
 #include <initializer_list>
@@ -65,6 +65,7 @@ __device__ __forceinline__ float ld_peer(uint32_t saddr, uint32_t rank) {
   return v;
 }
 
+template <bool SHARED>   // K > 1
 __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sb = smem_u32(smem);
@@ -73,15 +74,16 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
     return;
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rank = blockIdx.x % p.K, unit = blockIdx.x / p.K;   // consecutive blocks are a cluster
+  const int K = SHARED ? p.K : 1;
+  const int rank = SHARED ? blockIdx.x % K : 0, unit = SHARED ? blockIdx.x / K : blockIdx.x;   // consecutive blocks are a cluster
   const int blk = unit / p.slices, c0 = (unit % p.slices) * 128, b = blockIdx.y;
-  const int tiles = (p.L + TT - 1) / TT, first = tiles * rank / p.K, n2 = tiles * (rank + 1) / p.K - first;
-  const int n1 = rank < p.K - 1 ? n2 : 0, nt = n1 + n2;         // steps: n1 tiles for the summary, then n2 for the output
-  auto token = [&](int t) { return (first + (t < n1 ? t : t - n1)) * TT; };
+  const int tiles = (p.L + TT - 1) / TT, first = SHARED ? tiles * rank / K : 0, n2 = SHARED ? tiles * (rank + 1) / K - first : tiles;
+  const int n1 = SHARED && rank < K - 1 ? n2 : 0, nt = n1 + n2;         // steps: n1 tiles for the summary, then n2 for the output
+  auto token = [&](int t) { return SHARED ? (first + (t < n1 ? t : t - n1)) * TT : t * TT; };
   // shared memory: W_r, W_i (atoms each), u stages, y stages (two 64-channel atoms each), carries, barriers
   // and, with K > 1, the summary for the CTAs after this one (a product per group, the end state)
   const uint32_t SM_U = 2u * p.atoms * kWAtom, SM_Y = SM_U + 2u * p.atoms * kUAtom, SM_C = SM_Y + 4u * kUAtom,
-                 SM_SUM = SM_C + GROUPS * 128 * 4, SM_BAR = SM_SUM + (p.K > 1 ? kSummary : 0);
+                 SM_SUM = SM_C + GROUPS * 128 * 4, SM_BAR = SM_SUM + (SHARED ? kSummary : 0);
   const uint32_t B_W = sb + SM_BAR, B_FULL = B_W + 8, B_D = B_FULL + 16, B_EMPTY = B_D + 16, B_Y = B_EMPTY + 16,
                  B_OUT = B_Y + 16, B_CARRY = B_OUT + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SM_BAR + 8 * (11 + GROUPS));
@@ -103,9 +105,9 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
   // Cluster barrier 1: the summaries are written (and the call's state is read); 2: they have been read.  Threads that neither
   // write nor read arrive here at once and wait at the end.
   const bool writer = n1 > 0 && warp < NC / 32, reader = rank > 0 && warp < 4;
-  float S0 = 0.f;
-  if (warp < 4 && c0 + tid < p.n && seq::position0(p.offsets, p.offset, b) > 0) S0 = p.state[(int64_t)b * p.W + blk * p.n + c0 + tid];
-  if (p.K > 1 && !writer) cluster_arrive();
+  float given = 0.f;               // group 0: the state the call starts from
+  if (SHARED && warp < 4 && c0 + tid < p.n && seq::position0(p.offsets, p.offset, b) > 0) given = p.state[(int64_t)b * p.W + blk * p.n + c0 + tid];
+  if (SHARED && !writer) cluster_arrive();
 
   if (warp == NC / 32) {
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
@@ -186,9 +188,8 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
     const uint8_t* ucol = smem + SM_U + ((c0 + ch) >> 6) * kUAtom + (ch & 7) * 2;   // this channel's column of a stage
     const int chunk = ((c0 + ch) & 63) >> 3;
     float* sum = reinterpret_cast<float*>(smem + SM_SUM) + ch;
-    const float given = S0;          // group 0: the state the call starts from
-    if (n1 > 0) S0 = 0.f;
-    float prod = 1.f;
+    float S0 = n1 > 0 ? 0.f : given, prod = 1.f;
+    if (!SHARED && grp == 0 && live && seq::position0(p.offsets, p.offset, b) > 0) S0 = p.state[(int64_t)b * p.W + chan];
     for (int t = 0; t < nt; ++t) {
       const int x = t & 1, tok0 = token(t) + t0g;
       mbar_wait_bounded(B_D + 8 * x, (t >> 1) & 1, abort_flag, p.status, 1u << 21);
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
         mbar_wait_bounded(from, (grp > 0 ? t : t - 1) & 1, abort_flag, p.status, 1u << 22);
         S0 = *carry_in;
       }
-      if (grp == 0 && t == n1) {     // the output starts from what the CTAs before make of the call's state
+      if (SHARED && grp == 0 && t == n1) {     // the output starts from what the CTAs before make of the call's state
         S0 = given;
         if (reader) {
           cluster_wait();
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
       const float end = fmaf(pr, S0, sr);
       carry[grp * 128 + ch] = end;
       mbar_arrive(my_carry);
-      if (t < n1) {
+      if (SHARED && t < n1) {
         prod *= pr;
         if (t == n1 - 1) {
           sum[128 * grp] = prod;
@@ -265,10 +266,10 @@ __global__ void __launch_bounds__(NT, 1) rglru_tc_kernel(const __grid_constant__
         *at(i) = __float2bfloat16_rn(fmaf(P[i], S0, s[i]) * seq::gelu_tanh_t<bf16>(__bfloat162float(yv[i])));
       fence_proxy_async();
       mbar_arrive(B_OUT + 8 * yx);
-      if (live && grp == GROUPS - 1 && t == nt - 1 && rank == p.K - 1) p.state[(int64_t)b * p.W + chan] = end;
+      if (live && grp == GROUPS - 1 && t == nt - 1 && rank == K - 1) p.state[(int64_t)b * p.W + chan] = end;
     }
   }
-  if (p.K > 1) {
+  if (SHARED) {
     if (!reader) { cluster_wait(); cluster_arrive(); }
     cluster_wait();
   }
@@ -345,20 +346,22 @@ int launch_rglru_tc(const void* u, const void* y, const void* w, const void* rb,
       unsigned int* addr = nullptr;
       e = cudaGetSymbolAddress(reinterpret_cast<void**>(&addr), g_tc_status_rglru);
       if (e != cudaSuccess) return (int)e;
-      e = cudaFuncSetAttribute(rglru_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      e = cudaFuncSetAttribute(rglru_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) return (int)e;
+      e = cudaFuncSetAttribute(rglru_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) return (int)e;
       status[dev] = addr;
     }
     p.status = status[dev];
-    // The largest cluster of which all fit the device at once (a second wave costs more than a smaller cluster) and whose CTAs
-    // have two tiles or more (with one tile each the second pass, the exchange and the launch cost what the shorter chain
-    // saves).  Blocks of 256 leave no room for the summary in shared memory.
+    // The largest cluster of which all fit the device at once (a second wave costs more than a smaller cluster), where it is faster:
+    // a tile of a shared run takes 5.4 us in both passes and the exchange 2, a tile of an unshared sequence 3.0 (4 tiles 16.6 us
+    // unshared, 17.9 in two CTAs; 7 tiles 25.3, 19.1 in three).  Blocks of 256 leave no room for the summary in shared memory.
     if (smem + (int)kSummary <= 227 * 1024)
       for (int K = std::min(kMaxCluster, tiles / 2); K > 1; --K) {
         const int64_t units = (int64_t)blocks * p.slices * B;
-        if (units * K > 148) continue;
+        if (units * K > 148 || 9 * ((tiles + K - 1) / K) + 4 >= 5 * tiles) continue;
         short& r = room[dev][K][p.atoms - 1];
-        if (r == 0) r = (short)(1 + max_active_clusters(rglru_tc_kernel, K, NT, smem + (int)kSummary));
+        if (r == 0) r = (short)(1 + max_active_clusters(rglru_tc_kernel<true>, K, NT, smem + (int)kSummary));
         if (r - 1 < units) continue;
         p.K = K;
         smem += kSummary;
@@ -376,7 +379,7 @@ int launch_rglru_tc(const void* u, const void* y, const void* w, const void* rb,
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = p.K > 1 ? 1 : 0;
-  return launched((int)cudaLaunchKernelEx(&cfg, rglru_tc_kernel, p));
+  return launched((int)cudaLaunchKernelEx(&cfg, p.K > 1 ? rglru_tc_kernel<true> : rglru_tc_kernel<false>, p));
 }
 
 }  // namespace based

@@ -192,9 +192,10 @@ def test_rglru(W, blocks, dtype):
         assert rel_err(out.float().cpu(), ref) < (2e-5 if dtype == torch.float32 else 1e-2)
 
 
-@pytest.mark.parametrize("W,blocks,L,B", [(128, 1, 193, 2), (512, 2, 257, 1), (144, 1, 449, 1), (96, 1, 512, 2), (512, 4, 961, 1), (1024, 8, 1100, 3), (128, 2, 4096, 2), (256, 1, 700, 1)])
+@pytest.mark.parametrize("W,blocks,L,B", [(128, 1, 193, 2), (128, 1, 321, 2), (512, 2, 257, 1), (144, 1, 449, 1), (96, 1, 512, 2), (512, 4, 961, 1), (1024, 8, 1100, 3), (128, 2, 4096, 2), (256, 1, 700, 1)])
 def test_rglru_shared_sequences(W, blocks, L, B):
-    """Lengths at which 2, 4 or 8 CTAs share a sequence (4, 8 and 16 tiles of 64 tokens and one more), from the start and from a state."""
+    """Lengths at which 3, 4 or 8 CTAs share a sequence (6, 8 and 16 tiles of 64 tokens and one more) and at which none do (4, 5), from
+    the start and from a state."""
     from based_b200 import ops
     g = torch.Generator().manual_seed(L)
     n = W // blocks
