@@ -128,7 +128,7 @@ class BaseConv(nn.Module):
         finish = finish or ops.linear
         if inference_params is not None and inference_params.seqlen_offset > 0:
             state = self.conv._get_state(inference_params)
-            if (ops._decode_rows(u, self.in_proj.weight, fused=True)
+            if (ops._decode_rows(u, self.in_proj.weight)
                     and state.dtype == torch.bfloat16 and state.is_contiguous()
                     and state.shape[0] == u.shape[0] and u.shape[1] == 1 and self.d_inner % 8 == 0):
                 # decode step: in_proj, the convolution step on the state, silu and the gate in one launch

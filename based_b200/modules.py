@@ -57,7 +57,7 @@ class GatedMlp(nn.Module):
             act = "silu"
         else:
             raise NotImplementedError("GatedMlp: activation must be F.silu (SwiGLU) or F.sigmoid (GLU)")
-        if ops._decode_rows(x, self.fc1.weight, fused=True, gated=True) and self.fc1.weight.shape[0] % 16 == 0:
+        if ops._decode_rows(x, self.fc1.weight, gated=True) and self.fc1.weight.shape[0] % 16 == 0:
             # decode step: fc1 and the gated activation in one launch
             return ops.decode_linear(x, self.fc1.weight, self.fc1.bias, epilogue="gated", activation=act, out=out)
         return ops.gated_act(self.fc1(ops.dense(x)), act, out=out)

@@ -440,11 +440,13 @@ def gated_act(y: torch.Tensor, activation: str = "silu", out: Optional[torch.Ten
 # the weights from HBM, cuBLAS / ours (N x K, rows): 1024 x 1024 4.6 / 2.9 (16), 4.2 / 3.6 (32); 4096 x 1024 4.7 / 3.1, 4.8 / 4.3,
 # 4.9 / 6.3 (64); 1024 x 3072 8.6 / 3.5, 7.2 / 5.3; 1792 x 1792 5.2 / 3.6, 5.2 / 5.8; 7168 x 1792 7.4 / 6.9, 7.5 / 8.0, with the gated
 # activation 9.9 / 7.0, 9.9 / 8.5; 50280 x 1024 21 / 30.  So: up to 16 rows whatever K; up to 32 for a short K, for few enough
-# outputs that every block of the kernel has an SM, and where the epilogue saves a launch.
-# With the gated activation and one round of blocks, some more.  An MLP whose second product is the library's, library / ours (width x
-# hidden, 33 and 40 rows): 512 x 1024 9.5 / 8.1, 9.5 / 8.2; 768 x 1536 10.9 / 10.5, 10.9 / 10.6; 1024 x 1024 10.3 / 9.2, 10.3 / 9.4;
-# 1024 x 2048 12.3 / 12.2, 12.3 / 12.3, behind a norm 14.4 / 12.9, 14.4 / 13.1.  At 48 rows 1024 x 2048 is 12.4 / 12.6.
-DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_ROWS_GATED, DECODE_LINEAR_MAX_OUTPUTS = 32, 40, 8192
+# outputs that every block of the kernel has an SM, and where the gated activation saves a launch (the convolution does not there: a
+# BaseConv step of 24 rows, 7168 x 1792, 17.5 with the library, 20.0).
+# With the gated activation and one round of blocks, some more.  An MLP whose second product is the library's, library / ours at 33 and 40
+# rows (width x hidden): 512 x 1024 9.5 / 6.6, 9.5 / 6.7; 768 x 1536 10.9 / 10.0, 10.9 / 10.1; 1024 x 1024 10.3 / 8.8, 10.3 / 8.8; 1024 x 2048
+# 12.3 / 12.4, 12.3 / 12.6, behind a norm 14.4 / 13.2, 14.4 / 13.4.  At 48 rows 1024 x 2048 is 12.4 / 12.6.  Up to 2368 outputs of the product all
+# blocks have an SM: at 64 rows 512 x 1024 8.3 / 6.9, 1024 x 1024 10.4 / 9.0.
+DECODE_LINEAR_MAX_ROWS, DECODE_LINEAR_MAX_ROWS_GATED, DECODE_LINEAR_MAX_OUTPUTS = 32, (64, 40), 8192
 
 
 def decode_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, *,
@@ -563,19 +565,21 @@ def _observed() -> bool:
         n > 0 and any(type(torch._C._get_function_stack_at(i)) is not _DeviceContext for i in range(n)))
 
 
-def _decode_rows(x: torch.Tensor, weight: torch.Tensor, fused: bool = False, gated: bool = False) -> bool:
+def _decode_rows(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
     """True when ``x W^T`` is a decode-step product the library's own kernel should run: a few bf16 rows in a layout it takes, and
     nothing around the call that only a torch operator serves (autograd, autocast, forward mode, function transforms, tracing, modes).
-    ``fused``: its epilogue takes the place of another launch; ``gated``: that launch is the gated activation."""
+    ``gated``: its epilogue takes the place of the gated activation's launch."""
     if type(x) is NormRows:
         x = x.x
     K = x.shape[-1] if x.dim() else 0
-    most = DECODE_LINEAR_MAX_ROWS_GATED if gated and K <= 1024 and weight.shape[0] <= 2 * 8 * 296 else DECODE_LINEAR_MAX_ROWS
+    most = DECODE_LINEAR_MAX_ROWS
+    if gated and K <= 1024 and weight.shape[0] <= 2 * 8 * 296:
+        most = DECODE_LINEAR_MAX_ROWS_GATED[weight.shape[0] > 2 * 8 * 148]
     if not (0 < x.numel() <= K * most and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16):
         return False
     if type(x) is not torch.Tensor or type(weight) not in _PLAIN_TYPES or weight.dim() != 2 or weight.shape[0] > DECODE_LINEAR_MAX_OUTPUTS:
         return False
-    if x.numel() > 16 * K and not (K <= 1024 or (weight.shape[0] <= 8 * 148 and K <= 3072) or (fused and K <= 2048)):
+    if x.numel() > 16 * K and not (K <= 1024 or (weight.shape[0] <= 8 * 148 and K <= 3072) or (gated and K <= 2048)):
         return False
     return (K % 32 == 0 and weight.shape[1] == K and weight.shape[0] % 8 == 0 and weight.is_contiguous()
             and (x.is_contiguous() or (x.stride(-1) == 1 and all(st % 8 == 0 for st in x.stride()[:-1])))

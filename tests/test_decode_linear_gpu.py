@@ -132,6 +132,16 @@ def test_linear_takes_the_kernel_only_where_it_can(ops):
     assert xg.grad is not None
 
 
+def test_rows_that_take_the_kernel(ops):
+    """The borders of the dispatch, where a launch with the kernel and without cross."""
+    w = {(n, k): torch.zeros(n, k, device="cuda", dtype=torch.bfloat16) for n, k in ((1184, 3072), (1192, 3072), (7168, 1792), (4096, 1024), (4744, 1024), (2368, 1024), (2384, 1024))}
+    with torch.no_grad():
+        def most(n, k, **kind):
+            return max((m for m in (16, 17, 32, 33, 40, 41, 64, 65) if ops._decode_rows(torch.zeros(m, 1, k, device="cuda", dtype=torch.bfloat16), w[n, k], **kind)), default=0)
+        assert [most(1184, 3072), most(1192, 3072), most(7168, 1792), most(4096, 1024)] == [32, 16, 16, 32]
+        assert [most(2368, 1024, gated=True), most(2384, 1024, gated=True), most(4744, 1024, gated=True), most(7168, 1792, gated=True)] == [64, 40, 32, 32]
+
+
 def test_modes_see_the_products(ops, monkeypatch):
     """A FLOP counter and a function mode find every product of a few rows, as they do for many; a device context is no
     reason to leave the kernel."""
