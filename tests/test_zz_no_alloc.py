@@ -50,10 +50,12 @@ def test_static_workspace_matches_caller_workspace_twice_in_a_row():
     code, y0, kv0, _ = _call_static(q, k, v, 16)
     torch.cuda.synchronize()
     assert code == 0
-    free_before = torch.cuda.mem_get_info()[0]
     y = torch.empty_like(y0)
     kv = torch.empty_like(kv0)
     ks = torch.empty(1, 2, 1, 1, 273, dtype=torch.float32, device="cuda")
+    assert torch.equal(y.copy_(y0), y0) and torch.equal(kv.copy_(kv0), kv0)
+    y.zero_(), kv.zero_()
+    free_before = torch.cuda.mem_get_info()[0]     # behind the test's own tensors and comparisons, which may take a segment from the device
     lib = _capi.lib()
     for _ in range(2):
         code = lib.based_linattn_prefill_split_static(
