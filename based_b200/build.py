@@ -67,7 +67,8 @@ def build_native(force: bool = False) -> str:
 
 
 def build_library(force: bool = False, verbose: bool = False, part: str = None) -> str:
-    """Build (if stale) and return the path of the shared library.  Needs ``nvcc`` only; no GPU.  ``part`` names a subset
+    """Build (if stale) and return the path of the shared library, and build the extension module.  Needs ``nvcc``, a C++
+    compiler and Python's and torch's headers; no GPU.  ``part`` names a subset
     of the kernels that is enough for the caller: only those are compiled, unless the whole library is there already."""
     global _chosen
     build_native(force)

@@ -78,6 +78,8 @@ inline int max_active_clusters(void (*kernel)(P...), int K, int threads, int sme
 // another kernel writes or reads: it returns when the kernels before have ended and their writes are visible.  What stands
 // before it (launch latency, set-up, prefetches of weights into L2) overlaps with them.  Without the attribute both do nothing.
 // Data of other kernels is read by coherent loads only: the read-only path is for what no kernel in flight writes.
+// A kernel that allocates TMEM waits before it does, and calls pdl_trigger early only where the next kernel allocates none.
+// Worth it for small grids: with griddepcontrol in it a block costs a nanosecond or more.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 // 16-byte aligned, a multiple of 16 bytes

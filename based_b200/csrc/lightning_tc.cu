@@ -429,7 +429,9 @@ __global__ void __launch_bounds__(NT, 1) lightning_tc_kernel(const __grid_consta
 
 // What one segment adds to the state by its end: sum_j k_j (g^(end-1-j) v_j)^T over its tokens, without the state before it.
 // grid (H, B, column slices x (segments - 1)).  All warps load, apply silu and write the operands of a chunk into one of two
-// stages; one elected lane issues.  Bound by the loads' latency: a CTA has 2 to 6 chunks, one of them in registers ahead.
+// stages; one elected lane issues.  Bound by the loads' latency: a CTA has two chunks for a short sequence and p.per for a long one, one
+// of them in registers ahead.  It lets the kernel behind it start early although it holds TMEM: that one is the scan, which needs
+// none, and the kernel after it waits before it allocates.
 constexpr int kSegThreads = 512;
 __global__ void __launch_bounds__(kSegThreads, 1) lightning_segment_kernel(const __grid_constant__ Params p, const bf16* v, int64_t vb, int64_t vl) {
   pdl_trigger();
