@@ -98,31 +98,36 @@ struct NormParams {
 
 constexpr int NORM_THREADS = 128;
 
-// A kernel of one block per row has two forms.  FEW rows: a programmatic launch, and the weights are loaded with the row.  Else neither:
-// griddepcontrol makes a block cost a nanosecond or more, which a block of a few KB does not take at the HBM rate, and the weights'
-// registers cost occupancy.  us in chains, FEW / else: gated activation, 512 columns in, 300 rows 1.4 / 1.9, 2048 2.9 / 2.4, 32768
-// 34.7 / 18.3; residual add and norm, 1024 wide, 300 rows 2.2 / 2.7, 1200 3.9 / 3.5; 1792 wide, 300 rows 3.0 / 3.7, 8192 32.6 / 30.6; norm alone,
-// 1024 wide, 32768 rows 39.2 / 29.7.
-inline bool few_norm_rows(int64_t M, int D) { return M * D <= 600000; }
-inline bool few_rows(int64_t M) { return M <= 8 * 148; }   // little work per row: gated activation, gated norm
+// A kernel of one block per row has two forms.  PROGRAMMATIC: a programmatic launch, and the weights are loaded with the row.  Else
+// neither: griddepcontrol makes a block cost a nanosecond or more, which a row of less than 8 KB does not take at the HBM rate, and
+// the weights' registers cost occupancy once the rows come from HBM.  us in chains of one kernel, programmatic / else: gated activation,
+// 512 columns in, 300 rows 1.4 / 1.9, 2048 2.9 / 2.4, 32768 34.7 / 18.3, 4096 columns in, 4096 rows 6.1 / 6.5; residual add and norm, 1024 wide, 300 rows
+// 2.2 / 2.7, 1200 3.9 / 3.5, 4096 7.3 / 7.4; 1792 wide, 300 rows 3.0 / 3.7, 2048 7.1 / 7.9, 8192 32.6 / 30.6; norm alone, 1024 wide, 32768 rows 39.2 / 29.7.
+// In a prompt, between library products and outside a graph, the programmatic form saves more: a post-norm stack on 6001 tokens of
+// 1024, 81 such norms, 6.36 ms with it and 6.64 without.
+inline bool heavy_row(int64_t bytes) { return bytes >= 8192; }   // read and written per row
+inline bool programmatic_norm(int64_t M, int D, int64_t row_bytes) {
+  return M * D <= 600000 || (heavy_row(row_bytes) && M >= 2048 && M * D <= 8400000);
+}
+inline bool programmatic_rows(int64_t M, int64_t row_bytes) { return M <= 8 * 148 || heavy_row(row_bytes); }
 
 template <typename P>
-inline void launch_rows(bool few, void (*programmatic)(P), void (*plain)(P), unsigned grid, cudaStream_t stream, const P& p) {
-  if (few) launch_pdl(programmatic, grid, NORM_THREADS, 0, stream, p);
+inline void launch_rows(bool early, void (*programmatic)(P), void (*plain)(P), unsigned grid, cudaStream_t stream, const P& p) {
+  if (early) launch_pdl(programmatic, grid, NORM_THREADS, 0, stream, p);
   else plain<<<grid, NORM_THREADS, 0, stream>>>(p);
 }
 
 // One row per block; thread t owns the 8-value groups t, t + 128, ... (VPT of them, in registers
 // between the reduction and the scaling, so the row is read once).
-template <int VPT, bool FEW>
+template <int VPT, bool PROGRAMMATIC>
 __global__ void __launch_bounds__(NORM_THREADS) add_rmsnorm_kernel(const NormParams p) {
-  if constexpr (FEW) {
+  if constexpr (PROGRAMMATIC) {
     pdl_trigger();
     pdl_wait();
   }
   const int64_t row = blockIdx.x;
   const int ngroups = p.D >> 3;
-  constexpr bool kEarly = FEW && VPT <= 2;   // the weights' latency passes with the row's
+  constexpr bool kEarly = PROGRAMMATIC && VPT <= 2;   // the weights' latency passes with the row's
   float z[VPT][8], wv[kEarly ? VPT : 1][8];
   float ss = 0.f;
 #pragma unroll
@@ -215,9 +220,9 @@ struct StreamParams {
 };
 
 // One row per block; N values per access (8, or 1 for any D), VPT accesses per thread kept in registers.
-template <typename T, int N, int VPT, bool FEW>
+template <typename T, int N, int VPT, bool PROGRAMMATIC>
 __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamParams p) {
-  if constexpr (FEW) {
+  if constexpr (PROGRAMMATIC) {
     pdl_trigger();
     pdl_wait();
   }
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_norm_kernel(const StreamP
   const int64_t row = blockIdx.x;
   const int groups = p.D / N;
   float* res = p.residual + row * p.D;
-  constexpr bool kEarly = FEW && VPT <= 2;   // the weights' latency passes with the row's
+  constexpr bool kEarly = PROGRAMMATIC && VPT <= 2;   // the weights' latency passes with the row's
   float z[VPT][N], w1[kEarly ? VPT : 1][N], w2[kEarly ? VPT : 1][N];
   auto load_res = [&](int g, float (&v)[N]) {
     if constexpr (N == 8) load8(res, 0, 8 * g, v);
@@ -312,9 +317,9 @@ struct PostNormParams {
   float eps;
 };
 
-template <typename T, int N, int VPT, bool FEW>
+template <typename T, int N, int VPT, bool PROGRAMMATIC>
 __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const PostNormParams p) {
-  if constexpr (FEW) {
+  if constexpr (PROGRAMMATIC) {
     pdl_trigger();
     pdl_wait();
   }
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(NORM_THREADS) stream_post_norm_kernel(const Po
   const int groups = p.D / N;
   float* res = p.residual + row * p.D;
   const T* br = static_cast<const T*>(p.branch) + row * p.sb;
-  constexpr bool kEarly = FEW && VPT <= 2;   // the weight's latency passes with the row's
+  constexpr bool kEarly = PROGRAMMATIC && VPT <= 2;   // the weight's latency passes with the row's
   float z[VPT][N], r[VPT][N], w0[kEarly ? VPT : 1][N];
   float ss = 0.f;
 #pragma unroll
@@ -410,9 +415,9 @@ struct NormGateParams {
   float eps;
 };
 
-template <typename T, int N, int VPT, bool FEW>
+template <typename T, int N, int VPT, bool PROGRAMMATIC>
 __global__ void __launch_bounds__(NORM_THREADS) norm_gate_kernel(const NormGateParams p) {
-  if constexpr (FEW) {
+  if constexpr (PROGRAMMATIC) {
     pdl_trigger();
     pdl_wait();
   }
@@ -488,9 +493,9 @@ __device__ __forceinline__ float act_fn(float g, int act) {
 
 // One row per block; thread t owns the 16-byte vectors t, t + 128, ... of the row (VPT of them): a
 // warp's accesses are contiguous, all loads of a thread are issued before any arithmetic.
-template <typename T, int VPT, bool FEW>
+template <typename T, int VPT, bool PROGRAMMATIC>
 __global__ void __launch_bounds__(NORM_THREADS) gated_act_kernel(const ActParams p) {
-  if constexpr (FEW) {
+  if constexpr (PROGRAMMATIC) {
     pdl_trigger();
     pdl_wait();
   }
@@ -536,20 +541,20 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_act_scalar_kernel(const Ac
 template <typename T>
 int launch_stream_norm_t(const StreamParams& p, cudaStream_t stream) {
   const unsigned grid = (unsigned)p.M;
-  const bool few = few_norm_rows(p.M, p.D);
+  const bool early = programmatic_norm(p.M, p.D, (int64_t)p.D * (8 + (p.out2 ? 3 : 2) * sizeof(T)));
   const bool vec = p.D % 8 == 0 && aligned16(p.table) && aligned16(p.table_norm) && aligned16(p.branch) &&
                    aligned16(p.residual) && aligned16(p.w1) && aligned16(p.w2) && aligned16(p.out1) &&
                    aligned16(p.out2) && p.sb % 8 == 0;
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   if (vec) {
-    if (vpt <= 1) launch_rows(few, stream_norm_kernel<T, 8, 1, true>, stream_norm_kernel<T, 8, 1, false>, grid, stream, p);
-    else if (vpt <= 2) launch_rows(few, stream_norm_kernel<T, 8, 2, true>, stream_norm_kernel<T, 8, 2, false>, grid, stream, p);
-    else if (vpt <= 4) launch_rows(few, stream_norm_kernel<T, 8, 4, true>, stream_norm_kernel<T, 8, 4, false>, grid, stream, p);
-    else if (vpt <= 8) launch_rows(few, stream_norm_kernel<T, 8, 8, true>, stream_norm_kernel<T, 8, 8, false>, grid, stream, p);
+    if (vpt <= 1) launch_rows(early, stream_norm_kernel<T, 8, 1, true>, stream_norm_kernel<T, 8, 1, false>, grid, stream, p);
+    else if (vpt <= 2) launch_rows(early, stream_norm_kernel<T, 8, 2, true>, stream_norm_kernel<T, 8, 2, false>, grid, stream, p);
+    else if (vpt <= 4) launch_rows(early, stream_norm_kernel<T, 8, 4, true>, stream_norm_kernel<T, 8, 4, false>, grid, stream, p);
+    else if (vpt <= 8) launch_rows(early, stream_norm_kernel<T, 8, 8, true>, stream_norm_kernel<T, 8, 8, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 8192 wide
   } else {
-    if (vpt <= 4) launch_rows(few, stream_norm_kernel<T, 1, 4, true>, stream_norm_kernel<T, 1, 4, false>, grid, stream, p);
-    else if (vpt <= 32) launch_rows(few, stream_norm_kernel<T, 1, 32, true>, stream_norm_kernel<T, 1, 32, false>, grid, stream, p);
+    if (vpt <= 4) launch_rows(early, stream_norm_kernel<T, 1, 4, true>, stream_norm_kernel<T, 1, 4, false>, grid, stream, p);
+    else if (vpt <= 32) launch_rows(early, stream_norm_kernel<T, 1, 32, true>, stream_norm_kernel<T, 1, 32, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 4096 wide
   }
   return (int)cudaGetLastError();
@@ -561,16 +566,16 @@ int launch_post_norm_t(const PostNormParams& p, int64_t M, cudaStream_t stream) 
                    aligned16(p.w_out) && aligned16(p.out);
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
-  const bool few = few_norm_rows(M, p.D);
+  const bool early = programmatic_norm(M, p.D, (int64_t)p.D * (8 + 2 * sizeof(T)));
   if (vec) {
-    if (vpt <= 1) launch_rows(few, stream_post_norm_kernel<T, 8, 1, true>, stream_post_norm_kernel<T, 8, 1, false>, grid, stream, p);
-    else if (vpt <= 2) launch_rows(few, stream_post_norm_kernel<T, 8, 2, true>, stream_post_norm_kernel<T, 8, 2, false>, grid, stream, p);
-    else if (vpt <= 4) launch_rows(few, stream_post_norm_kernel<T, 8, 4, true>, stream_post_norm_kernel<T, 8, 4, false>, grid, stream, p);
-    else if (vpt <= 8) launch_rows(few, stream_post_norm_kernel<T, 8, 8, true>, stream_post_norm_kernel<T, 8, 8, false>, grid, stream, p);
+    if (vpt <= 1) launch_rows(early, stream_post_norm_kernel<T, 8, 1, true>, stream_post_norm_kernel<T, 8, 1, false>, grid, stream, p);
+    else if (vpt <= 2) launch_rows(early, stream_post_norm_kernel<T, 8, 2, true>, stream_post_norm_kernel<T, 8, 2, false>, grid, stream, p);
+    else if (vpt <= 4) launch_rows(early, stream_post_norm_kernel<T, 8, 4, true>, stream_post_norm_kernel<T, 8, 4, false>, grid, stream, p);
+    else if (vpt <= 8) launch_rows(early, stream_post_norm_kernel<T, 8, 8, true>, stream_post_norm_kernel<T, 8, 8, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 8192 wide
   } else {
-    if (vpt <= 4) launch_rows(few, stream_post_norm_kernel<T, 1, 4, true>, stream_post_norm_kernel<T, 1, 4, false>, grid, stream, p);
-    else if (vpt <= 32) launch_rows(few, stream_post_norm_kernel<T, 1, 32, true>, stream_post_norm_kernel<T, 1, 32, false>, grid, stream, p);
+    if (vpt <= 4) launch_rows(early, stream_post_norm_kernel<T, 1, 4, true>, stream_post_norm_kernel<T, 1, 4, false>, grid, stream, p);
+    else if (vpt <= 32) launch_rows(early, stream_post_norm_kernel<T, 1, 32, true>, stream_post_norm_kernel<T, 1, 32, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;   // rows up to 4096 wide
   }
   return (int)cudaGetLastError();
@@ -592,16 +597,16 @@ int launch_norm_gate_t(const NormGateParams& p, int64_t M, cudaStream_t stream) 
                    aligned16(p.gate) && aligned16(p.out);
   const int vpt = (p.D / (vec ? 8 : 1) + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
-  const bool few = few_rows(M);
+  const bool early = programmatic_rows(M, (int64_t)p.D * 3 * sizeof(T));
   if (vec) {
-    if (vpt <= 1) launch_rows(few, norm_gate_kernel<T, 8, 1, true>, norm_gate_kernel<T, 8, 1, false>, grid, stream, p);
-    else if (vpt <= 2) launch_rows(few, norm_gate_kernel<T, 8, 2, true>, norm_gate_kernel<T, 8, 2, false>, grid, stream, p);
-    else if (vpt <= 4) launch_rows(few, norm_gate_kernel<T, 8, 4, true>, norm_gate_kernel<T, 8, 4, false>, grid, stream, p);
-    else if (vpt <= 8) launch_rows(few, norm_gate_kernel<T, 8, 8, true>, norm_gate_kernel<T, 8, 8, false>, grid, stream, p);
+    if (vpt <= 1) launch_rows(early, norm_gate_kernel<T, 8, 1, true>, norm_gate_kernel<T, 8, 1, false>, grid, stream, p);
+    else if (vpt <= 2) launch_rows(early, norm_gate_kernel<T, 8, 2, true>, norm_gate_kernel<T, 8, 2, false>, grid, stream, p);
+    else if (vpt <= 4) launch_rows(early, norm_gate_kernel<T, 8, 4, true>, norm_gate_kernel<T, 8, 4, false>, grid, stream, p);
+    else if (vpt <= 8) launch_rows(early, norm_gate_kernel<T, 8, 8, true>, norm_gate_kernel<T, 8, 8, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;
   } else {
-    if (vpt <= 4) launch_rows(few, norm_gate_kernel<T, 1, 4, true>, norm_gate_kernel<T, 1, 4, false>, grid, stream, p);
-    else if (vpt <= 32) launch_rows(few, norm_gate_kernel<T, 1, 32, true>, norm_gate_kernel<T, 1, 32, false>, grid, stream, p);
+    if (vpt <= 4) launch_rows(early, norm_gate_kernel<T, 1, 4, true>, norm_gate_kernel<T, 1, 4, false>, grid, stream, p);
+    else if (vpt <= 32) launch_rows(early, norm_gate_kernel<T, 1, 32, true>, norm_gate_kernel<T, 1, 32, false>, grid, stream, p);
     else return BASED_ERR_SHAPE;
   }
   return (int)cudaGetLastError();
@@ -669,11 +674,12 @@ int launch_add_rmsnorm(const void* x, const void* residual, const void* weight, 
                io_dtype == BASED_BF16, res_dtype == BASED_BF16, w_dtype == BASED_BF16, round_input != 0, eps};
   const int groups = D / 8, vpt = (groups + NORM_THREADS - 1) / NORM_THREADS;
   const unsigned grid = (unsigned)M;
-  const bool few = few_norm_rows(M, D);
-  if (vpt <= 1) launch_rows(few, add_rmsnorm_kernel<1, true>, add_rmsnorm_kernel<1, false>, grid, stream, p);
-  else if (vpt <= 2) launch_rows(few, add_rmsnorm_kernel<2, true>, add_rmsnorm_kernel<2, false>, grid, stream, p);
-  else if (vpt <= 4) launch_rows(few, add_rmsnorm_kernel<4, true>, add_rmsnorm_kernel<4, false>, grid, stream, p);
-  else launch_rows(few, add_rmsnorm_kernel<8, true>, add_rmsnorm_kernel<8, false>, grid, stream, p);
+  const int io = io_dtype == BASED_BF16 ? 2 : 4, rs = res_dtype == BASED_BF16 ? 2 : 4;
+  const bool early = programmatic_norm(M, D, (int64_t)D * (2 * io + (residual ? rs : 0) + (residual_out ? rs : 0)));
+  if (vpt <= 1) launch_rows(early, add_rmsnorm_kernel<1, true>, add_rmsnorm_kernel<1, false>, grid, stream, p);
+  else if (vpt <= 2) launch_rows(early, add_rmsnorm_kernel<2, true>, add_rmsnorm_kernel<2, false>, grid, stream, p);
+  else if (vpt <= 4) launch_rows(early, add_rmsnorm_kernel<4, true>, add_rmsnorm_kernel<4, false>, grid, stream, p);
+  else launch_rows(early, add_rmsnorm_kernel<8, true>, add_rmsnorm_kernel<8, false>, grid, stream, p);
   return (int)cudaGetLastError();
 }
 
@@ -699,7 +705,7 @@ int launch_gated_act(const void* y, const void* gate, void* out, int64_t M, int 
   const int nvec = F / N, vpt = (nvec + NORM_THREADS - 1) / NORM_THREADS;
   ActParams p{y, gate, out, M, sy, sg, so, F, act};
   const unsigned grid = (unsigned)M;
-  const bool few = few_rows(M);
+  const bool early = programmatic_rows(M, (int64_t)F * 3 * (io_dtype == BASED_BF16 ? 2 : 4));
   if (F % N != 0 || vpt > 16 || !aligned16(y) || !aligned16(gate) || !aligned16(out) || sy % N || sg % N || so % N) {
     if (io_dtype == BASED_BF16) gated_act_scalar_kernel<__nv_bfloat16><<<grid, NORM_THREADS, 0, stream>>>(p);
     else gated_act_scalar_kernel<float><<<grid, NORM_THREADS, 0, stream>>>(p);
@@ -707,11 +713,11 @@ int launch_gated_act(const void* y, const void* gate, void* out, int64_t M, int 
   }
 #define BASED_LAUNCH_ACT(T)                                                                      \
   do {                                                                                           \
-    if (vpt <= 1) launch_rows(few, gated_act_kernel<T, 1, true>, gated_act_kernel<T, 1, false>, grid, stream, p); \
-    else if (vpt <= 2) launch_rows(few, gated_act_kernel<T, 2, true>, gated_act_kernel<T, 2, false>, grid, stream, p); \
-    else if (vpt <= 4) launch_rows(few, gated_act_kernel<T, 4, true>, gated_act_kernel<T, 4, false>, grid, stream, p); \
-    else if (vpt <= 8) launch_rows(few, gated_act_kernel<T, 8, true>, gated_act_kernel<T, 8, false>, grid, stream, p); \
-    else launch_rows(few, gated_act_kernel<T, 16, true>, gated_act_kernel<T, 16, false>, grid, stream, p); \
+    if (vpt <= 1) launch_rows(early, gated_act_kernel<T, 1, true>, gated_act_kernel<T, 1, false>, grid, stream, p); \
+    else if (vpt <= 2) launch_rows(early, gated_act_kernel<T, 2, true>, gated_act_kernel<T, 2, false>, grid, stream, p); \
+    else if (vpt <= 4) launch_rows(early, gated_act_kernel<T, 4, true>, gated_act_kernel<T, 4, false>, grid, stream, p); \
+    else if (vpt <= 8) launch_rows(early, gated_act_kernel<T, 8, true>, gated_act_kernel<T, 8, false>, grid, stream, p); \
+    else launch_rows(early, gated_act_kernel<T, 16, true>, gated_act_kernel<T, 16, false>, grid, stream, p); \
   } while (0)
   if (io_dtype == BASED_BF16) BASED_LAUNCH_ACT(__nv_bfloat16);
   else BASED_LAUNCH_ACT(float);

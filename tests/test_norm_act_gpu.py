@@ -120,14 +120,15 @@ def test_norm_act_full_size_properties(ops):
     assert rel_err(h[:64].cpu().double(), O.gated_act(y[:64].cpu().double(), "silu")) < TOL[torch.bfloat16]
 
 
+@pytest.mark.parametrize("M", [1185, 2048])
 @pytest.mark.parametrize("D", [512, 1024, 1792, 4096, 8192])
-def test_many_rows_equal_few(ops, D):
-    """Few rows run as a programmatic launch with the weights loaded early, many without either: the same arithmetic, so rows
-    of a large call equal those of a small one to the bit.  1185 rows is one above the gated activation's border; the norms'
-    lies between the two sizes for every width."""
+def test_many_rows_equal_few(ops, D, M):
+    """A call runs as a programmatic launch with the weights loaded early, or with neither: the same arithmetic, so rows of a large
+    call equal those of a small one to the bit.  1185 rows is one above the border for narrow rows, and every width's norms have
+    left the first range there; at 2048 the wide ones are programmatic again."""
     g = torch.Generator("cuda").manual_seed(D)
     r = lambda *s, dtype=torch.bfloat16: torch.randn(*s, generator=g, device="cuda").to(dtype)
-    M, m = 1185, 5
+    m = 5
     x, res, w, w2, gate = r(M, D), r(M, D, dtype=torch.float32), r(D), r(D), r(M, D)
 
     def all_ops(n):
