@@ -19,10 +19,10 @@ namespace {
 // flight while it builds the feature tables; the 32 vectors of a step lie in two rows known at compile time, so a product is added to one
 // of two sums (to one of all rows of a group: 16 instructions more a vector for bf16).
 // CTA size: 192 threads, four CTAs per SM, for many (batch, head) blocks with fp32 states, 128 and five with bf16 ones (their row
-// groups are half as many).  us at B=256, H=16, dv=64 (the bytes at the HBM rate): fp32 92 (89), with three CTAs, their first loads behind
-// the tables, 102.5; bf16 72.2 (44), 163 then.  256 threads (two per SM) for few blocks, where one block's latency counts (B=16, H=16,
-// bf16 state 7.5); 512 where every block has an SM of its own and more than eight row groups (B=8, H=16, dv=112, bf16 state, in a
-// chain of launches: 10.5 us with 256, 6.6 with 512).
+// groups are half as many).  us at B=256, H=16, dv=64, one launch after the other in a graph (the bytes at the HBM rate; a lone call takes
+// some 5 more): fp32 93 (89), with three CTAs, their first loads behind the tables, 102.5; bf16 73 (45), 163 then; dv=112 161 (155) and 122
+// (77).  256 threads (two per SM) for few blocks, where one block's latency counts (B=16, H=16, bf16 state 7.5); 512 where every block has
+// an SM of its own and more than eight row groups (B=8, H=16, dv=112, bf16 state, in a chain of launches: 10.5 us with 256, 6.6 with 512).
 constexpr int kTab = 288;     // table length: 273 + wrap-around + padding, multiple of 4
 constexpr int kVecPerGroup = kExpandedDim;  // 273 vectors of 16 B per row group
 constexpr int kIters = (kVecPerGroup + 31) / 32;  // 9
@@ -115,8 +115,8 @@ linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
     s_x[0][tid] = to_float(q[b * sq.b + h * sq.h + tid]);
   } else if (tid < 2 * kFeatureDim) {
     s_x[1][tid - kFeatureDim] = to_float(k[b * sk.b + h * sk.h + tid - kFeatureDim]);
-  } else if (tid - 2 * kFeatureDim < dv) {
-    s_v[tid - 2 * kFeatureDim] = to_float(v[b * sv.b + h * sv.h + tid - 2 * kFeatureDim]);
+  } else {   // (128 threads: more values than there are threads left)
+    for (int i = tid - 2 * kFeatureDim; i < dv; i += kThreads - 2 * kFeatureDim) s_v[i] = to_float(v[b * sv.b + h * sv.h + i]);
   }
   __syncthreads();
   for (int idx = tid; idx < 2 * kExpandedDim; idx += kThreads) {   // a feature once, into its places in the four copies
@@ -201,6 +201,7 @@ linattn_decode_kernel(const IO* q, const IO* k, const IO* v,
     }
   }
   __syncthreads();
+  static_assert(kThreads >= 128, "a thread per value of the output");
   if (tid < dv) {
     y[b * sy.b + h * sy.h + tid] = from_float<IO>(s_num[tid] / (s_den + eps));
   }

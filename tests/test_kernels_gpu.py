@@ -235,6 +235,36 @@ def test_linattn_decode_many_heads_vs_oracle(ops, io, st, B, H, dv):
     assert _capi.read_status() == 0
 
 
+# Block sizes by (batch, head) blocks: 192 threads (float32 states) or 128 (bf16) from 6 to an SM on, 512 for one to an SM with more than eight
+# row groups, 256 else; widths around what a block's threads load and write at once, the smallest and the largest.
+@pytest.mark.parametrize("B,H", [(2, 5), (37, 4), (149, 1), (111, 8), (74, 12), (256, 4)])
+@pytest.mark.parametrize("dv", [8, 64, 72, 96, 104, 112, 120, 128])
+@pytest.mark.parametrize("st", [torch.float32, torch.bfloat16])
+def test_linattn_decode_every_block_size(ops, B, H, dv, st):
+    """Every element of the states and of the output, two steps, against the sums in 64 bits."""
+    g = torch.Generator("cuda").manual_seed(B * dv)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    kv, ks = (0.02 * rnd(B, H, 1, dv, 273)).to(st), (1.0 + 0.02 * rnd(B, H, 1, 1, 273)).to(st)
+    for io in (torch.bfloat16, torch.float32):
+        q, k, v = (rnd(B, H, 1, 16) / 2).to(io), (rnd(B, H, 1, 16) / 2).to(io), rnd(B, H, 1, dv).to(io)
+        kv_ref, ks_ref = kv.double(), ks.double()
+        O.linattn_recurrent_step(kv_ref, ks_ref, q.double(), k.double(), v.double())
+        y = ops.linattn_decode(q, k, v, kv, ks)
+        # a state: features to a few 2^-24, one rounding to its type (2^-9 of the value)
+        for own, ref in ((kv, kv_ref), (ks, ks_ref)):
+            off = (own.double() - ref).abs()
+            assert bool((off <= ref.abs() * (2 ** -8 if st == torch.bfloat16 else 0) + 4e-6).all()), float(off.max())
+        # the output is read from the states as they are stored; 273 terms summed in float32, one rounding to its type
+        fq = O.taylor_exp(q.double())
+        terms = fq.unsqueeze(-2) * kv.double()
+        norm = fq.unsqueeze(-2) * ks.double()
+        y_ref = terms.sum(-1) / norm.sum(-1)
+        room = (terms.abs().sum(-1) + y_ref.abs() * norm.abs().sum(-1)) / norm.sum(-1).abs()
+        y_ref, room = (t.transpose(1, 2).reshape(B, 1, H * dv) for t in (y_ref, room))
+        off = (y.double() - y_ref).abs()
+        assert bool((off <= room * 1e-5 + y_ref.abs() * (2 ** -8 if io == torch.bfloat16 else 0)).all()), float((off / room).max())
+
+
 def test_linattn_decode_golden(ops):
     """Decode steps the reference itself ran (recurrent_forward), from its prefill state."""
     g = load_golden("linattn_qkv_f32_dv112.npz")
