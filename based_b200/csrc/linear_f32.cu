@@ -1,18 +1,22 @@
 // Linear layers of a prompt in float32, on the tensor cores: y[M, N] = x[M, K] W[N, K]^T (+ bias), W in up to four matrices one after the
 // other (the projections of one input are one product).
 //
-// A float32's 24 significant bits are exactly the sum of three bf16 values of 8 bits (h + m + l: the value cut after 8 bits, the rest cut
-// after 8, what is left).  A product is then nine bf16 products, exact in the tensor cores' float32 sums; the six of them that
-// reach 2^-24 of the product are computed (h h, h m, m h, m m, h l, l h), so an operand rounds no more than it did.  What is left
-// is the sum: the tensor cores cut a sum's low bits at every step (1e-9 K of it at K = 1024), so the h h products leave TMEM after every
-// 128 values of K and are added up in registers, rounded to nearest; the small ones, 2^-8 of them and less, stay in an accumulator of
-// their own.  Relative error against 64 bits (2-norm, normal values): 1.3e-7 to 2.0e-7 for K = 72 to 2048; the library's float32 product
-// 1.5e-7 to 8.1e-7.  (Values below 2^-110 lose m and l, which are subnormal there.)
+// A row of x or W is scaled by the power of two that takes its largest value to [1, 2), and a value's 24 significant bits are exactly the
+// sum of three bf16 values of 8 bits, each what is left rounded to nearest: h + m + l, |m| <= 2^-8 and |l| <= 2^-17 of the value's power of
+// two.  A product is then nine bf16 products, exact in the tensor cores' float32 sums; six of them are computed (h h, h m, m h, m m, h l,
+// l h).  The other three come to at most 2^-24 of the product, of either sign: as much as rounding it once.  (Values merely cut leave 2^-21,
+// always of the product's sign.)  Values below 2^-110 of their row's largest lose bits of m and l, which end at 2^-133 of it; small and
+// large rows lose none, and nothing overflows that the result does not.  What is left is the sum: the tensor cores cut a sum's low bits at
+// every step (1e-9 K of it at K = 1024), so the h h products leave TMEM after every 128 values of K and are added up in registers, rounded
+// to nearest; the small ones, 2^-8 of them and less, stay in an accumulator of their own.  Relative error against 64 bits (2-norm, normal
+// values, K = 256 to 1024) 1.25e-7 to 1.4e-7, the library's float32 product 2.9e-7 to 5.8e-7; the largest of an element in 2^-24 of its
+// products' absolute sum 0.8 to 2.2 and 4.5 to 6.7, all of one sign (K = 72 to 2048) 2.0 to 5.3 and 10 to 52.
 //
 // linear_f32_split_kernel writes the three planes of x and W; linear_f32_kernel multiplies them: a pair of CTAs per tile, a TMA producer, an
-// MMA issuer, eight warps that add.  The library's float32 product runs on the CUDA cores; us with it / here (rows; outputs x K): 512
-// 29 / 25, 2048 84 / 27, 8192 329 / 87 (1024 x 1024); 2048 141 / 40 (1536 x 1024); 2048 25 / 17 (512 x 512).  Of the 27, 5 are the split,
-// 19 the products: 1.2 a chunk of 64 values of K, 1.0 of it products at full rate.
+// MMA issuer, eight warps that add.  The library's float32 product runs on the CUDA cores; us with it / here, one after the other in a graph
+// (rows; outputs x K): 512 29 / 25, 2048 83 / 28.5, 8192 329 / 89 (1024 x 1024); 2048 141 / 42 (1536 x 1024); 2048 24.5 / 17.4 (512 x 512).  Of
+// the 28.5, 6 are the split, 19 the products: 1.2 a chunk of 64 values of K, 1.0 of it products at full rate.  The rows' scales take 1 to 2
+// of it (27 without): a row's largest value is found before its first is split, and each output is multiplied by two powers of two.
 #include "common.cuh"
 #include "tc_pair.cuh"
 
@@ -25,7 +29,7 @@ using namespace tc;
 
 __device__ unsigned int g_tc_status_f32;
 
-constexpr int kBM = 256, kBK = 64, kStages = 2, kRun = 2, kAddWarps = 8, kThreads = (kAddWarps + 2) * 32, kMaxParts = 5;
+constexpr int kBM = 256, kBK = 64, kStages = 2, kRun = 2, kAddWarps = 8, kThreads = (kAddWarps + 2) * 32, kMaxParts = 5, kHeld = 4;
 constexpr uint32_t kPlane = 128 * kBK * 2, kSlab = 4096;   // bytes of a plane's 128 rows in a stage; of 32 x 32 outputs
 constexpr unsigned kCode = 1u << 13;
 
@@ -34,45 +38,75 @@ struct SplitParams {   // up to kMaxParts matrices of K columns: row r of part i
   __nv_bfloat16* dst[kMaxParts];
   int64_t stride[kMaxParts], plane[kMaxParts];   // elements between rows of src, between planes of dst
   int first[kMaxParts + 1], at[kMaxParts];       // rows before the part, row of its first in dst
+  float2* power[kMaxParts];                      // of the planes' rows: the power of two to multiply them by, in two factors of some half of it
   int K, parts;
 };
 
-// A thread splits eight values.  Not a finite number: all in h (the products of its m and l would be NaN where the sum is infinite).
+// A warp splits a row.  Not a finite number: all in h (the products of its m and l would be NaN where the sum is infinite).
 __global__ void __launch_bounds__(256) linear_f32_split_kernel(const __grid_constant__ SplitParams p) {
   pdl_trigger();
   pdl_wait();
-  const int groups = p.K / 8;
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  int row = (int)(i / groups);
-  const int c = (int)(i - (int64_t)row * groups) * 8;
+  const int groups = p.K / 8, lane = threadIdx.x & 31;
+  int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= p.first[p.parts]) return;
   int part = 0;
   while (row >= p.first[part + 1]) ++part;
   row -= p.first[part];
-  const float* src = p.src[part] + row * p.stride[part] + c;
-  const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
-  const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  uint32_t h[8], m[8], l[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint32_t x = __float_as_uint(v[j]);
-    const bool finite = (x & 0x7f800000u) != 0x7f800000u;
-    h[j] = finite || !(x & 0x7fffffu) ? x & 0xffff0000u : 0x7fc00000u;
-    const float r = finite ? v[j] - __uint_as_float(h[j]) : 0.f;
-    m[j] = __float_as_uint(r) & 0xffff0000u;
-    l[j] = __float_as_uint(r - __uint_as_float(m[j]));   // eight bits are left
-  }
-  auto pack = [](const uint32_t (&x)[8]) {
-    return make_uint4(x[0] >> 16 | (x[1] & 0xffff0000u), x[2] >> 16 | (x[3] & 0xffff0000u), x[4] >> 16 | (x[5] & 0xffff0000u), x[6] >> 16 | (x[7] & 0xffff0000u));
+  const float4* src = reinterpret_cast<const float4*>(p.src[part] + row * p.stride[part]);
+  uint32_t most = 0;   // of the finite values' bits without the sign
+  auto see = [&](const float4& v) {
+    for (float e : {v.x, v.y, v.z, v.w}) {
+      const uint32_t x = __float_as_uint(e) & 0x7fffffffu;
+      most = max(most, x < 0x7f800000u ? x : 0u);
+    }
   };
-  __nv_bfloat16* dst = p.dst[part] + (int64_t)(p.at[part] + row) * p.K + c;
-  *reinterpret_cast<uint4*>(dst) = pack(h);
-  *reinterpret_cast<uint4*>(dst + p.plane[part]) = pack(m);
-  *reinterpret_cast<uint4*>(dst + 2 * p.plane[part]) = pack(l);
+  // up to 1024 values of a row stay in registers; what is behind them is read again
+  float4 held[2 * kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int at = lane + 32 * i;
+    held[2 * i] = held[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (at < groups) {
+      held[2 * i] = src[2 * at];
+      held[2 * i + 1] = src[2 * at + 1];
+    }
+  }
+  for (int at = 64 * kHeld + lane; at < 2 * groups; at += 32) see(src[at]);
+#pragma unroll
+  for (int i = 0; i < 2 * kHeld; ++i) see(held[i]);
+  most = __reduce_max_sync(0xffffffffu, most);
+  const int e = most ? min(max((int)(most >> 23) - 127, -126), 126) : 0;   // 2^-e is a normal number
+  const float scale = __uint_as_float((uint32_t)(127 - e) << 23);
+  if (lane == 0) {   // 2^e in two factors
+    const int half = e >> 1;
+    p.power[part][p.at[part] + row] = make_float2(__uint_as_float((uint32_t)(127 + half) << 23), __uint_as_float((uint32_t)(127 + e - half) << 23));
+  }
+  __nv_bfloat16* dst = p.dst[part] + (int64_t)(p.at[part] + row) * p.K;
+  auto split = [&](int at, const float4& lo, const float4& hi) {
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    float h[8], m[8], l[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float x = v[j] * scale;
+      h[j] = __bfloat162float(__float2bfloat16_rn(x));
+      const float r = fabsf(x) < __int_as_float(0x7f800000) ? x - h[j] : 0.f;
+      m[j] = __bfloat162float(__float2bfloat16_rn(r));
+      l[j] = r - m[j];
+    }
+    auto pack = [](const float (&x)[8]) { return make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7])); };
+    *reinterpret_cast<uint4*>(dst + 8 * at) = pack(h);
+    *reinterpret_cast<uint4*>(dst + p.plane[part] + 8 * at) = pack(m);
+    *reinterpret_cast<uint4*>(dst + 2 * p.plane[part] + 8 * at) = pack(l);
+  };
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i)
+    if (lane + 32 * i < groups) split(lane + 32 * i, held[2 * i], held[2 * i + 1]);
+  for (int at = 32 * kHeld + lane; at < groups; at += 32) split(at, src[2 * at], src[2 * at + 1]);
 }
 
 struct F32Params {
   int M, N, K, col_tiles;
+  const float2 *px, *pw;   // powers of the rows of x and of W
   const float* bias;
   unsigned int* status;
 };
@@ -99,6 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
+  __shared__ __align__(16) float2 powers[kAddWarps][kSpan];   // of a warp's columns
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = base + kStages * kStage;
   const uint32_t full = bars, empty = full + 8 * kStages, sum_full = empty + 8 * kStages, sum_empty = sum_full + 8;
@@ -193,6 +228,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int part = (warp >> 2) * kSpan;
     const uint32_t at = tmem + ((uint32_t)(warp & 3) << 21) + part, done = map_rank(sum_empty, 0);
     const float inf = __int_as_float(0x7f800000);
+    const int own = m0 + (warp & 3) * 32 + lane;
+    const float2 px = own < p.M ? p.px[own] : make_float2(1.f, 1.f);
+    for (int i = lane; i < kSpan; i += 32) powers[warp][i] = n0 + part + i < p.N ? p.pw[n0 + part + i] : make_float2(1.f, 1.f);
+    __syncwarp();
     float sum[kSpan];
 #pragma unroll
     for (int i = 0; i < kSpan; ++i) sum[i] = 0.f;
@@ -236,7 +275,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < 4; ++i) {
           const int col = 4 * q + i;
           const float big = sum[32 * j + col];
-          y[i] = fabsf(big) < inf ? big + __uint_as_float(r[col]) : big;
+          const float2 pw = powers[warp][32 * j + col];
+          // as one rounding: the factors are near one another, so where the first product is subnormal the second is nothing
+          y[i] = (fabsf(big) < inf ? big + __uint_as_float(r[col]) : big) * (px.x * pw.x) * (px.y * pw.y);
           if (p.bias && c0 + col < p.N) y[i] += p.bias[c0 + col];
         }
         st_shared16(slab + tma::sw128_offset(lane, q), __float_as_uint(y[0]), __float_as_uint(y[1]), __float_as_uint(y[2]), __float_as_uint(y[3]));
@@ -317,30 +358,32 @@ int read_tc_status_f32(unsigned int* out, int reset) {
   return 0;
 }
 
-size_t linear_f32_scratch_bytes(int M, int N, int K) { return 6 * ((size_t)M + N) * K; }
+// three planes of bf16, and a row's power of two
+size_t linear_f32_scratch_bytes(int M, int N, int K) { return (6 * (size_t)K + sizeof(float2)) * ((size_t)M + N); }
 
 int launch_linear_f32(const float* x, const float* const* w, const int* rows, int parts, const float* bias, float* out, int M, int N, int K, int64_t sx,
                       void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (K % 8 != 0 || N % 4 != 0) return BASED_ERR_SHAPE;
   if (sx % 4 != 0 || !aligned16(x) || !aligned16(out) || !aligned16(scratch)) return BASED_ERR_ALIGN;
   if (scratch_bytes < linear_f32_scratch_bytes(M, N, K)) return BASED_ERR_SCRATCH;
+  const int64_t blocks = ((int64_t)M + N + 7) / 8;
+  if (blocks > 2147483647LL / 8) return BASED_ERR_TOO_LARGE;
   __nv_bfloat16 *px = static_cast<__nv_bfloat16*>(scratch), *pw = px + 3 * (size_t)M * K;
+  float2 *power_w = reinterpret_cast<float2*>(pw + 3 * (size_t)N * K), *power_x = power_w + N;
   SplitParams sp{};
   sp.K = K;
   sp.parts = parts + 1;
-  sp.src[0] = x; sp.dst[0] = px; sp.stride[0] = sx; sp.plane[0] = (int64_t)M * K; sp.first[1] = M;
+  sp.src[0] = x; sp.dst[0] = px; sp.stride[0] = sx; sp.plane[0] = (int64_t)M * K; sp.first[1] = M; sp.power[0] = power_x;
   for (int i = 0, at = 0; i < parts; at += rows[i++]) {
     if (!aligned16(w[i])) return BASED_ERR_ALIGN;
-    sp.src[i + 1] = w[i]; sp.dst[i + 1] = pw; sp.stride[i + 1] = K; sp.plane[i + 1] = (int64_t)N * K;
+    sp.src[i + 1] = w[i]; sp.dst[i + 1] = pw; sp.stride[i + 1] = K; sp.plane[i + 1] = (int64_t)N * K; sp.power[i + 1] = power_w;
     sp.at[i + 1] = at; sp.first[i + 2] = M + at + rows[i];
   }
-  const int64_t blocks = (((int64_t)M + N) * (K / 8) + 255) / 256;
-  if (blocks > 2147483647LL) return BASED_ERR_TOO_LARGE;
   const int rc = launch_pdl(linear_f32_split_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, sp);
   if (rc != 0) return launched(rc);
   // the wide tile has more products to a byte, the other one fills the chip sooner: 2.15 and 1.2 us a round for 64 values of K
   const int64_t rounds = (M + kBM - 1) / kBM, wide = (rounds * ((N + 255) / 256) + 73) / 74, narrow = (rounds * ((N + 127) / 128) + 73) / 74;
-  const F32Params p{M, N, K, 0, bias, nullptr};
+  const F32Params p{M, N, K, 0, power_x, power_w, bias, nullptr};
   return wide * 215 <= narrow * 120 ? run_f32<true>(p, px, pw, out, stream) : run_f32<false>(p, px, pw, out, stream);
 }
 

@@ -780,14 +780,14 @@ def _split_rows(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -
     return all(_unwatched(x, w) for w in weights)
 
 
-# us with the library / linear_split (rows; outputs x K): 256 21 / 24, 512 29 / 25 (1024 x 1024); 1024 21 / 24, 2048 30 / 25 (256 x 1024);
-# 512 25 / 18 (2048 x 512); 1024 16.5 / 15.8 (512 x 512); 2048 9.8 / 12, 4096 14.5 / 13 (256 x 256).
+# us with the library / linear_split (rows; outputs x K): 256 21 / 25, 512 29 / 25 (1024 x 1024); 1024 21 / 25, 2048 29 / 26.5 (256 x 1024);
+# 512 24.5 / 17.6 (2048 x 512); 1024 16 / 16.2 (512 x 512); 2048 9.5 / 12.4, 4096 14.5 / 12.7 (256 x 256).
 SPLIT_MIN_OUTPUTS, SPLIT_MIN_PRODUCTS = 1 << 19, 1 << 28
 
 
 def linear_split(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x [W0; W1; ..]^T (+ bias)`` in fp32 on the tensor cores, for the rows of a prompt: x ``[..., K]``, up to four weights ``[n, K]``.
-    Operands are taken whole (three bf16 values each), sums are fp32."""
+    An operand is three bf16 values; what is left out of a product is no more than rounding it once; sums are fp32."""
     _need_cuda(x, *weights, bias)
     K = x.shape[-1]
     if any(t.dtype != torch.float32 for t in (x, *weights)) or any(w.shape[1] != K or not w.is_contiguous() for w in weights) or not 0 < len(weights) <= 4:
@@ -800,7 +800,7 @@ def linear_split(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) 
     M = x.numel() // K if K else 0
     out = torch.empty(*x.shape[:-1], N, dtype=torch.float32, device=x.device)
     if M > 0:
-        scratch = torch.empty(6 * (M + N) * K, dtype=torch.uint8, device=x.device)
+        scratch = torch.empty(_capi.lib().based_linear_f32_scratch_bytes(M, N, K), dtype=torch.uint8, device=x.device)
         none = 4 - len(weights)
         code = _capi.native().linear_f32(x2, *weights, *[None] * none, *[w.shape[0] for w in weights], *[0] * none, bias, out, M, K,
                                          _row_stride(x2, K), scratch, scratch.numel())

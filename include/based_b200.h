@@ -407,7 +407,8 @@ int based_prompt_linear_conv(const void* x, const void* w, const void* bias, voi
 
 /*
  * Linear layers of a prompt in fp32 on the tensor cores: out [M, n0 + n1 + n2 + n3] = x [W0; W1; W2; W3]^T (+ bias), Wi [ni, K]
- * contiguous (NULL and 0 from the first one that is not there on).  Each operand is taken as the exact sum of three bf16 values; sums are fp32.
+ * contiguous (NULL and 0 from the first one that is not there on).  Each operand is the exact sum of three bf16 values
+ * (under its row's largest by 2^110 and more: to 2^-133 of that); what is left out of a product is at most 2^-24 of it; sums are fp32.
  * scratch: based_linear_f32_scratch_bytes(M, N, K) bytes.  K a multiple of 8, N of 4, x rows sx (a multiple of 4) elements apart; all
  * pointers 16-byte aligned but bias.
  */

@@ -34,6 +34,47 @@ def test_split_products(ops, M, parts, K, scale):
     assert _capi.read_status() == 0
 
 
+# What a split may lose shows where nothing cancels: operands of one sign, constant ones, the largest part of a bf16 value (2^-7 - 2^-23 cut
+# after it leaves 2^-7), rows of very small and very large values.  Both tiles.
+@pytest.mark.parametrize("M,N", [(256, 128), (2048, 1536)])
+@pytest.mark.parametrize("K", [8, 200, 1024])
+@pytest.mark.parametrize("kind", ["1 + 2^-7 - 2^-23", "0.1", "1 - 2^-24", "positive", "signs", "tiny", "subnormal", "huge", "rows"])
+def test_split_products_element_by_element(ops, M, N, K, kind):
+    g = torch.Generator("cuda").manual_seed(K)
+    x, w = torch.rand(M, K, generator=g, device="cuda") + 0.5, torch.rand(N, K, generator=g, device="cuda") + 0.5
+    const = {"1 + 2^-7 - 2^-23": 1 + 2 ** -7 - 2 ** -23, "0.1": 0.1, "1 - 2^-24": 1 - 2 ** -24}.get(kind)
+    if const is not None:
+        x.fill_(const), w.fill_(const)
+    elif kind == "signs":
+        x, w = x * torch.randn_like(x).sign(), w * torch.randn_like(w).sign()
+    elif kind == "tiny":
+        x, w = x * 2.0 ** -118, w * 2.0 ** 30
+    elif kind == "subnormal":          # 2^-132 to 2^-131: 18 bits of the operand, exactly
+        x, w = x * 2.0 ** -131, w * 2.0 ** 60
+    elif kind == "huge":               # the products come near the largest float, their sums do not pass it
+        x, w = x * 2.0 ** 100, w * (2.0 ** 26 / K)
+    elif kind == "rows":
+        x = x * 2.0 ** torch.arange(M, device="cuda").remainder(120).sub(60)[:, None]
+        w = w * 2.0 ** torch.arange(N, device="cuda").remainder(100).sub(50)[:, None]
+    y, xd, wd = ops.linear_split(x, (w,)), x.double(), w.double()
+    ref, room = xd @ wd.T, xd.abs() @ wd.abs().T
+    off = ((y.double() - ref).abs() / room).max().item()
+    # a product to 2^-24, and 2^-24 more for each of the sums of the runs of 128 values and for what the tensor cores cut in a run
+    assert off < 2 ** -24 * (2 + K / 128 + 4), off * 2 ** 24
+
+
+def test_split_products_of_mixed_magnitudes(ops):
+    """Values far below their row's largest: to 2^-133 of it, which bounds what they may add.  A few products carry each sum, so that all of
+    the sixteen steps of the tensor cores may cut it, by 2^-23 each."""
+    K = 256
+    g = torch.Generator("cuda").manual_seed(1)
+    x, w = torch.rand(512, K, generator=g, device="cuda") + 0.5, torch.rand(256, K, generator=g, device="cuda") + 0.5
+    x[:, 1:] *= 2.0 ** -torch.randint(1, 140, (512, K - 1), generator=g, device="cuda").float()
+    w[:, 0], w[:, 1] = 0, 2.0 ** 40      # the row's largest of x meets nothing
+    y, ref, room = ops.linear_split(x, (w,)).double(), x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((y - ref).abs() <= room * 2 ** -23 * (K // 16) + K * 2.0 ** -132 * 2.0 ** 41).all())
+
+
 def test_split_products_of_special_values(ops):
     """Infinite and undefined sums as torch has them, for both tiles; the largest values do not overflow on the way."""
     for M, N in ((256, 128), (2048, 1536)):
