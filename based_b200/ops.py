@@ -777,6 +777,8 @@ def _split_rows(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -
     if bias is not None and not (type(bias) in _PLAIN_TYPES and bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == (N,)
                                  and bias.device == x.device and not _wrapped(bias)):
         return False
+    if torch.backends.cuda.matmul.fp32_precision not in ("none", "ieee"):   # the caller lets products round: the library's one pass
+        return False
     return all(_unwatched(x, w) for w in weights)
 
 

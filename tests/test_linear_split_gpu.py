@@ -109,3 +109,28 @@ def test_prompt_routes(ops, monkeypatch):
     with pytest.raises(RuntimeError):
         m(x)                         # the kernels have no backward
     assert len(calls) == 3
+
+
+def _set(where, name, value):
+    return lambda: setattr(where, name, value)
+
+
+@pytest.mark.parametrize("allow,forbid", [
+    (_set(torch.backends, "fp32_precision", "tf32"), _set(torch.backends, "fp32_precision", "none")),
+    (_set(torch.backends.cuda.matmul, "fp32_precision", "tf32"), _set(torch.backends.cuda.matmul, "fp32_precision", "none")),
+    (_set(torch.backends.cuda.matmul, "allow_tf32", True), _set(torch.backends.cuda.matmul, "allow_tf32", False)),
+    (lambda: torch.set_float32_matmul_precision("high"), lambda: torch.set_float32_matmul_precision("highest"))])
+def test_callers_that_let_products_round(ops, monkeypatch, allow, forbid):
+    """Who allows TF32 gets the library's one pass over rounded operands, by whichever switch; switched back, the exact products."""
+    calls, own = [], ops.linear_split
+    monkeypatch.setattr(ops, "linear_split", lambda *a, **k: calls.append(1) or own(*a, **k))
+    x, w = torch.randn(1024, 1024, device="cuda"), torch.randn(1024, 1024, device="cuda")
+    with torch.inference_mode():
+        y = ops.linear(x, w)
+        try:
+            allow()
+            z = ops.linear(x, w)
+            assert len(calls) == 1 and torch.equal(z, torch.nn.functional.linear(x, w)) and not torch.equal(y, z)
+        finally:
+            forbid()
+        assert torch.equal(ops.linear(x, w), y) and len(calls) == 2
