@@ -130,7 +130,7 @@ class LinearAttention(nn.Module):
             nq = self.feature_dim * self.num_heads
             qkv = ops.linear(hidden_states, self._fused_qkv_weight())
             q, k, v = qkv[..., :nq], qkv[..., nq:2 * nq], qkv[..., 2 * nq:]
-        elif (all(plain_linear(m) for m in (self.proj_q, self.proj_k, self.proj_v))
+        elif (all(plain_linear(m) and m.bias is None for m in (self.proj_q, self.proj_k, self.proj_v))
               and ops._split_rows(hidden_states, weights := (self.proj_q.weight, self.proj_k.weight, self.proj_v.weight))):
             # fp32 prompts: one product for the three, too
             nq = self.feature_dim * self.num_heads

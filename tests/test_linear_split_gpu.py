@@ -111,6 +111,26 @@ def test_prompt_routes(ops, monkeypatch):
     assert len(calls) == 3
 
 
+def test_projections_with_a_bias(ops):
+    """A projection that was replaced by one with a bias keeps it."""
+    from based_b200.mixers import LinearAttention
+    m = LinearAttention(512, num_heads=8, layer_idx=0, device="cuda").eval()
+    x = torch.randn(2, 1024, 512, device="cuda")
+    for name in ("proj_q", "proj_k", "proj_v"):
+        plain = getattr(m, name)
+        biased = torch.nn.Linear(512, plain.out_features, device="cuda")
+        with torch.inference_mode():
+            biased.weight.copy_(plain.weight)
+            biased.bias.fill_(0.5)
+            setattr(m, name, biased)
+            y = m(x)
+            h = biased.register_forward_hook(lambda *a: None)   # watched: called as a module
+            assert torch.allclose(y, m(x), rtol=1e-3, atol=1e-4)
+            h.remove()
+            setattr(m, name, plain)
+            assert not torch.allclose(y, m(x), rtol=1e-2, atol=1e-3)
+
+
 def _set(where, name, value):
     return lambda: setattr(where, name, value)
 
