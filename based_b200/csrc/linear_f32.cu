@@ -346,6 +346,27 @@ int run_f32(F32Params p, const void* px, const void* pw, float* out, cudaStream_
   return launched((int)cudaLaunchKernelEx(&cfg, linear_f32_kernel<WIDE>, mx, mw, mh, mo, p));
 }
 
+// three planes of bf16, and a row's power of two
+size_t row_bytes(int K) { return 6 * (size_t)K + sizeof(float2); }
+
+// Rows of x that are split at a time: all of them, or whole tiles that fit in what kScratch leaves beside W (kLeast, whatever W takes), as many
+// as make the fewest rounds of wide tiles over all parts.  us with all rows' planes at once
+// / in parts: 32768 rows 463 / 465, 65536 896 / 922 (1536 x 1024), 665 / 738 (1024 x 1024; the parts' last rounds are not full).
+constexpr size_t kScratch = (size_t)128 << 20;
+constexpr int kLeast = 2048;
+int rows_at_a_time(int M, int N, int K) {
+  const size_t w = row_bytes(K) * N;
+  const int64_t fit = std::max<int64_t>(w < kScratch ? (kScratch - w) / row_bytes(K) : 0, kLeast);
+  if (M <= fit) return M;
+  const int64_t most = fit / kBM, all = ((int64_t)M + kBM - 1) / kBM, cols = (N + 255) / 256;   // tiles
+  int64_t best = most, least = INT64_MAX;
+  for (int64_t t = most; t > most / 2; --t) {
+    const int64_t cost = all / t * ((t * cols + 73) / 74) + (all % t * cols + 73) / 74;
+    if (cost < least) { best = t; least = cost; }
+  }
+  return (int)(best * kBM);
+}
+
 }  // namespace
 
 int read_tc_status_f32(unsigned int* out, int reset) {
@@ -358,33 +379,40 @@ int read_tc_status_f32(unsigned int* out, int reset) {
   return 0;
 }
 
-// three planes of bf16, and a row's power of two
-size_t linear_f32_scratch_bytes(int M, int N, int K) { return (6 * (size_t)K + sizeof(float2)) * ((size_t)M + N); }
+size_t linear_f32_scratch_bytes(int M, int N, int K) { return row_bytes(K) * ((size_t)rows_at_a_time(M, N, K) + N); }
 
 int launch_linear_f32(const float* x, const float* const* w, const int* rows, int parts, const float* bias, float* out, int M, int N, int K, int64_t sx,
                       void* scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (K % 8 != 0 || N % 4 != 0) return BASED_ERR_SHAPE;
   if (sx % 4 != 0 || !aligned16(x) || !aligned16(out) || !aligned16(scratch)) return BASED_ERR_ALIGN;
   if (scratch_bytes < linear_f32_scratch_bytes(M, N, K)) return BASED_ERR_SCRATCH;
-  const int64_t blocks = ((int64_t)M + N + 7) / 8;
-  if (blocks > 2147483647LL / 8) return BASED_ERR_TOO_LARGE;
-  __nv_bfloat16 *px = static_cast<__nv_bfloat16*>(scratch), *pw = px + 3 * (size_t)M * K;
-  float2 *power_w = reinterpret_cast<float2*>(pw + 3 * (size_t)N * K), *power_x = power_w + N;
-  SplitParams sp{};
-  sp.K = K;
-  sp.parts = parts + 1;
-  sp.src[0] = x; sp.dst[0] = px; sp.stride[0] = sx; sp.plane[0] = (int64_t)M * K; sp.first[1] = M; sp.power[0] = power_x;
-  for (int i = 0, at = 0; i < parts; at += rows[i++]) {
+  const int step = rows_at_a_time(M, N, K);
+  if (((int64_t)step + N + 7) / 8 > 2147483647LL / 8) return BASED_ERR_TOO_LARGE;
+  for (int i = 0; i < parts; ++i)
     if (!aligned16(w[i])) return BASED_ERR_ALIGN;
-    sp.src[i + 1] = w[i]; sp.dst[i + 1] = pw; sp.stride[i + 1] = K; sp.plane[i + 1] = (int64_t)N * K; sp.power[i + 1] = power_w;
-    sp.at[i + 1] = at; sp.first[i + 2] = M + at + rows[i];
+  __nv_bfloat16 *px = static_cast<__nv_bfloat16*>(scratch), *pw = px + 3 * (size_t)step * K;
+  float2 *power_w = reinterpret_cast<float2*>(pw + 3 * (size_t)N * K), *power_x = power_w + N;
+  for (int64_t m0 = 0; m0 < M; m0 += step) {   // W is split with the first rows; a launch waits for the one before, so px is free again
+    const int m = (int)std::min<int64_t>(step, M - m0);
+    SplitParams sp{};
+    sp.K = K;
+    sp.parts = 1;
+    sp.src[0] = x + m0 * sx; sp.dst[0] = px; sp.stride[0] = sx; sp.plane[0] = (int64_t)m * K; sp.first[1] = m; sp.power[0] = power_x;
+    for (int i = 0, at = 0; i < parts && m0 == 0; at += rows[i++]) {
+      sp.parts = i + 2;
+      sp.src[i + 1] = w[i]; sp.dst[i + 1] = pw; sp.stride[i + 1] = K; sp.plane[i + 1] = (int64_t)N * K; sp.power[i + 1] = power_w;
+      sp.at[i + 1] = at; sp.first[i + 2] = m + at + rows[i];
+    }
+    int rc = launch_pdl(linear_f32_split_kernel, dim3((unsigned)((sp.first[sp.parts] + 7) / 8)), dim3(256), 0, stream, sp);
+    if (rc != 0) return launched(rc);
+    // the wide tile has more products to a byte, the other one fills the chip sooner: 2.15 and 1.2 us a round for 64 values of K
+    const int64_t rounds = (m + kBM - 1) / kBM, wide = (rounds * ((N + 255) / 256) + 73) / 74, narrow = (rounds * ((N + 127) / 128) + 73) / 74;
+    const F32Params p{m, N, K, 0, power_x, power_w, bias, nullptr};
+    float* y = out + m0 * N;
+    rc = wide * 215 <= narrow * 120 ? run_f32<true>(p, px, pw, y, stream) : run_f32<false>(p, px, pw, y, stream);
+    if (rc != 0) return rc;
   }
-  const int rc = launch_pdl(linear_f32_split_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, sp);
-  if (rc != 0) return launched(rc);
-  // the wide tile has more products to a byte, the other one fills the chip sooner: 2.15 and 1.2 us a round for 64 values of K
-  const int64_t rounds = (M + kBM - 1) / kBM, wide = (rounds * ((N + 255) / 256) + 73) / 74, narrow = (rounds * ((N + 127) / 128) + 73) / 74;
-  const F32Params p{M, N, K, 0, power_x, power_w, bias, nullptr};
-  return wide * 215 <= narrow * 120 ? run_f32<true>(p, px, pw, out, stream) : run_f32<false>(p, px, pw, out, stream);
+  return 0;
 }
 
 }  // namespace based

@@ -772,7 +772,7 @@ def _split_rows(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -
     N = sum(w.shape[0] for w in weights)
     if N % 4 or not 0 < len(weights) <= 4 or any(w.shape[0] == 0 for w in weights):
         return False
-    if x.numel() // K * N < SPLIT_MIN_OUTPUTS or x.numel() * N < SPLIT_MIN_PRODUCTS:
+    if x.numel() // K * N < SPLIT_MIN_OUTPUTS or x.numel() * N < SPLIT_MIN_PRODUCTS or N * K > SPLIT_MAX_WEIGHT:
         return False
     if bias is not None and not (type(bias) in _PLAIN_TYPES and bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == (N,)
                                  and bias.device == x.device and not _wrapped(bias)):
@@ -785,6 +785,9 @@ def _split_rows(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -
 # us with the library / linear_split (rows; outputs x K): 256 21 / 25, 512 29 / 25 (1024 x 1024); 1024 21 / 25, 2048 29 / 26.5 (256 x 1024);
 # 512 24.5 / 17.6 (2048 x 512); 1024 16 / 16.2 (512 x 512); 2048 9.5 / 12.4, 4096 14.5 / 12.7 (256 x 256).
 SPLIT_MIN_OUTPUTS, SPLIT_MIN_PRODUCTS = 1 << 19, 1 << 28
+# The call's scratch, 6 bytes an element of the weights and of as many rows as are split at a time, is at most 128 MB with up to
+# this many elements of weights (48 MB); a larger matrix (a model's head) stays with the library, which takes none.
+SPLIT_MAX_WEIGHT = 1 << 23
 
 
 def linear_split(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -409,7 +409,8 @@ int based_prompt_linear_conv(const void* x, const void* w, const void* bias, voi
  * Linear layers of a prompt in fp32 on the tensor cores: out [M, n0 + n1 + n2 + n3] = x [W0; W1; W2; W3]^T (+ bias), Wi [ni, K]
  * contiguous (NULL and 0 from the first one that is not there on).  Each operand is the exact sum of three bf16 values
  * (under its row's largest by 2^110 and more: to 2^-133 of that); what is left out of a product is at most 2^-24 of it; sums are fp32.
- * scratch: based_linear_f32_scratch_bytes(M, N, K) bytes.  K a multiple of 8, N of 4, x rows sx (a multiple of 4) elements apart; all
+ * scratch: based_linear_f32_scratch_bytes(M, N, K) bytes: 6 K + 8 for each row of W and of x, of x no more rows than make 128 MB of it (but
+ * 2048); many rows are taken in parts.  K a multiple of 8, N of 4, x rows sx (a multiple of 4) elements apart; all
  * pointers 16-byte aligned but bias.
  */
 int based_linear_f32(const void* x, const void* w0, const void* w1, const void* w2, const void* w3, int n0, int n1, int n2, int n3, const void* bias,

@@ -111,6 +111,35 @@ def test_prompt_routes(ops, monkeypatch):
     assert len(calls) == 3
 
 
+@pytest.mark.parametrize("M,parts,K", [(24000, (8, 500), 1024), (65536, (64, 64, 132), 512), (30001, (260,), 2048)])
+def test_many_rows_share_a_bounded_scratch(ops, M, parts, K):
+    """Rows in parts (two to six): the results of smaller calls, and no more memory than the bound."""
+    from based_b200 import _capi
+    assert 60 << 20 < _capi.lib().based_linear_f32_scratch_bytes(M, sum(parts), K) <= 128 << 20
+    g = torch.Generator("cuda").manual_seed(M)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, ws, b = r(M, K), [r(n, K) for n in parts], r(sum(parts))
+    with torch.inference_mode():
+        torch.cuda.synchronize()
+        held = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        y = ops.linear_split(x, ws, b)
+        assert torch.cuda.max_memory_allocated() - held <= (128 << 20) + y.numel() * 4 + 4096
+        for a in (0, 4096, M // 2 - 300, M - 700):
+            ref = x[a:a + 700].double() @ torch.cat(ws).double().T + b.double()
+            assert _rel(y[a:a + 700], ref) < 4e-7
+        w = torch.cat(ws)
+        wide = torch.nn.functional.linear(x, w, b)
+        assert float((y - wide).abs().max()) < 1e-4 * float(wide.abs().max())     # every row is there
+    assert _capi.read_status() == 0
+
+
+def test_large_weights_stay_with_the_library(ops):
+    x, w = torch.zeros(128, 1024, device="cuda"), torch.zeros(8200, 1024, device="cuda")
+    with torch.inference_mode():
+        assert ops._split_rows(x, (w[:8192],)) and not ops._split_rows(x, (w,))
+
+
 def test_projections_with_a_bias(ops):
     """A projection that was replaced by one with a bias keeps it."""
     from based_b200.mixers import LinearAttention
