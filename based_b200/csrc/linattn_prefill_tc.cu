@@ -110,7 +110,10 @@ __device__ __noinline__ void poly_pieces(uint32_t tlane, uint32_t tm_p, bool zer
       uint32_t sreg[32], pk[16];
       tmem_ld32(tlane + TM_S + piece * 32, sreg);
       tmem_ld_wait();
-      if (share == 1 && piece == 1) asm volatile("bar.arrive 1, 64;\n" ::: "memory");
+      if (share == 1 && piece == 1) {
+        fence_before_sync();
+        asm volatile("bar.arrive 1, 64;\n" ::: "memory");
+      }
       if (piece < qd) {   // left of the diagonal block: every column is visible
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -126,7 +129,10 @@ __device__ __noinline__ void poly_pieces(uint32_t tlane, uint32_t tm_p, bool zer
           pk[i] = pv & mask;
         }
       }
-      if (share == 2 && piece == p0) asm volatile("bar.sync 1, 64;\n" ::: "memory");
+      if (share == 2 && piece == p0) {
+        asm volatile("bar.sync 1, 64;\n" ::: "memory");
+        fence_after_sync();
+      }
       tmem_st16(tlane + tm_p + piece * 16, pk);
     } else if (zeros) {
       uint32_t z[16];

@@ -204,7 +204,9 @@ __global__ void __launch_bounds__(NT, PC <= 3 ? 2 : 1) swa_prefill_tc_kernel(con
   const int row = quad * 32 + lane;
   const float mine = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
   rowmax[half * TQ + row] = mine;
+  fence_before_sync();   // the other warp's P goes over the scores that this one has read
   asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quad) : "memory");   // the two warps of these rows
+  fence_after_sync();
   const float msc = fmaxf(mine, rowmax[(half ^ 1) * TQ + row]) * p.scale_log2e;
 #pragma unroll
   for (int pc = 0; pc < PC; ++pc) {

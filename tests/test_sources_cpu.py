@@ -52,3 +52,20 @@ def test_programmatic_kernels_read_activations_coherently(path):
         if "pdl_wait()" not in body[:600]:
             continue
         assert set(re.findall(r"\bconst\s+\w+\*\s*__restrict__\s+(\w+)", m.group(2))) <= TABLES, m.group(1)
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if "tmem_st" in open(p).read()], ids=os.path.basename)
+def test_tmem_hand_overs_between_warps_are_fenced(path):
+    """Accesses to TMEM are ordered between threads by the tcgen05 fences around what the threads meet at, not by the barrier: a named
+    barrier between reads of TMEM and writes of it has one before the arrival and one behind the wait."""
+    code = re.sub(r"\s+", " ", _code(path))
+    for m in re.finditer(r'asm volatile\("bar\.(sync|arrive)[^;]*;[^;]*;', code):
+        later = code[m.end():].split("__global__")[0]
+        writes, waits = later.find("tmem_st"), min((x for x in (later.find("mbar_"), later.find("__syncthreads")) if x >= 0), default=len(later))
+        if not 0 <= writes < waits:
+            continue                     # what is behind it does not write TMEM before the threads meet again
+        alone = m.group(1) == "arrive" or "bar.arrive" in code
+        if m.group(1) == "arrive" or not alone:
+            assert code[:m.start()].rstrip().endswith("fence_before_sync();"), m.group(0)
+        if m.group(1) == "sync":
+            assert later.lstrip().startswith("fence_after_sync();"), m.group(0)
