@@ -16,6 +16,7 @@ IMPL_SIMT = 1
 IMPL_TCGEN05 = 2
 IMPL_DECODE = 3
 TIED_DECODE_ROWS = 64
+TOKEN_SIDE_CLUSTER_ROWS = 192
 ERR_IMPL = -5
 
 _I64P = POINTER(c_int64)

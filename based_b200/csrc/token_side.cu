@@ -1,4 +1,4 @@
-// A layer's own input per token, for the few rows of a decode step, in one launch (bf16):
+// A layer's own input per token, for the few rows of a decode step or of a short prompt, in one launch (bf16):
 //   g = gelu_tanh(W_gate x) * table[token, column ..];  y = W_proj g;  stream <- stream + y / rms(y) * norm
 // and the new stream in bf16, plain or with a norm of its own.  The two products depend on one another through every
 // element, so a cluster of eight CTAs owns 16 rows: each takes an eighth of the gate's outputs, hands them to the others

@@ -10,9 +10,10 @@
 // cheaper than keeping it.  Where there are fewer row tiles than SMs each is shared out by its output columns; the first product and
 // the sums of squares are then made by every share, at the price of more reads of L2.  The stream comes and goes by TMA through slabs of
 // a warp's own, as in prompt_linear's ADD.
-// Measured at width 1024, 64 values, us as four launches / here, one after the other in a graph: 128 rows 9.0 / 12.4, 2048 13.5 / 13.2, 6001
-// 20.7 / 19.5, 18944 59 / 46.  Up to some 4000 rows a prompt of 27 such layers is bound by its launches instead: 5.9 ms / 5.1 (6001: 6.23 /
-// 6.05); hence also the few rows.  Three stages and a third slab of the stream: 13 at 128 rows, 19.9 at 6001.
+// Measured at width 1024, 64 values, us as four launches / here, one after the other in a graph: 512 rows 10.0 / 12.6, 2048 12.7 / 13.2, 4096
+// 16.4 / 16.3, 6001 19.8 / 19.4, 7168 24.0 / 22.4, 18944 57 / 48.  Up to some 4000 rows a prompt of 27 such layers is bound by its launches
+// instead: 5.55 to 5.9 ms / 4.85 to 5.2 (6001: 6.23 / 6.09); hence also the fewer rows, from where one round of token_side.cu's clusters ends
+// (128 rows there 6.8 us, 12.4 here).  Three stages and a third slab of the stream: 13 at 128 rows, 19.9 at 6001.
 #include "common.cuh"
 #include "seq_common.cuh"
 #include "tc_pair.cuh"

@@ -1350,10 +1350,19 @@ def token_gate(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, colum
     return out
 
 
-# A step's rows; from PROMPT_MIN_ROWS on, a whole tile of rows, there is a kernel on the tensor cores, and between the two the products of
-# the library are the quicker.
+# A step's rows; from PROMPT_MIN_ROWS on, a whole tile of rows, there is one launch for prompts, too.  us as four launches / in one, width 1024,
+# 64 values, in a graph: clusters of CTAs 64 9.0 / 6.4, 128 9.1 / 6.8, 192 9.4 / 7.5; beyond, on the tensor cores,
+# 512 10.0 / 12.6, 1024 11.1 / 12.8, 2048 12.7 / 13.2, 4096 16.4 / 16.3, 6400 21.5 / 22.3, 7168 24.0 / 22.4, 8192 27 / 23, 18944 57 / 48 (other
+# widths cross between 4096 and 7168).  A prompt that is not captured is bound by its launches (27 such layers, 130 to 4096 tokens 5.55 to 5.9
+# ms / 4.85 to 5.2) or loses less than 1 % of a layer, so there it is one launch at any length; a captured one from TOKEN_SIDE_CAPTURED_ROWS on.
 TOKEN_SIDE_MAX_ROWS = 64
+TOKEN_SIDE_CAPTURED_ROWS = 7168
 TOKEN_SIDE_MAX_WEIGHT = 200_000   # elements of one matrix up to which one cluster per 16 rows beats the separate launches
+
+
+def _one_launch(M, size) -> bool:
+    return (M >= TOKEN_SIDE_CAPTURED_ROWS or (M <= _capi.TOKEN_SIDE_CLUSTER_ROWS and size <= TOKEN_SIDE_MAX_WEIGHT)
+            or not torch.cuda.is_current_stream_capturing())
 
 
 def _prompt_side(residual, x, tokens, gate_weight, proj_weight, table, column, norm_weight) -> bool:
@@ -1379,7 +1388,7 @@ def token_side_step(residual: torch.Tensor, x: torch.Tensor, tokens: torch.Tenso
     if M <= TOKEN_SIDE_MAX_ROWS:
         if n * W > TOKEN_SIDE_MAX_WEIGHT:
             return None
-    elif not (M >= PROMPT_MIN_ROWS and out_weight is None and _prompt_side(residual, x, tokens, gate_weight, proj_weight, table, column, norm_weight)):
+    elif not (M >= PROMPT_MIN_ROWS and out_weight is None and _one_launch(M, n * W) and _prompt_side(residual, x, tokens, gate_weight, proj_weight, table, column, norm_weight)):
         return None
     _same_dtype(x, x=x, gate_weight=gate_weight, proj_weight=proj_weight, table=table, norm_weight=norm_weight, out_weight=out_weight)
     x2 = flat_rows(x)

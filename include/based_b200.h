@@ -627,9 +627,11 @@ int based_token_gate(const void* z, int64_t z_row_stride, const void* tokens, co
 /*
  * The whole token input of a layer for the few rows of a decode step (bf16): residual += norm(W_proj (gelu_tanh(W_gate x) *
  * table[token, column ..])) * norm_weight and out as in based_stream_post_norm; gate_weight [n, W], proj_weight [W, n]
- * contiguous.  Built for M <= 64 (more rows re-read the weights per 16) and, without out_weight, n <= 64, for M >= 128 (a prompt, on the
- * tensor cores).  BASED_ERR_IMPL: fp32, W or n no multiple of 8, n above 256, W above 8192 (M < 128), unaligned.
+ * contiguous.  Built for M <= BASED_TOKEN_SIDE_CLUSTER_ROWS (more rows re-read the weights per 16) and, without out_weight, n <= 64, for
+ * more (a prompt, on the tensor cores; matrices above 200 000 elements from M = 128 on).  BASED_ERR_IMPL: fp32, W or n no multiple of 8,
+ * n above 256, W above 8192 (but on the tensor cores), unaligned.
  */
+#define BASED_TOKEN_SIDE_CLUSTER_ROWS 192
 int based_token_side(const void* x, int64_t x_row_stride, const void* tokens, const void* gate_weight, const void* proj_weight,
                      const void* table, int64_t V, int64_t table_row_stride, int64_t column, const void* norm_weight, void* residual,
                      const void* out_weight, void* out, int M, int W, int n, float eps, int io_dtype, void* stream);
