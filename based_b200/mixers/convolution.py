@@ -72,8 +72,10 @@ class ShortConvolution(nn.Module):
         return state[:batch] if state.shape[0] != batch else state
 
     def takes_prompt(self) -> bool:
-        """True when :func:`ops.prompt_conv` has this convolution: three taps, no bias."""
-        return self.kernel_size == 3 and self._modules["conv"]._parameters.get("bias") is None
+        """True when :func:`ops.prompt_conv` has this convolution: three taps, no bias (one that is computed, by a parametrization or a
+        pruning, is not among the parameters)."""
+        own = self._modules["conv"]._parameters
+        return self.kernel_size == 3 and "bias" in own and own["bias"] is None
 
     def prompt_ok(self, u, inference_params) -> bool:
         """True when :func:`ops.prompt_conv` may stand for the projection ``u`` goes through and :meth:`gated`: bf16 taps it has, tokens

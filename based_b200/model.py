@@ -139,7 +139,9 @@ class Block(nn.Module):
             if type(m) is not RMSNorm or m._parameters.get("bias") is not None:
                 return None
         for m in (fc1, fc2, out) + ((mixer._modules["in_proj"],) if kind is BaseConv else ()):
-            own += [m._parameters.get("weight"), m._parameters.get("bias")]
+            if "bias" not in m._parameters:   # computed, by a parametrization or a pruning
+                return None
+            own += [m._parameters.get("weight"), m._parameters["bias"]]
         if own[0] is None or own[2] is None or own[4] is None or own[0].shape[0] % 16 or own[0].shape[1] % 8:
             return None
         taps = None

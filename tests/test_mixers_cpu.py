@@ -102,6 +102,35 @@ def test_model_assembly_keeps_the_reference_parameter_names():
     assert full.padded_vocab_size == 50280 and len(full.alt_mixer_layers) == 5
 
 
+def _small_block(layer=0):
+    from based_b200.model import BasedConfig, Block
+    return Block(BasedConfig(n_embd=64, n_layer=3, n_head=4, vocab_size=64, alt_mixer_layers=[1], alt_mixer_2_layers=[2]), layer).eval()
+
+
+class _Half(torch.nn.Module):
+    def forward(self, t):
+        return t / 2
+
+
+@pytest.mark.parametrize("name,field", [(n, f) for n in ("mixer.conv.conv", "mixer.in_proj", "mixer.out_proj", "mlp.fc1", "mlp.fc2") for f in ("weight", "bias")])
+@pytest.mark.parametrize("how", ["parametrization", "pruning"])
+def test_prompt_plans_leave_computed_parameters_to_the_modules(name, field, how):
+    """A weight or a bias that is computed is no parameter of its module: not one that is missing, either."""
+    from torch.nn.utils import parametrize, prune
+    block = _small_block()
+    assert block.prompt_plan(64) is not None
+    m = block.get_submodule(name)
+    if m.bias is None:
+        m.bias = torch.nn.Parameter(torch.ones(m.weight.shape[0]))
+    if how == "pruning":
+        prune.identity(m, field)
+    else:
+        parametrize.register_parametrization(m, field, _Half())
+    assert block.prompt_plan(64) is None
+    if name == "mixer.conv.conv" and field == "bias":
+        assert not block.mixer.conv.takes_prompt()
+
+
 def test_sample_token_policy():
     """Greedy, top-k support, nucleus support and temperature of the sampling policy (host logic, CPU tensors)."""
     import torch
