@@ -73,9 +73,10 @@ class ShortConvolution(nn.Module):
 
     def takes_prompt(self) -> bool:
         """True when :func:`ops.prompt_conv` has this convolution: three taps, no bias (one that is computed, by a parametrization or a
-        pruning, is not among the parameters)."""
+        pruning, is not among the parameters), and :meth:`gated` as it is here."""
         own = self._modules["conv"]._parameters
-        return self.kernel_size == 3 and "bias" in own and own["bias"] is None
+        return (self.kernel_size == 3 and "bias" in own and own["bias"] is None and type(self).gated is ShortConvolution.gated
+                and "gated" not in self.__dict__)
 
     def prompt_ok(self, u, inference_params) -> bool:
         """True when :func:`ops.prompt_conv` may stand for the projection ``u`` goes through and :meth:`gated`: bf16 taps it has, tokens

@@ -142,17 +142,18 @@ class LinearAttention(nn.Module):
         v = v.view(b, l, self.num_heads, self.head_dim).transpose(1, 2)
 
         self.is_inference = inference_params is not None
+        own = {} if finish is None else {"finish": finish}   # only where the model has looked at the mixer: others may not take it
         if inference_params is None:
-            return self.parallel_forward(hidden_states, q, k, v, finish=finish)
+            return self.parallel_forward(hidden_states, q, k, v, **own)
         if inference_params.seqlen_offset > 0:
             kv_state, k_state = self._get_inference_cache(inference_params)
             return self.recurrent_forward(hidden_states, kv_state, k_state, q, k, v, finish=finish)
         cached = inference_params.key_value_memory_dict.get(self.layer_idx)
         if cached is not None and cached[0].shape[0] == b:
             # pre-allocated (CUDA-graph) cache: the kernel writes the states in place
-            y, _, _ = self.parallel_forward(hidden_states, q, k, v, kv_state=cached[0], k_state=cached[1], finish=finish)
+            y, _, _ = self.parallel_forward(hidden_states, q, k, v, kv_state=cached[0], k_state=cached[1], **own)
             return y
-        y, kv_state, k_state = self.parallel_forward(hidden_states, q, k, v, finish=finish)
+        y, kv_state, k_state = self.parallel_forward(hidden_states, q, k, v, **own)
         if cached is not None:
             cached[0].copy_(kv_state)
             cached[1].copy_(k_state)

@@ -66,6 +66,7 @@ class BasedConfig:
 
 
 _MIXERS = (BaseConv, LinearAttention, SlidingAttention)
+_REPLACED = frozenset(("forward", "hidden", "parallel_forward"))   # methods a kernel stands for, where a module's instance has its own
 PLAN = ("fc1", "fc1 bias", "fc2", "fc2 bias", "activation", "out_proj", "out_proj bias", "in_proj", "in_proj bias", "taps", "norm1", "norm2")
 
 
@@ -128,7 +129,7 @@ class Block(nn.Module):
         if kind is not BaseConv and mixer.process_group is not None:
             return None
         for m in (self, mixer, mlp, norm1, norm2):
-            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            if m._forward_hooks or m._forward_pre_hooks or not _REPLACED.isdisjoint(m.__dict__):
                 return None
         fc1, fc2, out = mlp._modules["fc1"], mlp._modules["fc2"], mixer._modules["out_proj"]
         act = 0 if mlp.activation is F.silu else 1 if mlp.activation in (F.sigmoid, torch.sigmoid) else None

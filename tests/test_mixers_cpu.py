@@ -131,6 +131,42 @@ def test_prompt_plans_leave_computed_parameters_to_the_modules(name, field, how)
         assert not block.mixer.conv.takes_prompt()
 
 
+@pytest.mark.parametrize("layer,name,method", [(0, "", "forward"), (0, "mixer", "forward"), (0, "mlp", "hidden"), (0, "mlp", "forward"), (0, "mixer.conv", "gated"),
+                                               (0, "norm1", "forward"), (1, "mixer", "parallel_forward"), (1, "mlp", "hidden"), (2, "mixer", "forward")])
+def test_prompt_plans_leave_replaced_methods_to_be_called(layer, name, method):
+    block = _small_block(layer)
+    assert block.prompt_plan(64) is not None
+    m = block.get_submodule(name)
+    setattr(m, method, getattr(m, method))
+    assert block.prompt_plan(64) is None
+    if method == "gated":
+        assert not m.takes_prompt()
+
+
+def test_mixers_that_override_a_method_are_called_as_they_were():
+    """A subclass's methods have the arguments they always had."""
+    from based_b200.mixers import BaseConv
+    from based_b200.mixers.convolution import ShortConvolution
+
+    class Own(LinearAttention):
+        def parallel_forward(self, x, q, k, v, kv_state=None, k_state=None):
+            return x if not self.is_inference else (x, torch.zeros(2, 4, 1, 16, 273), torch.zeros(2, 4, 1, 1, 273))
+
+    class Gate(ShortConvolution):
+        def gated(self, u, inference_params=None):
+            return u
+
+    m, x = Own(64, num_heads=4, layer_idx=0).eval(), torch.zeros(2, 5, 64)
+    with torch.inference_mode():
+        assert m(x) is x
+        ip = InferenceParams(max_seqlen=8, max_batch_size=2)
+        assert m(x, inference_params=ip) is x and m(x, inference_params=ip) is x
+    c = BaseConv(64, l_max=64).conv
+    assert c.takes_prompt()
+    c.__class__ = Gate
+    assert not c.takes_prompt()
+
+
 def test_sample_token_policy():
     """Greedy, top-k support, nucleus support and temperature of the sampling policy (host logic, CPU tensors)."""
     import torch
