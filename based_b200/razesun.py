@@ -19,6 +19,7 @@ from .mixers.stateful import PackedLinear, pad_up
 from .modules import GatedMlp, unwatched
 
 MIXERS = {"latent_attention": LatentAttention, "delta": GatedDelta, "rglru": RGLRU}
+_GIVEN = (LatentAttention, GatedDelta, RGLRU)   # whose heads take the products with in_proj (and gate_proj) as given
 
 
 @dataclass
@@ -96,8 +97,8 @@ class ParallelBlock(nn.Module):
     def _first_products(self, h1, h2, hidden):
         """The mixer's projections of a step, and with them the MLP's hidden values, in one launch; None where they are several."""
         m, mlp = self.mixer, self.mlp
-        if (mlp is None or h1.numel() > h1.shape[-1] * ops.DECODE_LINEAR_MAX_ROWS or mlp.activation is not F.silu or "hidden" in vars(mlp)
-                or not unwatched(m.in_proj, PackedLinear)):
+        if (type(mlp) is not GatedMlp or h1.numel() > h1.shape[-1] * ops.DECODE_LINEAR_MAX_ROWS or mlp.activation is not F.silu or "hidden" in vars(mlp)
+                or type(m) not in _GIVEN or "heads" in vars(m) or not unwatched(m.in_proj, PackedLinear)):
             return None
         return ops.decode_beside(h1, m.in_proj.weight, m.in_proj.bias, getattr(m, "gate_proj", None), h2, mlp.fc1.weight, mlp.fc1.bias, "silu", hidden)
 

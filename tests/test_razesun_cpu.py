@@ -113,3 +113,43 @@ def test_oracle_mechanisms():
     a = torch.exp(-8 * R.softplus(lam))
     S = R.rglru_scan(u, one, one, lam)
     assert torch.allclose(S[:, 0], torch.sqrt(1 - a * a) * (1 - a ** torch.arange(1, 6)) / (1 - a))
+
+
+def test_first_products_are_left_to_other_mixers_and_mlps(monkeypatch):
+    """One launch for a layer's first products stands for this package's mixers and MLP, not for what is registered or put in their place."""
+    from based_b200 import ops
+    from based_b200.mixers import RGLRU
+    from based_b200.razesun import ParallelBlock, RazesunConfig
+
+    class Heads(RGLRU):
+        def heads(self, h, inference_params, out):
+            out.copy_(h[..., :out.shape[-1]])
+
+    class Mlp(torch.nn.Module):
+        def hidden(self, x, out=None):
+            return out.zero_()
+
+    class Plain(torch.nn.Module):
+        def heads(self, h, inference_params, out):
+            out.zero_()
+
+    monkeypatch.setattr(ops, "decode_beside", lambda *a: ("x", None))
+    layer = {"type": "rglru", "mixer": {"width": 64, "blocks": 2, "conv": 4}, "mlp": {"kind": "dense", "ff": 128}}
+    cfg = RazesunConfig.from_dict({"architecture": "Razesun", "vocab": 64, "width": 64, "layers": [layer], "norm": {"eps": 1e-6}, "residual_mult": 0.5, "logit_scale": 1.0})
+    h = torch.zeros(2, 1, 64)
+
+    def block(change=lambda b: None):
+        b = ParallelBlock(cfg, 0)
+        change(b)
+        return b
+
+    with torch.inference_mode():
+        assert block()._first_products(h, h, torch.zeros(2, 1, 128)) == ("x", None)
+        for change in (lambda b: setattr(b.mixer, "__class__", Heads), lambda b: setattr(b, "mlp", Mlp()), lambda b: setattr(b, "mixer", Plain()),
+                       lambda b: setattr(b.mixer, "heads", lambda h, ip, out: out.zero_()), lambda b: setattr(b.mlp, "hidden", lambda x, out=None: out.zero_())):
+            b = block(change)
+            assert b._first_products(h, h, torch.zeros(2, 1, 128)) is None
+            if not isinstance(b.mlp, Mlp) and "hidden" not in vars(b.mlp):
+                b.mlp.hidden = lambda x, out=None: out.zero_()      # (its kernel is for CUDA tensors)
+            if type(b.mixer) is not RGLRU or "heads" in vars(b.mixer):
+                assert b(h, h, None).shape == h.shape
