@@ -11,7 +11,7 @@ steps split of based/generation.py:93-204, and optional CUDA-graph replay of the
 (:689-739).  Training, dropout, tensor-parallel embeddings and sampling strategies are not.
 """
 from dataclasses import dataclass, field, fields
-from typing import List, Optional
+from typing import List, NamedTuple, Optional
 
 import torch
 import torch.nn as nn
@@ -66,8 +66,25 @@ class BasedConfig:
 
 
 _MIXERS = (BaseConv, LinearAttention, SlidingAttention)
-_REPLACED = frozenset(("forward", "hidden", "parallel_forward"))   # methods a kernel stands for, where a module's instance has its own
-PLAN = ("fc1", "fc1 bias", "fc2", "fc2 bias", "activation", "out_proj", "out_proj bias", "in_proj", "in_proj bias", "taps", "norm1", "norm2")
+
+
+class PromptPlan(NamedTuple):
+    """What a prompt's pass through a layer without launches for the norms needs.  ``in_proj``, its bias and ``taps`` are a BaseConv layer's."""
+    mixer: nn.Module
+    norm1: RMSNorm
+    norm2: RMSNorm
+    fc1: torch.Tensor
+    fc1_bias: Optional[torch.Tensor]
+    fc2: torch.Tensor
+    fc2_bias: Optional[torch.Tensor]
+    activation: int
+    out_proj: torch.Tensor
+    out_bias: Optional[torch.Tensor]
+    in_proj: Optional[torch.Tensor]
+    in_bias: Optional[torch.Tensor]
+    taps: Optional[torch.Tensor]
+    norm1_weight: torch.Tensor
+    norm2_weight: torch.Tensor
 
 
 class Block(nn.Module):
@@ -115,10 +132,9 @@ class Block(nn.Module):
                 and weights[-3][0].shape[0] == weights[-1][0].shape[0] == width)
 
     def prompt_plan(self, width):
-        """What a prompt's pass through this layer without launches for the norms needs, as ``(mixer, norm1, norm2, weights)`` with the
-        weights of :data:`PLAN`; None where :meth:`forward` has to run instead: somebody watches a module or has put another forward on
-        one, the stream is not fp32, or a module is not of the kind or form the kernels stand for.  Modules' own dictionaries are read,
-        because a module's attribute look-up costs a microsecond and this runs for every layer of every prompt."""
+        """This layer's :class:`PromptPlan`; None where :meth:`forward` has to run instead: somebody watches a module or has put another
+        forward on one, the stream is not fp32, or a module is not of the kind or form the kernels stand for.  Modules' own dictionaries
+        are read, because a module's attribute look-up costs a microsecond and this runs for every layer of every prompt."""
         mods = self._modules
         mixer, mlp, norms = mods["mixer"], mods["mlp"], (mods["norm1"], mods["norm2"])
         kind, norm1, norm2 = type(mixer), *norms
@@ -129,8 +145,10 @@ class Block(nn.Module):
         if kind is not BaseConv and mixer.process_group is not None:
             return None
         for m in (self, mixer, mlp, norm1, norm2):
-            if m._forward_hooks or m._forward_pre_hooks or not _REPLACED.isdisjoint(m.__dict__):
+            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
                 return None
+        if "hidden" in mlp.__dict__ or "parallel_forward" in mixer.__dict__:
+            return None
         fc1, fc2, out = mlp._modules["fc1"], mlp._modules["fc2"], mixer._modules["out_proj"]
         act = 0 if mlp.activation is F.silu else 1 if mlp.activation in (F.sigmoid, torch.sigmoid) else None
         if act is None or not plain_linear(fc1) or not plain_linear(out):   # a prompt calls these two as modules
@@ -140,9 +158,10 @@ class Block(nn.Module):
             if type(m) is not RMSNorm or m._parameters.get("bias") is not None:
                 return None
         for m in (fc1, fc2, out) + ((mixer._modules["in_proj"],) if kind is BaseConv else ()):
-            if "bias" not in m._parameters:   # computed, by a parametrization or a pruning
+            tensors = m._parameters
+            if "bias" not in tensors:   # computed, by a parametrization or a pruning
                 return None
-            own += [m._parameters.get("weight"), m._parameters["bias"]]
+            own += [tensors.get("weight"), tensors["bias"]]
         if own[0] is None or own[2] is None or own[4] is None or own[0].shape[0] % 16 or own[0].shape[1] % 8:
             return None
         taps = None
@@ -153,25 +172,26 @@ class Block(nn.Module):
                 return None
         if own[2].shape[0] != width or own[4].shape[0] != width or own[2].shape[1] % 8 or own[4].shape[1] % 8:
             return None
-        return mixer, norm1, norm2, (*own[:4], act, *own[4:6], *(own[6:] or (None, None)), taps, norm1._parameters["weight"], norm2._parameters["weight"])
+        w1, b1, w2, b2, wo, bo, wi, bi = own if kind is BaseConv else (*own, None, None)
+        return PromptPlan(mixer, norm1, norm2, w1, b1, w2, b2, act, wo, bo, wi, bi, taps, norm1._parameters["weight"], norm2._parameters["weight"])
 
     def prompt(self, rows, residual, inference_params, plan, next_norm):
         """:meth:`forward` of a prompt with the :meth:`prompt_plan` of this layer: ``rows`` is what ``norm1`` gives (a tensor, or a
         :class:`ops.NormRows`), ``residual`` is updated in place; returns what ``next_norm`` gives, or without one the MLP's output."""
-        mixer, norm1, norm2, (w1, b1, w2, b2, act, wo, bo, wi, bi, taps, _, n2) = plan
+        p: PromptPlan = plan
         x, ss, eps = (rows.x, rows.ss, rows.eps) if type(rows) is ops.NormRows else (rows, None, 0.0)
         B, L, _ = x.shape
         first = (None,) * 7
-        if taps is not None:
-            state = mixer.conv._prefill_state(inference_params, B, clear=False)
+        if p.taps is not None:
+            state = p.mixer.conv._prefill_state(inference_params, B, clear=False)
             if L >= 3 and (state is None or (state.dtype == torch.bfloat16 and state.is_contiguous() and state.data_ptr() % 16 == 0)):
-                first = wi, bi, taps, state, wo, bo, n2
+                first = p.in_proj, p.in_bias, p.taps, state, p.out_proj, p.out_bias, p.norm2_weight
         if first[0] is None:
-            rows = mixer(rows, inference_params=inference_params,
-                         finish=lambda x, weight, bias: ops.prompt_add_norm(x, weight, bias, residual, n2, eps=norm2.eps))
+            rows = p.mixer(rows, inference_params=inference_params,
+                           finish=lambda x, weight, bias: ops.prompt_add_norm(x, weight, bias, residual, p.norm2_weight, eps=p.norm2.eps))
             x, ss, eps = rows.x, rows.ss, rows.eps
-        x, ss = ops.prompt_layer(x, ss, eps, residual, L, *first, norm2.eps, w1, b1, act, w2, b2, None if next_norm is None else next_norm.weight,
-                                 0.0 if next_norm is None else next_norm.eps)
+        x, ss = ops.prompt_layer(x, ss, eps, residual, L, *first, p.norm2.eps, p.fc1, p.fc1_bias, p.activation, p.fc2, p.fc2_bias,
+                                 None if next_norm is None else next_norm.weight, 0.0 if next_norm is None else next_norm.eps)
         return x if next_norm is None else ops.NormRows(x, ss, next_norm.eps)
 
     def step(self, hidden_states, residual, inference_params, next_norm):
@@ -230,7 +250,7 @@ class BasedModel(nn.Module):
                 and not torch.nn.modules.module._has_any_global_hook()):
             return None
         plans = [layer.prompt_plan(h.shape[-1]) for layer in layers]
-        if any(p is None for p in plans) or not ops.plain_bf16(h, *(w for p in plans for w in p[3] if torch.is_tensor(w))):
+        if any(p is None for p in plans) or not ops.plain_bf16(h, *(w for p in plans for w in p[3:] if torch.is_tensor(w))):
             return None
         return plans
 
@@ -239,7 +259,7 @@ class BasedModel(nn.Module):
         step = inference_params is not None and inference_params.seqlen_offset > 0
         plans = None if step else self._prompt_plans(hidden_states)
         if plans is not None:
-            layers, norms = list(self.layers), [p[1] for p in plans[1:]] + [None]
+            layers, norms = list(self.layers), [p.norm1 for p in plans[1:]] + [None]
             hidden_states, residual = layers[0].norm1(hidden_states, prenorm=True, residual_in_fp32=True, round_input=True)
             for layer, plan, norm in zip(layers, plans, norms):
                 hidden_states = layer.prompt(hidden_states, residual, inference_params, plan, norm)

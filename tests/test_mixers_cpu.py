@@ -131,6 +131,17 @@ def test_prompt_plans_leave_computed_parameters_to_the_modules(name, field, how)
         assert not block.mixer.conv.takes_prompt()
 
 
+@pytest.mark.parametrize("layer", [0, 1, 2])
+def test_prompt_plans_name_the_modules_parameters(layer):
+    block = _small_block(layer)
+    plan, conv = block.prompt_plan(64), layer == 0
+    for field, name in (("fc1", "mlp.fc1.weight"), ("fc1_bias", "mlp.fc1.bias"), ("fc2", "mlp.fc2.weight"), ("fc2_bias", "mlp.fc2.bias"),
+                        ("out_proj", "mixer.out_proj.weight"), ("out_bias", "mixer.out_proj.bias"), ("norm1_weight", "norm1.weight"), ("norm2_weight", "norm2.weight"),
+                        ("in_proj", "mixer.in_proj.weight"), ("in_bias", "mixer.in_proj.bias"), ("taps", "mixer.conv.conv.weight")):
+        assert getattr(plan, field) is dict(block.named_parameters()).get(name), field
+    assert (plan.taps is not None) == conv and plan.mixer is block.mixer and plan.norm1 is block.norm1 and plan.norm2 is block.norm2
+
+
 @pytest.mark.parametrize("layer,name,method", [(0, "", "forward"), (0, "mixer", "forward"), (0, "mlp", "hidden"), (0, "mlp", "forward"), (0, "mixer.conv", "gated"),
                                                (0, "norm1", "forward"), (1, "mixer", "parallel_forward"), (1, "mlp", "hidden"), (2, "mixer", "forward")])
 def test_prompt_plans_leave_replaced_methods_to_be_called(layer, name, method):
