@@ -68,14 +68,16 @@ class GatedMlp(nn.Module):
             act = "silu"
         else:
             raise NotImplementedError("GatedMlp: activation must be F.silu (SwiGLU) or F.sigmoid (GLU)")
-        if ops._decode_rows(x, self.fc1.weight, gated=True) and self.fc1.weight.shape[0] % 16 == 0:
+        fc1 = self.fc1
+        weight = fc1.weight
+        if ops._decode_rows(x, weight, gated=True) and weight.shape[0] % 16 == 0:
             # decode step: fc1 and the gated activation in one launch
-            return ops.decode_linear(x, self.fc1.weight, self.fc1.bias, epilogue="gated", activation=act, out=out)
-        if ops._prompt_rows(x, self.fc1.weight, self.fc1.bias) and self.fc1.weight.shape[0] % 16 == 0 and plain_linear(self.fc1) and (
+            return ops.decode_linear(x, weight, fc1.bias, epilogue="gated", activation=act, out=out)
+        if ops._prompt_rows(x, weight, fc1.bias) and weight.shape[0] % 16 == 0 and plain_linear(fc1) and (
                 out is None or (out.dtype == torch.bfloat16 and out.stride(-1) == 1 and out.data_ptr() % 16 == 0
                                 and all(st % 8 == 0 for st in out.stride()[:-1]))):
-            return ops.prompt_linear(x, self.fc1.weight, self.fc1.bias, epilogue="gated", activation=act, out=out)
-        return ops.gated_act(self.fc1(ops.dense(x)), act, out=out)
+            return ops.prompt_linear(x, weight, fc1.bias, epilogue="gated", activation=act, out=out)
+        return ops.gated_act(fc1(ops.dense(x)), act, out=out)
 
     def forward(self, x, finish=None):
         """``finish(hidden, weight, bias)``, when given, stands for the product with fc2 and what comes behind it."""

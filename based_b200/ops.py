@@ -685,7 +685,7 @@ def prompt_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
         o2 = _rows(out, n_out)
         if o2.shape[0] != M:
             raise ValueError("out must have a row for each of x's")
-        so, out = o2.stride(0), o2.reshape(shape)
+        so, out = o2.stride(0), out if out.shape == shape else o2.reshape(shape)
     if M > 0:
         code = _capi.native().prompt_linear(x2, weight, bias, o2, M, N, K, _row_stride(x2, K), K, so, epi, _ACTS[activation],
                                             None if rows is None else rows.ss, 0 if rows is None else rows.ss.shape[1],
@@ -752,9 +752,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if _decode_rows(x, weight) and (bias is None or (type(bias) in _PLAIN_TYPES and bias.dtype == torch.bfloat16
                                                      and bias.shape == weight.shape[:1] and bias.device == x.device)):
         return decode_linear(x, weight, bias)
-    if type(x) is NormRows and _prompt_rows(x, weight, bias):
-        return prompt_linear(x, weight, bias)
-    if _split_rows(x, (weight,), bias):
+    if type(x) is NormRows:
+        if _prompt_rows(x, weight, bias):
+            return prompt_linear(x, weight, bias)
+    elif x.dtype == torch.float32 and _split_rows(x, (weight,), bias):
         return linear_split(x, (weight,), bias)
     return torch.nn.functional.linear(dense(x), weight, bias)
 

@@ -153,3 +153,18 @@ def test_first_products_are_left_to_other_mixers_and_mlps(monkeypatch):
                 b.mlp.hidden = lambda x, out=None: out.zero_()      # (its kernel is for CUDA tensors)
             if type(b.mixer) is not RGLRU or "heads" in vars(b.mixer):
                 assert b(h, h, None).shape == h.shape
+
+
+@pytest.mark.parametrize("B,L,asks", [(32, 1, True), (1, 32, True), (33, 1, False), (2, 17, False), (1, 200, False)])
+def test_prompts_do_not_ask_for_a_steps_launch(monkeypatch, B, L, asks):
+    """Each layer of a prompt paid 3 us for the slice and the checks of a launch that takes up to 32 rows."""
+    from based_b200.razesun import ParallelBlock, RazesunConfig
+    layer = {"type": "rglru", "mixer": {"width": 64, "blocks": 2, "conv": 4}, "mlp": {"kind": "dense", "ff": 128}}
+    cfg = RazesunConfig.from_dict({"architecture": "Razesun", "vocab": 64, "width": 64, "layers": [layer], "norm": {"eps": 1e-6}, "residual_mult": 0.5, "logit_scale": 1.0})
+    b, asked = ParallelBlock(cfg, 0), []
+    monkeypatch.setattr(b, "_first_products", lambda *a: asked.append(1))
+    b.mixer.heads = lambda h, ip, out: out.zero_()
+    b.mlp.hidden = lambda x, out=None: out.zero_()
+    with torch.inference_mode():
+        b(torch.zeros(B, L, 64), torch.zeros(B, L, 64), None)
+    assert bool(asked) == asks
