@@ -64,9 +64,11 @@ class ShortConvolution(nn.Module):
         is cleared only where it holds more rows than that."""
         if inference_params is None:
             return None
-        held = inference_params.key_value_memory_dict.get(self.layer_idx[0], {}) if isinstance(self.layer_idx, tuple) else {}
-        state = held.get(self.layer_idx[1]) if held else None
-        if clear or state is None or state.shape[0] != batch:
+        if not clear:
+            held = inference_params.key_value_memory_dict.get(self.layer_idx[0], {}) if isinstance(self.layer_idx, tuple) else {}
+            state = held.get(self.layer_idx[1]) if held else None
+            clear = state is None or state.shape[0] != batch
+        if clear:
             self._init_state(inference_params)
         state = self._get_state(inference_params)
         return state[:batch] if state.shape[0] != batch else state
@@ -144,26 +146,27 @@ class BaseConv(nn.Module):
         """u ``[B, L, d_model]`` -> ``[B, L, d_model]``; with ``inference_params`` the prompt pass
         fills the convolution state and later single-token calls step it.  ``finish(v, weight, bias)``, when
         given, stands for the product with out_proj and what comes behind it."""
-        finish = finish or ops.linear
+        finish, in_proj = finish or ops.linear, self.in_proj
         if inference_params is not None and inference_params.seqlen_offset > 0:
             state = self.conv._get_state(inference_params)
-            if (ops._decode_rows(u, self.in_proj.weight)
+            if (ops._decode_rows(u, in_proj.weight)
                     and state.dtype == torch.bfloat16 and state.is_contiguous()
                     and state.shape[0] == u.shape[0] and u.shape[1] == 1 and self.d_inner % 8 == 0):
                 # decode step: in_proj, the convolution step on the state, silu and the gate in one launch
-                v = ops.decode_linear(u, self.in_proj.weight, self.in_proj.bias, epilogue="conv", conv_state=state,
+                v = ops.decode_linear(u, in_proj.weight, in_proj.bias, epilogue="conv", conv_state=state,
                                       conv_weight=self.conv.conv.weight, conv_bias=self.conv.conv.bias)
                 return finish(v, self.out_proj.weight, self.out_proj.bias)
-        if ops._prompt_rows(u, self.in_proj.weight, self.in_proj.bias) and self.d_inner % 8 == 0 and self.conv.prompt_ok(u, inference_params):
+        if (type(u) is ops.NormRows or u.numel() >= ops.PROMPT_MIN_ROWS * u.shape[-1]) and (
+                ops._prompt_rows(u, in_proj.weight, in_proj.bias)) and self.d_inner % 8 == 0 and self.conv.prompt_ok(u, inference_params):
             # prompt: in_proj, the convolution, silu and the gate in one launch
             state = self.conv._prefill_state(inference_params, u.shape[0], clear=False)
             own = state if state is None or (state.dtype == torch.bfloat16 and state.is_contiguous()) else torch.empty(
                 state.shape, dtype=torch.bfloat16, device=state.device)
-            v = ops.prompt_conv(u, self.in_proj.weight, self.in_proj.bias, self.conv.conv.weight, state=own)
+            v = ops.prompt_conv(u, in_proj.weight, in_proj.bias, self.conv.conv.weight, state=own)
             if own is not state:
                 state.copy_(own)
             return finish(v, self.out_proj.weight, self.out_proj.bias)
-        u = ops.linear(u, self.in_proj.weight, self.in_proj.bias)
+        u = ops.linear(u, in_proj.weight, in_proj.bias)
         v = self.conv.gated(u, inference_params=inference_params)
         return finish(v, self.out_proj.weight, self.out_proj.bias)
 

@@ -73,7 +73,9 @@ class GatedMlp(nn.Module):
         if ops._decode_rows(x, weight, gated=True) and weight.shape[0] % 16 == 0:
             # decode step: fc1 and the gated activation in one launch
             return ops.decode_linear(x, weight, fc1.bias, epilogue="gated", activation=act, out=out)
-        if ops._prompt_rows(x, weight, fc1.bias) and weight.shape[0] % 16 == 0 and plain_linear(fc1) and (
+        # (few rows are not looked at further: half a microsecond for every layer of a short prompt)
+        if (type(x) is ops.NormRows or x.numel() >= ops.PROMPT_MIN_ROWS * x.shape[-1]) and (
+                ops._prompt_rows(x, weight, fc1.bias)) and weight.shape[0] % 16 == 0 and plain_linear(fc1) and (
                 out is None or (out.dtype == torch.bfloat16 and out.stride(-1) == 1 and out.data_ptr() % 16 == 0
                                 and all(st % 8 == 0 for st in out.stride()[:-1]))):
             return ops.prompt_linear(x, weight, fc1.bias, epilogue="gated", activation=act, out=out)

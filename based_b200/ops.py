@@ -755,9 +755,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if type(x) is NormRows:
         if _prompt_rows(x, weight, bias):
             return prompt_linear(x, weight, bias)
-    elif x.dtype == torch.float32 and _split_rows(x, (weight,), bias):
+        x = dense(x)
+    elif x.dtype is torch.float32 and _split_rows(x, (weight,), bias):
         return linear_split(x, (weight,), bias)
-    return torch.nn.functional.linear(dense(x), weight, bias)
+    return torch.nn.functional.linear(x, weight, bias)
 
 
 def _split_rows(x: torch.Tensor, weights, bias: Optional[torch.Tensor] = None) -> bool:
