@@ -20,7 +20,7 @@ import torch.nn.functional as F
 from . import ops
 from .generation import GenerationMixin, sample_token  # noqa: F401
 from .mixers import BaseConv, LinearAttention, SlidingAttention, TaylorExp
-from .modules import GatedMlp, RMSNorm, plain_linear
+from .modules import GatedMlp, RMSNorm
 
 
 @dataclass
@@ -132,8 +132,8 @@ class Block(nn.Module):
                 and weights[-3][0].shape[0] == weights[-1][0].shape[0] == width)
 
     def prompt_plan(self, width):
-        """This layer's :class:`PromptPlan`; None where :meth:`forward` has to run instead: somebody watches a module or has put another
-        forward on one, the stream is not fp32, or a module is not of the kind or form the kernels stand for.  Modules' own dictionaries
+        """This layer's :class:`PromptPlan`; None where :meth:`forward` has to run instead: somebody watches a module (hooks on all modules
+        are the caller's to look for) or has put another forward on one, the stream is not fp32, or a module is not of the kind or form the kernels stand for.  Modules' own dictionaries
         are read, because a module's attribute look-up costs a microsecond and this runs for every layer of every prompt."""
         mods = self._modules
         mixer, mlp, norms = mods["mixer"], mods["mlp"], (mods["norm1"], mods["norm2"])
@@ -144,14 +144,14 @@ class Block(nn.Module):
             return None
         if kind is not BaseConv and mixer.process_group is not None:
             return None
-        for m in (self, mixer, mlp, norm1, norm2):
+        fc1, fc2, out = mlp._modules["fc1"], mlp._modules["fc2"], mixer._modules["out_proj"]
+        for m in (self, mixer, mlp, norm1, norm2, fc1, out):   # a prompt calls fc1 and out_proj as modules, too
             if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
                 return None
         if "hidden" in mlp.__dict__ or "parallel_forward" in mixer.__dict__:
             return None
-        fc1, fc2, out = mlp._modules["fc1"], mlp._modules["fc2"], mixer._modules["out_proj"]
         act = 0 if mlp.activation is F.silu else 1 if mlp.activation in (F.sigmoid, torch.sigmoid) else None
-        if act is None or not plain_linear(fc1) or not plain_linear(out):   # a prompt calls these two as modules
+        if act is None or type(fc1) is not nn.Linear or type(out) is not nn.Linear:
             return None
         own = []
         for m in norms:
