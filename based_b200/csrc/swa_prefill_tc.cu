@@ -18,8 +18,9 @@
 // next tile are asked for when S is done, V when O is done, and the output leaves under the next S.  A tile takes a CTA 3.7 us; with
 // the copies issued by a softmax warp it took 4.7 (700 to 900 cycles each time: coordinates, descriptors, the wait for the store), and
 // as a CTA of its own, three to an SM, 4.1 for two at a time.
-// us, a CTA per tile with O beside S and a thread per row / now (B x H x L, head, window; floor at the HBM rate): 8x16x8192, 64, 64 116.8 / 103.6
-// (82); 4x16x8192, 64, 32 57 / 47 (41); 64, 128 123 / 93 (41); 112, 64 174 / 92 (72); 2x16x8192, 128, 128 106 / 62 (41).
+// us, one after the other in a graph, a CTA per tile with O beside S and a thread per row / now (B x H x L, head, window; floor at the HBM
+// rate): 8x16x8192, 64, 64 116.8 / 104 (82; a lone call 125); 4x16x8192, 64, 32 57 / 46 (41); 64, 128 123 / 93 (41); 112, 64 174 / 91 (72);
+// 2x16x8192, 128, 128 106 / 61 (41).
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "tma.cuh"

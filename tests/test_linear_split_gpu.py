@@ -27,7 +27,7 @@ def test_split_products(ops, M, parts, K, scale):
     got = ops.linear_split(x, ws).split(list(parts), -1)
     for y, w in zip(got, ws):
         ref = x.double() @ w.double().T
-        # 6 products of 2^-24 or less each, two sums of at most 128 / 16 steps a run, one rounding a run: measured 1.3e-7 to 2e-7
+        # what is left out of a product 2^-24 of it at most, two sums of at most 128 / 16 steps a run, one rounding a run: measured 1.25e-7 to 1.4e-7
         assert _rel(y, ref) < 4e-7, (_rel(y, ref), _rel(torch.nn.functional.linear(x, w), ref))
     y = ops.linear_split(x, ws, b)
     assert _rel(y, x.double() @ torch.cat(ws).double().T + b.double()) < 4e-7
