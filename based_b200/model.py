@@ -133,8 +133,9 @@ class Block(nn.Module):
 
     def prompt_plan(self, width):
         """This layer's :class:`PromptPlan`; None where :meth:`forward` has to run instead: somebody watches a module (hooks on all modules
-        are the caller's to look for) or has put another forward on one, the stream is not fp32, or a module is not of the kind or form the kernels stand for.  Modules' own dictionaries
-        are read, because a module's attribute look-up costs a microsecond and this runs for every layer of every prompt."""
+        are the caller's to look for) or has put another forward on one, the stream is not fp32, or a module is not of the kind or form
+        the kernels stand for.  Modules' own dictionaries are read, because a module's attribute look-up costs a microsecond and this
+        runs for every layer of every prompt."""
         mods = self._modules
         mixer, mlp, norms = mods["mixer"], mods["mlp"], (mods["norm1"], mods["norm2"])
         kind, norm1, norm2 = type(mixer), *norms
